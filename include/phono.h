@@ -92,7 +92,8 @@ typedef struct phono_desc {
   int max_steps;                 /* capacity: source samples and surface records */
   int record_every;              /* record uz[:, :, 0] after every k-th step; 0 = off */
   int tile_j;                    /* tile height along y: 4, 8 or 16; 0 = default (F32K 4, else 8) */
-  int x_segment;                 /* planes per block segment; -L: L-plane segments, the last 2L planes in four shorter ones; 0 = default (24) */
+  int x_segment;                 /* planes per block segment; -L: L-plane segments, the last 2L planes in four shorter ones; 0 = default (24).
+                                  * Both 0: the form of phono_step that suits the mesh, not necessarily tiles */
 } phono_desc;
 
 typedef struct phono_handle phono_handle;
@@ -113,7 +114,11 @@ int phono_create(const phono_desc *desc, phono_handle **out);
 int phono_set_source(phono_handle *h, const double *samples, int n);
 
 /* Advance nsteps time steps; per step a tile launch and a face launch (one
- * launch when ny == 3), replayed from captured CUDA graphs of 12 steps.  Replaces the loop body of BaseSolver.run
+ * launch when ny == 3), or in the two-launch form a stress launch and an
+ * update launch per chunk of planes, replayed from captured CUDA graphs of 12
+ * steps.  The two-launch form is that of handles with the default tile shape
+ * (tile_j = x_segment = 0) in FP64, and in FP32 up to 400,000 nodes; results
+ * are the same bits.  Replaces the loop body of BaseSolver.run
  * (base_solver.py:245-266): source, update_T, update_T_BC, update_u,
  * update_u_BC, time_step.  Asynchronous on the handle's stream. */
 int phono_step(phono_handle *h, int nsteps);
@@ -121,8 +126,8 @@ int phono_step(phono_handle *h, int nsteps);
 /* Advance nsteps time steps like phono_step, but without the graph and with
  * a CUDA event before and after each launch, so that the two kernels of a
  * step are timed apart: *tile_ms = the summed device time of the tile
- * launches (the fused launch when ny == 3), *face_ms = that of the face
- * launches.  Blocks until done.  Results are those of phono_step.  No
+ * launches (the fused launch when ny == 3, all launches of the two-launch
+ * form), *face_ms = that of the face launches.  Blocks until done.  Results are those of phono_step.  No
  * reference counterpart (measurement). */
 int phono_time_kernels(phono_handle *h, int nsteps, float *tile_ms, float *face_ms);
 
@@ -331,7 +336,8 @@ int phono_batch_sync(phono_batch *b);
 int phono_batch_last_step_ms(phono_batch *b, float *ms);
 void phono_batch_destroy(phono_batch *b);
 
-/* Change the tile shape of a handle (0 keeps a value): tile_j rows per block
+/* Change the tile shape of a handle (0 keeps a value, both 0 change nothing):
+ * steps then take the tile pass.  tile_j rows per block
  * (4, 8, 16) and x_segment planes per block column (-L: tapered, as in
  * phono_desc; PHONO_ERR_ARG when that takes more than 64 segments).  Results
  * do not depend on the tile shape; the tuner (phonomena_gb300/autotune.py) calls this to

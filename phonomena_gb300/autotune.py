@@ -1,9 +1,10 @@
 """Tile-shape autotuner for the fused step kernel, single meshes and batches.
 
-``tune``: for one mesh shape and arithmetic scheme it times every
-(tile_j, x_segment) candidate on a scratch simulation of that shape (CUDA
-events around a chunk of steps from the zero state; ``phono_set_tiling``
-switches the candidate in place) and keeps the fastest.
+``tune``: for one mesh shape and arithmetic scheme it times the library's
+default and every (tile_j, x_segment) candidate on a scratch simulation of
+that shape (CUDA events around a chunk of steps from the zero state;
+``phono_set_tiling`` switches the candidate in place) and keeps the fastest;
+(0, 0) means the default.
 
 ``tune_batch``: for a mix of mesh shapes stepped as one batch it picks the
 batch's tile height and each instance's x segment, i.e. how many
@@ -137,12 +138,13 @@ def tune(spacing, mat, table, dt, precision="f32k", steps=None, candidates=None,
             return int(tj), (tuple(xs) if isinstance(xs, list) else int(xs))
     if steps is None:
         steps = 48 if precision == "f32k" else 12
-    cands = candidates or candidates_for(shape)
+    cands = [(0, 0)] + list(candidates or candidates_for(shape))  # (0, 0): the library's own choice, tiles or not
     results = []
-    sim = _scratch(shape, precision, (steps + 12) * len(cands) + 12)
+    sim = _scratch(shape, precision, (steps + 12) * len(cands) + 12, tile_j=0, x_segment=0)
     try:
         for tj, xs in cands:
-            sim.set_tiling(tj, xs)
+            if tj or xs:
+                sim.set_tiling(tj, xs)
             sim.step(12)  # warm up: graph capture
             sim.sync()
             sim.step(steps)

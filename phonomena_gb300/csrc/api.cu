@@ -9,7 +9,7 @@
 
 #include "../../include/phono.h"
 #include <cudaTypedefs.h>
-#include "fdtd_common.cuh"
+#include "split_common.cuh"
 
 namespace phono {
 cudaError_t configure_step_f64(int tj);
@@ -18,6 +18,7 @@ cudaError_t launch_step_f64(const StepArgs<double>& a, int tj, int n_face_blocks
 cudaError_t launch_step_f32k(const StepArgs<float>& a, int tj, int n_face_blocks, cudaStream_t st);
 cudaError_t configure_step_f64v(int tj);
 cudaError_t launch_step_f64v(const StepArgs<double>& a, int tj, int n_face_blocks, cudaStream_t st);
+cudaError_t launch_split(int precision, const void* args, bool stress, cudaStream_t st);
 cudaError_t launch_energy(const EnergyArgs& a, double2* partial, int nblocks, double* out, cudaStream_t st);
 cudaError_t batch_step_any(int precision, const void* ba, int tj, int grid_tiles, int grid_faces, cudaStream_t st);
 cudaError_t batch_advance_any(int precision, const void* ba, int n_active_cap, int n, cudaStream_t st);
@@ -86,6 +87,16 @@ struct phono_handle {
   int tj = 8, xseg = 64, ntj = 0, ntk = 0, nseg = 0, n_tile = 0, n_face = 0, separate_faces = 1;
   FaceTable faces{};
   std::vector<int> seg_start;  // first plane of each x segment, + nx-1
+  // two-launch step (split_step.cu): stress window of `win` planes (0: this
+  // mesh has none).  split: the handle steps that way (default tile shape);
+  // the velocity forms' v and Kahan terms then stay in buffer 0
+  int win = 0, tsy = 0;
+  bool split = false;
+  bool resplit = false;        // in a persistent batch (tile pass): back to the two-launch form when it leaves
+  char* stress = nullptr;      // leapfrog: the window
+  SoftRec* rec = nullptr;      // leapfrog: table entries as records, 16 per material
+  void* spd[6] = {};           // divisors of the two-launch step (records, or sp)
+  double* vals = nullptr;      // leapfrog: values of all records
   cudaStream_t stream = nullptr;
   cudaGraphExec_t graph = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -174,30 +185,28 @@ static int upload_materials(phono_handle* h, const uint8_t* mat, const double* t
 static int upload_table(phono_handle* h, const double* table, int nmat, int id000) {
   const double dt = h->d.dt;
   const double dt2 = dt * dt;
+  const bool leapfrog = h->d.precision == PHONO_F64;
+  std::vector<double> t(16 * nmat, 0.0);
+  for (int m = 0; m < nmat; m++) {
+    const double* row = table + m * PHONO_TABLE_COLS;
+    for (int q = 0; q < 12; q++) t[m * 16 + q] = row[q];
+    // (dt**2 / P) of base_solver.py:443 for the leapfrog, dt / P for the velocity form
+    t[m * 16 + 12] = leapfrog ? dt2 / row[12] : dt / row[12];
+    t[m * 16 + 13] = row[12];
+    t[m * 16 + 14] = dt;
+  }
+  std::vector<float> t32;
+  std::vector<SoftRec> rec;
   if (h->es == 8) {
-    const bool leapfrog = h->d.precision == PHONO_F64;
-    std::vector<double> t(16 * nmat, 0.0);
-    for (int m = 0; m < nmat; m++) {
-      const double* row = table + m * PHONO_TABLE_COLS;
-      for (int q = 0; q < 12; q++) t[m * 16 + q] = row[q];
-      // (dt**2 / P) of base_solver.py:443 for the leapfrog, dt / P for the velocity form
-      t[m * 16 + 12] = leapfrog ? dt2 / row[12] : dt / row[12];
-      t[m * 16 + 13] = row[12];
-      t[m * 16 + 14] = dt;
-    }
     CK(cudaMemcpyAsync(h->tab, t.data(), t.size() * 8, cudaMemcpyHostToDevice, h->stream));
-    CK(cudaStreamSynchronize(h->stream));
   } else {
-    std::vector<float> t(16 * nmat, 0.0f);
-    for (int m = 0; m < nmat; m++) {
-      const double* row = table + m * PHONO_TABLE_COLS;
-      for (int q = 0; q < 12; q++) t[m * 16 + q] = (float)row[q];
-      t[m * 16 + 12] = (float)(dt / row[12]);
-      t[m * 16 + 13] = (float)row[12];
-      t[m * 16 + 14] = (float)dt;
-    }
-    CK(cudaMemcpyAsync(h->tab, t.data(), t.size() * 4, cudaMemcpyHostToDevice, h->stream));
-    CK(cudaStreamSynchronize(h->stream));
+    t32.assign(t.begin(), t.end());
+    CK(cudaMemcpyAsync(h->tab, t32.data(), t32.size() * 4, cudaMemcpyHostToDevice, h->stream));
+  }
+  if (leapfrog) {  // the same entries for the two-launch step
+    for (size_t q = 0; q < t.size(); q++) rec.push_back(soft_record(t[q], false, (uint32_t)q));
+    CK(cudaMemcpyAsync(h->rec, rec.data(), rec.size() * sizeof(SoftRec), cudaMemcpyHostToDevice, h->stream));
+    CK(cudaMemcpyAsync(h->vals, t.data(), t.size() * 8, cudaMemcpyHostToDevice, h->stream));
   }
   CK(cudaMemcpyAsync(h->tab13, table, (size_t)nmat * PHONO_TABLE_COLS * 8, cudaMemcpyHostToDevice, h->stream));
   CK(cudaStreamSynchronize(h->stream));
@@ -263,8 +272,95 @@ static StepArgs<R> make_args(const phono_handle* h, int step_off) {
   return a;
 }
 
+// Two-launch step: the stresses and the update of one chunk of planes after
+// another (one chunk when the stress window holds the whole mesh).  A chunk's
+// update reads the stresses from two planes behind it to one ahead.
+template <class R, class D>
+static cudaError_t split_step(const phono_handle* h, int step_off, int step_end, cudaStream_t st) {
+  SplitArgs<R, D> a{};
+  a.g = h->g;
+  const D** sp[6] = {&a.fdx, &a.fdy, &a.fdz, &a.sdx, &a.sdy, &a.sdz};
+  for (int q = 0; q < 6; q++) *sp[q] = (const D*)h->spd[q];
+  a.mat = h->mat;
+  a.tab = (const R*)h->tab;
+  a.rec = h->rec;
+  a.vals = h->vals;
+  a.dtab = h->dtab;
+  a.src = h->src;
+  a.ubase = (R*)h->ubase;
+  a.vbase = (R*)h->vbase;
+  a.cbase = (R*)h->cbase;
+  for (int q = 0; q < 8; q++) a.abc[q] = (R)h->abc[q];
+  a.dt = (R)h->d.dt;
+  a.surf = (R*)h->surf;
+  a.record_every = h->d.record_every;
+  a.nrec_cap = h->nrec_cap;
+  a.step_base = h->step_base;
+  a.step_off = step_off;
+  a.step_end = step_end;
+  a.surface_mode = h->d.surface_mode;
+  a.bc = h->d.bc;
+  a.source_mode = h->d.source_mode;
+  a.err = h->err;
+  const int nx = h->d.nx, ny = h->d.ny, nz = h->d.nz;
+  a.W = h->win;
+  if (h->stress) {  // leapfrog
+    a.tsy = h->tsy;
+    a.tsx = (unsigned)(ny * h->tsy);
+    a.tcs = (long long)h->win * a.tsx;
+    a.Ta = (R*)h->stress + SPLIT_KOFF;
+    a.Tb = a.Ta + 3 * a.tcs;
+  } else {  // velocity forms: the layout of the fields
+    a.tsy = (int)h->g.sy;
+    a.tsx = (unsigned)h->g.sx;
+    a.tcs = h->g.fstride;
+    a.Ta = a.vbase + 3 * a.tcs + h->g.o0;
+    a.Tb = a.cbase + 3 * a.tcs + h->g.o0;
+  }
+  a.dz1 = fast_div(nz - 1);
+  a.dy1 = fast_div(ny - 1);
+  // points of each component on no face: nj rows (from 1), nk columns (from 0),
+  // planes up to xn, the last of them and the outer rows and column next to a face
+  int xn[3], nj[3], nk[3];
+  for (int c = 0; c < 3; c++) {
+    xn[c] = nx - 2 - (c == 0);
+    nj[c] = ny - 2 - (c == 1);
+    nk[c] = nz - 1 - (c == 2);
+    a.uy_[c] = fast_div(std::max(nj[c] - 2, 1));
+    a.uz_[c] = fast_div(std::max(nk[c] - 1, 1));
+    a.per[c] = fast_div(std::min(nj[c], 2) * nk[c] + std::max(nj[c] - 2, 0));
+    a.nk[c] = fast_div(nk[c]);
+  }
+  const int len = h->win >= nx ? nx : h->win - SPLIT_BEHIND;
+  cudaError_t e = cudaSuccess;
+  for (int p = 0, done = 0; p < nx && e == cudaSuccess; p += len) {
+    a.pa = p;
+    a.pb = std::min(p + len, nx);
+    a.sa = done;
+    a.sb = done = std::min(a.pb + 1, nx);
+    for (int c = 0; c < 3; c++) {
+      const int planes = std::max(0, std::min(a.pb, xn[c]) - p);
+      a.off[c + 1] = a.off[c] + planes * a.per[c].d + (p <= xn[c] && xn[c] < a.pb ? nj[c] * nk[c] : 0);
+    }
+    for (int c = 0; c < 3; c++) {
+      const int planes = std::max(0, std::min(a.pb, xn[c]) - p);
+      a.off[c + 4] = a.off[c + 3] + planes * std::max(nj[c] - 2, 0) * (nk[c] - 1);
+    }
+    e = launch_split(h->d.precision, &a, true, st);
+    if (e == cudaSuccess) e = launch_split(h->d.precision, &a, false, st);
+  }
+  return e;
+}
+
+static cudaError_t split_step_any(const phono_handle* h, int step_off, int step_end, cudaStream_t st) {
+  if (h->d.precision == PHONO_F64) return split_step<double, SoftRec>(h, step_off, step_end, st);
+  if (h->d.precision == PHONO_F64V) return split_step<double, double>(h, step_off, step_end, st);
+  return split_step<float, float>(h, step_off, step_end, st);
+}
+
 // one time step (parts: the handle's form; or 2 tile launch only, 3 face launch only)
 static cudaError_t launch_one(phono_handle* h, int step_off, int parts = -1) {
+  if (h->split) return parts == 3 ? cudaSuccess : split_step_any(h, step_off, 0x7fffffff, h->stream);
   const int form = parts < 0 ? h->separate_faces : parts;
   if (h->d.precision == PHONO_F64) return launch_step_f64(make_args<double>(h, step_off), h->tj, form, h->stream);
   if (h->d.precision == PHONO_F64V) return launch_step_f64v(make_args<double>(h, step_off), h->tj, form, h->stream);
@@ -280,6 +376,70 @@ static long long field_row(int nz, int es) {
 }
 static long long mat_row(int nz) { return round_up(MKOFF + nz + 1, 16); }
 
+// Planes of the stress window of the two-launch step; 0: the mesh steps with
+// the tile pass.
+//  * FP64 (both schemes) is bound by the FP64 pipe: every mesh takes the
+//    two-launch form (256x256x128 cells: 1.07 ms a step against 2.0 for the
+//    best tile shape of the leapfrog, 1.03 against 1.17 for the velocity form).
+//  * FP32 moves 60 more bytes a node than the tile pass, and wins only where
+//    the tile pass has too few planes to march: 7.7 us against 10.3 for the
+//    best tile shape at 35 k nodes, 16 against 20 at 270 k, 45 against 38 at
+//    0.9 M.
+// The velocity forms' stresses fit in the second buffers of v and the Kahan
+// term.  The leapfrog's window is the whole mesh up to 128 MB, else the planes
+// that fill 128 MB and at least 36: chunks cost a tail each (256x256x128: 1.08
+// ms at 64 MB, 1.03 with all 463 MB), and the footprint should not grow by the
+// six stresses of a large mesh.  With ny == 3 a face point can be the point
+// another face's chain starts from (the tile pass's one-launch form has that).
+constexpr long long kSplitF32Nodes = 400000;
+static int split_window(int nx, int ny, int nz, int precision) {
+  if (ny == 3) return 0;
+  if (precision == PHONO_F32K && (long long)nx * ny * nz > kSplitF32Nodes) return 0;
+  long long win = nx;
+  if (precision == PHONO_F64)
+    win = std::min(win, std::max<long long>((128LL << 20) / (6LL * ny * round_up(SPLIT_KOFF + nz, 8) * 8), 36));
+  // flattened points of a launch are 31-bit
+  return 3LL * win * ny * nz <= 0x7fff0000LL ? (int)win : 0;
+}
+// bytes of the leapfrog's window (the velocity forms need none)
+static size_t split_bytes(int nx, int ny, int nz, int precision) {
+  if (precision != PHONO_F64) return 0;
+  return (size_t)6 * split_window(nx, ny, nz, precision) * ny * round_up(SPLIT_KOFF + nz, 8) * 8;
+}
+
+// One allocation holds what depends on the mesh alone: per axis the spacings
+// as the kernels use them (with one value 1 before and two after, so that the
+// tile pass reads the x spacings of its planes -1..nx without range tests;
+// the padding only reaches values whose results are discarded), their FP64
+// reciprocals (energy) and, for the leapfrog, the divisor table and the
+// records of the two-launch step with their values (16 per material id first).
+struct ConstBlock {
+  size_t sp[6], rsp[6], spd[6], div, rec, vals, bytes;
+};
+static ConstBlock const_block(int nx, int ny, int nz, int precision) {
+  const int es = precision == PHONO_F32K ? 4 : 8;
+  const int lens[6] = {nx - 1, ny - 1, nz - 1, nx - 2, ny - 2, nz - 2};
+  ConstBlock c{};
+  auto take = [&](size_t n) {
+    const size_t at = c.bytes;
+    c.bytes += (n + 511) / 512 * 512;
+    return at;
+  };
+  for (int a = 0; a < 6; a++) c.sp[a] = take((size_t)(lens[a] + 3) * es);
+  for (int a = 0; a < 6; a++) c.rsp[a] = take((size_t)lens[a] * 8);
+  if (precision == PHONO_F64) {
+    c.div = take(sizeof(double) * 4 * DIV_TABLE_SLOTS_MAX);
+    size_t n = 256 * 16;
+    for (int a = 0; a < 6; a++) {
+      c.spd[a] = take((size_t)(lens[a] + 3) * sizeof(SoftRec));
+      n += lens[a] + 1;
+    }
+    c.rec = take(256 * 16 * sizeof(SoftRec));
+    c.vals = take(n * 8);
+  }
+  return c;
+}
+
 // Bytes of device memory phono_create allocates for a handle (each cudaMalloc
 // rounded up to 512 bytes).
 static size_t handle_bytes(int nx, int ny, int nz, int precision, int max_steps, int record_every) {
@@ -289,8 +449,7 @@ static size_t handle_bytes(int nx, int ny, int nz, int precision, int max_steps,
   const size_t field_elems = (size_t)(nx + 2) * (ny + 2) * field_row(nz, es);
   const size_t fb = field_elems * es * 3 * nbuf;
   size_t total = r(fb) * (precision == PHONO_F64 ? 1 : 3);
-  const int lens[6] = {nx - 1, ny - 1, nz - 1, nx - 2, ny - 2, nz - 2};
-  for (int a = 0; a < 6; a++) total += r((size_t)(lens[a] + 3) * es) + r((size_t)lens[a] * 8);
+  total += r(const_block(nx, ny, nz, precision).bytes);
   total += r((size_t)(nx + 2) * (ny + 2) * mat_row(nz));
   total += r((size_t)256 * 16 * es) + r((size_t)256 * PHONO_TABLE_COLS * 8);
   const int cap = max_steps > 0 ? max_steps : 1;
@@ -298,7 +457,7 @@ static size_t handle_bytes(int nx, int ny, int nz, int precision, int max_steps,
   const int nrec = record_every > 0 ? max_steps / record_every : 0;
   if (nrec > 0) total += r((size_t)nrec * nx * ny * es);
   total += r(sizeof(int) * 2) + r(sizeof(double2) * kEnergyBlocks) + r(sizeof(double) * 2);
-  if (precision == PHONO_F64) total += r(sizeof(double) * 4 * DIV_TABLE_SLOTS_MAX);
+  total += r(split_bytes(nx, ny, nz, precision));
   return total;
 }
 
@@ -371,9 +530,25 @@ static void* field_ptr(phono_handle* h, int field) {
   int b = t & 1;
   if (field <= PHONO_FIELD_UZ) return arr(h, h->ubase, b, comp);
   if (field <= PHONO_FIELD_UZ_OLD) return nullptr;
+  if (h->split) b = 0;
   if (field <= PHONO_FIELD_VZ) return arr(h, h->vbase, b, comp);
   if (field <= PHONO_FIELD_CZ) return arr(h, h->cbase, b, comp);
   return nullptr;
+}
+
+// Switch a handle between the two-launch form (v and the Kahan term in buffer
+// 0) and the tile pass (in the buffer of the step's parity).
+static cudaError_t set_split(phono_handle* h, bool on) {
+  if (h->split == on) return cudaSuccess;
+  h->split = on;
+  cudaError_t e = cudaSuccess;
+  if (h->vbase && (h->steps_done & 1)) {
+    const size_t n = 3 * h->field_elems * h->es;
+    for (char* b : {h->vbase, h->cbase})
+      if (e == cudaSuccess)
+        e = cudaMemcpyAsync(on ? b : b + n, on ? b + n : b, n, cudaMemcpyDeviceToDevice, h->stream);
+  }
+  return e;
 }
 
 // Tile decomposition of a handle: tile_j rows x 32 z-points per block, the
@@ -585,52 +760,71 @@ int phono_create(const phono_desc* d, phono_handle** out) {
     TRYC(cudaMemsetAsync(h->cbase, 0, fb, h->stream));
   }
 
-  // spacings
+  // spacings and what derives from them, in one allocation and one copy
   const double* arrs[6] = {d->fdx, d->fdy, d->fdz, d->sdx, d->sdy, d->sdz};
   int lens[6] = {nx - 1, ny - 1, nz - 1, nx - 2, ny - 2, nz - 2};
-  // FP64 leapfrog: divisor table (div_tab in div_table.cuh) over the distinct
-  // spacing values and 1.0, the divisors the step uses
-  // (allocated for every FP64 handle, so that phono_footprint is exact)
-  if (f64) {
-    std::vector<double> tbl;
-    double* tab_dev = nullptr;
-    TRY(dalloc(h, (void**)&tab_dev, sizeof(double) * 4 * DIV_TABLE_SLOTS_MAX));
+  {
+    const ConstBlock cb = const_block(nx, ny, nz, d->precision);
+    std::vector<char> host(cb.bytes, 0);
+    char* dev = nullptr;
+    TRY(dalloc(h, (void**)&dev, cb.bytes));
     std::vector<double> divisors{1.0};
-    for (int a = 0; a < 6; a++) divisors.insert(divisors.end(), arrs[a], arrs[a] + lens[a]);
-    if (build_div_table(divisors, tbl, &h->dtab.mult, &h->dtab.shift)) {
-      TRYC(cudaMemcpy(tab_dev, tbl.data(), tbl.size() * sizeof(double), cudaMemcpyHostToDevice));
-      h->dtab.tab = tab_dev;
+    uint32_t nval = 256 * 16;  // the table's values come first (upload_table)
+    double* vals = f64 ? (double*)(host.data() + cb.vals) : nullptr;
+    for (int a = 0; a < 6; a++) {
+      h->h_sp0[a] = arrs[a][0];
+      h->sp_host[a].assign(arrs[a], arrs[a] + lens[a]);
+      h->sp[a] = dev + cb.sp[a] + h->es;
+      h->spd[a] = f64 ? (void*)((SoftRec*)(dev + cb.spd[a]) + 1) : h->sp[a];
+      h->rsp64[a] = (double*)(dev + cb.rsp[a]);
+      SoftRec* rec = (SoftRec*)(host.data() + cb.spd[a]);
+      const uint32_t one = nval;  // the padding's divisor
+      if (f64) vals[nval++] = 1.0;
+      for (int q = -1; q < lens[a] + 2; q++) {
+        const bool in = q >= 0 && q < lens[a];
+        const double v = in ? arrs[a][q] : 1.0;
+        // F64: raw spacings; the velocity forms: reciprocals
+        if (h->es == 4) ((float*)(host.data() + cb.sp[a]))[q + 1] = (float)(1.0 / v);
+        else ((double*)(host.data() + cb.sp[a]))[q + 1] = f64 ? v : 1.0 / v;
+        if (in) ((double*)(host.data() + cb.rsp[a]))[q] = 1.0 / v;
+        if (f64) {
+          rec[q + 1] = soft_record(v, true, in ? nval : one);
+          if (in) vals[nval++] = v;
+        }
+      }
+      divisors.insert(divisors.end(), arrs[a], arrs[a] + lens[a]);
     }
-  }
-  // device copies carry one value 1 before and two after the array, so the
-  // tile pass reads the x spacings of its planes -1..nx without range tests
-  // (the padding only reaches values whose results are discarded)
-  for (int a = 0; a < 6; a++) {
-    h->h_sp0[a] = arrs[a][0];
-    h->sp_host[a].assign(arrs[a], arrs[a] + lens[a]);
-    void* spb = nullptr;
-    TRY(dalloc(h, &spb, (size_t)(lens[a] + 3) * h->es));
-    h->sp[a] = (char*)spb + h->es;
-    TRY(dalloc(h, (void**)&h->rsp64[a], (size_t)lens[a] * 8));
-    {
-      std::vector<double> rec(lens[a]);
-      for (int q = 0; q < lens[a]; q++) rec[q] = 1.0 / arrs[a][q];
-      TRYC(cudaMemcpy(h->rsp64[a], rec.data(), (size_t)lens[a] * 8, cudaMemcpyHostToDevice));
+    if (f64) {
+      h->rec = (SoftRec*)(dev + cb.rec);
+      h->vals = (double*)(dev + cb.vals);
+      // divisor table (div_tab in div_table.cuh) over the distinct spacing
+      // values and 1.0, the divisors the step uses
+      std::vector<double> tbl;
+      if (build_div_table(divisors, tbl, &h->dtab.mult, &h->dtab.shift)) {
+        std::memcpy(host.data() + cb.div, tbl.data(), tbl.size() * sizeof(double));
+        h->dtab.tab = (const double*)(dev + cb.div);
+      }
     }
-    if (h->es == 8) {  // F64: raw spacings; F64V: reciprocals in double
-      std::vector<double> r(lens[a] + 3, 1.0);
-      for (int q = 0; q < lens[a]; q++) r[q + 1] = f64 ? arrs[a][q] : 1.0 / arrs[a][q];
-      TRYC(cudaMemcpy(spb, r.data(), r.size() * 8, cudaMemcpyHostToDevice));
-    } else {
-      std::vector<float> r(lens[a] + 3, 1.0f);
-      for (int q = 0; q < lens[a]; q++) r[q + 1] = (float)(1.0 / arrs[a][q]);
-      TRYC(cudaMemcpy(spb, r.data(), r.size() * 4, cudaMemcpyHostToDevice));
-    }
+    TRYC(cudaMemcpy(dev, host.data(), host.size(), cudaMemcpyHostToDevice));
   }
   // materials: padded id layout and the 16-entry device rows (capacity 256 ids)
   TRY(dalloc(h, (void**)&h->mat, h->mat_bytes));
   TRYC(cudaMemset(h->mat, 0, h->mat_bytes));
   TRY(dalloc(h, &h->tab, (size_t)256 * 16 * h->es));
+  // two-launch step; the leapfrog's window is zero outside the points the
+  // stress pass writes, and a mesh whose window does not fit keeps to the tiles
+  h->win = split_window(nx, ny, nz, d->precision);
+  if (const size_t sb = split_bytes(nx, ny, nz, d->precision)) {
+    h->tsy = (int)round_up(SPLIT_KOFF + nz, 8);
+    if (dalloc(h, (void**)&h->stress, sb)) {
+      h->win = 0;
+      cudaGetLastError();
+      g_err.clear();
+    } else {
+      TRYC(cudaMemsetAsync(h->stress, 0, sb, h->stream));
+    }
+  }
+  h->split = h->win > 0 && !d->tile_j && !d->x_segment;
   TRY(dalloc(h, (void**)&h->tab13, (size_t)256 * PHONO_TABLE_COLS * 8));
   TRY(upload_materials(h, d->mat, d->table, d->nmat));
   TRY(encode_tensor_maps(h));
@@ -775,6 +969,7 @@ int phono_test_wait_timeout(phono_handle* h, int polls, int skip_plane) {
   if (h->batch) return fail(PHONO_ERR_STATE, "handle is in a batch");
   if (polls < 0 || skip_plane < -1 || skip_plane > h->d.nx) return fail(PHONO_ERR_ARG, "polls >= 0, skip_plane in -1..nx");
   CK(cudaStreamSynchronize(h->stream));
+  if (polls || skip_plane >= 0) CK(set_split(h, false));  // the two-launch form waits for nothing
   h->wait_polls = polls;
   h->skip_plane = skip_plane;
   if (h->graph) {  // the hook is a kernel argument baked into the graph
@@ -1070,7 +1265,7 @@ void* phono_stream(phono_handle* h) { return h ? (void*)h->stream : nullptr; }
 // switch a handle to tile height tj and the given x segments, keeping the old
 // shape if the new one cannot be set up
 static int retile(phono_handle* h, int tj, int xseg, const std::vector<int>& starts) {
-  if (tj == h->tj && starts == h->seg_start) {
+  if (!h->split && tj == h->tj && starts == h->seg_start) {
     h->xseg = xseg;
     return PHONO_OK;
   }
@@ -1088,6 +1283,7 @@ static int retile(phono_handle* h, int tj, int xseg, const std::vector<int>& sta
     g_err = m;
     return rc;
   }
+  CK(set_split(h, false));
   if (h->graph) {  // the captured launches hold the old grid and tensor maps
     cudaGraphExecDestroy(h->graph);
     h->graph = nullptr;
@@ -1098,9 +1294,11 @@ static int retile(phono_handle* h, int tj, int xseg, const std::vector<int>& sta
 int phono_set_tiling(phono_handle* h, int tile_j, int x_segment) {
   if (!h) return fail(PHONO_ERR_ARG, "handle is NULL");
   if (h->batch) return fail(PHONO_ERR_STATE, "handle is in a batch");
+  const bool keep = tile_j == 0;
   if (tile_j == 0) tile_j = h->tj;
   if (tile_j != 4 && tile_j != 8 && tile_j != 16) return fail(PHONO_ERR_ARG, "tile_j must be 0, 4, 8 or 16");
   if (x_segment < -4096) return fail(PHONO_ERR_ARG, "x_segment out of range");
+  if (x_segment == 0 && tile_j == h->tj && keep) return PHONO_OK;
   if (x_segment == 0)  // keep the current segments (a list included)
     return retile(h, tile_j, h->xseg, h->seg_start);
   return retile(h, tile_j, x_segment, segment_starts(h->d.nx - 1, x_segment));
@@ -1180,11 +1378,19 @@ static void batch_detach(phono_batch* b, const phono_handle* h) {
     }
 }
 
+// the batch's work is done: the handle is on its own again
+static cudaError_t leave_batch(phono_handle* h) {
+  h->batch = nullptr;
+  if (!h->resplit) return cudaSuccess;
+  h->resplit = false;
+  return set_split(h, true);
+}
+
 static void batch_release(phono_batch* b) {
   if (!b) return;
   if (b->stream) cudaStreamSynchronize(b->stream);
   for (phono_handle* h : b->slot)
-    if (h) h->batch = nullptr;
+    if (h) leave_batch(h);
   if (b->graph) cudaGraphExecDestroy(b->graph);
   for (cudaGraphExec_t g : b->igraph)
     if (g) cudaGraphExecDestroy(g);
@@ -1283,6 +1489,7 @@ static int batch_rebuild(phono_batch* b) {
 // one step of instance s on stream st, with the handle's own kernels and tiles
 static cudaError_t chain_launch(phono_batch* b, int s, int step_off, cudaStream_t st) {
   phono_handle* h = b->slot[s];
+  if (h->split) return split_step_any(h, step_off, b->step_end[s], st);
   if (h->d.precision == PHONO_F32K) {
     StepArgs<float> a = make_args<float>(h, step_off);
     a.step_end = b->step_end[s];
@@ -1494,6 +1701,10 @@ int phono_batch_add(phono_batch* b, phono_handle* h, int nsteps) {
     if (s < 0 && !b->slot[q]) s = q;
   }
   if (s < 0) return fail(PHONO_ERR_NOMEM, "batch is full");
+  if (!b->streams && h->split) {
+    CK(set_split(h, false));
+    h->resplit = true;
+  }
   CK(cudaStreamSynchronize(h->stream));
   CK(cudaStreamSynchronize(b->stream));
   if (b->precision == PHONO_F32K) {
@@ -1516,7 +1727,7 @@ int phono_batch_add(phono_batch* b, phono_handle* h, int nsteps) {
 int phono_batch_remove(phono_batch* b, int s) {
   if (!b || s < 0 || s >= b->cap || !b->slot[s]) return fail(PHONO_ERR_ARG, "no instance in that slot");
   CK(cudaStreamSynchronize(b->stream));
-  b->slot[s]->batch = nullptr;
+  CK(leave_batch(b->slot[s]));
   b->slot[s] = nullptr;
   b->remaining[s] = 0;
   b->dirty = true;

@@ -1,0 +1,346 @@
+// Two-launch step: all stresses of a chunk of planes into a stress window in
+// global memory, then every displacement point of the chunk, faces included.
+//
+// Each stress is computed once and each thread owns one point of a flattened
+// box, so no lane idles on a ragged z or y extent, no block waits at a barrier
+// and a mesh of a few thousand nodes still spreads over all SMs.  The stresses
+// cost a write and a read of 24 (FP32) or 48 bytes a node.  The velocity forms
+// keep them in the second buffers of v and of the Kahan term; the leapfrog has
+// a window of at most a few dozen planes of a large mesh, and a step walks
+// through it in chunks.  The result is that of the tile pass, bit for bit.
+//
+// Bound (one GB300, us a step, the best tile shape of the tile pass first):
+// FP64 by the FP64 pipe and, nearly as much, by instruction issue (18 FP64 of
+// 1500 instructions a stress point, FP64 pipe 38% and ALU 52% busy); small
+// meshes by two dependent launches (1.2 us each) of three or four L2
+// latencies.
+//   nodes       25x21x13  41x41x21  61x61x21  150x131x47  194x162x98  257x257x129
+//   F64         25 / 11   32 / 12   47 / 15   354 / 118   969 / 391   2012 / 1071
+//   F64V        13 / 8    21 / 10   29 / 14   197 / 121   559 / 378   1174 / 1037
+//   F32K        9 / 6     10 / 7    12 / 8    38 / -      80 / -      154 / -
+#include "scheme.cuh"
+#include "split_common.cuh"
+
+namespace phono {
+
+__device__ __forceinline__ float ldd(const float* p) { return __ldg(p); }
+__device__ __forceinline__ double ldd(const double* p) { return __ldg(p); }
+__device__ __forceinline__ SoftRec ldd(const SoftRec* p) {
+  const uint4 v = __ldg(reinterpret_cast<const uint4*>(p));
+  return SoftRec{v.x, v.y, v.z, v.w};
+}
+
+// velocity forms: reciprocal spacings, coefficients as stored
+template <class B>
+struct VelOps {
+  using Base = B;
+  using R = typename B::R;
+  using D = R;
+  using Args = SplitArgs<R, D>;
+  static constexpr int STRESS_BLOCKS = sizeof(R) == 8 ? 6 : 12, UPDATE_BLOCKS = sizeof(R) == 8 ? 9 : 8;
+  static __device__ __forceinline__ void normals(const Args& a, int id, R d1, R d2, R d3, D x, D y, D z, R* t) {
+    const R* row = a.tab + 16 * id;
+    R c[9];
+    if constexpr (sizeof(R) == 4) {
+      const float4 q0 = __ldg(reinterpret_cast<const float4*>(row)), q1 = __ldg(reinterpret_cast<const float4*>(row) + 1);
+      c[0] = q0.x, c[1] = q0.y, c[2] = q0.z, c[3] = q0.w, c[4] = q1.x, c[5] = q1.y, c[6] = q1.z, c[7] = q1.w;
+      c[8] = __ldg(row + 8);
+    } else {
+      for (int q = 0; q < 9; q++) c[q] = __ldg(row + q);
+    }
+    for (int q = 0; q < 3; q++) t[q] = B::tn1(a.dtab, c + 3 * q, d1, d2, d3, x, y, z);
+  }
+  static __device__ __forceinline__ R shear(const Args& a, int id, int col, R d1, D x, R d2, D y) {
+    return B::ts(a.dtab, __ldg(a.tab + 16 * id + col), d1, x, d2, y);
+  }
+  static __device__ __forceinline__ R div3(const Args& a, R d1, D x, R d2, D y, R d3, D z) {
+    return B::div3(a.dtab, d1, x, d2, y, d3, z);
+  }
+  static __device__ __forceinline__ R update(const Args& a, int id, R u, Pw<R> pw, R dv, R& vn, R& cn) {
+    return update_value<B>(u, pw, dv, __ldg(a.tab + 16 * id + 12), a.dt, vn, cn);
+  }
+};
+
+// the leapfrog: multiplications by constants and divisions in integer
+// arithmetic (soft_f64.cuh), additions on the FP64 pipe
+__device__ __noinline__ double slow_div(double x, double b, DivTable k) { return k.tab ? div_tab(x, b, k) : __ddiv_rn(x, b); }
+
+struct LeapOps {
+  using Base = F64;
+  using R = double;
+  using D = SoftRec;
+  using Args = SplitArgs<double, SoftRec>;
+  // resident blocks the registers are allotted for: 6 and 7 gave 1071 us a
+  // step on 256x256x128 cells, 5 and 7 1112, 8 and 8 1116, 9 and 12 1160
+  static constexpr int STRESS_BLOCKS = 6, UPDATE_BLOCKS = 7;
+  struct Num {
+    double x;
+    SoftNum n;
+    bool ok;
+  };
+  static __device__ __forceinline__ Num split(double x) {
+    Num v;
+    v.x = x;
+    v.n = soft_split(x, v.ok);
+    return v;
+  }
+  // a zero's quotient or product keeps its sign (the other operand's sign is in `flip`)
+  static __device__ __forceinline__ bool zero(double x) {
+    return ((uint32_t)__double2hiint(x) << 1 | (uint32_t)__double2loint(x)) == 0u;
+  }
+  static __device__ __forceinline__ double signed_zero(double x, uint32_t flip) {
+    return soft_double(((uint32_t)__double2hiint(x) ^ flip) & 0x80000000u, 0u);
+  }
+  static __device__ __forceinline__ double divide(const Args& a, double x, const SoftRec& d) {
+    const Num v = split(x);
+    if (v.ok && (int)d.hi < 0) return soft_join(soft_div(v.n, d, [&] { return __ldg(a.vals + d.idx); }));
+    return zero(x) ? signed_zero(x, 0u) : slow_div(x, __ldg(a.vals + d.idx), a.dtab);
+  }
+  static __device__ __forceinline__ double times(const Args& a, double x, const SoftRec& c) {
+    const Num v = split(x);
+    if (v.ok && (int)c.hi < 0) return soft_join(soft_mul(v.n, c));
+    return zero(x) ? signed_zero(x, c.de) : __dmul_rn(__ldg(a.vals + c.idx), x);
+  }
+  // (c * x) / d, both roundings
+  static __device__ __forceinline__ double scaled(const Args& a, const Num& v, const SoftRec& c, const SoftRec& d) {
+    if (v.ok && (int)(c.hi & d.hi) < 0)
+      return soft_join(soft_div(soft_mul(v.n, c), d, [&] { return __ldg(a.vals + d.idx); }));
+    if (zero(v.x)) return signed_zero(v.x, c.de);
+    const double y = __dmul_rn(__ldg(a.vals + c.idx), v.x);
+    return zero(y) ? y : slow_div(y, __ldg(a.vals + d.idx), a.dtab);
+  }
+  static __device__ __forceinline__ void normals(const Args& a, int id, R d1, R d2, R d3, const D& x, const D& y,
+                                                 const D& z, R* t) {
+    const SoftRec* c = a.rec + 16 * id;
+    const Num v1 = split(d1), v2 = split(d2), v3 = split(d3);
+#pragma unroll
+    for (int q = 0; q < 3; q++)
+      t[q] = __dadd_rn(__dadd_rn(scaled(a, v1, ldd(c + 3 * q), x), scaled(a, v2, ldd(c + 3 * q + 1), y)),
+                       scaled(a, v3, ldd(c + 3 * q + 2), z));
+  }
+  static __device__ __forceinline__ R shear(const Args& a, int id, int col, R d1, const D& x, R d2, const D& y) {
+    return times(a, __dadd_rn(divide(a, d1, x), divide(a, d2, y)), ldd(a.rec + 16 * id + col));
+  }
+  static __device__ __forceinline__ R div3(const Args& a, R d1, const D& x, R d2, const D& y, R d3, const D& z) {
+    return __dadd_rn(__dadd_rn(divide(a, d1, x), divide(a, d2, y)), divide(a, d3, z));
+  }
+  static __device__ __forceinline__ R update(const Args& a, int id, R u, Pw<R> pw, R dv, R& vn, R& cn) {
+    vn = cn = 0;
+    // 2u is exact, so the FMA rounds as the reference's 2u - u_old
+    return __dadd_rn(__fma_rn(2.0, u, -pw.p0), times(a, dv, ldd(a.rec + 16 * id + 12)));
+  }
+};
+
+__device__ __forceinline__ int fdiv(int n, const FastDiv& f) { return (int)(__umulhi(2u * (unsigned)n, f.mult) >> f.shift); }
+
+// ---------------------------------------------------------------------------
+// stresses of planes [sa, sb): one thread per node of [sa, sb) x [0, ny-1) x
+// [0, nz-1).  Zero where the reference never writes (base_solver.py:329-433).
+// ---------------------------------------------------------------------------
+template <class O>
+__global__ void __launch_bounds__(SPLIT_THREADS, O::STRESS_BLOCKS) split_stress_kernel(const __grid_constant__ typename O::Args a) {
+  using R = typename O::R;
+  using B = typename O::Base;
+  const int tt = __ldg(a.step_base) + a.step_off;
+  if (tt >= a.step_end) return;
+  const Geo& g = a.g;
+  const int nx = g.nx;
+  int n = blockIdx.x * SPLIT_THREADS + threadIdx.x;
+  const int q1 = fdiv(n, a.dz1), k = n - q1 * a.dz1.d;
+  const int q2 = fdiv(q1, a.dy1), j = q1 - q2 * a.dy1.d;
+  const int i = a.sa + q2;
+  if (i >= a.sb) return;
+  const Roles<R> r = roles<B>(a, tt);
+  const unsigned sx = (unsigned)g.sx, sy = (unsigned)g.sy;
+  const unsigned o = (unsigned)g.o0 + (unsigned)i * sx + (unsigned)j * sy + (unsigned)k;
+  const R *X = r.u_cur + o, *Y = X + r.fs, *Z = Y + r.fs;
+  const uint8_t* M = a.mat + g.mo0 + (long long)i * g.msx + (long long)j * g.msy + k;
+  const bool kz = k == 0;
+  const int up = kz ? 0 : 1;  // shear moduli of T4, T5: one layer down, except in the z = 0 row
+  const bool i_n = i >= 1 && i <= nx - 2, i_s = i <= nx - 2, j_n = j >= 1;
+  const R x0 = X[0], y0 = Y[0];
+  R z0 = Z[0];
+  if (i == 0 && (a.source_mode == 1 || kz)) z0 = (R)__ldg(a.src + tt);  // source overwrite (base_solver.py:251)
+  const R x_k = X[1], x_j = X[sy], y_k = Y[1], y_i = Y[sx], z_j = Z[sy], z_i = Z[sx];
+  R t[6] = {R(0), R(0), R(0), R(0), R(0), R(0)};
+  if (i_n && j_n)
+    O::normals(a, M[0], B::sub(x0, *(X - sx)), B::sub(y0, *(Y - sy)), B::sub(z0, Z[-1]), ldd(a.sdx + (kz ? 0 : i - 1)),
+               ldd(a.sdy + (kz ? 0 : j - 1)), ldd(a.sdz + (kz ? 0 : k - 1)), t);
+  if (kz) t[2] = R(0);  // base_solver.py:418
+  // shears; the z = 0 row's substituted spacings are base_solver.py:420-433's
+  if (i_n)
+    t[3] = O::shear(a, M[g.msy + up], 9, B::sub(y_k, y0), ldd(kz ? a.fdy : a.fdz + k), B::sub(z_j, z0),
+                    ldd(kz ? a.fdz : a.fdy + j));
+  if (i_s && j_n)
+    t[4] = O::shear(a, M[g.msx + up], 10, B::sub(x_k, x0), ldd(kz ? a.fdx : a.fdz + k), B::sub(z_i, z0),
+                    ldd(kz ? a.fdz : a.fdx + i));
+  if (i_s)
+    t[5] = O::shear(a, M[g.msx + g.msy], 11, B::sub(x_j, x0), ldd(kz ? a.fdx : a.fdy + j), B::sub(y_i, y0),
+                    ldd(kz ? a.fdz : a.fdx + i));
+  const unsigned to = (unsigned)(i % a.W) * a.tsx + (unsigned)(j * a.tsy + k);
+#pragma unroll
+  for (int q = 0; q < 3; q++) {
+    a.Ta[to + q * a.tcs] = t[q];
+    a.Tb[to + q * a.tcs] = t[q + 3];
+  }
+}
+
+// ---------------------------------------------------------------------------
+// new state of planes [pa, pb): one thread per point of each component that is
+// on no face, those next to a face first.  A face point's value is a chain of at most four face formulas
+// (base_solver.py:540-554, in the order x=N, y=0, y=N, z=N) from the new value
+// of one such point: the thread of that point writes it (in warps of their own:
+// with the z = N points in the lanes above them, the FP64 step was 20% slower).
+// The velocity forms
+// update v and the Kahan term in place (no other thread reads them), which
+// leaves their second buffers to the stresses.
+// ---------------------------------------------------------------------------
+template <class O>
+__global__ void __launch_bounds__(SPLIT_THREADS, O::UPDATE_BLOCKS) split_update_kernel(const __grid_constant__ typename O::Args a) {
+  using R = typename O::R;
+  using B = typename O::Base;
+  const int tt = __ldg(a.step_base) + a.step_off;
+  if (tt >= a.step_end) return;
+  const Geo& g = a.g;
+  int n = blockIdx.x * SPLIT_THREADS + threadIdx.x;
+  if (n >= a.off[6]) return;
+  int c, i, j, k;
+  const bool edge = n < a.off[3];
+  if (!edge) {
+    c = (n >= a.off[4]) + (n >= a.off[5]);
+    n -= a.off[3 + c];
+    const FastDiv fz = a.uz_[c], fy = a.uy_[c];
+    const int q1 = fdiv(n, fz), q2 = fdiv(q1, fy);
+    k = n - q1 * fz.d, j = q1 - q2 * fy.d + 2, i = a.pa + q2;
+  } else {  // points next to a face: per plane the rows j = 1 and jN-1, then the rest of k = kN-1
+    c = (n >= a.off[1]) + (n >= a.off[2]);
+    n -= a.off[c];
+    const int xi = ext_x(g, c) - 1, nj = ext_y(g, c) - 2, nk = ext_z(g, c) - 1, rows = min(nj, 2) * nk;
+    const int planes = max(min(a.pb, xi - 1) - a.pa, 0);
+    i = fdiv(n, a.per[c]);
+    if (i < planes) {
+      n -= i * a.per[c].d;
+      i += a.pa;
+      if (n < nk) j = 1, k = n;
+      else if (n < rows) j = nj, k = n - nk;
+      else j = 2 + n - rows, k = nk - 1;
+    } else {  // the plane next to x = N: all of it
+      n -= planes * a.per[c].d;
+      i = xi - 1;
+      j = fdiv(n, a.nk[c]);
+      k = n - j++ * nk;
+    }
+  }
+  Roles<R> r = roles<B>(a, tt);
+  if constexpr (B::kahan) {
+    r.v_in = r.v_out = a.vbase;
+    r.c_in = r.c_out = a.cbase;
+  }
+  const unsigned o = (unsigned)g.o0 + (unsigned)i * (unsigned)g.sx + (unsigned)j * (unsigned)g.sy + (unsigned)k;
+  const R* uc = r.cur(c);
+  const R u = __ldg(uc + o);
+  // faces next to the point (x = N; y = 0 or N; z = N), and the old values of
+  // the up to 2 x 2 x 2 points they span, read here because they are off the
+  // path of the update
+  const int nfx = edge && i == ext_x(g, c) - 2, nfz = edge && k == ext_z(g, c) - 2;
+  int fj = !edge ? 0 : j == 1 ? -1 : j == ext_y(g, c) - 2 ? 1 : 0;
+  const bool two_y = fj < 0 && j == ext_y(g, c) - 2;
+  R old[8];  // [z][y][x]
+  auto read_old = [&] {
+    const R s = (R)__ldg(a.src + tt);
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+      const bool fx = q & 1, fy = q & 2, fk = q & 4;
+      if ((fx && !nfx) || (fy && !fj) || (fk && !nfz)) continue;
+      old[q] = __ldg(uc + (o + (fx ? (unsigned)g.sx : 0u) + (fy ? (unsigned)(fj * (int)g.sy) : 0u) + (fk ? 1u : 0u)));
+      if (c == 2 && i == 0 && !fx && (a.source_mode == 1 || (k == 0 && !fk))) old[q] = s;  // source overwrite (base_solver.py:251)
+    }
+  };
+  if (edge) read_old();
+  R val, vn = R(0), cn = R(0);
+  if (c == 0 || i >= 1) {
+    const bool kz = k == 0;
+    Pw<R> pw;
+    if constexpr (B::kahan) pw = Pw<R>{r.v_in[c * r.fs + o], r.c_in[c * r.fs + o]};
+    else pw = load_pw<B>(r, c, o);
+    const unsigned s0 = (unsigned)i % a.W, sp = s0 + 1 == a.W ? 0 : s0 + 1, sm = s0 == 0 ? a.W - 1 : s0 - 1;
+    const unsigned ro = (unsigned)(j * a.tsy + k);
+    const R *A = a.Ta + ro, *Bc = a.Tb + ro + s0 * a.tsx, *Bm = a.Tb + ro + sm * a.tsx;  // T4..T6 of planes i, i-1
+    const R* Ac = A + s0 * a.tsx;
+    const long long tc = a.tcs;
+    const uint8_t* M = a.mat + g.mo0 + (long long)i * g.msx + (long long)j * g.msy + k;
+    R d1, d2, d3;
+    const typename O::D *ax, *ay, *az;
+    int id;
+    if (c == 0) {  // base_solver.py:441-447, 495-501
+      d1 = B::sub(*(A + sp * a.tsx), Ac[0]);
+      d2 = B::sub(Bc[2 * tc], *(Bc + 2 * tc - a.tsy));
+      d3 = B::sub(Bc[tc], *(Bc + tc - 1));
+      ax = a.fdx + (kz ? 0 : i), ay = a.sdy + (kz ? 0 : j - 1), az = a.sdz + (kz ? 0 : k - 1);
+      id = M[g.msx];
+    } else if (c == 1) {  // base_solver.py:449-455, 503-509
+      d1 = B::sub(Bc[2 * tc], Bm[2 * tc]);
+      d2 = B::sub(*(Ac + tc + a.tsy), Ac[tc]);
+      d3 = B::sub(Bc[0], *(Bc - 1));
+      ax = a.sdx + (kz ? 0 : i - 1), ay = a.fdy + (kz ? 0 : j), az = a.sdz + (kz ? 0 : k - 1);
+      id = M[g.msy];
+    } else {  // base_solver.py:457-463, 511-516: as written, :516 adds T3[..,1] undivided
+      d1 = B::sub(Bc[tc], Bm[tc]);
+      d2 = B::sub(Bc[0], *(Bc - a.tsy));
+      d3 = B::sub(Ac[2 * tc + 1], Ac[2 * tc]);
+      ax = a.sdx + (kz ? 0 : i - 1), ay = a.sdy + (kz ? 0 : j - 1);
+      az = a.fdz + (kz ? (a.surface_mode == 0 ? -1 : 0) : k);
+      id = kz ? M[0] : M[1];
+    }
+    const R dv = O::div3(a, d1, ldd(ax), d2, ldd(ay), d3, ldd(az));
+    val = O::update(a, id, u, pw, dv, vn, cn);
+    store_point<B>(r, c, o, val, vn, cn);
+  } else {  // uy, uz at i = 0: not written by the reference, keeps its state
+    val = u;
+    r.out(c)[o] = u;
+  }
+  if (c == 2 && k == 0) record(a, tt, i, j, val);
+  if (!edge) return;
+  for (;;) {
+    // every face point whose chain starts here: x = N first, then y, then z = N
+    R w[8];
+    w[0] = val;
+#pragma unroll
+    for (int q = 1; q < 8; q++) {
+      const bool fx = q & 1, fy = q & 2, fk = q & 4;
+      if ((fx && !nfx) || (fy && !fj) || (fk && !nfz)) continue;
+      const int from = q & (fk ? 3 : fy ? 1 : 0);
+      const R f = fk ? (c == 2 ? a.abc[7] : a.abc[6])
+                     : !fy ? (c == 0 ? a.abc[0] : a.abc[1])
+                           : fj < 0 ? (c == 1 ? a.abc[3] : a.abc[2]) : (c == 1 ? a.abc[5] : a.abc[4]);
+      w[q] = a.bc == 1 ? R(0) : B::abc(f, w[from], old[q], old[from]);
+      store_point<B>(r, c, o + (fx ? (unsigned)g.sx : 0u) + (fy ? (unsigned)(fj * (int)g.sy) : 0u) + (fk ? 1u : 0u), w[q],
+                     R(0), R(0));
+      if (c == 2 && k == 0 && !fk) record(a, tt, i + fx, fy ? j + fj : j, w[q]);
+    }
+    if (!two_y || fj > 0) break;
+    fj = 1;  // a single row between the two y faces
+    read_old();
+  }
+}
+
+template <class O>
+static cudaError_t split_launch(const typename O::Args& a, bool stress, cudaStream_t st) {
+  if (stress) {
+    const long long n = (long long)(a.sb - a.sa) * a.dy1.d * a.dz1.d;
+    if (n > 0) split_stress_kernel<O><<<(int)((n + SPLIT_THREADS - 1) / SPLIT_THREADS), SPLIT_THREADS, 0, st>>>(a);
+  } else {
+    const long long n = a.off[6];
+    if (n > 0) split_update_kernel<O><<<(int)((n + SPLIT_THREADS - 1) / SPLIT_THREADS), SPLIT_THREADS, 0, st>>>(a);
+  }
+  return cudaGetLastError();
+}
+
+// one pass over the planes set in the arguments; precision as in phono.h
+cudaError_t launch_split(int precision, const void* args, bool stress, cudaStream_t st) {
+  if (precision == 0) return split_launch<LeapOps>(*(const LeapOps::Args*)args, stress, st);
+  if (precision == 2) return split_launch<VelOps<F64V>>(*(const VelOps<F64V>::Args*)args, stress, st);
+  return split_launch<VelOps<F32K>>(*(const VelOps<F32K>::Args*)args, stress, st);
+}
+
+}  // namespace phono

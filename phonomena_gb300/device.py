@@ -84,6 +84,7 @@ class DeviceSimulation:
         self._h = h
         self.tile_j = int(tile_j) or (4 if precision == "f32k" else 8)
         self.x_segment = int(x_segment) or 24
+        self._default_shape = not tile_j and not x_segment and segments is None  # the library picks the step's form
         self.surface_mode, self.bc, self.source_mode = surface_mode, bc, source_mode
         self._source = None
         if segments is not None:
@@ -128,6 +129,8 @@ class DeviceSimulation:
             check(self._L.phono_set_tiling(self._h, int(tile_j), int(x_segment)))
             self.x_segment = int(x_segment) or self.x_segment
         self.tile_j = int(tile_j) or self.tile_j
+        if np.ndim(x_segment) or tile_j or x_segment:
+            self._default_shape = False
 
     def set_lattice(self, lat, table):
         """Material ids built on the device from a hole lattice (crystal.lattice)
@@ -263,8 +266,8 @@ class DeviceSimulation:
         for k, v in self._sp.items():
             ck[k] = v
         listed = isinstance(self.x_segment, tuple)
-        ck["meta"] = np.array([self.dt, self.max_steps, self.record_every, self.tile_j,
-                               0 if listed else self.x_segment], np.float64)
+        ck["meta"] = np.array([self.dt, self.max_steps, self.record_every, 0 if self._default_shape else self.tile_j,
+                               0 if listed or self._default_shape else self.x_segment], np.float64)
         ck["segments"] = np.array(self.x_segment if listed else [], np.int32)
         ck["modes"] = np.array([self.precision, self.surface_mode, self.bc, self.source_mode])
         return ck
