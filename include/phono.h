@@ -117,8 +117,9 @@ int phono_set_source(phono_handle *h, const double *samples, int n);
  * launch when ny == 3), or in the two-launch form a stress launch and an
  * update launch per chunk of planes, replayed from captured CUDA graphs of 12
  * steps.  The two-launch form is that of handles with the default tile shape
- * (tile_j = x_segment = 0) in FP64, and in FP32 up to 400,000 nodes; results
- * are the same bits.  Replaces the loop body of BaseSolver.run
+ * (tile_j = x_segment = 0) in FP64, and in FP32 up to 170,000 nodes.  Otherwise
+ * handles with the default tile shape pick their own tiles.  Results are the
+ * same bits.  Replaces the loop body of BaseSolver.run
  * (base_solver.py:245-266): source, update_T, update_T_BC, update_u,
  * update_u_BC, time_step.  Asynchronous on the handle's stream. */
 int phono_step(phono_handle *h, int nsteps);
@@ -304,8 +305,9 @@ int phono_energy_static(const phono_energy_dense *in, double *out_dev, void *str
  * object (base_solver.py:245-266) and has no counterpart; the per-instance
  * arithmetic is that of phono_step, bit for bit.  Instances are handles made
  * by phono_create with the batch's precision and ny >= 4 (and the batch's
- * tile_j in the persistent scheme); each keeps its own x segments.  While a
- * handle is in a batch, phono_step, phono_reset, phono_set_materials,
+ * tile_j in the persistent scheme); each keeps its own x segments, cut
+ * shorter where the persistent launch would have fewer than three items a
+ * block.  While a handle is in a batch, phono_step, phono_reset, phono_set_materials,
  * phono_upload and phono_set_tiling on it return PHONO_ERR_STATE; call
  * phono_batch_sync before reading it.  A handle destroyed while in a batch
  * leaves the batch. */

@@ -55,6 +55,13 @@ void set_last_error(const char* msg) { g_err = msg; }
 static const int kGraphSteps = 12;  // multiple of 2 and 3: buffer rotations line up
 static const int kEnergyBlocks = 1024;
 
+// tile decomposition of the tile pass and the TMA descriptors of its boxes
+struct Tiling {
+  int tj = 0, xseg = 64, ntj = 0, ntk = 0, nseg = 0, n_tile = 0;
+  std::vector<int> seg_start;  // first plane of each x segment, + nx-1
+  CUtensorMap tm_u{}, tm_mat{}, tm_pw0{}, tm_pw1{};
+};
+
 struct phono_handle {
   phono_desc d;  // scalar copy; pointers not kept
   int es = 8;
@@ -66,7 +73,6 @@ struct phono_handle {
   char* ubase = nullptr;   // nbuf x 3 padded arrays, buffer-major
   char* vbase = nullptr;   // F32K: 2 x 3 velocity arrays
   char* cbase = nullptr;   // F32K: 2 x 3 Kahan arrays
-  CUtensorMap tm_u{}, tm_mat{}, tm_pw0{}, tm_pw1{};
   void* sp[6] = {};       // R spacings (F64 raw, F32K reciprocals)
   double* rsp64[6] = {};  // reciprocal double spacings 1/fd, 1/sd (energy)
   double h_sp0[6] = {};   // first elements (raw)
@@ -84,9 +90,10 @@ struct phono_handle {
   double2* partial = nullptr;
   double* energy_out = nullptr;
   double abc[8] = {};
-  int tj = 8, xseg = 64, ntj = 0, ntk = 0, nseg = 0, n_tile = 0, n_face = 0, separate_faces = 1;
+  Tiling t;                    // the tile shape the caller knows
+  Tiling own;                  // a default handle's own shape for its single steps (own.tj 0: t)
+  int n_face = 0, separate_faces = 1;
   FaceTable faces{};
-  std::vector<int> seg_start;  // first plane of each x segment, + nx-1
   // two-launch step (split_step.cu): stress window of `win` planes (0: this
   // mesh has none).  split: the handle steps that way (default tile shape);
   // the velocity forms' v and Kahan terms then stay in buffer 0
@@ -216,7 +223,7 @@ static int upload_table(phono_handle* h, const double* table, int nmat, int id00
 }
 
 template <class R>
-static StepArgs<R> make_args(const phono_handle* h, int step_off) {
+static StepArgs<R> make_args(const phono_handle* h, const Tiling& t, int step_off) {
   StepArgs<R> a{};
   a.g = h->g;
   a.sp.fdx = (const R*)h->sp[0];
@@ -239,10 +246,10 @@ static StepArgs<R> make_args(const phono_handle* h, int step_off) {
   a.mat = h->mat;
   a.tab = (const R*)h->tab;
   a.src = h->src;
-  a.tm_u = h->tm_u;
-  a.tm_mat = h->tm_mat;
-  a.tm_pw0 = h->tm_pw0;
-  a.tm_pw1 = h->tm_pw1;
+  a.tm_u = t.tm_u;
+  a.tm_mat = t.tm_mat;
+  a.tm_pw0 = t.tm_pw0;
+  a.tm_pw1 = t.tm_pw1;
   a.nmat = h->nmat;
   a.ubase = (R*)h->ubase;
   a.vbase = (R*)h->vbase;
@@ -258,12 +265,12 @@ static StepArgs<R> make_args(const phono_handle* h, int step_off) {
   a.surface_mode = h->d.surface_mode;
   a.bc = h->d.bc;
   a.source_mode = h->d.source_mode;
-  a.ntj = h->ntj;
-  a.ntk = h->ntk;
-  a.nseg = h->nseg;
-  for (int q = 0; q <= SEG_TABLE && q < (int)h->seg_start.size(); q++) a.seg_start[q] = h->seg_start[q];
-  a.xseg = h->xseg;
-  a.n_tile_blocks = h->n_tile;
+  a.ntj = t.ntj;
+  a.ntk = t.ntk;
+  a.nseg = t.nseg;
+  for (int q = 0; q <= SEG_TABLE && q < (int)t.seg_start.size(); q++) a.seg_start[q] = t.seg_start[q];
+  a.xseg = t.xseg;
+  a.n_tile_blocks = t.n_tile;
   a.faces = h->faces;
   a.err = h->err;
   a.step_end = 0x7fffffff;
@@ -358,13 +365,24 @@ static cudaError_t split_step_any(const phono_handle* h, int step_off, int step_
   return split_step<float, float>(h, step_off, step_end, st);
 }
 
+// one step of the tile pass, in a handle's own shape
+static cudaError_t tile_step(const phono_handle* h, int step_off, int step_end, int form, cudaStream_t st) {
+  const Tiling& t = h->own.tj ? h->own : h->t;
+  if (h->d.precision == PHONO_F32K) {
+    StepArgs<float> a = make_args<float>(h, t, step_off);
+    a.step_end = step_end;
+    return launch_step_f32k(a, t.tj, form, st);
+  }
+  StepArgs<double> a = make_args<double>(h, t, step_off);
+  a.step_end = step_end;
+  return h->d.precision == PHONO_F64 ? launch_step_f64(a, t.tj, form, st) : launch_step_f64v(a, t.tj, form, st);
+}
+
 // one time step (parts: the handle's form; or 2 tile launch only, 3 face launch only)
 static cudaError_t launch_one(phono_handle* h, int step_off, int parts = -1) {
   if (h->split) return parts == 3 ? cudaSuccess : split_step_any(h, step_off, 0x7fffffff, h->stream);
   const int form = parts < 0 ? h->separate_faces : parts;
-  if (h->d.precision == PHONO_F64) return launch_step_f64(make_args<double>(h, step_off), h->tj, form, h->stream);
-  if (h->d.precision == PHONO_F64V) return launch_step_f64v(make_args<double>(h, step_off), h->tj, form, h->stream);
-  return launch_step_f32k(make_args<float>(h, step_off), h->tj, form, h->stream);
+  return tile_step(h, step_off, 0x7fffffff, form, h->stream);
 }
 
 // Padded device layout: planes -1..nx, rows -1..ny, a KOFF-element front pad
@@ -382,16 +400,16 @@ static long long mat_row(int nz) { return round_up(MKOFF + nz + 1, 16); }
 //    two-launch form (256x256x128 cells: 1.07 ms a step against 2.0 for the
 //    best tile shape of the leapfrog, 1.03 against 1.17 for the velocity form).
 //  * FP32 moves 60 more bytes a node than the tile pass, and wins only where
-//    the tile pass has too few planes to march: 7.7 us against 10.3 for the
-//    best tile shape at 35 k nodes, 16 against 20 at 270 k, 45 against 38 at
-//    0.9 M.
+//    a launch is too short to fill its pipeline (us a step, two launches
+//    against the default tiles: 7.5 / 10.1 at 78 k nodes, 9.2 / 9.7 at 139 k,
+//    12.0 / 11.2 at 208 k, 16.2 / 12.8 at 310 k, 147 / 67 at 3.1 M).
 // The velocity forms' stresses fit in the second buffers of v and the Kahan
 // term.  The leapfrog's window is the whole mesh up to 128 MB, else the planes
 // that fill 128 MB and at least 36: chunks cost a tail each (256x256x128: 1.08
 // ms at 64 MB, 1.03 with all 463 MB), and the footprint should not grow by the
 // six stresses of a large mesh.  With ny == 3 a face point can be the point
 // another face's chain starts from (the tile pass's one-launch form has that).
-constexpr long long kSplitF32Nodes = 400000;
+constexpr long long kSplitF32Nodes = 170000;
 static int split_window(int nx, int ny, int nz, int precision) {
   if (ny == 3) return 0;
   if (precision == PHONO_F32K && (long long)nx * ny * nz > kSplitF32Nodes) return 0;
@@ -576,7 +594,7 @@ static std::vector<int> segment_starts(int planes, int xseg) {
 constexpr int kExplicitSegments = INT_MIN;
 
 // tile height tj and x segments starting at starts[0..n) (+ nx-1 at the end)
-static int apply_tiling(phono_handle* h, int tj, int xseg, const std::vector<int>& starts) {
+static int apply_tiling(phono_handle* h, Tiling& t, int tj, int xseg, const std::vector<int>& starts) {
   const int nx = h->d.nx, ny = h->d.ny, nz = h->d.nz;
   const int ntj = (ny - 1 + tj - 1) / tj, ntk = (nz - 1 + TK - 1) / TK, nseg = (int)starts.size() - 1;
   if (xseg <= 0 && nseg > SEG_TABLE) return fail(PHONO_ERR_ARG, "tapered or listed x segments: more than 64 segments");
@@ -597,14 +615,14 @@ static int apply_tiling(phono_handle* h, int tj, int xseg, const std::vector<int
   faces.off[12] = (int)acc;
   const long long nface = (acc + TK * tj - 1) / (TK * tj);
   if (ntile + nface > 0x7fffffffLL || acc > 0x7fffffffLL) return fail(PHONO_ERR_ARG, "grid too large for one launch");
-  h->tj = tj;
-  h->xseg = xseg;
-  h->seg_start = starts;
-  h->ntj = ntj;
-  h->ntk = ntk;
-  h->nseg = nseg;
+  t.tj = tj;
+  t.xseg = xseg;
+  t.seg_start = starts;
+  t.ntj = ntj;
+  t.ntk = ntk;
+  t.nseg = nseg;
+  t.n_tile = (int)ntile;
   h->faces = faces;
-  h->n_tile = (int)ntile;
   h->n_face = (int)nface;
   // faces in a second launch that reads the tile pass's interior values; the
   // chain end of a face point can itself be a face point only when ny == 3
@@ -613,13 +631,41 @@ static int apply_tiling(phono_handle* h, int tj, int xseg, const std::vector<int
 }
 
 static int set_tiling(phono_handle* h, int tj, int xseg) {
-  return apply_tiling(h, tj, xseg, segment_starts(h->d.nx - 1, xseg));
+  return apply_tiling(h, h->t, tj, xseg, segment_starts(h->d.nx - 1, xseg));
+}
+
+// A default FP32 handle's own tiles: the vectorised tile pass at height 16, or
+// 8 where 16 rows waste more than 3% of the y extent (256x256x128 cells: 134
+// against 136 us a step; 130 rows are 9 tiles of 16 but 17 of 8).  Segments of
+// about 12 planes (a segment reads two planes more than it updates; long ones
+// let neighbouring blocks drift apart until their common halo rows have left
+// L2: 169 us at 37 planes, 134 at 10, 138 at 4), as many as fill the last wave
+// of resident blocks (3 an SM of height 16, 5 of height 8; 160x128x64 cells:
+// 31 us with 448 blocks of 456, 37 with 480).  Beside other instances (a
+// streams batch) there is no last wave to fill: even segments of at most 24
+// planes (12 crystals of 6.2 M nodes in all: 120 us a step, 163 with each
+// instance's single-run segments).
+static int own_tiling(phono_handle* h, bool alone) {
+  int dev = 0, nsm = 152;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  cudaGetLastError();
+  const int planes = h->d.nx - 1, rows = h->d.ny - 1;
+  const long long r16 = round_up(rows, 16), r8 = round_up(rows, 8);
+  const int tj = r16 * 100 > r8 * 103 ? 8 : 16;
+  const long long tiles = (tj == 16 ? r16 : r8) / tj * ((h->d.nz - 1 + TK - 1) / TK), wave = (long long)nsm * (tj == 16 ? 3 : 5);
+  const long long want = tiles * ((planes + 11) / 12), waves = (want + wave - 1) / wave;
+  const int nseg = alone ? (int)std::min<long long>(std::max<long long>(waves * wave / tiles, 1), planes) : (planes + 23) / 24;
+  std::vector<int> starts;
+  for (int q = 0; q <= nseg; q++) starts.push_back((int)((long long)planes * q / nseg));
+  // more segments than a launch describes by table: even ones
+  if (nseg > SEG_TABLE) return apply_tiling(h, h->own, tj, (planes + nseg - 1) / nseg, segment_starts(planes, (planes + nseg - 1) / nseg));
+  return apply_tiling(h, h->own, tj, kExplicitSegments, starts);
 }
 
 // TMA descriptors: a 4-D (k, j, i, array) map over the u allocation with a
 // (KW, TJ+2, 1, 3) box (one plane tile of the three components of a buffer)
 // and a 3-D (k, j, i) map over the material ids with a (48, TJ+2, 1) box.
-static int encode_tensor_maps(phono_handle* h) {
+static int encode_tensor_maps(const phono_handle* h, Tiling& t) {
   static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
   if (!encode) {
     void* fn = nullptr;
@@ -633,25 +679,25 @@ static int encode_tensor_maps(phono_handle* h) {
   cuuint64_t dims[4] = {(cuuint64_t)h->g.sy, (cuuint64_t)(h->d.ny + 2), (cuuint64_t)(h->d.nx + 2),
                         (cuuint64_t)(h->nbuf * 3)};
   cuuint64_t strides[3] = {(cuuint64_t)h->g.sy * es, (cuuint64_t)h->g.sx * es, (cuuint64_t)h->field_elems * es};
-  cuuint32_t box[4] = {(cuuint32_t)kw, (cuuint32_t)(h->tj + 2), 1, 3};
+  cuuint32_t box[4] = {(cuuint32_t)kw, (cuuint32_t)(t.tj + 2), 1, 3};
   cuuint32_t estr[4] = {1, 1, 1, 1};
-  CUresult r = encode(&h->tm_u, es == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4,
+  CUresult r = encode(&t.tm_u, es == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4,
                       h->ubase, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                       CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(PHONO_ERR_CUDA, "cuTensorMapEncodeTiled (fields) failed: " + std::to_string(r));
   cuuint64_t mdims[3] = {(cuuint64_t)h->g.msy, (cuuint64_t)(h->d.ny + 2), (cuuint64_t)(h->d.nx + 2)};
   cuuint64_t mstr[2] = {(cuuint64_t)h->g.msy, (cuuint64_t)h->g.msx};
-  cuuint32_t mbox[3] = {(cuuint32_t)MKW, (cuuint32_t)(h->tj + 2), 1};
-  r = encode(&h->tm_mat, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, h->mat, mdims, mstr, mbox, estr,
+  cuuint32_t mbox[3] = {(cuuint32_t)MKW, (cuuint32_t)(t.tj + 2), 1};
+  r = encode(&t.tm_mat, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, h->mat, mdims, mstr, mbox, estr,
              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(PHONO_ERR_CUDA, "cuTensorMapEncodeTiled (materials) failed: " + std::to_string(r));
   // pointwise state, own points only: a (32, TJ, 1, 3) box over u_old (F64)
   // or over v and the Kahan terms (velocity forms)
-  cuuint32_t pbox[4] = {(cuuint32_t)TK, (cuuint32_t)h->tj, 1, 3};
+  cuuint32_t pbox[4] = {(cuuint32_t)TK, (cuuint32_t)t.tj, 1, 3};
   const bool f64 = h->d.precision == PHONO_F64;
   void* pw[2] = {f64 ? h->ubase : h->vbase, f64 ? h->ubase : h->cbase};
-  CUtensorMap* maps[2] = {&h->tm_pw0, &h->tm_pw1};
+  CUtensorMap* maps[2] = {&t.tm_pw0, &t.tm_pw1};
   for (int q = 0; q < 2; q++) {
     r = encode(maps[q], es == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, pw[q], dims,
                strides, pbox, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
@@ -713,10 +759,11 @@ int phono_create(const phono_desc* d, phono_handle** out) {
   h->g.mo0 = h->g.msx + h->g.msy + MKOFF;
   h->mat_bytes = (size_t)(nx + 2) * h->g.msx;
 
-  // tiles
-  // default tile: height 4 for FP32 (one row a thread), 8 for FP64; 24 planes
-  // per segment (the tuned shapes of the 256x256x128 crystal on GB300)
-  if (set_tiling(h, d->tile_j ? d->tile_j : (d->precision == PHONO_F32K ? 4 : 8), d->x_segment ? d->x_segment : 24)) {
+  // tiles: the shape the caller knows by default is height 4 for FP32, 8 for
+  // FP64, and 24 planes per segment
+  int rt = set_tiling(h, d->tile_j ? d->tile_j : (d->precision == PHONO_F32K ? 4 : 8), d->x_segment ? d->x_segment : 24);
+  if (!rt && d->precision == PHONO_F32K && !d->tile_j && !d->x_segment) rt = own_tiling(h, true);
+  if (rt) {
     std::string m_ = g_err;
     delete h;
     g_err = m_;
@@ -746,8 +793,9 @@ int phono_create(const phono_desc* d, phono_handle** out) {
       return fail(PHONO_ERR_CUDA, std::string(#x) + ": " + cudaGetErrorString(e_));     \
     }                                                                                   \
   } while (0)
-  TRYC(f64 ? configure_step_f64(h->tj)
-           : (d->precision == PHONO_F64V ? configure_step_f64v(h->tj) : configure_step_f32k(h->tj)));
+  TRYC(f64 ? configure_step_f64(h->t.tj)
+           : (d->precision == PHONO_F64V ? configure_step_f64v(h->t.tj) : configure_step_f32k(h->t.tj)));
+  if (h->own.tj) TRYC(configure_step_f32k(h->own.tj));
   TRYC(cudaEventCreate(&h->ev0));
   TRYC(cudaEventCreate(&h->ev1));
   const size_t fb = h->field_elems * h->es * 3 * h->nbuf;
@@ -827,7 +875,8 @@ int phono_create(const phono_desc* d, phono_handle** out) {
   h->split = h->win > 0 && !d->tile_j && !d->x_segment;
   TRY(dalloc(h, (void**)&h->tab13, (size_t)256 * PHONO_TABLE_COLS * 8));
   TRY(upload_materials(h, d->mat, d->table, d->nmat));
-  TRY(encode_tensor_maps(h));
+  TRY(encode_tensor_maps(h, h->t));
+  if (h->own.tj) TRY(encode_tensor_maps(h, h->own));
   // source table, surface records, counters
   int cap = d->max_steps > 0 ? d->max_steps : 1;
   TRY(dalloc(h, (void**)&h->src, (size_t)cap * 8));
@@ -1265,24 +1314,19 @@ void* phono_stream(phono_handle* h) { return h ? (void*)h->stream : nullptr; }
 // switch a handle to tile height tj and the given x segments, keeping the old
 // shape if the new one cannot be set up
 static int retile(phono_handle* h, int tj, int xseg, const std::vector<int>& starts) {
-  if (!h->split && tj == h->tj && starts == h->seg_start) {
-    h->xseg = xseg;
+  if (!h->split && !h->own.tj && tj == h->t.tj && starts == h->t.seg_start) {
+    h->t.xseg = xseg;
     return PHONO_OK;
   }
   CK(cudaStreamSynchronize(h->stream));
   const int p = h->d.precision;
   CK(p == PHONO_F64 ? configure_step_f64(tj) : (p == PHONO_F64V ? configure_step_f64v(tj) : configure_step_f32k(tj)));
-  const int old_tj = h->tj, old_xs = h->xseg;
-  const std::vector<int> old_starts = h->seg_start;
-  int rc = apply_tiling(h, tj, xseg, starts);
-  if (!rc) rc = encode_tensor_maps(h);
-  if (rc) {
-    std::string m = g_err;
-    apply_tiling(h, old_tj, old_xs, old_starts);
-    encode_tensor_maps(h);
-    g_err = m;
-    return rc;
-  }
+  Tiling t;
+  int rc = apply_tiling(h, t, tj, xseg, starts);
+  if (!rc) rc = encode_tensor_maps(h, t);
+  if (rc) return rc;
+  h->t = t;
+  h->own = Tiling();
   CK(set_split(h, false));
   if (h->graph) {  // the captured launches hold the old grid and tensor maps
     cudaGraphExecDestroy(h->graph);
@@ -1295,19 +1339,19 @@ int phono_set_tiling(phono_handle* h, int tile_j, int x_segment) {
   if (!h) return fail(PHONO_ERR_ARG, "handle is NULL");
   if (h->batch) return fail(PHONO_ERR_STATE, "handle is in a batch");
   const bool keep = tile_j == 0;
-  if (tile_j == 0) tile_j = h->tj;
+  if (tile_j == 0) tile_j = h->t.tj;
   if (tile_j != 4 && tile_j != 8 && tile_j != 16) return fail(PHONO_ERR_ARG, "tile_j must be 0, 4, 8 or 16");
   if (x_segment < -4096) return fail(PHONO_ERR_ARG, "x_segment out of range");
-  if (x_segment == 0 && tile_j == h->tj && keep) return PHONO_OK;
+  if (x_segment == 0 && keep) return PHONO_OK;
   if (x_segment == 0)  // keep the current segments (a list included)
-    return retile(h, tile_j, h->xseg, h->seg_start);
+    return retile(h, tile_j, h->t.xseg, h->t.seg_start);
   return retile(h, tile_j, x_segment, segment_starts(h->d.nx - 1, x_segment));
 }
 
 int phono_set_segments(phono_handle* h, int tile_j, const int* lengths, int n) {
   if (!h || !lengths) return fail(PHONO_ERR_ARG, "NULL argument");
   if (h->batch) return fail(PHONO_ERR_STATE, "handle is in a batch");
-  if (tile_j == 0) tile_j = h->tj;
+  if (tile_j == 0) tile_j = h->t.tj;
   if (tile_j != 4 && tile_j != 8 && tile_j != 16) return fail(PHONO_ERR_ARG, "tile_j must be 0, 4, 8 or 16");
   if (n < 1 || n > PHONO_MAX_SEGMENTS) return fail(PHONO_ERR_ARG, "n must be 1..PHONO_MAX_SEGMENTS");
   std::vector<int> starts{0};
@@ -1354,6 +1398,7 @@ struct phono_batch {
   cudaEvent_t fork = nullptr;
   std::vector<int> order;     // active slots, costliest first
   std::vector<int> step_end;  // per slot: the instance's budget end
+  std::vector<int> cut;       // persistent scheme, per slot: segment limit its device arguments were written with (-1: none)
   std::vector<cudaGraphExec_t> igraph;  // streams scheme: per slot, 12 steps with its budget baked in
   cudaStream_t capture = nullptr;       // streams scheme: capture stream (always idle)
 };
@@ -1378,9 +1423,22 @@ static void batch_detach(phono_batch* b, const phono_handle* h) {
     }
 }
 
+// a default FP32 handle's tiles for single steps or for steps beside others
+static int reshape_own(phono_handle* h, bool alone) {
+  if (!h->own.tj) return PHONO_OK;
+  int rc = own_tiling(h, alone);
+  if (!rc) rc = encode_tensor_maps(h, h->own);
+  if (h->graph) {
+    cudaGraphExecDestroy(h->graph);
+    h->graph = nullptr;
+  }
+  return rc;
+}
+
 // the batch's work is done: the handle is on its own again
 static cudaError_t leave_batch(phono_handle* h) {
   h->batch = nullptr;
+  reshape_own(h, true);
   if (!h->resplit) return cudaSuccess;
   h->resplit = false;
   return set_split(h, true);
@@ -1431,6 +1489,42 @@ static BatchArgs<float> batch_args(const phono_batch* b, int step_off) {
 static_assert(sizeof(BatchArgs<float>) == sizeof(BatchArgs<double>), "batch argument layouts differ");
 static_assert(PHONO_MAX_SEGMENTS == SEG_TABLE, "segment list limit and the kernel table differ");
 
+// a handle's tiles with every x segment cut evenly to at most `limit` planes (0: as they are)
+static Tiling cut_segments(const phono_handle* h, int limit) {
+  Tiling t = h->t;
+  if (!limit) return t;
+  const int planes = h->d.nx - 1;
+  std::vector<int> starts{0};
+  for (int q = 0, p = 0; q < t.nseg; q++) {
+    const int end = t.nseg <= SEG_TABLE ? t.seg_start[q + 1] : std::min(planes, p + t.xseg);
+    const int n = (end - p + limit - 1) / limit;
+    for (int c = 1; c <= n; c++) starts.push_back(p + (int)((long long)(end - p) * c / n));
+    p = end;
+  }
+  if ((int)starts.size() - 1 > SEG_TABLE) starts = segment_starts(planes, limit);  // even: beyond the table
+  t.xseg = limit;
+  t.n_tile = t.n_tile / t.nseg * ((int)starts.size() - 1);
+  t.nseg = (int)starts.size() - 1;
+  t.seg_start = starts;
+  return t;
+}
+
+// device arguments of the instance in slot s
+static int write_instance(phono_batch* b, int s, const Tiling& t) {
+  const phono_handle* h = b->slot[s];
+  char* dst = b->d_inst + (size_t)s * b->inst_size;
+  if (b->precision == PHONO_F32K) {
+    StepArgs<float> a = make_args<float>(h, t, 0);
+    a.step_end = b->step_end[s];
+    CK(cudaMemcpy(dst, &a, sizeof a, cudaMemcpyHostToDevice));
+  } else {
+    StepArgs<double> a = make_args<double>(h, t, 0);
+    a.step_end = b->step_end[s];
+    CK(cudaMemcpy(dst, &a, sizeof a, cudaMemcpyHostToDevice));
+  }
+  return PHONO_OK;
+}
+
 // work items (costliest instances first), face-block prefix, active list
 static int batch_rebuild(phono_batch* b) {
   std::vector<int> act;
@@ -1441,24 +1535,47 @@ static int batch_rebuild(phono_batch* b) {
   // updates left), each instance's chunks queued before the next one's
   auto cost = [&](int x) {
     const phono_handle* h = b->slot[x];
-    return b->streams ? (long long)h->d.nx * h->d.ny * h->d.nz * b->remaining[x] : (long long)h->n_tile;
+    return b->streams ? (long long)h->d.nx * h->d.ny * h->d.nz * b->remaining[x] : (long long)h->t.n_tile;
   };
   std::sort(act.begin(), act.end(), [&](int x, int y) {
     const long long cx = cost(x), cy = cost(y);
     return cx != cy ? cx > cy : x < y;
   });
+  b->order = act;
+  if (b->streams) {  // the instances' own launches: no work list
+    b->dirty = false;
+    return PHONO_OK;
+  }
   std::vector<int2> items;
   std::vector<int> prefix, finst;
   int fb = 0;
+  // With fewer than three items a block, segments are cut
+  // to 12 planes, so that no block is left with a long one at the end of the
+  // launch (12 crystals of 6.2 M nodes, tiles of height 8: 184 us a step
+  // against 240 with their segments of 32 planes; 24 crystals of 29 M nodes
+  // fill the launch and stay at 730).
+  long long own_items = 0;
+  for (int s : act) own_items += b->slot[s]->t.n_tile;
+  const int limit = own_items < 3LL * b->grid_tiles ? 12 : 0;
+  for (int s : act)
+    if (b->cut[s] != limit) {
+      CK(cudaStreamSynchronize(b->stream));  // launches that read the old arguments
+      break;
+    }
   for (int s : act) {
     const phono_handle* h = b->slot[s];
-    for (int t = 0; t < h->n_tile; t++) items.push_back(make_int2(s, t));
+    const Tiling t = cut_segments(h, limit);
+    for (int q = 0; q < t.n_tile; q++) items.push_back(make_int2(s, q));
+    if (b->cut[s] != limit) {
+      int rc = write_instance(b, s, t);
+      if (rc) return rc;
+      b->cut[s] = limit;
+    }
     prefix.push_back(fb);
     finst.push_back(s);
     fb += (h->faces.off[12] + 255) / 256;
   }
   prefix.push_back(fb);
-  b->order = act;
   if ((int)items.size() > b->item_cap) {
     int cap = std::max<int>((int)items.size(), 2 * b->item_cap);
     void* p = nullptr;
@@ -1490,15 +1607,7 @@ static int batch_rebuild(phono_batch* b) {
 static cudaError_t chain_launch(phono_batch* b, int s, int step_off, cudaStream_t st) {
   phono_handle* h = b->slot[s];
   if (h->split) return split_step_any(h, step_off, b->step_end[s], st);
-  if (h->d.precision == PHONO_F32K) {
-    StepArgs<float> a = make_args<float>(h, step_off);
-    a.step_end = b->step_end[s];
-    return launch_step_f32k(a, h->tj, h->separate_faces, st);
-  }
-  StepArgs<double> a = make_args<double>(h, step_off);
-  a.step_end = b->step_end[s];
-  return h->d.precision == PHONO_F64 ? launch_step_f64(a, h->tj, h->separate_faces, st)
-                                     : launch_step_f64v(a, h->tj, h->separate_faces, st);
+  return tile_step(h, step_off, b->step_end[s], h->separate_faces, st);
 }
 
 static cudaError_t batch_launch_steps(phono_batch* b, int first_off, int n) {
@@ -1611,6 +1720,7 @@ int phono_batch_create(int capacity, int precision, int tile_j, phono_batch** ou
   b->slot.assign(capacity, nullptr);
   b->remaining.assign(capacity, 0);
   b->step_end.assign(capacity, 0);
+  b->cut.assign(capacity, -1);
   b->igraph.assign(capacity, nullptr);
 #define BTRY(x)              \
   do {                       \
@@ -1689,7 +1799,7 @@ int phono_batch_add(phono_batch* b, phono_handle* h, int nsteps) {
   if (!b || !h) return fail(PHONO_ERR_ARG, "NULL argument");
   if (h->batch) return fail(PHONO_ERR_ARG, h->batch == b ? "handle already in the batch" : "handle is in another batch");
   if (h->d.precision != b->precision) return fail(PHONO_ERR_ARG, "handle precision differs from the batch");
-  if (!b->streams && h->tj != b->tj) return fail(PHONO_ERR_ARG, "handle tile_j differs from the batch");
+  if (!b->streams && h->t.tj != b->tj) return fail(PHONO_ERR_ARG, "handle tile_j differs from the batch");
   if (!h->separate_faces) return fail(PHONO_ERR_ARG, "batched instances need ny >= 4");
   if (h->nmat > BATCH_TAB_ROWS)
     return fail(PHONO_ERR_ARG, "batched instances hold at most " + std::to_string(BATCH_TAB_ROWS) + " materials");
@@ -1701,24 +1811,19 @@ int phono_batch_add(phono_batch* b, phono_handle* h, int nsteps) {
     if (s < 0 && !b->slot[q]) s = q;
   }
   if (s < 0) return fail(PHONO_ERR_NOMEM, "batch is full");
-  if (!b->streams && h->split) {
+  if (b->streams && reshape_own(h, false)) return PHONO_ERR_ARG;
+  // the persistent launch is a tile pass; beside others FP32's two launches
+  // only move more bytes (12 crystals: 120 us a step, 142 with the small ones split)
+  if (h->split && (!b->streams || b->precision == PHONO_F32K)) {
     CK(set_split(h, false));
     h->resplit = true;
   }
   CK(cudaStreamSynchronize(h->stream));
   CK(cudaStreamSynchronize(b->stream));
-  if (b->precision == PHONO_F32K) {
-    StepArgs<float> a = make_args<float>(h, 0);
-    a.step_end = h->steps_done + nsteps;
-    CK(cudaMemcpy(b->d_inst + (size_t)s * b->inst_size, &a, sizeof a, cudaMemcpyHostToDevice));
-  } else {
-    StepArgs<double> a = make_args<double>(h, 0);
-    a.step_end = h->steps_done + nsteps;
-    CK(cudaMemcpy(b->d_inst + (size_t)s * b->inst_size, &a, sizeof a, cudaMemcpyHostToDevice));
-  }
   b->slot[s] = h;
   b->remaining[s] = nsteps;
   b->step_end[s] = h->steps_done + nsteps;
+  b->cut[s] = -1;  // its device arguments are written with the next work list
   b->dirty = true;
   h->batch = b;
   return s;

@@ -249,22 +249,22 @@ struct SmemPlan {
   static_assert((PWC * sizeof(R)) % 128 == 0 && (TF::SU * sizeof(R)) % 128 == 0, "ring tiles must stay 128-byte aligned");
 };
 
-// Rows of one z column a tile-pass thread owns: two for the FP32 velocity
-// form at tile heights 8 and 16 (the per-plane work shared by two nodes; 128
-// or 256 threads a block), one otherwise.
+// FP32 tiles of height 8 and 16 take the vectorised pass (tile_vec.cuh); at
+// height 4 one updating warp does not pay for the halo warp (256x256x128
+// cells: 192 us a step against 154 with one row a thread).
 template <class S, int TJ>
-struct RowsPerThread {
-  static constexpr int value = (S::kahan && sizeof(typename S::R) == 4 && TJ >= 8) ? 2 : 1;
-};
+__host__ __device__ constexpr bool vec_tile() { return sizeof(typename S::R) == 4 && TJ >= 8; }
 
 #include "tile_rows.cuh"
+#include "tile_vec.cuh"
 
-// the tile pass of one block: one row per thread or RowsPerThread rows
+// the tile pass of one block
 template <class S, int TJ>
 __device__ __forceinline__ bool run_tile(const StepArgs<typename S::R>& a, unsigned char* base,
                                          const Roles<typename S::R>& r, const typename S::R s, const int tt,
                                          const int tid, const int b, const StepArgs<typename S::R>* maps) {
-  return tile_block_rows<S, TJ>(a, base, r, s, tt, tid, b, maps);
+  if constexpr (vec_tile<S, TJ>()) return tile_block_vec<TJ>(a, base, r, s, tt, tid, b, maps);
+  else return tile_block_rows<S, TJ>(a, base, r, s, tt, tid, b, maps);
 }
 
 // ---------------------------------------------------------------------------
@@ -277,10 +277,16 @@ __device__ __forceinline__ bool run_tile(const StepArgs<typename S::R>& a, unsig
 // registers).  FP64: 16 warps per SM.
 template <class R, int TJ, bool BATCH = false>
 struct MinBlocks {
-  static constexpr int value = sizeof(R) == 8 ? (TJ < 16 ? 16 / TJ : 1) : (TJ == 4 ? 6 : (TJ == 8 ? 4 : 2));
+  static constexpr int value = sizeof(R) == 8 ? (TJ < 16 ? 16 / TJ : 1) : (TJ == 4 ? 6 : (TJ == 8 ? 5 : 3));
 };
 template <class S, int TJ>
-__host__ __device__ constexpr int step_threads() { return TK * TJ / RowsPerThread<S, TJ>::value; }
+__host__ __device__ constexpr int step_threads() {
+  return vec_tile<S, TJ>() ? VecPlan<TJ>::NT : TK * TJ;
+}
+template <class S, int TJ>
+__host__ __device__ constexpr size_t step_smem(int table_rows) {
+  return vec_tile<S, TJ>() ? VecPlan<TJ>::bytes(table_rows) : SmemPlan<S, TJ>::bytes(table_rows);
+}
 template <class S, int TJ>
 __global__ void __launch_bounds__(step_threads<S, TJ>(), MinBlocks<typename S::R, TJ>::value)
     fdtd_step_kernel(const __grid_constant__ StepArgs<typename S::R> a) {
@@ -313,7 +319,7 @@ __global__ void __launch_bounds__(step_threads<S, TJ>(), MinBlocks<typename S::R
 template <class S, int TJ>
 static cudaError_t configure_tj() {
   return cudaFuncSetAttribute(fdtd_step_kernel<S, TJ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)SmemPlan<S, TJ>::bytes(TAB_ROWS_MAX));
+                              (int)step_smem<S, TJ>(TAB_ROWS_MAX));
 }
 
 template <class S>
@@ -336,7 +342,7 @@ static cudaError_t launch_tj(const StepArgs<typename S::R>& a, int separate_face
   dim3 block(TK, NT / TK);
   // fused: face points handled by extra blocks of the same launch
   dim3 grid(a.n_tile_blocks + (separate_faces ? 0 : (nfaces + NT - 1) / NT));
-  if (separate_faces != 3) fdtd_step_kernel<S, TJ><<<grid, block, SmemPlan<S, TJ>::bytes(a.nmat), st>>>(a);
+  if (separate_faces != 3) fdtd_step_kernel<S, TJ><<<grid, block, step_smem<S, TJ>(a.nmat), st>>>(a);
   if ((separate_faces == 1 || separate_faces == 3) && nfaces > 0)
     fdtd_face_kernel<S><<<(nfaces + 255) / 256, 256, 0, st>>>(a);
   return cudaGetLastError();
@@ -419,7 +425,7 @@ template <class S, int TJ>
 static cudaError_t batch_launch_tj(const BatchArgs<typename S::R>& ba, int grid_tiles, int grid_faces,
                                    cudaStream_t st) {
   batch_step_kernel<S, TJ>
-      <<<grid_tiles, dim3(TK, step_threads<S, TJ>() / TK), SmemPlan<S, TJ>::bytes(BATCH_TAB_ROWS), st>>>(ba);
+      <<<grid_tiles, dim3(TK, step_threads<S, TJ>() / TK), step_smem<S, TJ>(BATCH_TAB_ROWS), st>>>(ba);
   batch_face_kernel<S><<<grid_faces, 256, 0, st>>>(ba);
   return cudaGetLastError();
 }
@@ -436,7 +442,7 @@ cudaError_t batch_step(const BatchArgs<typename S::R>& ba, int tj, int grid_tile
 
 template <class S, int TJ>
 static cudaError_t batch_configure_tj(int* blocks_per_sm) {
-  const int smem = (int)SmemPlan<S, TJ>::bytes(BATCH_TAB_ROWS);
+  const int smem = (int)step_smem<S, TJ>(BATCH_TAB_ROWS);
   cudaError_t e = cudaFuncSetAttribute(batch_step_kernel<S, TJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
   return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, batch_step_kernel<S, TJ>, step_threads<S, TJ>(),

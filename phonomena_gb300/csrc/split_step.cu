@@ -17,7 +17,7 @@
 //   nodes       25x21x13  41x41x21  61x61x21  150x131x47  194x162x98  257x257x129
 //   F64         25 / 11   32 / 12   47 / 15   354 / 118   969 / 391   2012 / 1071
 //   F64V        13 / 8    21 / 10   29 / 14   197 / 121   559 / 378   1174 / 1037
-//   F32K        9 / 6     10 / 7    12 / 8    38 / -      80 / -      154 / -
+//   F32K        9 / 6     10 / 7    12 / 8    (larger meshes: tile_vec.cuh)
 #include "scheme.cuh"
 #include "split_common.cuh"
 

@@ -3,16 +3,14 @@
 // A block owns a (TJ x 32) tile of the (y, z) plane and marches along x over
 // planes [ib, ie).  Planes of u (3 components, 1-node halo), material ids and
 // the pointwise state of the own points (u_old, or v and the Kahan terms)
-// arrive by TMA in a 4-slot ring.  A thread owns JR rows of one z column
-// (rows j0 + ty*JR .. + JR-1; JR = RowsPerThread: 2 for FP32 at tile heights
-// 8 and 16, else 1), so the per-plane work that does not depend on the row
-// (ring waits, barriers, slot addresses, x spacings, the plane's range tests)
-// is shared by JR nodes.  Every smem access uses offsets fixed per thread
-// and row (own position Lu / Lm, neighbours at constant distance), the range
-// predicates of the reference's slices are split into per-row (j, k) and
-// per-plane (i) parts computed once, ring values and material ids are carried
-// from plane to plane, and the per-axis spacings live in registers, so the
-// inner loop is the stencil arithmetic plus shared-memory traffic.  The
+// arrive by TMA in a 4-slot ring.  A thread owns one z column of one row.
+// Every smem access uses offsets fixed per thread (own position Lu / Lm,
+// neighbours at constant distance), the range predicates of the reference's
+// slices are split into per-thread (j, k) and per-plane (i) parts computed
+// once, ring values and material ids are carried from plane to plane, and the
+// per-axis spacings live in registers, so the inner loop is the stencil
+// arithmetic plus shared-memory traffic.  FP64 tiles take this pass, and FP32
+// tiles of height 4 (the others: tile_vec.cuh).  The
 // arithmetic goes through the same scheme primitives (tn1, ts, div3,
 // update_value) as the face path, operation for operation.
 // Included inside namespace phono, after SmemPlan and the scheme primitives.
@@ -25,8 +23,7 @@ __device__ __forceinline__ bool tile_block_rows(const StepArgs<typename S::R>& a
   using R = typename S::R;
   using P = SmemPlan<S, TJ>;
   using TF = TileShape<R, TJ>;
-  constexpr int JR = RowsPerThread<S, TJ>::value;
-  constexpr int NT = TK * TJ / JR;
+  constexpr int NT = TK * TJ;
   constexpr int W = P::W, PL = P::PL;
   constexpr int KW = TF::KW, KB = TF::KB, CW = TF::CW, SU = TF::SU, SM = TF::SM;
   constexpr int XO = 0, YO = CW, ZO = 2 * CW;  // component offsets inside a ring slot
@@ -54,11 +51,11 @@ __device__ __forceinline__ bool tile_block_rows(const StepArgs<typename S::R>& a
   const int ibase = ib - 1;
   const int plast = ie + 1;  // last plane the segment reads
   const int tx = threadIdx.x, ty = threadIdx.y;
-  const int jb = j0 + ty * JR, k = k0 + tx;  // first own row, own column
-  const int L = (ty * JR + 1) * W + tx + 1;    // own entry of the stress planes (row r: + r*W)
-  const int Lu = (ty * JR + 1) * KW + tx + KB;  // own entry of a u component tile (row r: + r*KW)
-  const int Lm = (ty * JR + 1) * MKW + tx + MKOFF;
-  const int Lp = ty * JR * TK + tx;            // own entry of a pointwise component tile (row r: + r*TK)
+  const int j = j0 + ty, k = k0 + tx;  // own row and column
+  const int L = (ty + 1) * W + tx + 1;    // own entry of the stress planes
+  const int Lu = (ty + 1) * KW + tx + KB;  // own entry of a u component tile
+  const int Lm = (ty + 1) * MKW + tx + MKOFF;
+  const int Lp = ty * TK + tx;            // own entry of a pointwise component tile
 
   // the whole material table (nmat <= 256 rows) is staged in shared memory
   for (int q = tid; q < a.nmat * 16; q += NT) stab[q] = __ldg(a.tab + q);
@@ -73,25 +70,21 @@ __device__ __forceinline__ bool tile_block_rows(const StepArgs<typename S::R>& a
   // spacings as used by the z = 0 row or the interior (the x ones are per plane)
   const R t123_d = kz ? a.sp.sdz0 : sdz_m;  // T1..T3 z; uy and ux z-divergence
   const R uz_c = kz ? (a.surface_mode == 0 ? R(1) : a.sp.fdz0) : fdz_k;
-  bool j_n[JR], j_s[JR], own_y[JR], own_z[JR], own_x[JR];
-  R sb[JR], fdy_j[JR], uy_b[JR];
-  #pragma unroll
-  for (int q = 0; q < JR; q++) {
-    const int j = jb + q;
-    const bool active = (j < ny - 1) && k_in;
-    j_n[q] = j >= 1 && j <= ny - 2;  // T1..T3, T5: j in [1, ny-2]
-    j_s[q] = j <= ny - 2;            // T4, T6: j in [0, ny-2]
-    const R sdy_m = j_n[q] ? __ldg(a.sp.sdy + j - 1) : R(1);
-    fdy_j[q] = j_s[q] ? __ldg(a.sp.fdy + j) : R(1);
-    sb[q] = kz ? a.sp.sdy0 : sdy_m;  // T1..T3 y; uz and ux y-divergence
-    uy_b[q] = kz ? a.sp.fdy0 : fdy_j[q];
-    // output classification (component extents, faces, V0 sets): uy has its
-    // y faces at 0 and ny-2, uz at y = 0 and z = N (nz-2), ux at y = 0 (the
-    // x = N plane is checked per plane); face points are the face pass's
-    own_y[q] = active && !(j == 0 || j == ny - 2);
-    own_z[q] = active && !(j == 0 || k == nz - 2);
-    own_x[q] = active && j != 0;
-  }
+  bool j_n, j_s, own_y, own_z, own_x;
+  R sb, fdy_j, uy_b;
+  const bool active = (j < ny - 1) && k_in;
+  j_n = j >= 1 && j <= ny - 2;  // T1..T3, T5: j in [1, ny-2]
+  j_s = j <= ny - 2;            // T4, T6: j in [0, ny-2]
+  const R sdy_m = j_n ? __ldg(a.sp.sdy + j - 1) : R(1);
+  fdy_j = j_s ? __ldg(a.sp.fdy + j) : R(1);
+  sb = kz ? a.sp.sdy0 : sdy_m;  // T1..T3 y; uz and ux y-divergence
+  uy_b = kz ? a.sp.fdy0 : fdy_j;
+  // output classification (component extents, faces, V0 sets): uy has its
+  // y faces at 0 and ny-2, uz at y = 0 and z = N (nz-2), ux at y = 0 (the
+  // x = N plane is checked per plane); face points are the face pass's
+  own_y = active && !(j == 0 || j == ny - 2);
+  own_z = active && !(j == 0 || k == nz - 2);
+  own_x = active && j != 0;
   // The z = N face point above an (i, j) that is on no x / y face is one face
   // formula applied to the value this thread computes at k = kz - 1
   // (base_solver.py:552-554, applied last); the thread writes it.  Points on
@@ -107,7 +100,7 @@ __device__ __forceinline__ bool tile_block_rows(const StepArgs<typename S::R>& a
     const int q = p - ibase, sl = q & (NSLOT - 1);
     const bool pw = p >= ib && p < ie;
     mbar_expect_tx(&bars[sl], P::tx_bytes + (pw ? P::pw_bytes : 0u));
-    // test hook (skip_plane >= 0; -1 is off, and plane -1 is a real padding
+    // test hook (skip_plane >= 0; -1 is off_i, and plane -1 is a real padding
     // plane that segment 0 loads): armed, no copy, so the wait on it runs out
     if (a.skip_plane >= 0 && p == a.skip_plane) return;
     // padded coordinates: k + KOFF, j + 1, i + 1; the u tiles start at k0-KB, j0-1
@@ -245,8 +238,8 @@ __device__ __forceinline__ bool tile_block_rows(const StepArgs<typename S::R>& a
   // values one iteration earlier), the material ids of plane i the previous
   // plane's loads fetched.  Prologue: T5, T6 of plane ib-1 and the ring
   // values of planes ib-1, ib.
-  R t1m[JR], t5m[JR], t6m[JR], uxm[JR], uxm_up[JR], uyc_n[JR], uzc_n[JR];
-  int id_c[JR], id_z[JR], id_y[JR];
+  R t1m, t5m, t6m, uxm, uxm_up, uyc_n, uzc_n;
+  int id_c, id_z, id_y;
   {
     const int i = ib - 1;
     const bool i_s = i >= 0 && i <= nx - 2;
@@ -254,42 +247,38 @@ __device__ __forceinline__ bool tile_block_rows(const StepArgs<typename S::R>& a
     const R* U0 = uslot(i);
     const R* Up = uslot(i + 1);
     const uint8_t* Mp = mslot(i + 1);
-    #pragma unroll
-    for (int q = 0; q < JR; q++) {
-      const int lu = Lu + q * KW, lm = Lm + q * MKW;
-      t5m[q] = R(0);
-      t6m[q] = R(0);
-      if (i_s && j_n[q] && k_in) {  // T5 (base_solver.py:360-365, 425-428)
-        const R c = tab[16 * Mp[lm + (kz ? 0 : 1)] + 10];
-        t5m[q] = S::ts(a.dtab, c, S::sub(U0[XO + lu + 1], U0[XO + lu]), kz ? a.sp.fdx0 : fdz_k,
-                       S::sub(Up[ZO + lu], U0[ZO + lu]), kz ? a.sp.fdz0 : fx);
-      }
-      if (i_s && j_s[q] && k_in) {  // T6 (base_solver.py:367-372, 430-433)
-        const R c = tab[16 * Mp[lm + MKW] + 11];
-        t6m[q] = S::ts(a.dtab, c, S::sub(U0[XO + lu + KW], U0[XO + lu]), kz ? a.sp.fdx0 : fdy_j[q],
-                       S::sub(Up[YO + lu], U0[YO + lu]), kz ? a.sp.fdz0 : fx);
-      }
-      t1m[q] = R(0);
-      uxm_up[q] = R(0);
-      uxm[q] = U0[XO + lu];
-      uyc_n[q] = Up[YO + lu];
-      uzc_n[q] = Up[ZO + lu];
-      id_c[q] = Mp[lm];
-      id_z[q] = Mp[lm + 1];
-      id_y[q] = Mp[lm + MKW];
+      t5m = R(0);
+    t6m = R(0);
+    if (i_s && j_n && k_in) {  // T5 (base_solver.py:360-365, 425-428)
+      const R c = tab[16 * Mp[Lm + (kz ? 0 : 1)] + 10];
+      t5m = S::ts(a.dtab, c, S::sub(U0[XO + Lu + 1], U0[XO + Lu]), kz ? a.sp.fdx0 : fdz_k,
+                     S::sub(Up[ZO + Lu], U0[ZO + Lu]), kz ? a.sp.fdz0 : fx);
     }
+    if (i_s && j_s && k_in) {  // T6 (base_solver.py:367-372, 430-433)
+      const R c = tab[16 * Mp[Lm + MKW] + 11];
+      t6m = S::ts(a.dtab, c, S::sub(U0[XO + Lu + KW], U0[XO + Lu]), kz ? a.sp.fdx0 : fdy_j,
+                     S::sub(Up[YO + Lu], U0[YO + Lu]), kz ? a.sp.fdz0 : fx);
+    }
+    t1m = R(0);
+    uxm_up = R(0);
+    uxm = U0[XO + Lu];
+    uyc_n = Up[YO + Lu];
+    uzc_n = Up[ZO + Lu];
+    id_c = Mp[Lm];
+    id_z = Mp[Lm + 1];
+    id_y = Mp[Lm + MKW];
   }
 
-  // the surface record this step writes (none: nullptr), at the own column of row jb
+  // the surface record this step writes (none: nullptr), at the own column
   R* rec = nullptr;
   if (kz && a.record_every > 0 && (tt + 1) % a.record_every == 0) {
     const int slot = (tt + 1) / a.record_every - 1 - a.rec_base;
-    if (slot >= 0 && slot < a.nrec_cap) rec = a.surf + ((long long)slot * nx) * ny + jb;
+    if (slot >= 0 && slot < a.nrec_cap) rec = a.surf + ((long long)slot * nx) * ny + j;
   }
 
   // element offsets inside one array fit in 32 bits (checked at handle creation)
-  const unsigned off_j = (unsigned)(g.o0 + (long long)jb * g.sy + k);  // row r: + r*sy
-  const unsigned sxu = (unsigned)g.sx, syu = (unsigned)g.sy;
+  const unsigned off_j = (unsigned)(g.o0 + (long long)j * g.sy + k);
+  const unsigned sxu = (unsigned)g.sx;
 
   // x spacings of plane p: fdx[p] (T5, T6 at p; ux at p+1) and sdx[p-1]
   // (T1..T3 at p; uy, uz at p), read one plane ahead so that their latency
@@ -300,7 +289,7 @@ __device__ __forceinline__ bool tile_block_rows(const StepArgs<typename S::R>& a
   R fx_prev = fx_at(ib - 1), fx_cur = fx_at(ib), sx_cur = sx_at(ib);
 
   for (int i = ib; i <= ie; i++) {
-    const unsigned off_i = off_j + (unsigned)i * sxu;  // (i, jb, k)
+    const unsigned off_i = off_j + (unsigned)i * sxu;  // (i, j, k)
     const R fx_next = fx_at(i + 1), sx_next = sx_at(i + 1);
     // per-plane (uniform) predicates and spacings
     const bool i_n = i >= 1 && i <= nx - 2;  // T1..T4
@@ -319,66 +308,61 @@ __device__ __forceinline__ bool tile_block_rows(const StepArgs<typename S::R>& a
     const uint8_t* M0 = mslot(i);
     const uint8_t* Mp = mslot(i + 1);
     // own stresses of plane i, row by row, each ring value read once
-    R uxc[JR], uyc[JR], uzc[JR], uxc_up[JR], t1c[JR], t2c[JR], t3c[JR], t4c[JR], t5c[JR], t6c[JR];
-    int idp_c[JR], idp_z[JR], idp_y[JR];
-    #pragma unroll
-    for (int q = 0; q < JR; q++) {
-      const int lu = Lu + q * KW, lm = Lm + q * MKW;
-      uxc[q] = U0[XO + lu];
-      uyc[q] = uyc_n[q];
-      uzc[q] = uzc_n[q];
-      uyc_n[q] = Up[YO + lu];
-      uzc_n[q] = Up[ZO + lu];
-      uxc_up[q] = U0[XO + lu + 1];  // ux(i, j, k+1): T5, and the z = N face input of the next plane's ux
-      idp_c[q] = Mp[lm];
-      idp_z[q] = Mp[lm + 1];
-      idp_y[q] = Mp[lm + MKW];
-      t1c[q] = t2c[q] = t3c[q] = R(0);
-      if (i_n && j_n[q] && k_in) {
-        // T1..T3 (base_solver.py:329-351, 408-418): material of the own node
-        const R* row = tab + 16 * id_c[q];
-        R cc[9];
-        if constexpr (sizeof(R) == 4) {
-          const float4 q0 = *reinterpret_cast<const float4*>(row), q1 = *reinterpret_cast<const float4*>(row + 4);
-          cc[0] = q0.x, cc[1] = q0.y, cc[2] = q0.z, cc[3] = q0.w, cc[4] = q1.x, cc[5] = q1.y, cc[6] = q1.z,
-          cc[7] = q1.w;
-          cc[8] = row[8];
-        } else {
-          for (int c = 0; c < 9; c++) cc[c] = row[c];
-        }
-        const R d1 = S::sub(uxc[q], uxm[q]);
-        const R d2 = S::sub(uyc[q], U0[YO + lu - KW]);
-        const R d3 = S::sub(uzc[q], U0[ZO + lu - 1]);
-        t1c[q] = S::tn1(a.dtab, cc, d1, d2, d3, SA, sb[q], t123_d);
-        t2c[q] = S::tn1(a.dtab, cc + 3, d1, d2, d3, SA, sb[q], t123_d);
-        if (!kz) t3c[q] = S::tn1(a.dtab, cc + 6, d1, d2, d3, SA, sb[q], t123_d);  // T3[1:-1,1:-1,0] = 0 (:418)
+    R uxc, uyc, uzc, uxc_up, t1c, t2c, t3c, t4c, t5c, t6c;
+    int idp_c, idp_z, idp_y;
+      uxc = U0[XO + Lu];
+    uyc = uyc_n;
+    uzc = uzc_n;
+    uyc_n = Up[YO + Lu];
+    uzc_n = Up[ZO + Lu];
+    uxc_up = U0[XO + Lu + 1];  // ux(i, j, k+1): T5, and the z = N face input of the next plane's ux
+    idp_c = Mp[Lm];
+    idp_z = Mp[Lm + 1];
+    idp_y = Mp[Lm + MKW];
+    t1c = t2c = t3c = R(0);
+    if (i_n && j_n && k_in) {
+      // T1..T3 (base_solver.py:329-351, 408-418): material of the own node
+      const R* row = tab + 16 * id_c;
+      R cc[9];
+      if constexpr (sizeof(R) == 4) {
+        const float4 q0 = *reinterpret_cast<const float4*>(row), q1 = *reinterpret_cast<const float4*>(row + 4);
+        cc[0] = q0.x, cc[1] = q0.y, cc[2] = q0.z, cc[3] = q0.w, cc[4] = q1.x, cc[5] = q1.y, cc[6] = q1.z,
+        cc[7] = q1.w;
+        cc[8] = row[8];
+      } else {
+        for (int c = 0; c < 9; c++) cc[c] = row[c];
       }
-      t4c[q] = t5c[q] = t6c[q] = R(0);
-      if (i_n && j_s[q] && k_in) {  // T4 (base_solver.py:353-358, 420-423)
-        const R c = tab[16 * (kz ? id_y[q] : (int)M0[lm + MKW + 1]) + 9];
-        const R d1 = S::sub(U0[YO + lu + 1], uyc[q]);
-        const R d2 = S::sub(U0[ZO + lu + KW], uzc[q]);
-        t4c[q] = S::ts(a.dtab, c, d1, kz ? a.sp.fdy0 : fdz_k, d2, kz ? a.sp.fdz0 : fdy_j[q]);
-      }
-      if (i_s && j_n[q] && k_in) {  // T5 (base_solver.py:360-365, 425-428)
-        const R c = tab[16 * (kz ? idp_c[q] : idp_z[q]) + 10];
-        const R d1 = S::sub(uxc_up[q], uxc[q]);
-        const R d2 = S::sub(uzc_n[q], uzc[q]);
-        t5c[q] = S::ts(a.dtab, c, d1, kz ? a.sp.fdx0 : fdz_k, d2, SX5);
-      }
-      if (i_s && j_s[q] && k_in) {  // T6 (base_solver.py:367-372, 430-433)
-        const R c = tab[16 * idp_y[q] + 11];
-        const R d1 = S::sub(U0[XO + lu + KW], uxc[q]);
-        const R d2 = S::sub(uyc_n[q], uyc[q]);
-        t6c[q] = S::ts(a.dtab, c, d1, kz ? a.sp.fdx0 : fdy_j[q], d2, SX5);
-      }
-      const int l = L + q * W;
-      sT2[l] = t2c[q];
-      sT3[l] = t3c[q];
-      sT4[l] = t4c[q];
-      sT5[p * PL + l] = t5c[q];
-      sT6[p * PL + l] = t6c[q];
+      const R d1 = S::sub(uxc, uxm);
+      const R d2 = S::sub(uyc, U0[YO + Lu - KW]);
+      const R d3 = S::sub(uzc, U0[ZO + Lu - 1]);
+      t1c = S::tn1(a.dtab, cc, d1, d2, d3, SA, sb, t123_d);
+      t2c = S::tn1(a.dtab, cc + 3, d1, d2, d3, SA, sb, t123_d);
+      if (!kz) t3c = S::tn1(a.dtab, cc + 6, d1, d2, d3, SA, sb, t123_d);  // T3[1:-1,1:-1,0] = 0 (:418)
     }
+    t4c = t5c = t6c = R(0);
+    if (i_n && j_s && k_in) {  // T4 (base_solver.py:353-358, 420-423)
+      const R c = tab[16 * (kz ? id_y : (int)M0[Lm + MKW + 1]) + 9];
+      const R d1 = S::sub(U0[YO + Lu + 1], uyc);
+      const R d2 = S::sub(U0[ZO + Lu + KW], uzc);
+      t4c = S::ts(a.dtab, c, d1, kz ? a.sp.fdy0 : fdz_k, d2, kz ? a.sp.fdz0 : fdy_j);
+    }
+    if (i_s && j_n && k_in) {  // T5 (base_solver.py:360-365, 425-428)
+      const R c = tab[16 * (kz ? idp_c : idp_z) + 10];
+      const R d1 = S::sub(uxc_up, uxc);
+      const R d2 = S::sub(uzc_n, uzc);
+      t5c = S::ts(a.dtab, c, d1, kz ? a.sp.fdx0 : fdz_k, d2, SX5);
+    }
+    if (i_s && j_s && k_in) {  // T6 (base_solver.py:367-372, 430-433)
+      const R c = tab[16 * idp_y + 11];
+      const R d1 = S::sub(U0[XO + Lu + KW], uxc);
+      const R d2 = S::sub(uyc_n, uyc);
+      t6c = S::ts(a.dtab, c, d1, kz ? a.sp.fdx0 : fdy_j, d2, SX5);
+    }
+    sT2[L] = t2c;
+    sT3[L] = t3c;
+    sT4[L] = t4c;
+    sT5[p * PL + L] = t5c;
+    sT6[p * PL + L] = t6c;
     // this thread's halo stress of plane i (set up before the loop)
     if (hk >= 0) {
       R v = R(0);
@@ -420,9 +404,7 @@ __device__ __forceinline__ bool tile_block_rows(const StepArgs<typename S::R>& a
     // ux is updated one plane behind: its pointwise state is taken from the
     // slot of plane i-1 before that slot is refilled
     const R* PWm = pwring + ((i - 1 - ibase) & (NSLOT - 1)) * P::PWS + Lp;  // pointwise, plane i-1
-    Pw<R> pwx[JR];
-    #pragma unroll
-    for (int q = 0; q < JR; q++) pwx[q] = Pw<R>{PWm[q * TK], S::kahan ? PWm[3 * P::PWC + q * TK] : R(0)};
+    const Pw<R> pwx{PWm[0], S::kahan ? PWm[3 * P::PWC] : R(0)};
     // The slot of plane i-1 is refilled by a TMA copy (async proxy) that
     // thread 0 issues after the barrier.  A barrier orders shared-memory
     // accesses of the block's threads only: without this proxy fence a read
@@ -439,82 +421,77 @@ __device__ __forceinline__ bool tile_block_rows(const StepArgs<typename S::R>& a
     const bool plane_yz = i < ie;                     // uy, uz of plane i belong to this segment
     const bool plane_x = i > ib && i - 1 != nx - 2;  // ux of plane i-1 (not the x = N face)
     const int pm = p ^ 1;
-    #pragma unroll
-    for (int q = 0; q < JR; q++) {
-      const int l = L + q * W, lu = Lu + q * KW;
-      const unsigned off = off_i + (unsigned)q * syu;
-      if (plane_yz) {
-        // uy_new(i, j, k)   (base_solver.py:449-455, 503-509)
-        if (own_y[q]) {
-          R val;
-          if (i_n) {
-            // at k = 0 the T4(k-1) halo entry is 0, so T4 - 0 is the z = 0 row's "T4 - 0"
-            const R* row = tab + 16 * id_y[q];
-            const R dv = S::div3(a.dtab, S::sub(t6c[q], t6m[q]), SA, S::sub(sT2[l + W], t2c[q]), uy_b[q],
-                                 S::sub(t4c[q], sT4[l - 1]), t123_d);
-            R vn, cn;
-            val = update_value<S>(uyc[q], Pw<R>{PW0[P::PWC + q * TK], S::kahan ? PW0[4 * P::PWC + q * TK] : R(0)},
-                                  dv, row[12], a.dt, vn, cn);
-            store_point<S>(r, 1, off, val, vn, cn);
-          } else {
-            val = store_stale<S>(r, 1, off);
-          }
-          if (zface_xy)  // uy on z = N from its inner neighbour (base_solver.py:553)
-            store_point<S>(r, 1, off + 1, rigid ? R(0) : S::abc(a.abc[6], val, U0[YO + lu + 1], uyc[q]), R(0), R(0));
-        }
-        // uz_new(i, j, k)   (base_solver.py:457-463, 511-516)
-        if (own_z[q]) {
-          R val;
-          if (i_n && j_n[q]) {
-            // z = 0 row: density at z index 0 (base_solver.py:513); T3(k) = 0 there,
-            // and the reference precedence (:516) adds T3[..,1] with factor 1
-            const R* row = tab + 16 * (kz ? id_c[q] : id_z[q]);
-            const R dv = S::div3(a.dtab, S::sub(t5c[q], t5m[q]), SA, S::sub(t4c[q], sT4[l - W]), sb[q],
-                                 S::sub(sT3[l + 1], t3c[q]), uz_c);
-            R vn, cn;
-            val = update_value<S>(uzc[q],
-                                  Pw<R>{PW0[2 * P::PWC + q * TK], S::kahan ? PW0[5 * P::PWC + q * TK] : R(0)}, dv,
-                                  row[12], a.dt, vn, cn);
-            store_point<S>(r, 2, off, val, vn, cn);
-          } else {
-            val = store_stale<S>(r, 2, off);
-          }
-          if (kz) {  // surface uz (base_solver.py:114-116) and the non-finite guard
-            if (rec) rec[(long long)i * ny + q] = val;
-            if (!isfinite(val)) atomicOr(a.err, 1);
-          }
-          if (zface_z)  // uz on z = N from its inner neighbour (base_solver.py:554)
-            store_point<S>(r, 2, off + 1, rigid ? R(0) : S::abc(a.abc[7], val, U0[ZO + lu + 1], uzc[q]), R(0), R(0));
-        }
-      }
-      if (plane_x && own_x[q]) {
-        // ux_new(i-1, j, k)   (base_solver.py:441-447, 495-501)
-        const unsigned offm = off - sxu;
+    if (plane_yz) {
+      // uy_new(i, j, k)   (base_solver.py:449-455, 503-509)
+      if (own_y) {
         R val;
-        if (j_n[q]) {
-          const R* row = tab + 16 * id_c[q];  // P[(i-1)+1, j, k]
-          // at k = 0 the T5(k-1) halo entry is 0 (the z = 0 row's "T5 - 0")
-          const R dv = S::div3(a.dtab, S::sub(t1c[q], t1m[q]), kz ? a.sp.fdx0 : fdx_im,
-                               S::sub(sT6[pm * PL + l], sT6[pm * PL + l - W]), sb[q],
-                               S::sub(sT5[pm * PL + l], sT5[pm * PL + l - 1]), t123_d);
+        if (i_n) {
+          // at k = 0 the T4(k-1) halo entry is 0, so T4 - 0 is the z = 0 row's "T4 - 0"
+          const R* row = tab + 16 * id_y;
+          const R dv = S::div3(a.dtab, S::sub(t6c, t6m), SA, S::sub(sT2[L + W], t2c), uy_b,
+                               S::sub(t4c, sT4[L - 1]), t123_d);
           R vn, cn;
-          val = update_value<S>(uxm[q], pwx[q], dv, row[12], a.dt, vn, cn);
-          store_point<S>(r, 0, offm, val, vn, cn);
+          val = update_value<S>(uyc, Pw<R>{PW0[P::PWC], S::kahan ? PW0[4 * P::PWC] : R(0)},
+                                dv, row[12], a.dt, vn, cn);
+          store_point<S>(r, 1, off_i, val, vn, cn);
         } else {
-          val = store_stale<S>(r, 0, offm);
+          val = store_stale<S>(r, 1, off_i);
         }
-        if (zface_xy)  // ux on z = N from its inner neighbour (base_solver.py:552)
-          store_point<S>(r, 0, offm + 1, rigid ? R(0) : S::abc(a.abc[6], val, uxm_up[q], uxm[q]), R(0), R(0));
+        if (zface_xy)  // uy on z = N from its inner neighbour (base_solver.py:553)
+          store_point<S>(r, 1, off_i + 1, rigid ? R(0) : S::abc(a.abc[6], val, U0[YO + Lu + 1], uyc), R(0), R(0));
       }
-      t1m[q] = t1c[q];
-      t5m[q] = t5c[q];
-      t6m[q] = t6c[q];
-      uxm[q] = uxc[q];
-      uxm_up[q] = uxc_up[q];
-      id_c[q] = idp_c[q];
-      id_z[q] = idp_z[q];
-      id_y[q] = idp_y[q];
+      // uz_new(i, j, k)   (base_solver.py:457-463, 511-516)
+      if (own_z) {
+        R val;
+        if (i_n && j_n) {
+          // z = 0 row: density at z index 0 (base_solver.py:513); T3(k) = 0 there,
+          // and the reference precedence (:516) adds T3[..,1] with factor 1
+          const R* row = tab + 16 * (kz ? id_c : id_z);
+          const R dv = S::div3(a.dtab, S::sub(t5c, t5m), SA, S::sub(t4c, sT4[L - W]), sb,
+                               S::sub(sT3[L + 1], t3c), uz_c);
+          R vn, cn;
+          val = update_value<S>(uzc,
+                                Pw<R>{PW0[2 * P::PWC], S::kahan ? PW0[5 * P::PWC] : R(0)}, dv,
+                                row[12], a.dt, vn, cn);
+          store_point<S>(r, 2, off_i, val, vn, cn);
+        } else {
+          val = store_stale<S>(r, 2, off_i);
+        }
+        if (kz) {  // surface uz (base_solver.py:114-116) and the non-finite guard
+          if (rec) rec[(long long)i * ny] = val;
+          if (!isfinite(val)) atomicOr(a.err, 1);
+        }
+        if (zface_z)  // uz on z = N from its inner neighbour (base_solver.py:554)
+          store_point<S>(r, 2, off_i + 1, rigid ? R(0) : S::abc(a.abc[7], val, U0[ZO + Lu + 1], uzc), R(0), R(0));
+      }
     }
+    if (plane_x && own_x) {
+      // ux_new(i-1, j, k)   (base_solver.py:441-447, 495-501)
+      const unsigned offm = off_i - sxu;
+      R val;
+      if (j_n) {
+        const R* row = tab + 16 * id_c;  // P[(i-1)+1, j, k]
+        // at k = 0 the T5(k-1) halo entry is 0 (the z = 0 row's "T5 - 0")
+        const R dv = S::div3(a.dtab, S::sub(t1c, t1m), kz ? a.sp.fdx0 : fdx_im,
+                             S::sub(sT6[pm * PL + L], sT6[pm * PL + L - W]), sb,
+                             S::sub(sT5[pm * PL + L], sT5[pm * PL + L - 1]), t123_d);
+        R vn, cn;
+        val = update_value<S>(uxm, pwx, dv, row[12], a.dt, vn, cn);
+        store_point<S>(r, 0, offm, val, vn, cn);
+      } else {
+        val = store_stale<S>(r, 0, offm);
+      }
+      if (zface_xy)  // ux on z = N from its inner neighbour (base_solver.py:552)
+        store_point<S>(r, 0, offm + 1, rigid ? R(0) : S::abc(a.abc[6], val, uxm_up, uxm), R(0), R(0));
+    }
+    t1m = t1c;
+    t5m = t5c;
+    t6m = t6c;
+    uxm = uxc;
+    uxm_up = uxc_up;
+    id_c = idp_c;
+    id_z = idp_z;
+    id_y = idp_y;
     fx_prev = fx_cur;
     fx_cur = fx_next;
     sx_cur = sx_next;
