@@ -19,7 +19,7 @@ cudaError_t launch_step_f32k(const StepArgs<float>& a, int tj, int n_face_blocks
 cudaError_t configure_step_f64v(int tj);
 cudaError_t launch_step_f64v(const StepArgs<double>& a, int tj, int n_face_blocks, cudaStream_t st);
 cudaError_t launch_split(int precision, const void* args, bool stress, cudaStream_t st);
-cudaError_t launch_energy(const EnergyArgs& a, double2* partial, int nblocks, double* out, cudaStream_t st);
+cudaError_t launch_energy(const EnergyArgs& a, double2* partial, int nblocks, double* out, bool pairs, cudaStream_t st);
 cudaError_t batch_step_any(int precision, const void* ba, int tj, int grid_tiles, int grid_faces, cudaStream_t st);
 cudaError_t batch_advance_any(int precision, const void* ba, int n_active_cap, int n, cudaStream_t st);
 cudaError_t batch_configure_any(int precision, int tj, int* blocks_per_sm);
@@ -54,6 +54,9 @@ void set_last_error(const char* msg) { g_err = msg; }
 
 static const int kGraphSteps = 12;  // multiple of 2 and 3: buffer rotations line up
 static const int kEnergyBlocks = 1024;
+// FP32 meshes from here on sum their energy in pairs of floats: on smaller
+// ones FP64 takes less than the launches around it
+static const double kEnergyPairNodes = 200000;
 
 // tile decomposition of the tile pass and the TMA descriptors of its boxes
 struct Tiling {
@@ -1124,10 +1127,17 @@ int phono_energy(phono_handle* h, double out[2]) {
   a.mat = h->mat;
   a.tab = h->tab13;
   a.nmat = h->nmat;
-  CK(launch_energy(a, h->partial, kEnergyBlocks, h->energy_out, h->stream));
-  CK(cudaMemcpyAsync(out, h->energy_out, sizeof(double) * 2, cudaMemcpyDeviceToHost, h->stream));
-  CK(cudaStreamSynchronize(h->stream));
-  return PHONO_OK;
+  const double n = (double)h->d.nx * h->d.ny * h->d.nz;
+  bool pairs = h->es == 4 && n >= kEnergyPairNodes;
+  for (;; pairs = false) {
+    CK(launch_energy(a, h->partial, kEnergyBlocks, h->energy_out, pairs, h->stream));
+    CK(cudaMemcpyAsync(out, h->energy_out, sizeof(double) * 2, cudaMemcpyDeviceToHost, h->stream));
+    CK(cudaStreamSynchronize(h->stream));
+    // terms of 1e-6 to 1e30 on average keep every intermediate of the pairs
+    // within FP32's range (a pair's low part is 2^-48 of its term); a zero, tiny,
+    // huge or non-finite energy is computed again in FP64
+    if (!pairs || (out[0] > 1e-6 * n && out[0] < 1e30 && out[1] > 1e-6 * n && out[1] < 1e30)) return PHONO_OK;
+  }
 }
 
 int phono_reset(phono_handle* h) {

@@ -23,15 +23,50 @@ __device__ __forceinline__ double ld(const void* p, int f32, long long off) {
 constexpr int EN_THREADS = 256;
 constexpr int EN_WARPS = EN_THREADS / 32;
 
+// Material row of the reductions: the quadratic form of the normal strains
+// (c00, c11, c22, c01 + c10, c02 + c20, c12 + c21), the shear moduli, rho.
+constexpr int EN_COLS = 10;
+__device__ __forceinline__ double en_coef(const double* row, int q) {
+  switch (q) {
+    case 0: return __ldg(row);
+    case 1: return __ldg(row + 4);
+    case 2: return __ldg(row + 8);
+    case 3: return __dadd_rn(__ldg(row + 1), __ldg(row + 3));
+    case 4: return __dadd_rn(__ldg(row + 2), __ldg(row + 6));
+    case 5: return __dadd_rn(__ldg(row + 5), __ldg(row + 7));
+    default: return __ldg(row + 3 + q);  // 6..8: columns 9..11; 9: rho
+  }
+}
+
+// sums of the block's threads, halved, into its partial
+__device__ __forceinline__ void block_partial(double ek, double es, double2* partial) {
+  __shared__ double sk[EN_THREADS], ss[EN_THREADS];
+  sk[threadIdx.x] = 0.5 * ek;
+  ss[threadIdx.x] = 0.5 * es;
+  __syncthreads();
+  for (int w = EN_THREADS / 2; w > 0; w >>= 1) {
+    if ((int)threadIdx.x < w) {
+      sk[threadIdx.x] += sk[threadIdx.x + w];
+      ss[threadIdx.x] += ss[threadIdx.x + w];
+    }
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) *partial = make_double2(sk[0], ss[0]);
+}
+
 // One warp per (i, j) row of the mesh, lanes along k (coalesced loads of every
 // array), rows dealt to the warps of the grid in a fixed order.  Spacings come
 // as FP64 reciprocals (the strain is a difference times 1/spacing) and the
-// material table is staged in shared memory, so a node costs FP64 multiplies
-// and adds only.  Element type T of the displacement / velocity arrays.
+// material table is staged in shared memory, so a node costs about 40 FP64
+// operations, which bounds the kernel (one FP64 instruction takes a
+// multiprocessor 16 cycles): 0.57 ms of FP64 pipe at 8.5 M nodes, 0.70 ms
+// measured (0.79 with two resident blocks instead of four), 1.27 with separate
+// multiplications and additions and all nine stiffnesses.  Element type T of the displacement / velocity arrays.
 template <class T>
-__global__ void __launch_bounds__(EN_THREADS) energy_partial_kernel(EnergyArgs a, double2* __restrict__ partial) {
-  extern __shared__ double etab[];  // nmat rows of 13
-  for (int q = threadIdx.x; q < a.nmat * 13; q += EN_THREADS) etab[q] = __ldg(a.tab + q);
+__global__ void __launch_bounds__(EN_THREADS, 4) energy_partial_kernel(EnergyArgs a, double2* __restrict__ partial) {
+  extern __shared__ double etab[];  // nmat rows of EN_COLS
+  for (int q = threadIdx.x; q < a.nmat * EN_COLS; q += EN_THREADS)
+    etab[q] = en_coef(a.tab + 13 * (q / EN_COLS), q % EN_COLS);
   __syncthreads();
   const Geo& g = a.g;
   const int nx = g.nx, ny = g.ny, nz = g.nz;
@@ -44,7 +79,7 @@ __global__ void __launch_bounds__(EN_THREADS) energy_partial_kernel(EnergyArgs a
   const T* vy = (const T*)a.vy;
   const T* vz = (const T*)a.vz;
   const uint8_t* mat = a.mat;
-  double ek = 0.0, es = 0.0;  // sums of rho v^2 and of T . e (the 1/2 is applied once)
+  double ek = 0.0, es = 0.0;  // sums of rho v^2 (leapfrog: of rho (u - u_old)^2) and of T . e
   for (int r = blockIdx.x * EN_WARPS + (threadIdx.x >> 5); r < nx * ny; r += nwarps) {
     const int i = r / ny, j = r - (r / ny) * ny;
     const long long o = g.o0 + (long long)i * g.sx + (long long)j * g.sy;      // field (i, j, 0)
@@ -58,65 +93,199 @@ __global__ void __launch_bounds__(EN_THREADS) energy_partial_kernel(EnergyArgs a
       const long long p = o + k;
       const bool kin = k <= nz - 2, kn = k >= 1 && k <= nz - 2;
       const double rsdz = kn ? __ldg(a.rsdz + k - 1) : 0.0, rfdz = kn ? __ldg(a.rfdz + k) : 0.0;
+      auto at = [&](const T* f, long long q) { return (double)__ldg(f + q); };
       // kinetic energy at the interior displacement points, absorbing faces excluded
-      auto vel = [&](const T* u, const T* v) {
-        const double x = (double)__ldg(v + p);
-        return a.vgiven ? x : ((double)__ldg(u + p) - x) * a.inv_dt;
-      };
-      if (ix_in && jx_in && kin) {
-        const double v = vel(ux, vx);
-        ek += etab[13 * mat[mo + g.msx + k] + 12] * v * v;
-      }
-      if (iyz_in && jy_in && kin) {
-        const double v = vel(uy, vy);
-        ek += etab[13 * mat[mo + g.msy + k] + 12] * v * v;
-      }
-      if (iyz_in && jx_in && k <= nz - 3) {
-        const double v = vel(uz, vz);
-        ek += etab[13 * mat[mo + k + 1] + 12] * v * v;
-      }
+      auto vel = [&](const T* u, const T* v) { return a.vgiven ? at(v, p) : at(u, p) - at(v, p); };
+      auto square = [&](double& sum, double c, double x) { sum = __fma_rn(__dmul_rn(c, x), x, sum); };
+      if (ix_in && jx_in && kin) square(ek, etab[EN_COLS * mat[mo + g.msx + k] + 9], vel(ux, vx));
+      if (iyz_in && jy_in && kin) square(ek, etab[EN_COLS * mat[mo + g.msy + k] + 9], vel(uy, vy));
+      if (iyz_in && jx_in && k <= nz - 3) square(ek, etab[EN_COLS * mat[mo + k + 1] + 9], vel(uz, vz));
       if (!kn) continue;  // every strain term below needs 1 <= k <= nz-2
+      const double x0 = at(ux, p), y0 = at(uy, p), z0 = at(uz, p);
       // strain energy: normal stresses at interior nodes
       if (iyz_in && jx_in) {
-        const double* c = etab + 13 * mat[mo + k];
-        const double e1 = ((double)__ldg(ux + p) - (double)__ldg(ux + p - g.sx)) * rsdx;
-        const double e2 = ((double)__ldg(uy + p) - (double)__ldg(uy + p - g.sy)) * rsdy;
-        const double e3 = ((double)__ldg(uz + p) - (double)__ldg(uz + p - 1)) * rsdz;
-        const double t1 = c[0] * e1 + c[1] * e2 + c[2] * e3;
-        const double t2 = c[3] * e1 + c[4] * e2 + c[5] * e3;
-        const double t3 = c[6] * e1 + c[7] * e2 + c[8] * e3;
-        es += t1 * e1 + t2 * e2 + t3 * e3;
+        const double* c = etab + EN_COLS * mat[mo + k];
+        const double e1 = (x0 - at(ux, p - g.sx)) * rsdx, e2 = (y0 - at(uy, p - g.sy)) * rsdy, e3 = (z0 - at(uz, p - 1)) * rsdz;
+        es = __fma_rn(__fma_rn(c[0], e1, __fma_rn(c[3], e2, __dmul_rn(c[4], e3))), e1, es);
+        es = __fma_rn(__fma_rn(c[1], e2, __dmul_rn(c[5], e3)), e2, es);
+        square(es, c[2], e3);
       }
       // shears at edges
-      if (iyz_in && jsh) {
-        const double gam = ((double)__ldg(uy + p + 1) - (double)__ldg(uy + p)) * rfdz +
-                           ((double)__ldg(uz + p + g.sy) - (double)__ldg(uz + p)) * rfdy;
-        es += etab[13 * mat[mo + g.msy + k + 1] + 9] * gam * gam;
-      }
-      if (ish && jx_in) {
-        const double gam = ((double)__ldg(ux + p + 1) - (double)__ldg(ux + p)) * rfdz +
-                           ((double)__ldg(uz + p + g.sx) - (double)__ldg(uz + p)) * rfdx;
-        es += etab[13 * mat[mo + g.msx + k + 1] + 10] * gam * gam;
-      }
-      if (ish && jsh) {
-        const double gam = ((double)__ldg(ux + p + g.sy) - (double)__ldg(ux + p)) * rfdy +
-                           ((double)__ldg(uy + p + g.sx) - (double)__ldg(uy + p)) * rfdx;
-        es += etab[13 * mat[mo + g.msx + g.msy + k] + 11] * gam * gam;
-      }
+      if (iyz_in && jsh)
+        square(es, etab[EN_COLS * mat[mo + g.msy + k + 1] + 6],
+               __fma_rn(at(uy, p + 1) - y0, rfdz, __dmul_rn(at(uz, p + g.sy) - z0, rfdy)));
+      if (ish && jx_in)
+        square(es, etab[EN_COLS * mat[mo + g.msx + k + 1] + 7],
+               __fma_rn(at(ux, p + 1) - x0, rfdz, __dmul_rn(at(uz, p + g.sx) - z0, rfdx)));
+      if (ish && jsh)
+        square(es, etab[EN_COLS * mat[mo + g.msx + g.msy + k] + 8],
+               __fma_rn(at(ux, p + g.sy) - x0, rfdy, __dmul_rn(at(uy, p + g.sx) - y0, rfdx)));
     }
   }
-  __shared__ double sk[EN_THREADS], ss[EN_THREADS];
-  sk[threadIdx.x] = 0.5 * ek;
-  ss[threadIdx.x] = 0.5 * es;
-  __syncthreads();
-  for (int w = EN_THREADS / 2; w > 0; w >>= 1) {
-    if ((int)threadIdx.x < w) {
-      sk[threadIdx.x] += sk[threadIdx.x + w];
-      ss[threadIdx.x] += ss[threadIdx.x + w];
+  block_partial(a.vgiven ? ek : ek * (a.inv_dt * a.inv_dt), es, partial + blockIdx.x);
+}
+
+// ---------------------------------------------------------------------------
+// FP32 fields of large meshes: the same sums in pairs of floats (an
+// unevaluated sum h + l, 48 bits), on the FP32 pipe, whose rate is 64 times
+// the FP64 pipe's.  Differences of floats are exact pairs; constants enter as
+// three floats (72 bits) and the low parts' product is kept in squares, so
+// that no rounding is biased; a product or sum of pairs is off by 2^-47 of its
+// value at random, which over the terms of a large mesh averages out below
+// the FP64 rounding of the result (against 128-bit sums on meshes of 0.2 to 3 M
+// nodes: 2.6e-16 at most, 2.7e-16 for the FP64 kernel).  A thread's sums go to
+// FP64 every few planes (every 32: 9.6e-16).  Terms must stay clear of
+// the FP32 range: the caller checks the result and repeats in FP64 otherwise.
+// ---------------------------------------------------------------------------
+struct Pair {
+  float h, l;
+};
+__device__ __forceinline__ Pair pair_diff(float x, float y) {  // x - y, exact (Knuth's two-sum)
+  const float d = __fsub_rn(x, y), t = __fsub_rn(d, x);
+  return Pair{d, __fsub_rn(__fsub_rn(x, __fsub_rn(d, t)), __fadd_rn(y, t))};
+}
+__device__ __forceinline__ Pair pair_fast(float h, float l) {  // |h| >= |l|
+  const float s = __fadd_rn(h, l);
+  return Pair{s, __fsub_rn(l, __fsub_rn(s, h))};
+}
+__device__ __forceinline__ Pair pair_add(Pair x, Pair y) {
+  const float s = __fadd_rn(x.h, y.h), t = __fsub_rn(s, x.h);
+  const float e = __fadd_rn(__fsub_rn(x.h, __fsub_rn(s, t)), __fsub_rn(y.h, t));
+  return pair_fast(s, __fadd_rn(e, __fadd_rn(x.l, y.l)));
+}
+__device__ __forceinline__ Pair pair_scale(Pair x, const float3 c) {  // x times a constant of three floats
+  const float p = __fmul_rn(x.h, c.x);
+  float e = __fmaf_rn(x.h, c.x, -p);
+  e = __fmaf_rn(x.h, c.z, e);
+  e = __fmaf_rn(x.l, c.y, e);
+  e = __fmaf_rn(x.h, c.y, e);
+  e = __fmaf_rn(x.l, c.x, e);
+  return pair_fast(p, e);
+}
+// sum += x * y
+__device__ __forceinline__ void pair_acc(Pair& sum, Pair x, Pair y) {
+  const float p = __fmul_rn(x.h, y.h);
+  float e = __fmaf_rn(x.h, y.h, -p);
+  e = __fmaf_rn(x.l, y.l, e);
+  e = __fmaf_rn(x.h, y.l, e);
+  e = __fmaf_rn(x.l, y.h, e);
+  const float s = __fadd_rn(sum.h, p), t = __fsub_rn(s, sum.h);
+  sum.l = __fadd_rn(sum.l, __fadd_rn(__fadd_rn(__fsub_rn(sum.h, __fsub_rn(s, t)), __fsub_rn(p, t)), e));
+  sum.h = s;
+}
+__device__ __forceinline__ float3 triple(double c) {
+  const float x = __double2float_rn(c);
+  const double r = __dsub_rn(c, (double)x);
+  const float y = __double2float_rn(r);
+  return make_float3(x, y, __double2float_rn(__dsub_rn(r, (double)y)));
+}
+
+constexpr int EN_PLANES = 64;  // most planes of an item
+constexpr int EN_FLUSH = 4;    // planes after which a thread's sums go to FP64: a pair's low part drifts by 2^-49 a term
+
+// what plane i of a column adds to the last plane's values
+struct EnPlane {
+  float x0, xk, xj;      // ux(i), ux(i, k+1), ux(i, j+1)
+  float y1, yk, yj;      // uy(i+1), uy(i, k+1), uy(i, j-1)
+  float z1, zk, zj;      // uz(i+1), uz(i, k-1), uz(i, j+1)
+  float vx, vy, vz;
+  int id, id_z, id_y, id_yz;  // plane i+1: own, k+1, j+1, both
+};
+
+// A block takes (column tile of 8 rows x 32 z, 1/nit of the planes) items in a
+// fixed order; a warp owns a row of the tile, a lane a z column, and marches
+// along x with the values of the last plane in registers and those of the next
+// one on their way.  256x256x128 cells: 191 us, 1510 for the FP64 form, which the
+// FP64 pipe bounds; without the loads a plane ahead 380 us.  Bound by
+// instruction issue (71% of the slots, 430 instructions a node).
+__global__ void __launch_bounds__(EN_THREADS, 2) energy_pair_kernel(EnergyArgs a, int nit, double2* __restrict__ partial) {
+  extern __shared__ float4 ptab[];  // nmat rows of EN_COLS constants (x, y, z of a float4), then the x spacings of an item
+  float4* px = ptab + a.nmat * EN_COLS;
+  for (int q = threadIdx.x; q < a.nmat * EN_COLS; q += EN_THREADS) {
+    const float3 c = triple(en_coef(a.tab + 13 * (q / EN_COLS), q % EN_COLS));
+    ptab[q] = make_float4(c.x, c.y, c.z, 0.f);
+  }
+  const Geo& g = a.g;
+  const int nx = g.nx, ny = g.ny, nz = g.nz;
+  const int lane = threadIdx.x & 31, row = threadIdx.x >> 5;
+  const int nkt = (nz - 1 + 31) / 32, njt = (ny - 1 + EN_WARPS - 1) / EN_WARPS;
+  const long long sx = g.sx, sy = g.sy, msx = g.msx, msy = g.msy;
+  double ek = 0.0, es = 0.0;
+  for (int item = blockIdx.x; item < nkt * njt * nit; item += gridDim.x) {
+    const int kt = item % nkt, rest = item / nkt, jt = rest % njt, part = rest / njt;
+    const int i0 = (int)((long long)(nx - 1) * part / nit), i1 = (int)((long long)(nx - 1) * (part + 1) / nit);
+    __syncthreads();
+    for (int q = threadIdx.x; q < 2 * (i1 - i0); q += EN_THREADS) {
+      const int i = i0 + (q >> 1);  // 1/sdx[i-1], 1/fdx[i]
+      const float3 c = triple(q & 1 ? __ldg(a.rfdx + i) : (i >= 1 && i <= nx - 2 ? __ldg(a.rsdx + i - 1) : 0.0));
+      px[q] = make_float4(c.x, c.y, c.z, 0.f);
     }
     __syncthreads();
+    const int j = jt * EN_WARPS + row, k = kt * 32 + lane;
+    if (j > ny - 2 || k > nz - 2) continue;  // no term there
+    const bool j_n = j >= 1, jy = j >= 1 && j <= ny - 3, kn = k >= 1, kz = k <= nz - 3;
+    const float3 rsy = triple(j_n ? __ldg(a.rsdy + j - 1) : 0.0), rfy = triple(__ldg(a.rfdy + j));
+    const float3 rsz = triple(kn ? __ldg(a.rsdz + k - 1) : 0.0), rfz = triple(__ldg(a.rfdz + k));
+    const long long o = g.o0 + (long long)i0 * sx + (long long)j * sy + k;
+    const float *ux = (const float*)a.ux + o, *uy = (const float*)a.uy + o, *uz = (const float*)a.uz + o;
+    const float *vx = (const float*)a.vx + o, *vy = (const float*)a.vy + o, *vz = (const float*)a.vz + o;
+    const uint8_t* m = a.mat + g.mo0 + (long long)i0 * msx + (long long)j * msy + k;
+    float xm = __ldg(ux - sx), y0 = __ldg(uy), z0 = __ldg(uz);
+    int id = m[0], id_z = m[1], id_y = m[msy], id_yz = m[msy + 1];
+    // the padding makes every neighbour of planes up to nx-1 readable
+    auto read = [&] {
+      EnPlane p;
+      p.x0 = __ldg(ux), p.xk = __ldg(ux + 1), p.xj = __ldg(ux + sy);
+      p.y1 = __ldg(uy + sx), p.yk = __ldg(uy + 1), p.yj = __ldg(uy - sy);
+      p.z1 = __ldg(uz + sx), p.zk = __ldg(uz - 1), p.zj = __ldg(uz + sy);
+      p.vx = __ldg(vx), p.vy = __ldg(vy), p.vz = __ldg(vz);
+      p.id = m[msx], p.id_z = m[msx + 1], p.id_y = m[msx + msy], p.id_yz = m[msx + msy + 1];
+      ux += sx, uy += sx, uz += sx, vx += sx, vy += sx, vz += sx, m += msx;
+      return p;
+    };
+    Pair k2{0.f, 0.f}, s2{0.f, 0.f};
+    auto coef = [&](int mid, int q) {
+      const float4 c = ptab[EN_COLS * mid + q];
+      return make_float3(c.x, c.y, c.z);
+    };
+    EnPlane next = read();
+    for (int i = i0; i < i1; i++) {
+      const EnPlane p = next;
+      if (i + 1 < i1) next = read();
+      const bool i_n = i >= 1, in = i_n && j_n;  // i <= nx-2 here
+      // kinetic energy
+      auto kinetic = [&](int mid, float v) { pair_acc(k2, pair_scale(Pair{v, 0.f}, coef(mid, 9)), Pair{v, 0.f}); };
+      if (j_n && i <= nx - 3) kinetic(p.id, p.vx);
+      if (i_n && jy) kinetic(id_y, p.vy);
+      if (in && kz) kinetic(id_z, p.vz);
+      if (kn) {
+        const float4 sx4 = px[2 * (i - i0)], fx4 = px[2 * (i - i0) + 1];
+        const float3 rsx = make_float3(sx4.x, sx4.y, sx4.z), rfx = make_float3(fx4.x, fx4.y, fx4.z);
+        if (in) {
+          const Pair e1 = pair_scale(pair_diff(p.x0, xm), rsx), e2 = pair_scale(pair_diff(y0, p.yj), rsy),
+                     e3 = pair_scale(pair_diff(z0, p.zk), rsz);
+          pair_acc(s2, pair_add(pair_scale(e1, coef(id, 0)), pair_add(pair_scale(e2, coef(id, 3)), pair_scale(e3, coef(id, 4)))), e1);
+          pair_acc(s2, pair_add(pair_scale(e2, coef(id, 1)), pair_scale(e3, coef(id, 5))), e2);
+          pair_acc(s2, pair_scale(e3, coef(id, 2)), e3);
+        }
+        auto shear = [&](int mid, int q, Pair d1, float3 r1, Pair d2, float3 r2) {
+          const Pair gam = pair_add(pair_scale(d1, r1), pair_scale(d2, r2));
+          pair_acc(s2, pair_scale(gam, coef(mid, q)), gam);
+        };
+        if (i_n) shear(id_yz, 6, pair_diff(p.yk, y0), rfz, pair_diff(p.zj, z0), rfy);
+        if (j_n) shear(p.id_z, 7, pair_diff(p.xk, p.x0), rfz, pair_diff(p.z1, z0), rfx);
+        shear(p.id_y, 8, pair_diff(p.xj, p.x0), rfy, pair_diff(p.y1, y0), rfx);
+      }
+      xm = p.x0, y0 = p.y1, z0 = p.z1;
+      id = p.id, id_z = p.id_z, id_y = p.id_y, id_yz = p.id_yz;
+      if ((i + 1 - i0) % EN_FLUSH == 0 || i + 1 == i1) {
+        ek = __dadd_rn(ek, __dadd_rn((double)k2.h, (double)k2.l));
+        es = __dadd_rn(es, __dadd_rn((double)s2.h, (double)s2.l));
+        k2 = s2 = Pair{0.f, 0.f};
+      }
+    }
   }
-  if (threadIdx.x == 0) partial[blockIdx.x] = make_double2(sk[0], ss[0]);
+  block_partial(ek, es, partial + blockIdx.x);
 }
 
 __global__ void __launch_bounds__(EN_THREADS) energy_final_kernel(const double2* __restrict__ partial, int n,
@@ -143,13 +312,31 @@ __global__ void __launch_bounds__(EN_THREADS) energy_final_kernel(const double2*
   }
 }
 
-// partial must hold nblocks double2 values; out two doubles (device)
-cudaError_t launch_energy(const EnergyArgs& a, double2* partial, int nblocks, double* out, cudaStream_t st) {
-  const size_t smem = (size_t)a.nmat * 13 * sizeof(double);
-  if (a.f32)
-    energy_partial_kernel<float><<<nblocks, EN_THREADS, smem, st>>>(a, partial);
-  else
-    energy_partial_kernel<double><<<nblocks, EN_THREADS, smem, st>>>(a, partial);
+// partial must hold nblocks double2 values; out two doubles (device).
+// pairs: FP32 fields in pairs of floats (energy_pair_kernel)
+cudaError_t launch_energy(const EnergyArgs& a, double2* partial, int nblocks, double* out, bool pairs, cudaStream_t st) {
+  if (pairs) {
+    const size_t smem = ((size_t)a.nmat * EN_COLS + 2 * EN_PLANES) * sizeof(float4);
+    nblocks = nblocks < 304 ? nblocks : 304;  // two resident blocks on each of 152 SMs
+    // x parts: as many items as fill the blocks' last round best
+    const int tiles = ((a.g.nz + 30) / 32) * ((a.g.ny - 1 + EN_WARPS - 1) / EN_WARPS);
+    const int least = (a.g.nx - 1 + EN_PLANES - 1) / EN_PLANES, most = (a.g.nx - 1 + 7) / 8;
+    int nit = least;
+    double best = 0.0;
+    for (int n = least; n <= most && n <= least + 16; n++) {
+      const int rounds = (tiles * n + nblocks - 1) / nblocks;
+      // a round takes its planes and about two more for the start of a column
+      const double use = 1.0 / (rounds * ((double)(a.g.nx - 1) / n + 2.0));
+      if (use > best) best = use, nit = n;
+    }
+    energy_pair_kernel<<<nblocks, EN_THREADS, smem, st>>>(a, nit, partial);
+  } else {
+    const size_t smem = (size_t)a.nmat * EN_COLS * sizeof(double);
+    if (a.f32)
+      energy_partial_kernel<float><<<nblocks, EN_THREADS, smem, st>>>(a, partial);
+    else
+      energy_partial_kernel<double><<<nblocks, EN_THREADS, smem, st>>>(a, partial);
+  }
   energy_final_kernel<<<1, EN_THREADS, 0, st>>>(partial, nblocks, out);
   return cudaGetLastError();
 }
