@@ -18,7 +18,7 @@ cudaError_t launch_step_f64(const StepArgs<double>& a, int tj, int n_face_blocks
 cudaError_t launch_step_f32k(const StepArgs<float>& a, int tj, int n_face_blocks, cudaStream_t st);
 cudaError_t configure_step_f64v(int tj);
 cudaError_t launch_step_f64v(const StepArgs<double>& a, int tj, int n_face_blocks, cudaStream_t st);
-cudaError_t launch_split(int precision, const void* args, bool stress, cudaStream_t st);
+cudaError_t launch_split(int precision, const void* args, bool stress, bool after_kernel, cudaStream_t st);
 cudaError_t launch_energy(const EnergyArgs& a, double2* partial, int nblocks, double* out, bool pairs, cudaStream_t st);
 cudaError_t batch_step_any(int precision, const void* ba, int tj, int grid_tiles, int grid_faces, cudaStream_t st);
 cudaError_t batch_advance_any(int precision, const void* ba, int n_active_cap, int n, cudaStream_t st);
@@ -356,8 +356,9 @@ static cudaError_t split_step(const phono_handle* h, int step_off, int step_end,
       const int planes = std::max(0, std::min(a.pb, xn[c]) - p);
       a.off[c + 4] = a.off[c + 3] + planes * std::max(nj[c] - 2, 0) * (nk[c] - 1);
     }
-    e = launch_split(h->d.precision, &a, true, st);
-    if (e == cudaSuccess) e = launch_split(h->d.precision, &a, false, st);
+    // the first launch of a chunk of steps waits for all before it
+    e = launch_split(h->d.precision, &a, true, step_off > 0 || p > 0, st);
+    if (e == cudaSuccess) e = launch_split(h->d.precision, &a, false, true, st);
   }
   return e;
 }

@@ -14,50 +14,35 @@
 // 1500 instructions a stress point, FP64 pipe 38% and ALU 52% busy); small
 // meshes by two dependent launches (1.2 us each) of three or four L2
 // latencies.
-//   nodes       25x21x13  41x41x21  61x61x21  150x131x47  194x162x98  257x257x129
-//   F64         25 / 11   32 / 12   47 / 15   354 / 118   969 / 391   2012 / 1071
-//   F64V        13 / 8    21 / 10   29 / 14   197 / 121   559 / 378   1174 / 1037
-//   F32K        9 / 6     10 / 7    12 / 8    (larger meshes: tile_vec.cuh)
-#include "scheme.cuh"
-#include "split_common.cuh"
+//   nodes       25x21x13   41x41x21   61x61x21   150x131x47  194x162x98  257x257x129
+//   F64         25 / 11.6  32 / 12.6  47 / 15.0  354 / 116   969 / 378   2012 / 1033
+//   F64V        13 / 7.4   21 / 9.1   29 / 13.8  197 / 121   559 / 385   1174 / 1064
+//   F32K        9 / 5.3    10 / 5.7   12 / 6.7   (split_f32.cu; larger meshes: tile_vec.cuh)
+#include "split_point.cuh"
 
 namespace phono {
 
-__device__ __forceinline__ float ldd(const float* p) { return __ldg(p); }
-__device__ __forceinline__ double ldd(const double* p) { return __ldg(p); }
-__device__ __forceinline__ SoftRec ldd(const SoftRec* p) {
-  const uint4 v = __ldg(reinterpret_cast<const uint4*>(p));
-  return SoftRec{v.x, v.y, v.z, v.w};
-}
-
-// velocity forms: reciprocal spacings, coefficients as stored
-template <class B>
+// the velocity form in FP64: reciprocal spacings, coefficients as stored
 struct VelOps {
-  using Base = B;
-  using R = typename B::R;
+  using Base = F64V;
+  using R = double;
   using D = R;
   using Args = SplitArgs<R, D>;
-  static constexpr int STRESS_BLOCKS = sizeof(R) == 8 ? 6 : 12, UPDATE_BLOCKS = sizeof(R) == 8 ? 9 : 8;
+  static constexpr int STRESS_BLOCKS = 6, UPDATE_BLOCKS = 7;
   static __device__ __forceinline__ void normals(const Args& a, int id, R d1, R d2, R d3, D x, D y, D z, R* t) {
     const R* row = a.tab + 16 * id;
     R c[9];
-    if constexpr (sizeof(R) == 4) {
-      const float4 q0 = __ldg(reinterpret_cast<const float4*>(row)), q1 = __ldg(reinterpret_cast<const float4*>(row) + 1);
-      c[0] = q0.x, c[1] = q0.y, c[2] = q0.z, c[3] = q0.w, c[4] = q1.x, c[5] = q1.y, c[6] = q1.z, c[7] = q1.w;
-      c[8] = __ldg(row + 8);
-    } else {
-      for (int q = 0; q < 9; q++) c[q] = __ldg(row + q);
-    }
-    for (int q = 0; q < 3; q++) t[q] = B::tn1(a.dtab, c + 3 * q, d1, d2, d3, x, y, z);
+    for (int q = 0; q < 9; q++) c[q] = __ldg(row + q);
+    for (int q = 0; q < 3; q++) t[q] = F64V::tn1(a.dtab, c + 3 * q, d1, d2, d3, x, y, z);
   }
   static __device__ __forceinline__ R shear(const Args& a, int id, int col, R d1, D x, R d2, D y) {
-    return B::ts(a.dtab, __ldg(a.tab + 16 * id + col), d1, x, d2, y);
+    return F64V::ts(a.dtab, __ldg(a.tab + 16 * id + col), d1, x, d2, y);
   }
   static __device__ __forceinline__ R div3(const Args& a, R d1, D x, R d2, D y, R d3, D z) {
-    return B::div3(a.dtab, d1, x, d2, y, d3, z);
+    return F64V::div3(a.dtab, d1, x, d2, y, d3, z);
   }
   static __device__ __forceinline__ R update(const Args& a, int id, R u, Pw<R> pw, R dv, R& vn, R& cn) {
-    return update_value<B>(u, pw, dv, __ldg(a.tab + 16 * id + 12), a.dt, vn, cn);
+    return update_value<F64V>(u, pw, dv, __ldg(a.tab + 16 * id + 12), a.dt, vn, cn);
   }
 };
 
@@ -70,9 +55,9 @@ struct LeapOps {
   using R = double;
   using D = SoftRec;
   using Args = SplitArgs<double, SoftRec>;
-  // resident blocks the registers are allotted for: 6 and 7 gave 1071 us a
-  // step on 256x256x128 cells, 5 and 7 1112, 8 and 8 1116, 9 and 12 1160
-  static constexpr int STRESS_BLOCKS = 6, UPDATE_BLOCKS = 7;
+  // resident blocks the registers are allotted for (us a step on 256x256x128
+  // cells): 7 and 8 1033, 6 and 8 1048, 6 and 7 1089, 5 and 7 1127
+  static constexpr int STRESS_BLOCKS = 7, UPDATE_BLOCKS = 8;
   struct Num {
     double x;
     SoftNum n;
@@ -131,8 +116,6 @@ struct LeapOps {
   }
 };
 
-__device__ __forceinline__ int fdiv(int n, const FastDiv& f) { return (int)(__umulhi(2u * (unsigned)n, f.mult) >> f.shift); }
-
 // ---------------------------------------------------------------------------
 // stresses of planes [sa, sb): one thread per node of [sa, sb) x [0, ny-1) x
 // [0, nz-1).  Zero where the reference never writes (base_solver.py:329-433).
@@ -141,6 +124,7 @@ template <class O>
 __global__ void __launch_bounds__(SPLIT_THREADS, O::STRESS_BLOCKS) split_stress_kernel(const __grid_constant__ typename O::Args a) {
   using R = typename O::R;
   using B = typename O::Base;
+  last_launch_done();
   const int tt = __ldg(a.step_base) + a.step_off;
   if (tt >= a.step_end) return;
   const Geo& g = a.g;
@@ -199,38 +183,14 @@ template <class O>
 __global__ void __launch_bounds__(SPLIT_THREADS, O::UPDATE_BLOCKS) split_update_kernel(const __grid_constant__ typename O::Args a) {
   using R = typename O::R;
   using B = typename O::Base;
+  last_launch_done();
   const int tt = __ldg(a.step_base) + a.step_off;
   if (tt >= a.step_end) return;
   const Geo& g = a.g;
   int n = blockIdx.x * SPLIT_THREADS + threadIdx.x;
   if (n >= a.off[6]) return;
   int c, i, j, k;
-  const bool edge = n < a.off[3];
-  if (!edge) {
-    c = (n >= a.off[4]) + (n >= a.off[5]);
-    n -= a.off[3 + c];
-    const FastDiv fz = a.uz_[c], fy = a.uy_[c];
-    const int q1 = fdiv(n, fz), q2 = fdiv(q1, fy);
-    k = n - q1 * fz.d, j = q1 - q2 * fy.d + 2, i = a.pa + q2;
-  } else {  // points next to a face: per plane the rows j = 1 and jN-1, then the rest of k = kN-1
-    c = (n >= a.off[1]) + (n >= a.off[2]);
-    n -= a.off[c];
-    const int xi = ext_x(g, c) - 1, nj = ext_y(g, c) - 2, nk = ext_z(g, c) - 1, rows = min(nj, 2) * nk;
-    const int planes = max(min(a.pb, xi - 1) - a.pa, 0);
-    i = fdiv(n, a.per[c]);
-    if (i < planes) {
-      n -= i * a.per[c].d;
-      i += a.pa;
-      if (n < nk) j = 1, k = n;
-      else if (n < rows) j = nj, k = n - nk;
-      else j = 2 + n - rows, k = nk - 1;
-    } else {  // the plane next to x = N: all of it
-      n -= planes * a.per[c].d;
-      i = xi - 1;
-      j = fdiv(n, a.nk[c]);
-      k = n - j++ * nk;
-    }
-  }
+  const bool edge = update_point(a, g, n, c, i, j, k);
   Roles<R> r = roles<B>(a, tt);
   if constexpr (B::kahan) {
     r.v_in = r.v_out = a.vbase;
@@ -238,31 +198,16 @@ __global__ void __launch_bounds__(SPLIT_THREADS, O::UPDATE_BLOCKS) split_update_
   }
   const unsigned o = (unsigned)g.o0 + (unsigned)i * (unsigned)g.sx + (unsigned)j * (unsigned)g.sy + (unsigned)k;
   const R* uc = r.cur(c);
-  const R u = __ldg(uc + o);
-  // faces next to the point (x = N; y = 0 or N; z = N), and the old values of
-  // the up to 2 x 2 x 2 points they span, read here because they are off the
-  // path of the update
-  const int nfx = edge && i == ext_x(g, c) - 2, nfz = edge && k == ext_z(g, c) - 2;
-  int fj = !edge ? 0 : j == 1 ? -1 : j == ext_y(g, c) - 2 ? 1 : 0;
-  const bool two_y = fj < 0 && j == ext_y(g, c) - 2;
-  R old[8];  // [z][y][x]
-  auto read_old = [&] {
-    const R s = (R)__ldg(a.src + tt);
-#pragma unroll
-    for (int q = 0; q < 8; q++) {
-      const bool fx = q & 1, fy = q & 2, fk = q & 4;
-      if ((fx && !nfx) || (fy && !fj) || (fk && !nfz)) continue;
-      old[q] = __ldg(uc + (o + (fx ? (unsigned)g.sx : 0u) + (fy ? (unsigned)(fj * (int)g.sy) : 0u) + (fk ? 1u : 0u)));
-      if (c == 2 && i == 0 && !fx && (a.source_mode == 1 || (k == 0 && !fk))) old[q] = s;  // source overwrite (base_solver.py:251)
-    }
-  };
-  if (edge) read_old();
+  const R u = uc[o];
+  // old values for the face points, read early: they are off the path of the update
+  FacePoints<B, typename O::Args> faces(a, r, uc, c, i, j, k, tt, o, edge);
+  if (edge) faces.read();
   R val, vn = R(0), cn = R(0);
   if (c == 0 || i >= 1) {
     const bool kz = k == 0;
     Pw<R> pw;
     if constexpr (B::kahan) pw = Pw<R>{r.v_in[c * r.fs + o], r.c_in[c * r.fs + o]};
-    else pw = load_pw<B>(r, c, o);
+    else pw = Pw<R>{r.old(c)[o], R(0)};
     const unsigned s0 = (unsigned)i % a.W, sp = s0 + 1 == a.W ? 0 : s0 + 1, sm = s0 == 0 ? a.W - 1 : s0 - 1;
     const unsigned ro = (unsigned)(j * a.tsy + k);
     const R *A = a.Ta + ro, *Bc = a.Tb + ro + s0 * a.tsx, *Bm = a.Tb + ro + sm * a.tsx;  // T4..T6 of planes i, i-1
@@ -300,47 +245,25 @@ __global__ void __launch_bounds__(SPLIT_THREADS, O::UPDATE_BLOCKS) split_update_
     r.out(c)[o] = u;
   }
   if (c == 2 && k == 0) record(a, tt, i, j, val);
-  if (!edge) return;
-  for (;;) {
-    // every face point whose chain starts here: x = N first, then y, then z = N
-    R w[8];
-    w[0] = val;
-#pragma unroll
-    for (int q = 1; q < 8; q++) {
-      const bool fx = q & 1, fy = q & 2, fk = q & 4;
-      if ((fx && !nfx) || (fy && !fj) || (fk && !nfz)) continue;
-      const int from = q & (fk ? 3 : fy ? 1 : 0);
-      const R f = fk ? (c == 2 ? a.abc[7] : a.abc[6])
-                     : !fy ? (c == 0 ? a.abc[0] : a.abc[1])
-                           : fj < 0 ? (c == 1 ? a.abc[3] : a.abc[2]) : (c == 1 ? a.abc[5] : a.abc[4]);
-      w[q] = a.bc == 1 ? R(0) : B::abc(f, w[from], old[q], old[from]);
-      store_point<B>(r, c, o + (fx ? (unsigned)g.sx : 0u) + (fy ? (unsigned)(fj * (int)g.sy) : 0u) + (fk ? 1u : 0u), w[q],
-                     R(0), R(0));
-      if (c == 2 && k == 0 && !fk) record(a, tt, i + fx, fy ? j + fj : j, w[q]);
-    }
-    if (!two_y || fj > 0) break;
-    fj = 1;  // a single row between the two y faces
-    read_old();
-  }
+  if (edge) faces.write(val);
 }
 
 template <class O>
-static cudaError_t split_launch(const typename O::Args& a, bool stress, cudaStream_t st) {
-  if (stress) {
-    const long long n = (long long)(a.sb - a.sa) * a.dy1.d * a.dz1.d;
-    if (n > 0) split_stress_kernel<O><<<(int)((n + SPLIT_THREADS - 1) / SPLIT_THREADS), SPLIT_THREADS, 0, st>>>(a);
-  } else {
-    const long long n = a.off[6];
-    if (n > 0) split_update_kernel<O><<<(int)((n + SPLIT_THREADS - 1) / SPLIT_THREADS), SPLIT_THREADS, 0, st>>>(a);
-  }
-  return cudaGetLastError();
+static cudaError_t launch_pass(const void* args, bool stress, bool after_kernel, cudaStream_t st) {
+  const typename O::Args& a = *(const typename O::Args*)args;
+  return stress ? split_launch(split_stress_kernel<O>, a, (long long)(a.sb - a.sa) * a.dy1.d * a.dz1.d, after_kernel, st)
+                : split_launch(split_update_kernel<O>, a, a.off[6], after_kernel, st);
 }
 
-// one pass over the planes set in the arguments; precision as in phono.h
-cudaError_t launch_split(int precision, const void* args, bool stress, cudaStream_t st) {
-  if (precision == 0) return split_launch<LeapOps>(*(const LeapOps::Args*)args, stress, st);
-  if (precision == 2) return split_launch<VelOps<F64V>>(*(const VelOps<F64V>::Args*)args, stress, st);
-  return split_launch<VelOps<F32K>>(*(const VelOps<F32K>::Args*)args, stress, st);
+cudaError_t launch_split_f32(const void* args, bool stress, bool after_kernel, cudaStream_t st);
+
+// one pass over the planes set in the arguments; precision as in phono.h;
+// after_kernel: the launch before it on the stream is a pass of the same chunk
+// of steps (nothing between the two changed a constant or the step counter)
+cudaError_t launch_split(int precision, const void* args, bool stress, bool after_kernel, cudaStream_t st) {
+  if (precision == 0) return launch_pass<LeapOps>(args, stress, after_kernel, st);
+  if (precision == 2) return launch_pass<VelOps>(args, stress, after_kernel, st);
+  return launch_split_f32(args, stress, after_kernel, st);
 }
 
 }  // namespace phono
