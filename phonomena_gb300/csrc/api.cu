@@ -105,6 +105,7 @@ struct phono_handle {
   bool resplit = false;        // in a persistent batch (tile pass): back to the two-launch form when it leaves
   char* stress = nullptr;      // leapfrog: the window
   SoftRec* rec = nullptr;      // leapfrog: table entries as records, 16 per material
+  int shared = 0;              // leapfrog: the normal stresses share terms (split_step.cu)
   void* spd[6] = {};           // divisors of the two-launch step (records, or sp)
   double* vals = nullptr;      // leapfrog: values of all records
   cudaStream_t stream = nullptr;
@@ -214,6 +215,12 @@ static int upload_table(phono_handle* h, const double* table, int nmat, int id00
     CK(cudaMemcpyAsync(h->tab, t32.data(), t32.size() * 4, cudaMemcpyHostToDevice, h->stream));
   }
   if (leapfrog) {  // the same entries for the two-launch step
+    h->shared = 1;
+    for (int m = 0; m < nmat; m++) {
+      const double* c = table + m * PHONO_TABLE_COLS;
+      auto same = [&](int p, int q) { return soft_bits(c[p]) == soft_bits(c[q]); };  // zeros with their signs
+      h->shared &= same(3, 6) && same(1, 7) && same(2, 5);
+    }
     for (size_t q = 0; q < t.size(); q++) rec.push_back(soft_record(t[q], false, (uint32_t)q));
     CK(cudaMemcpyAsync(h->rec, rec.data(), rec.size() * sizeof(SoftRec), cudaMemcpyHostToDevice, h->stream));
     CK(cudaMemcpyAsync(h->vals, t.data(), t.size() * 8, cudaMemcpyHostToDevice, h->stream));
@@ -295,6 +302,7 @@ static cudaError_t split_step(const phono_handle* h, int step_off, int step_end,
   a.tab = (const R*)h->tab;
   a.rec = h->rec;
   a.vals = h->vals;
+  a.shared = h->shared;
   a.dtab = h->dtab;
   a.src = h->src;
   a.ubase = (R*)h->ubase;

@@ -88,7 +88,7 @@ SOFT_HD SoftNum soft_split(double x, bool& ok) {
   n.hi = (xh << 11) | (xl >> 21) | 0x80000000u;
   n.lo = xl << 11;
   n.se = xh & 0xfff00000u;
-  ok = ((xh >> 20) & 0x7ffu) - SOFT_EXP_MIN <= SOFT_EXP_SPAN;
+  ok = xh * 2u - (SOFT_EXP_MIN << 21) <= ((SOFT_EXP_SPAN << 21) | 0x1fffffu);  // a multiply-add and a compare
   return n;
 }
 

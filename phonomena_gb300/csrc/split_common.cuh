@@ -32,6 +32,7 @@ struct SplitArgs {
   const R* tab;          // velocity forms: 16 entries per material id
   const SoftRec* rec;    // leapfrog: the same entries as records
   const double* vals;    // leapfrog: values of the records (fallback division)
+  int shared;            // leapfrog: c10 = c20, c01 = c21, c02 = c12 in every material
   DivTable dtab;
   const double* src;
   R *ubase, *vbase, *cbase;

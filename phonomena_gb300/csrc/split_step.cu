@@ -10,12 +10,12 @@
 // through it in chunks.  The result is that of the tile pass, bit for bit.
 //
 // Bound (one GB300, us a step, the best tile shape of the tile pass first):
-// FP64 by the FP64 pipe and, nearly as much, by instruction issue (18 FP64 of
-// 1500 instructions a stress point, FP64 pipe 38% and ALU 52% busy); small
+// FP64 by instruction issue and the FP64 pipe together (18 FP64 of 1220
+// instructions a stress point; issue 61%, ALU 61%, FP64 pipe 57% busy); small
 // meshes by two dependent launches (1.2 us each) of three or four L2
 // latencies.
 //   nodes       25x21x13   41x41x21   61x61x21   150x131x47  194x162x98  257x257x129
-//   F64         25 / 11.6  32 / 12.6  47 / 15.0  354 / 116   969 / 378   2012 / 1033
+//   F64         25 / 10.9  32 / 11.1  47 / 13.5  354 / 102   969 / 337   2012 / 924
 //   F64V        13 / 7.4   21 / 9.1   29 / 13.8  197 / 121   559 / 385   1174 / 1064
 //   F32K        9 / 5.3    10 / 5.7   12 / 6.7   (split_f32.cu; larger meshes: tile_vec.cuh)
 #include "split_point.cuh"
@@ -50,13 +50,17 @@ struct VelOps {
 // arithmetic (soft_f64.cuh), additions on the FP64 pipe
 __device__ __noinline__ double slow_div(double x, double b, DivTable k) { return k.tab ? div_tab(x, b, k) : __ddiv_rn(x, b); }
 
+// SHARED: every material has c10 = c20, c01 = c21 and c02 = c12 (isotropic and
+// cubic ones do), so that the normal stresses share three of their nine terms
+// (256x256x128 cells: 924 us a step, 1008 without).
+template <bool SHARED>
 struct LeapOps {
   using Base = F64;
   using R = double;
   using D = SoftRec;
   using Args = SplitArgs<double, SoftRec>;
   // resident blocks the registers are allotted for (us a step on 256x256x128
-  // cells): 7 and 8 1033, 6 and 8 1048, 6 and 7 1089, 5 and 7 1127
+  // cells): 7 and 8 924, 6 and 8 954, 8 and 8 926, 7 and 7 962
   static constexpr int STRESS_BLOCKS = 7, UPDATE_BLOCKS = 8;
   struct Num {
     double x;
@@ -98,10 +102,19 @@ struct LeapOps {
                                                  const D& z, R* t) {
     const SoftRec* c = a.rec + 16 * id;
     const Num v1 = split(d1), v2 = split(d2), v3 = split(d3);
-#pragma unroll
-    for (int q = 0; q < 3; q++)
-      t[q] = __dadd_rn(__dadd_rn(scaled(a, v1, ldd(c + 3 * q), x), scaled(a, v2, ldd(c + 3 * q + 1), y)),
-                       scaled(a, v3, ldd(c + 3 * q + 2), z));
+    if constexpr (SHARED) {
+      const R x1 = scaled(a, v1, ldd(c + 3), x), y0 = scaled(a, v2, ldd(c + 1), y), z0 = scaled(a, v3, ldd(c + 2), z);
+      t[0] = __dadd_rn(__dadd_rn(scaled(a, v1, ldd(c), x), y0), z0);
+      t[1] = __dadd_rn(__dadd_rn(x1, scaled(a, v2, ldd(c + 4), y)), z0);
+      t[2] = __dadd_rn(__dadd_rn(x1, y0), scaled(a, v3, ldd(c + 8), z));
+    } else {
+      // not unrolled: the instructions of three copies miss the cache (1033 us
+      // a step on 256x256x128 cells, 1008 so)
+#pragma unroll 1
+      for (int q = 0; q < 3; q++)
+        t[q] = __dadd_rn(__dadd_rn(scaled(a, v1, ldd(c + 3 * q), x), scaled(a, v2, ldd(c + 3 * q + 1), y)),
+                         scaled(a, v3, ldd(c + 3 * q + 2), z));
+    }
   }
   static __device__ __forceinline__ R shear(const Args& a, int id, int col, R d1, const D& x, R d2, const D& y) {
     return times(a, __dadd_rn(divide(a, d1, x), divide(a, d2, y)), ldd(a.rec + 16 * id + col));
@@ -261,7 +274,10 @@ cudaError_t launch_split_f32(const void* args, bool stress, bool after_kernel, c
 // after_kernel: the launch before it on the stream is a pass of the same chunk
 // of steps (nothing between the two changed a constant or the step counter)
 cudaError_t launch_split(int precision, const void* args, bool stress, bool after_kernel, cudaStream_t st) {
-  if (precision == 0) return launch_pass<LeapOps>(args, stress, after_kernel, st);
+  if (precision == 0) {
+    if (((const LeapOps<false>::Args*)args)->shared) return launch_pass<LeapOps<true>>(args, stress, after_kernel, st);
+    return launch_pass<LeapOps<false>>(args, stress, after_kernel, st);
+  }
   if (precision == 2) return launch_pass<VelOps>(args, stress, after_kernel, st);
   return launch_split_f32(args, stress, after_kernel, st);
 }

@@ -54,6 +54,28 @@ def test_two_launch_step_equals_oracle(gpu_lib, oracle, precision, shape, modes)
         assert np.array_equal(sim.read_surface(), want_surf)
 
 
+@pytest.mark.parametrize("flip", [None, 3, 6, 1, 7, 2, 5])
+def test_shared_stress_terms(gpu_lib, oracle, flip):
+    """Materials whose normal stresses share terms, and the same with one of
+    the stiffnesses a little different or a zero of the other sign."""
+    from phonomena_gb300.device import DeviceSimulation
+
+    sp, ids, dt, src = _problem((13, 12, 37), 3, 20)
+    tab = TABLE.copy()
+    tab[0, [3, 6]], tab[0, [1, 7]], tab[0, [2, 5]] = 61e9, 63e9, 65e9
+    if flip is not None:
+        tab[0, flip] *= 1 + 2.0 ** -40
+        tab[1, flip] = -0.0
+    prob = oracle.OracleProblem(sp, ids, tab, dt, src, surface_mode=1)
+    want, _ = oracle.run_f64(prob)
+    with DeviceSimulation(sp, ids, tab, dt, precision="f64", surface_mode="corrected", max_steps=20) as sim:
+        sim.set_source(src)
+        sim.step(20)
+        sim.sync()
+        for key, w in zip(("ux", "uy", "uz"), want.u):
+            assert np.array_equal(sim.download(key), w), key
+
+
 @pytest.mark.parametrize("precision", ["f64", "f64v"])
 def test_chunked_window_equals_tile_pass(gpu_lib, precision):
     """A mesh of several chunks (77 planes of 270 x 180 nodes: 128 MB hold 57)."""
