@@ -397,12 +397,11 @@ static cudaError_t launch_one(phono_handle* h, int step_off, int parts = -1) {
   return tile_step(h, step_off, 0x7fffffff, form, h->stream);
 }
 
-// Padded device layout: planes -1..nx, rows -1..ny, a KOFF-element front pad
-// in z and rows rounded up to 128 bytes; material ids with an MKOFF front pad
+// Padded device layout: planes -1..nx, rows -1..ny, z rows with KPAD zeros
+// behind them, rounded up to 128 bytes; material ids with an MKOFF front pad
 // and 16-byte rows.
 static long long field_row(int nz, int es) {
-  const long long koff = es == 8 ? Lay<double>::KOFF : Lay<float>::KOFF;
-  return round_up(koff + nz + 1, 128 / es);
+  return round_up((es == 8 ? Lay<double>::KPAD : Lay<float>::KPAD) + nz + 1, 128 / es);
 }
 static long long mat_row(int nz) { return round_up(MKOFF + nz + 1, 16); }
 
@@ -647,13 +646,13 @@ static int set_tiling(phono_handle* h, int tj, int xseg) {
 }
 
 // A default FP32 handle's own tiles: the vectorised tile pass at height 16, or
-// 8 where 16 rows waste more than 3% of the y extent (256x256x128 cells: 134
-// against 136 us a step; 130 rows are 9 tiles of 16 but 17 of 8).  Segments of
+// 8 where 16 rows waste more than 3% of the y extent (256x256x128 cells: 128
+// us a step either way; 130 rows are 9 tiles of 16 but 17 of 8).  Segments of
 // about 12 planes (a segment reads two planes more than it updates; long ones
 // let neighbouring blocks drift apart until their common halo rows have left
-// L2: 169 us at 37 planes, 134 at 10, 138 at 4), as many as fill the last wave
+// L2: 512x512x256 cells 802 us at 12 planes, 917 at 57), as many as fill the last wave
 // of resident blocks (3 an SM of height 16, 5 of height 8; 160x128x64 cells:
-// 31 us with 448 blocks of 456, 37 with 480).  Beside other instances (a
+// 26 us with 448 blocks of 456, 35 with 480).  Beside other instances (a
 // streams batch) there is no last wave to fill: even segments of at most 24
 // planes (12 crystals of 6.2 M nodes in all: 120 us a step, 163 with each
 // instance's single-run segments).
@@ -749,8 +748,7 @@ int phono_create(const phono_desc* d, phono_handle** out) {
   const bool f64 = d->precision == PHONO_F64;  // leapfrog state (u_old, u, u_new)
   h->es = d->precision == PHONO_F32K ? 4 : 8;
   const int nx = d->nx, ny = d->ny, nz = d->nz;
-  // padded layout: planes -1..nx, rows -1..ny, 32-byte front pad in z
-  const long long koff = h->es == 8 ? Lay<double>::KOFF : Lay<float>::KOFF;
+  // padded layout: planes -1..nx, rows -1..ny
   const long long pz = field_row(nz, h->es);
   h->nbuf = f64 ? 3 : 2;
   h->g.nx = nx;
@@ -758,7 +756,7 @@ int phono_create(const phono_desc* d, phono_handle** out) {
   h->g.nz = nz;
   h->g.sy = pz;
   h->g.sx = (long long)(ny + 2) * pz;
-  h->g.o0 = h->g.sx + h->g.sy + koff;
+  h->g.o0 = h->g.sx + h->g.sy;
   h->field_elems = (size_t)(nx + 2) * h->g.sx;
   if (h->field_elems >= (1ull << 32)) {  // the tile pass addresses an array with 32-bit offsets
     delete h;

@@ -11,7 +11,8 @@
 // nbuf x 3 arrays (buffer-major, then component ux, uy, uz), each with the
 // padded extents
 //   element (i, j, k) at  o0 + i*sx + j*sy + k,   i in [-1, nx], j in [-1, ny],
-//   k in [-KOFF, sy-KOFF) with the (0,0,0) row start 32-byte aligned,
+//   k in [0, sy) with every row start 128-byte aligned; k = -1 is the last
+//   element of the row before,
 // so that one 4-D TMA box (k, j, i, component) loads a plane tile of all three
 // components.  The padding is zero and never written: the 1-node halo of every
 // stencil read exists without bounds checks.  Component extents inside that
@@ -40,13 +41,13 @@ template <class R>
 struct Lay;
 template <>
 struct Lay<double> {
-  static constexpr int KOFF = 4;   // field front pad in k (elements): 32 bytes
+  static constexpr int KPAD = 4;   // zeros behind a row's nz + 1 elements (at least)
   static constexpr int KW = 36;    // tile width in k: k0-2 .. k0+34 (288 bytes)
   static constexpr int KB = 2;     // column of k0 inside the tile
 };
 template <>
 struct Lay<float> {
-  static constexpr int KOFF = 8;
+  static constexpr int KPAD = 8;
   static constexpr int KW = 40;    // k0-4 .. k0+36 (160 bytes)
   static constexpr int KB = 4;
 };

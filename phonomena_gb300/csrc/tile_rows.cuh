@@ -103,13 +103,13 @@ __device__ __forceinline__ bool tile_block_rows(const StepArgs<typename S::R>& a
     // test hook (skip_plane >= 0; -1 is off_i, and plane -1 is a real padding
     // plane that segment 0 loads): armed, no copy, so the wait on it runs out
     if (a.skip_plane >= 0 && p == a.skip_plane) return;
-    // padded coordinates: k + KOFF, j + 1, i + 1; the u tiles start at k0-KB, j0-1
-    tma_load_4d(uring + sl * SU, &maps->tm_u, k0 - KB + Lay<R>::KOFF, j0, p + 1, r.rcur * 3, &bars[sl]);
+    // padded coordinates: k, j + 1, i + 1; the u tiles start at k0-KB (columns before 0: zeros), j0-1
+    tma_load_4d(uring + sl * SU, &maps->tm_u, k0 - KB, j0, p + 1, r.rcur * 3, &bars[sl]);
     tma_load_3d(mring + sl * SM, &maps->tm_mat, k0, j0, p + 1, &bars[sl]);
     if (pw) {
       R* d = pwring + sl * P::PWS;
-      tma_load_4d(d, &maps->tm_pw0, k0 + Lay<R>::KOFF, j0 + 1, p + 1, pw_buf, &bars[sl]);
-      if constexpr (S::kahan) tma_load_4d(d + 3 * P::PWC, &maps->tm_pw1, k0 + Lay<R>::KOFF, j0 + 1, p + 1, pw_buf, &bars[sl]);
+      tma_load_4d(d, &maps->tm_pw0, k0, j0 + 1, p + 1, pw_buf, &bars[sl]);
+      if constexpr (S::kahan) tma_load_4d(d + 3 * P::PWC, &maps->tm_pw1, k0, j0 + 1, p + 1, pw_buf, &bars[sl]);
     }
   };
   bool ok = true;

@@ -21,14 +21,17 @@
 //      ux of plane i will need.
 // Segment ends need only T1 of the first plane behind them.
 //
-// Bound by DRAM traffic on large meshes (512x512x256 cells: 845 us a step,
-// 5.84 TB/s of the 73 bytes a node, 86% of the measured copy bandwidth), and by
+// Bound by DRAM traffic on large meshes (512x512x256 cells: 805 us a step,
+// 6.16 TB/s of the 73 bytes a node, 90% of the measured copy bandwidth), and by
 // the latency of a plane (1.7 us for a block alone) with the ramp and tail of
 // the launch on small ones.  The form before it, one node a thread with all
 // stresses exchanged through shared memory and two barriers a plane, issued
-// 507 instructions a node against 220 here and was bound by that.  us a step,
-// best tiles before and now: 512x512x256 1043 / 845, 256x256x128 154 / 134,
-// 193x161x97 80 / 67, 160x128x64 39.5 / 31, 149x130x46 38 / 25.
+// 507 instructions a node against 220 here and was bound by that.  Rows start
+// on 128-byte lines, so that a row of the tile's state is one line for the
+// copies in and for the stores (87 bytes of DRAM traffic a node when rows
+// started 32 bytes into a line, 80 now).  us a step, best tiles before, this
+// form, with aligned rows: 512x512x256 1043 / 850 / 805, 256x256x128 154 / 138
+// / 128, 193x161x97 80 / 66 / 63, 160x128x64 39.5 / 31 / 26.
 // Included inside namespace phono, after the TMA helpers and the schemes.
 #pragma once
 
@@ -107,12 +110,12 @@ __device__ __forceinline__ bool tile_block_vec(const StepArgs<float>& a, unsigne
     mbar_expect_tx(&bars[sl], P::tx_bytes + (pw ? P::pw_bytes : 0u));
     // test hook (skip_plane >= 0; -1 is off): armed, no copy, so the wait on it runs out
     if (a.skip_plane >= 0 && p == a.skip_plane) return;
-    tma_load_4d(uring + sl * P::SU, &maps->tm_u, k0 - KB + Lay<float>::KOFF, j0, p + 1, sbuf, &bars[sl]);
+    tma_load_4d(uring + sl * P::SU, &maps->tm_u, k0 - KB, j0, p + 1, sbuf, &bars[sl]);
     tma_load_3d(mring + sl * P::SM, &maps->tm_mat, k0, j0, p + 1, &bars[sl]);
     if (pw) {
       float* d = pwring + sl * P::PWS;
-      tma_load_4d(d, &maps->tm_pw0, k0 + Lay<float>::KOFF, j0 + 1, p, sbuf, &bars[sl]);
-      tma_load_4d(d + 3 * P::PWC, &maps->tm_pw1, k0 + Lay<float>::KOFF, j0 + 1, p, sbuf, &bars[sl]);
+      tma_load_4d(d, &maps->tm_pw0, k0, j0 + 1, p, sbuf, &bars[sl]);
+      tma_load_4d(d + 3 * P::PWC, &maps->tm_pw1, k0, j0 + 1, p, sbuf, &bars[sl]);
     }
   };
   if (tid == 0) {
