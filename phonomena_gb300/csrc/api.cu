@@ -645,17 +645,39 @@ static int set_tiling(phono_handle* h, int tj, int xseg) {
   return apply_tiling(h, h->t, tj, xseg, segment_starts(h->d.nx - 1, xseg));
 }
 
+// Segments that keep the resident blocks busy to the end: every wave of blocks
+// takes segments of one length, the last the shortest, since blocks of equal
+// length that share the memory bandwidth drift apart and leave it idle at the
+// end.  For `depth` planes a block slot and at most `waves` waves; the lengths
+// grow by 1/0.6 from the shortest up to 17 planes.
+static std::vector<double> wave_lengths(double depth, int waves, double shortest) {
+  std::vector<double> len{shortest};
+  double sum = shortest;
+  while ((int)len.size() < waves) {
+    const double next = std::min(len.back() / 0.6, 17.0);
+    if (sum + next > depth) break;
+    len.push_back(next);
+    sum += next;
+  }
+  for (double& l : len) l *= depth / sum;
+  std::reverse(len.begin(), len.end());
+  return len;
+}
+
 // A default FP32 handle's own tiles: the vectorised tile pass at height 16, or
-// 8 where 16 rows waste more than 3% of the y extent (256x256x128 cells: 128
-// us a step either way; 130 rows are 9 tiles of 16 but 17 of 8).  Segments of
-// about 12 planes (a segment reads two planes more than it updates; long ones
-// let neighbouring blocks drift apart until their common halo rows have left
-// L2: 512x512x256 cells 802 us at 12 planes, 917 at 57), as many as fill the last wave
-// of resident blocks (3 an SM of height 16, 5 of height 8; 160x128x64 cells:
-// 26 us with 448 blocks of 456, 35 with 480).  Beside other instances (a
-// streams batch) there is no last wave to fill: even segments of at most 24
-// planes (12 crystals of 6.2 M nodes in all: 120 us a step, 163 with each
-// instance's single-run segments).
+// 8 where 16 rows waste more than 3% of the y extent (130 rows are 9 tiles of
+// 16 but 17 of 8).  Segments: at least as many as fill one wave of resident
+// blocks (3 an SM of height 16, 5 of height 8; 160x128x64 cells: 31 us with 448
+// blocks of 456, 37 with 480); meshes of a few waves in lengths that fall from
+// wave to wave (us a step, even segments before: 256x256x128 129 / 122,
+// 329x199x149 146 / 138, 119x149x288 83 / 78, 193x161x97 63 / 61); where less
+// than three segments fill a wave, even ones of about 12 planes (a segment
+// reads two planes more than it updates; long ones let neighbouring blocks
+// drift apart until their common halo rows have left L2: 512x512x256 cells 802
+// us at 12 planes, 917 at 57).  Beside other instances (a streams batch) there
+// is no last wave to fill: even segments of at most 24 planes (12 crystals of
+// 6.2 M nodes in all: 120 us a step, 163 with each instance's single-run
+// segments).
 static int own_tiling(phono_handle* h, bool alone) {
   int dev = 0, nsm = 152;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
@@ -664,10 +686,24 @@ static int own_tiling(phono_handle* h, bool alone) {
   const long long r16 = round_up(rows, 16), r8 = round_up(rows, 8);
   const int tj = r16 * 100 > r8 * 103 ? 8 : 16;
   const long long tiles = (tj == 16 ? r16 : r8) / tj * ((h->d.nz - 1 + TK - 1) / TK), wave = (long long)nsm * (tj == 16 ? 3 : 5);
-  const long long want = tiles * ((planes + 11) / 12), waves = (want + wave - 1) / wave;
-  const int nseg = alone ? (int)std::min<long long>(std::max<long long>(waves * wave / tiles, 1), planes) : (planes + 23) / 24;
   std::vector<int> starts;
-  for (int q = 0; q <= nseg; q++) starts.push_back((int)((long long)planes * q / nseg));
+  auto even = [&](int nseg) {
+    for (int q = 0; q <= nseg; q++) starts.push_back((int)((long long)planes * q / nseg));
+  };
+  const int fill = (int)std::min<long long>(wave / tiles, planes);  // segments that fill a wave
+  if (!alone) {
+    even((planes + 23) / 24);
+  } else if (fill >= 3) {
+    double at = 0;
+    starts.push_back(0);
+    for (double l : wave_lengths((double)planes / fill, SEG_TABLE / fill, tj == 16 ? 3.6 : 4.4))
+      for (int q = 0; q < fill; q++) starts.push_back((int)std::lround(at += l));
+    starts.back() = planes;
+  } else {
+    const long long want = tiles * ((planes + 11) / 12), waves = (want + wave - 1) / wave;
+    even((int)std::min<long long>(std::max<long long>(waves * wave / tiles, 1), planes));
+  }
+  const int nseg = (int)starts.size() - 1;
   // more segments than a launch describes by table: even ones
   if (nseg > SEG_TABLE) return apply_tiling(h, h->own, tj, (planes + nseg - 1) / nseg, segment_starts(planes, (planes + nseg - 1) / nseg));
   return apply_tiling(h, h->own, tj, kExplicitSegments, starts);
