@@ -664,9 +664,10 @@ static std::vector<double> wave_lengths(double depth, int waves, double shortest
   return len;
 }
 
-// A default FP32 handle's own tiles: the vectorised tile pass at height 16, or
-// 8 where 16 rows waste more than 3% of the y extent (130 rows are 9 tiles of
-// 16 but 17 of 8).  Segments: at least as many as fill one wave of resident
+// A default FP32 handle's own tiles: the vectorised tile pass at height 16,
+// which needs no face launch, or 8 where 16 rows waste more than half of
+// the y extent (us a step at 8 / 16: 8 rows, 1399x8x16 cells 13.5 / 15.5; 24
+// rows 23.9 / 23.5, 130 rows 25.6 / 22.4, 256 rows 124 / 118).  Segments: at least as many as fill one wave of resident
 // blocks (3 an SM of height 16, 5 of height 8; 160x128x64 cells: 31 us with 448
 // blocks of 456, 37 with 480); meshes of a few waves in lengths that fall from
 // wave to wave (us a step, even segments before: 256x256x128 129 / 122,
@@ -684,7 +685,7 @@ static int own_tiling(phono_handle* h, bool alone) {
   cudaGetLastError();
   const int planes = h->d.nx - 1, rows = h->d.ny - 1;
   const long long r16 = round_up(rows, 16), r8 = round_up(rows, 8);
-  const int tj = r16 * 100 > r8 * 103 ? 8 : 16;
+  const int tj = r16 > r8 + r8 / 2 ? 8 : 16;
   const long long tiles = (tj == 16 ? r16 : r8) / tj * ((h->d.nz - 1 + TK - 1) / TK), wave = (long long)nsm * (tj == 16 ? 3 : 5);
   std::vector<int> starts;
   auto even = [&](int nseg) {
@@ -1444,7 +1445,7 @@ struct phono_batch {
   cudaGraphExec_t graph = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   bool timed = false, dirty = true;
-  int grid_tiles = 0, grid_faces = 0;
+  int grid_tiles = 0, grid_faces = 0, face_blocks = 0;
   int streams = 0;  // PHONO_BATCH_STREAMS: per-instance launches on this many worker streams
   std::vector<cudaStream_t> workers;
   std::vector<cudaEvent_t> joins;
@@ -1626,9 +1627,15 @@ static int batch_rebuild(phono_batch* b) {
     }
     prefix.push_back(fb);
     finst.push_back(s);
-    fb += (h->faces.off[12] + 255) / 256;
+    if (!writes_faces(b->precision == PHONO_F32K, b->tj, h->d.ny)) fb += (h->faces.off[12] + 255) / 256;
   }
   prefix.push_back(fb);
+  const int grid_faces = fb ? b->face_blocks : 0;  // no face launch where the tiles write the faces
+  if (grid_faces != b->grid_faces) {
+    b->grid_faces = grid_faces;
+    if (b->graph) cudaGraphExecDestroy(b->graph);  // captured with or without it
+    b->graph = nullptr;
+  }
   if ((int)items.size() > b->item_cap) {
     int cap = std::max<int>((int)items.size(), 2 * b->item_cap);
     void* p = nullptr;
@@ -1809,7 +1816,7 @@ int phono_batch_create(int capacity, int precision, int tile_j, phono_batch** ou
   BTRYC(cudaGetDevice(&dev));
   BTRYC(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
   b->grid_tiles = std::max(1, bps) * nsm;
-  b->grid_faces = 8 * nsm;
+  b->face_blocks = 8 * nsm;
 #undef BTRY
 #undef BTRYC
   *out = b;

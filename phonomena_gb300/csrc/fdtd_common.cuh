@@ -37,6 +37,11 @@ constexpr int MKW = 48;     // material tile width in k (bytes): k0-8 .. k0+40
 constexpr int TAB_ROWS_MAX = 256;  // material rows a table may hold (uint8 ids)
 constexpr int BATCH_TAB_ROWS = 32;  // material rows of a batched instance
 
+constexpr int VEC_TJ = 8;         // the FP32 tile pass is the vectorised one from this tile height on
+// It writes the face points itself (no face launch) on meshes with no row next
+// to two y faces, and at the height whose halo warp has the time.
+__host__ __device__ constexpr bool writes_faces(bool f32, int tj, int ny) { return f32 && tj >= 16 && ny >= 5; }
+
 template <class R>
 struct Lay;
 template <>

@@ -253,7 +253,7 @@ struct SmemPlan {
 // height 4 one updating warp does not pay for the halo warp (256x256x128
 // cells: 192 us a step against 154 with one row a thread).
 template <class S, int TJ>
-__host__ __device__ constexpr bool vec_tile() { return sizeof(typename S::R) == 4 && TJ >= 8; }
+__host__ __device__ constexpr bool vec_tile() { return sizeof(typename S::R) == 4 && TJ >= VEC_TJ; }
 
 #include "tile_rows.cuh"
 #include "tile_vec.cuh"
@@ -334,10 +334,11 @@ cudaError_t configure_step(int tj) {
 
 // separate_faces: 0 one fused launch (face points in extra blocks), 1 the tile
 // launch then the face launch; 2 only the tile launch and 3 only the face
-// launch of the separate form (phono_time_kernels times them apart)
+// launch of the separate form (phono_time_kernels times them apart).  No face
+// launch where the tile pass writes the faces.
 template <class S, int TJ>
 static cudaError_t launch_tj(const StepArgs<typename S::R>& a, int separate_faces, cudaStream_t st) {
-  const int nfaces = a.faces.off[12];
+  const int nfaces = writes_faces(sizeof(typename S::R) == 4, TJ, a.g.ny) ? 0 : a.faces.off[12];
   constexpr int NT = step_threads<S, TJ>();
   dim3 block(TK, NT / TK);
   // fused: face points handled by extra blocks of the same launch
@@ -426,7 +427,7 @@ static cudaError_t batch_launch_tj(const BatchArgs<typename S::R>& ba, int grid_
                                    cudaStream_t st) {
   batch_step_kernel<S, TJ>
       <<<grid_tiles, dim3(TK, step_threads<S, TJ>() / TK), step_smem<S, TJ>(BATCH_TAB_ROWS), st>>>(ba);
-  batch_face_kernel<S><<<grid_faces, 256, 0, st>>>(ba);
+  if (grid_faces > 0) batch_face_kernel<S><<<grid_faces, 256, 0, st>>>(ba);
   return cudaGetLastError();
 }
 

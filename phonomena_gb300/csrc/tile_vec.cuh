@@ -21,17 +21,30 @@
 //      ux of plane i will need.
 // Segment ends need only T1 of the first plane behind them.
 //
-// Bound by DRAM traffic on large meshes (512x512x256 cells: 805 us a step,
-// 6.16 TB/s of the 73 bytes a node, 90% of the measured copy bandwidth), and by
+// The face points are written here too (meshes of TILE_FACES_NY rows and
+// more).  The halo warp of a block with a row next to y = 0 or y = N evaluates
+// that face's points of plane i-1 from the new state the block has just
+// written: it reads it behind the barrier of iteration i and uses it before
+// the next one.  The x = N points come after the last plane, from the threads
+// of the rows.  A face launch of its own costs 4 to 5 us a step (with it and
+// without, us a step: 512x512x256 cells 805 / 778, 256x256x128 122 / 118,
+// 160x128x64 25.8 / 24.5); the same from the registers of the updating threads
+// made their loop slower for every block (256x256x128: 138).  At height 8 the
+// halo warp has half the time for it, and the launch is the better one (12
+// crystals in a persistent batch 174 us a step with it, 208 without).
+//
+// Bound by DRAM traffic on large meshes (512x512x256 cells: 778 us a step,
+// 6.37 TB/s of the 73 bytes a node, 94% of the measured copy bandwidth), and by
 // the latency of a plane (1.7 us for a block alone) with the ramp and tail of
 // the launch on small ones.  The form before it, one node a thread with all
 // stresses exchanged through shared memory and two barriers a plane, issued
 // 507 instructions a node against 220 here and was bound by that.  Rows start
 // on 128-byte lines, so that a row of the tile's state is one line for the
 // copies in and for the stores (87 bytes of DRAM traffic a node when rows
-// started 32 bytes into a line, 80 now).  us a step, best tiles before, this
-// form, with aligned rows: 512x512x256 1043 / 850 / 805, 256x256x128 154 / 138
-// / 128, 193x161x97 80 / 66 / 63, 160x128x64 39.5 / 31 / 26.
+// started 32 bytes into a line, 80 now).  us a step, best tiles of the form
+// before, this form, with aligned rows, now: 512x512x256 1043 / 850 / 805 /
+// 778, 256x256x128 154 / 138 / 128 / 118, 193x161x97 80 / 66 / 63 / 59,
+// 160x128x64 39.5 / 31 / 26 / 24.5.
 // Included inside namespace phono, after the TMA helpers and the schemes.
 #pragma once
 
@@ -75,6 +88,38 @@ __device__ __forceinline__ void store_vec(const Roles<float>& r, int c, unsigned
   *reinterpret_cast<float4*>(r.out(c) + o) = make_float4(u[0], u[1], u[2], u[3]);
   *reinterpret_cast<float4*>(r.vout(c) + o) = make_float4(v[0], v[1], v[2], v[3]);
   *reinterpret_cast<float4*>(r.cout(c) + o) = make_float4(kc[0], kc[1], kc[2], kc[3]);
+}
+
+// Four points of a face row, or of a row next to one, of component c: plane p,
+// row j, from z = k on.
+struct FaceRow {
+  float v[4], v4;  // old values (uz of plane 0: the source), and the one above
+  __device__ __forceinline__ void read(const StepArgs<float>& a, const Roles<float>& r, const float s, int c, int p, int j, int k) {
+    const float* src = r.cur(c) + fidx(a.g, p, j, k);
+    const float4 t = *reinterpret_cast<const float4*>(src);
+    v[0] = t.x, v[1] = t.y, v[2] = t.z, v[3] = t.w, v4 = src[4];
+    if (c == 2 && p == 0) {  // source overwrite (base_solver.py:251)
+      if (a.source_mode == 1) v[0] = v[1] = v[2] = v[3] = v4 = s;
+      else if (k == 0) v[0] = s;
+    }
+  }
+  // u: new values of the points; stored with the z = N point above them
+  __device__ __forceinline__ void write(const StepArgs<float>& a, const Roles<float>& r, int tt, int c, int p, int j, int k,
+                                        float (&u)[4]) const {
+    if (c == 2 && k == 0) record(a, tt, p, j, u[0]);
+    float vn[4] = {0.f, 0.f, 0.f, 0.f}, cn[4] = {0.f, 0.f, 0.f, 0.f};
+    store_vec(r, c, (unsigned)fidx(a.g, p, j, k), (c == 2 ? a.g.nz - 3 : a.g.nz - 2) - k, a.bc == 1, c == 2 ? a.abc[7] : a.abc[6],
+              v, v4, u, vn, cn);
+  }
+  // new values from those of the next row inward, `in` and its old values
+  __device__ __forceinline__ void face(const StepArgs<float>& a, const float f, const float (&in)[4], const FaceRow& old,
+                                       float (&u)[4]) const {
+#pragma unroll
+    for (int q = 0; q < 4; q++) u[q] = a.bc == 1 ? 0.f : F32K::abc(f, in[q], v[q], old.v[q]);
+  }
+};
+__device__ __forceinline__ float y_face_coef(const StepArgs<float>& a, int c, int dj) {
+  return dj < 0 ? a.abc[c == 1 ? 3 : 2] : a.abc[c == 1 ? 5 : 4];
 }
 
 template <int TJ>
@@ -188,6 +233,33 @@ __device__ __forceinline__ bool tile_block_vec(const StepArgs<float>& a, unsigne
     const int u_top = (TJ + 1) * KW + KB + lane, u_bot = KB + lane, u_col = (l + 1) * KW + KB - 1, u_right = u_col + 1 + TK;
     const int m_top = (TJ + 1) * MKW + MKOFF + lane, m_bot = MKW + MKOFF + lane;
     const int m_t4c = (l + 2) * MKW + MKOFF, m_t5c = (l + 1) * MKW + MKOFF, m_right = m_t5c + TK;
+    // y faces: a lane takes four points of a component's row next to y = 0 or,
+    // from the end, y = N; a tile with both does the second on the spot
+    const int fc = lane >> 3, fk = k0 + 4 * (lane & 7), f_hi = ny - 2 - (fc == 1 ? 1 : 0);
+    const bool f_on = writes_faces(true, TJ, ny) && fc < 3 && fk <= nz - 2, hi = f_on && f_hi >= j0 && f_hi < j0 + TJ;
+    const int fd = !f_on ? 0 : j0 == 0 ? -1 : hi ? 1 : 0, fj = fd < 0 ? 1 : f_hi;
+    float fn[4];
+    FaceRow f_in, f_out;
+    auto face_read = [&](int p, int j, int dj) {
+      const float4 t = *reinterpret_cast<const float4*>(r.out(fc) + fidx(g, p, j, fk));
+      fn[0] = t.x, fn[1] = t.y, fn[2] = t.z, fn[3] = t.w;
+      f_in.read(a, r, s, fc, p, j, fk);
+      f_out.read(a, r, s, fc, p, j + dj, fk);
+    };
+    auto face_write = [&](int p, int j, int dj) {
+      float u[4];
+      f_out.face(a, y_face_coef(a, fc, dj), fn, f_in, u);
+      f_out.write(a, r, tt, fc, p, j + dj, fk, u);
+    };
+    // plane p's points, their values read before; then those of the other face
+    auto face_rows = [&](int p, bool read) {
+#pragma unroll 1
+      for (int j = fj, dj = fd; dj; read = true) {
+        if (read) face_read(p, j, dj);
+        face_write(p, j, dj);
+        dj = dj < 0 && hi ? 1 : 0, j = f_hi;
+      }
+    };
     float xt_m = 0.f, xr_m = 0.f;  // ux one plane back at u_top, u_right
     {
       const float* U = uring;
@@ -237,6 +309,7 @@ __device__ __forceinline__ bool tile_block_vec(const StepArgs<float>& a, unsigne
             xr_m = x;
           }
         }
+        if (fd && i >= ib + 2) face_rows(i - 2, false);
       }
       // The slot of plane i is refilled by TMA (async proxy) after the
       // barrier: order this thread's reads of it first (a barrier orders
@@ -250,10 +323,14 @@ __device__ __forceinline__ bool tile_block_vec(const StepArgs<float>& a, unsigne
         issue(i + 3, s0);
         issued = i + 3;
       }
+      if (fd && i > ib) face_read(i - 1, fj, fd);  // plane i-1 is complete
       s0 = s1;
       if (++s1 == NS) s1 = 0, par ^= 1;
       advance(i);
     }
+    if (ok && fd && ie - ib >= 2) face_rows(ie - 2, false);
+    __syncthreads();  // the last plane is written
+    if (ok && fd && !(fc == 0 && ie == nx - 1)) face_rows(ie - 1, true);  // ux ends at plane nx-2, its x = N face
   } else {
     // ---------------- updating warps ----------------
     const int lr = lane >> 3, lc = lane & 7, jl = 4 * warp + lr, j = j0 + jl, k = k0 + 4 * lc;
@@ -493,6 +570,31 @@ __device__ __forceinline__ bool tile_block_vec(const StepArgs<float>& a, unsigne
       }
       update_x(ie, t1, pwring + s0 * P::PWS, qx, fx_prev);
     }
+    // x = N (with its y = 0, y = N and z = N edges): the rows of the plane next
+    // to it, as written above (ux of plane nx-3 may be the segment before's)
+    if (ok && ie >= nx - 2 && row && writes_faces(true, TJ, ny)) {
+#pragma unroll 1
+      for (int c = 0; c < 3; c++) {
+        if (c == 1 && !row_y) continue;
+        const int p = c == 0 ? nx - 3 : nx - 2;
+        if (p < ib || p >= ie) continue;
+        const float4 t = *reinterpret_cast<const float4*>(r.out(c) + fidx(g, p, j, k));
+        const float un[4] = {t.x, t.y, t.z, t.w};
+        FaceRow in, out, edge_old;
+        in.read(a, r, s, c, p, j, k);
+        out.read(a, r, s, c, p + 1, j, k);
+        const int dj = j == 1 ? -1 : j == ny - 2 - (c == 1 ? 1 : 0) ? 1 : 0;
+        float u[4], w[4];
+        out.face(a, a.abc[c == 0 ? 0 : 1], un, in, u);
+        if (dj) {
+          edge_old.read(a, r, s, c, p + 1, j + dj, k);
+          edge_old.face(a, y_face_coef(a, c, dj), u, out, w);
+          edge_old.write(a, r, tt, c, p + 1, j + dj, k, w);
+        }
+        out.write(a, r, tt, c, p + 1, j, k, u);
+      }
+    }
+    __syncthreads();  // see the halo warp
   }
   if (!ok && producer) {
     // A wait ran out: flag it and drain the copies this block issued, so that
