@@ -46,12 +46,12 @@ def parse():
     p.add_argument("--warmup", type=int, default=3)
     p.add_argument("--impl", default="ours", choices=["ours", "reference"])
     p.add_argument("--workload", default="crystal", choices=["crystal", "batch", "serve", "precision"],
-                   help="crystal: the 256x256x128 crystal (default); batch: 64 uneven crystals in one persistent "
-                        "launch; serve: Poisson request stream; precision: 1024x1024x256 FP32K vs FP64 error")
+                   help="crystal: the 256x256x128 crystal (default); batch: 64 uneven crystals stepped "
+                        "together; serve: Poisson request stream; precision: 1024x1024x256 FP32K vs FP64 error")
     p.add_argument("--fdtd-steps", type=int, default=None)
     p.add_argument("--instances", type=int, default=64)
     p.add_argument("--batch-streams", type=int, default=64,
-                   help="batch and serving: worker streams of the streams batch scheme (0: the persistent scheme only)")
+                   help="batch and serving: worker streams of the streams batch scheme (0: the default scheme only)")
     p.add_argument("--requests", type=int, default=2000, help="serve: FP32K requests")
     p.add_argument("--rate", type=float, default=0.0, help="serve: FP32K arrivals per second (0: 70%% load)")
     p.add_argument("--requests-f64", type=int, default=40, help="serve: plain FP64 requests")
@@ -129,10 +129,12 @@ class ClockSampler:
                 "power_w_max": max((float(r[3]) for r in rows if r[3].replace(".", "").isdigit()), default=None)}
 
 
-def graph_launches(nsteps, separate_faces=True):
-    """Kernels launched by phono_step(nsteps): per step the tile pass and the
-    face pass, plus one step-counter update per 12-step graph and remainder."""
-    per = 2 if separate_faces else 1
+def graph_launches(nsteps, tile_j, ny):
+    """Kernels launched by phono_step(nsteps) of an FP32 simulation: per step
+    the tile pass (heights 16 and 0, the default, write the faces too; the
+    other heights need a face pass unless ny is 3), plus one step-counter
+    update per 12-step graph and remainder."""
+    per = 2 if ny == 4 or (ny > 4 and tile_j not in (0, 16)) else 1
     full, rem = divmod(nsteps, GRAPH_CHUNK)
     return full * (per * GRAPH_CHUNK + 1) + per * rem + (1 if rem else 0)
 
@@ -164,12 +166,10 @@ def traffic_per_node(kernel):
     return d.get(kernel, {}).get("dram_bytes_per_node")
 
 
-def traffic_bounds(scheme, nodes):
-    """DRAM bytes per batch step bounded from the committed ncu summary where
-    the scheme's traffic is not observable directly (streams: ncu serialises
-    the side-by-side launches); None for the persistent scheme."""
-    if scheme == "persistent":
-        return None
+def traffic_bounds(nodes):
+    """DRAM bytes per batch step bounded from the committed ncu summary: the
+    traffic is not observable directly (ncu serialises the side-by-side
+    launches)."""
     p = ROOT / "profiles" / "traffic.json"
     if not p.exists():
         return None
@@ -282,10 +282,9 @@ def reference_arm(args, rank, world):
 def bench_batch(args, rank, world, local, torch, dist):
     """64 uneven seeded crystals (sizes {64..192}^2 x {32..96} cells, a in
     {8,12,16}, f ~ U[20, 60] MHz), 1500 steps each, FP32 Kahan, with a
-    graph-captured step loop, in both batch schemes: one persistent tile
-    launch per time step, and every instance's own kernels on worker streams;
-    tile height and per-instance x segments from the batch autotuner for
-    each.  The faster scheme is the line's value.  One bench step = the whole
+    graph-captured step loop, in both batch schemes (every instance's own
+    kernels on worker streams; tiles picked by the batch, or tile height and
+    per-instance x segments from the batch autotuner).  The faster scheme is the line's value.  One bench step = the whole
     batch from the zero state to its last step."""
     from phonomena_gb300 import autotune, crystal
     from phonomena_gb300.batch import Batch
@@ -318,7 +317,7 @@ def bench_batch(args, rank, world, local, torch, dist):
             b.remove(q)
         return ms
 
-    schemes = {"persistent": 0}
+    schemes = {"default": 0}
     if args.batch_streams > 0:
         schemes["streams"] = args.batch_streams
     timed = {}
@@ -429,7 +428,7 @@ def bench_batch(args, rank, world, local, torch, dist):
     launch_ms = ms / (args.steps * S)
     hbm_peak, peak_kind = measured_peaks()
     achieved = BYTES_PER_NODE * node_sum / (launch_ms / 1e3) / 1e9
-    tpn = traffic_per_node("batch_step_kernel_f32k" if scheme == "persistent" else "fdtd_step_kernel_f32k_batch")
+    tpn = traffic_per_node("fdtd_step_kernel_f32k_batch")
     if rank == 0:
         line = {
             "metric": "Gcell-updates/s", "value": round(value, 4), "unit": "Gcell-updates/s", "n_gpus": world,
@@ -462,19 +461,15 @@ def bench_batch(args, rank, world, local, torch, dist):
             "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": hbm_peak, "unit": "GB/s",
                          "frac": round(achieved / hbm_peak, 4), "peak_kind": peak_kind,
                          "traffic": (round(tpn * node_sum) if tpn else None),
-                         "traffic_bounds_per_launch": traffic_bounds(scheme, node_sum),
+                         "traffic_bounds_per_launch": traffic_bounds(node_sum),
                          "algorithmic_bytes_per_launch": BYTES_PER_NODE * node_sum,
                          "avg_launch_ms": round(launch_ms, 5),
-                         "launch_timing": ("one time step = persistent tile launch + batched face launch "
-                                           "(+1/12 counter update)" if scheme == "persistent" else
-                                           "one time step = every instance's tile and face launches on the worker "
-                                           "streams (+1/12 counter update)")
-                                          + "; the whole step is charged to the stencil kernel"},
+                         "launch_timing": "one time step = every instance's launches on the worker streams (+1/12 "
+                                          "counter update); the whole step is charged to the stencil kernel"},
             "cpu_baseline": None,
             "e2e": {"value": round(e2e, 4), "unit": "Gcell-updates/s", "h2d_bytes_per_step": int(h2d),
                     "d2h_bytes_per_step": int(d2h)},
-            "gpu_launches": (graph_launches(S, True) if scheme == "persistent"
-                             else len(specs) * 2 * S + -(-S // GRAPH_CHUNK)) * args.steps,
+            "gpu_launches": sum(graph_launches(S, 0 if scheme == "default" else tj, sp.nodes[1]) for sp in specs) * args.steps,
             "clocks": clocks,
         }
         print(json.dumps(line), flush=True)
@@ -564,7 +559,7 @@ def serve_study(args, rank):
     rate64 = serve.rate_for_load(SERVE_GCELL["f64"], 0.7)
     out["fp64"].append(serve_summary(serve_stream("f64", args.serve_requests_f64, rate64, rank + 1000,
                                                   args.budget_gb, streams=args.batch_streams), 0.7))
-    out["batch_scheme"] = "streams" if args.batch_streams > 0 else "persistent"
+    out["batch_scheme"] = "streams" if args.batch_streams > 0 else "default"
     return out
 
 
@@ -701,7 +696,6 @@ def main():
 
     # ---- FP32 Kahan: device-resident throughput ----
     sim = DeviceSimulation(sp, m.ids, m.table, m.dt, precision="f32k", **kw("f32k"))
-    separate_faces = g.y.size >= 4
     sim.set_source(src)
     stream = torch.cuda.ExternalStream(sim.stream_ptr)
     for _ in range(args.warmup):
@@ -863,13 +857,13 @@ def main():
                          "face_launch_ms": round(face_ms / KT, 5),
                          "whole_step": {"ms": round(step_ms, 5), "achieved": round(step_achieved, 1),
                                         "frac": round(step_achieved / hbm_peak, 4),
-                                        "note": "graph-replayed step of the timed region: tile + face launch "
-                                                "(+1/12 counter update), all charged to the stencil"}},
+                                        "note": "graph-replayed step of the timed region: all its launches "
+                                                "(+1/12 counter update) charged to the stencil"}},
             "tile": list(shapes["f32k"]),
             "cpu_baseline": cpu,
             "e2e": {"value": round(e2e, 4), "unit": "Gcell-updates/s", "h2d_bytes_per_step": int(h2d),
                     "d2h_bytes_per_step": int(d2h)},
-            "gpu_launches": graph_launches(S, separate_faces) * args.steps,
+            "gpu_launches": graph_launches(S, shapes["f32k"][0], g.y.size) * args.steps,
             "clocks": clocks,
             "precision_config3": prec3,
             "serve": served,

@@ -299,33 +299,29 @@ typedef struct phono_energy_dense {
 
 int phono_energy_static(const phono_energy_dense *in, double *out_dev, void *stream);
 
-/* Batches: many simulations stepped together.  In the default (persistent)
- * scheme every time step is one persistent tile launch (CTAs pull (instance,
- * tile) work items until none are left) and one face launch for all active
- * instances, replayed from a captured CUDA graph; phono_batch_set_mode
- * selects the other scheme.  The reference runs one simulation per solver
- * object (base_solver.py:245-266) and has no counterpart; the per-instance
- * arithmetic is that of phono_step, bit for bit.  Instances are handles made
- * by phono_create with the batch's precision and ny >= 4 (and the batch's
- * tile_j in the persistent scheme); each keeps its own x segments, cut
- * shorter where the persistent launch would have fewer than three items a
- * block.  While a handle is in a batch, phono_step, phono_reset, phono_set_materials,
- * phono_upload and phono_set_tiling on it return PHONO_ERR_STATE; call
- * phono_batch_sync before reading it.  A handle destroyed while in a batch
- * leaves the batch. */
+/* Batches: many simulations stepped together.  Every instance runs its own
+ * step kernels on a worker stream, so that instances run side by side; each
+ * replays its own graph of 12 steps (captured when it joins) and starts its
+ * next chunk as soon as its previous one is done.  phono_batch_step returns
+ * once every worker's work is queued, and the batch stream waits for all of
+ * them.  In the default scheme the batch has up to 64 workers and FP32
+ * instances step in tiles that it picks for all of them;
+ * phono_batch_set_mode selects the other scheme.  The reference runs one
+ * simulation per solver object (base_solver.py:245-266) and has no
+ * counterpart; the per-instance arithmetic is that of phono_step, bit for
+ * bit.  Instances are handles made by phono_create with the batch's precision
+ * and ny >= 4 (and the batch's tile_j in the default scheme).  While a handle
+ * is in a batch, phono_step, phono_reset, phono_set_materials, phono_upload
+ * and phono_set_tiling on it return PHONO_ERR_STATE; call phono_batch_sync
+ * before reading it.  A handle destroyed while in a batch leaves the batch. */
 typedef struct phono_batch phono_batch;
 
 int phono_batch_create(int capacity, int precision, int tile_j, phono_batch **out);
-/* Launch scheme of an empty batch (PHONO_ERR_STATE once it holds an
- * instance).  PHONO_BATCH_PERSISTENT (the default): the persistent tile
- * launch above, every instance at the batch's tile_j.  PHONO_BATCH_STREAMS:
- * every instance runs its own step kernels (those of phono_step, with its own
- * tile_j and x segments) on one of `streams` worker streams (1..256), so that
- * instances run side by side.  Each instance replays its own graph of 12
- * steps (captured when it joins) and starts its next chunk as soon as its
- * previous one is done; phono_batch_step returns once every worker's work is
- * queued and the batch stream waits for all of them.  Results are those of
- * phono_step in both schemes. */
+/* Scheme of an empty batch (PHONO_ERR_STATE once it holds an instance).
+ * PHONO_BATCH_PERSISTENT: the default one above (the name is that of the
+ * kernel it once launched).  PHONO_BATCH_STREAMS: `streams` worker streams
+ * (1..256), instances of any tile_j, and those made with a tile shape keep
+ * it.  Results are those of phono_step in both. */
 #define PHONO_BATCH_PERSISTENT 0
 #define PHONO_BATCH_STREAMS 1
 int phono_batch_set_mode(phono_batch *b, int mode, int streams);

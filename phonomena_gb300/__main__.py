@@ -25,7 +25,7 @@ def main(argv=None):
     p.add_argument("--x-segments", default="", help="explicit x segment lengths, comma separated (phono_set_segments)")
     p.add_argument("--batch", type=int, default=0, help="run this many crystals of the batching mix instead")
     p.add_argument("--batch-streams", type=int, default=0,
-                   help="with --batch: worker streams of the streams scheme (0: the persistent kernel)")
+                   help="with --batch: worker streams of the streams scheme (0: the default scheme)")
     p.add_argument("--seed", type=int, default=0)
     a = p.parse_args(argv)
 

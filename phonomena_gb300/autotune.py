@@ -7,9 +7,8 @@ that shape (CUDA events around a chunk of steps from the zero state;
 (0, 0) means the default.
 
 ``tune_batch``: for a mix of mesh shapes stepped as one batch it picks the
-batch's tile height and each instance's x segment, i.e. how many
-(instance, tile) work items every instance contributes to the persistent
-launch.  Stage 1 times the whole mix for every tile height and one common
+batch's tile height and each instance's x segment (in the default scheme FP32
+instances step in tiles of the batch's choice, whatever these are).  Stage 1 times the whole mix for every tile height and one common
 x segment; stage 2 revisits the x segment of each group of instances with
 the same x extent, keeping a change only when the whole batch gets faster.
 
@@ -172,7 +171,7 @@ def tune_batch(shapes, precision="f32k", steps=24, tile_js=TILE_J, use_cache=Tru
     """Tile height of a batch and the x segment of each instance.
 
     shapes: mesh node counts (nx, ny, nz) of the instances, in batch order.
-    streams: 0 times the persistent scheme, W > 0 the streams scheme on W
+    streams: 0 times the default scheme, W > 0 the streams scheme on W
     worker streams (every instance at the chosen tile height).
     Returns (tile_j, [x_segment per instance]).
     """
@@ -198,7 +197,7 @@ def tune_batch(shapes, precision="f32k", steps=24, tile_js=TILE_J, use_cache=Tru
         with Batch(len(sims), precision=precision, tile_j=tj, streams=streams) as b:
             for sim in sims:
                 b.add(sim, steps + 12)
-            b.step(12)  # work list upload, graph capture
+            b.step(12)  # graph capture
             b.sync()
             b.step(steps)
             ms = b.last_step_ms() / steps

@@ -1,21 +1,18 @@
 """Many simulations stepped together (phono_batch_* of include/phono.h).
 
 A ``Batch`` holds up to ``capacity`` device simulations of one arithmetic
-scheme.  Two launch schemes:
+scheme.  Every instance runs its own step kernels on a worker stream, so that
+the instances' launches run side by side on the GPU; each instance replays
+its own 12-step graph (captured when it joins) and does not wait for the
+others between chunks.  Two schemes:
 
-* persistent (``streams=0``, the default): every instance at the batch's
-  tile height; each time step is one persistent tile launch in which the
-  CTAs pull (instance, tile) work items, costliest instances first, plus one
-  face launch for all instances;
-* streams (``streams=W``): every instance runs its own step kernels, with
-  its own tile height and x segments, on one of W worker streams, so that
-  the instances' launches run side by side on the GPU; each instance
-  replays its own 12-step graph (captured when it joins) and does not wait
-  for the others between chunks.
+* ``streams=0``, the default: up to 64 workers; FP32 instances step in tiles
+  the batch picks from what all of them amount to, whatever shape they were
+  made with (their ``tile_j`` has to be the batch's);
+* ``streams=W``: W workers; an instance made with a tile shape keeps it.
 
-Chunks of 12 steps are replayed from captured CUDA graphs.  Instances
-keep their own step counters and budgets, so a batch can hold simulations of
-different sizes at different points of their runs, and instances can join
+Instances keep their own step counters and budgets, so a batch can hold
+simulations of different sizes at different points of their runs, and instances can join
 and leave between calls.  Results are those of stepping each alone.
 """
 from __future__ import annotations

@@ -20,9 +20,6 @@ cudaError_t configure_step_f64v(int tj);
 cudaError_t launch_step_f64v(const StepArgs<double>& a, int tj, int n_face_blocks, cudaStream_t st);
 cudaError_t launch_split(int precision, const void* args, bool stress, bool after_kernel, cudaStream_t st);
 cudaError_t launch_energy(const EnergyArgs& a, double2* partial, int nblocks, double* out, bool pairs, cudaStream_t st);
-cudaError_t batch_step_any(int precision, const void* ba, int tj, int grid_tiles, int grid_faces, cudaStream_t st);
-cudaError_t batch_advance_any(int precision, const void* ba, int n_active_cap, int n, cudaStream_t st);
-cudaError_t batch_configure_any(int precision, int tj, int* blocks_per_sm);
 cudaError_t launch_lattice_ids(uint8_t* mat, const Geo& g, int pitch, int ncx, int ncy, const double* radius,
                                const uint8_t* kind, int depth, uint8_t host, cudaStream_t st);
 cudaError_t launch_inclusion_ids(uint8_t* mat, const Geo& g, const double* x, const double* y, const double4* incl,
@@ -94,7 +91,9 @@ struct phono_handle {
   double* energy_out = nullptr;
   double abc[8] = {};
   Tiling t;                    // the tile shape the caller knows
-  Tiling own;                  // a default handle's own shape for its single steps (own.tj 0: t)
+  Tiling own;                  // a default handle's own shape (own.tj 0: t)
+  int own_limit = 0;           // longest segment of it in a batch (0: alone)
+  bool lent = false;           // not a default handle: own is its batch's choice
   int n_face = 0, separate_faces = 1;
   FaceTable faces{};
   // two-launch step (split_step.cu): stress window of `win` planes (0: this
@@ -102,7 +101,7 @@ struct phono_handle {
   // the velocity forms' v and Kahan terms then stay in buffer 0
   int win = 0, tsy = 0;
   bool split = false;
-  bool resplit = false;        // in a persistent batch (tile pass): back to the two-launch form when it leaves
+  bool resplit = false;        // in a batch (tile pass): back to the two-launch form when it leaves
   char* stress = nullptr;      // leapfrog: the window
   SoftRec* rec = nullptr;      // leapfrog: table entries as records, 16 per material
   int shared = 0;              // leapfrog: the normal stresses share terms (split_step.cu)
@@ -645,6 +644,13 @@ static int set_tiling(phono_handle* h, int tj, int xseg) {
   return apply_tiling(h, h->t, tj, xseg, segment_starts(h->d.nx - 1, xseg));
 }
 
+static int sm_count() {
+  int dev = 0, nsm = 152;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  cudaGetLastError();
+  return nsm;
+}
+
 // Segments that keep the resident blocks busy to the end: every wave of blocks
 // takes segments of one length, the last the shortest, since blocks of equal
 // length that share the memory bandwidth drift apart and leave it idle at the
@@ -675,14 +681,11 @@ static std::vector<double> wave_lengths(double depth, int waves, double shortest
 // than three segments fill a wave, even ones of about 12 planes (a segment
 // reads two planes more than it updates; long ones let neighbouring blocks
 // drift apart until their common halo rows have left L2: 512x512x256 cells 802
-// us at 12 planes, 917 at 57).  Beside other instances (a streams batch) there
-// is no last wave to fill: even segments of at most 24 planes (12 crystals of
-// 6.2 M nodes in all: 120 us a step, 163 with each instance's single-run
-// segments).
-static int own_tiling(phono_handle* h, bool alone) {
-  int dev = 0, nsm = 152;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  cudaGetLastError();
+// us at 12 planes, 917 at 57). Beside other
+// instances (a batch) there is no last wave to fill: even segments of at most
+// `limit` planes (0: alone), see batch_rebuild.
+static int own_tiling(phono_handle* h, int limit) {
+  const int nsm = sm_count();
   const int planes = h->d.nx - 1, rows = h->d.ny - 1;
   const long long r16 = round_up(rows, 16), r8 = round_up(rows, 8);
   const int tj = r16 > r8 + r8 / 2 ? 8 : 16;
@@ -692,8 +695,8 @@ static int own_tiling(phono_handle* h, bool alone) {
     for (int q = 0; q <= nseg; q++) starts.push_back((int)((long long)planes * q / nseg));
   };
   const int fill = (int)std::min<long long>(wave / tiles, planes);  // segments that fill a wave
-  if (!alone) {
-    even((planes + 23) / 24);
+  if (limit) {
+    even((planes + limit - 1) / limit);
   } else if (fill >= 3) {
     double at = 0;
     starts.push_back(0);
@@ -809,7 +812,7 @@ int phono_create(const phono_desc* d, phono_handle** out) {
   // tiles: the shape the caller knows by default is height 4 for FP32, 8 for
   // FP64, and 24 planes per segment
   int rt = set_tiling(h, d->tile_j ? d->tile_j : (d->precision == PHONO_F32K ? 4 : 8), d->x_segment ? d->x_segment : 24);
-  if (!rt && d->precision == PHONO_F32K && !d->tile_j && !d->x_segment) rt = own_tiling(h, true);
+  if (!rt && d->precision == PHONO_F32K && !d->tile_j && !d->x_segment) rt = own_tiling(h, 0);
   if (rt) {
     std::string m_ = g_err;
     delete h;
@@ -1429,33 +1432,21 @@ void phono_destroy(phono_handle* h) { release(h); }
 // ---------------------------------------------------------------------------
 struct phono_batch {
   int cap = 0, precision = 0, tj = 8;
-  size_t inst_size = 0;  // sizeof(StepArgs<R>)
-  std::vector<void*> allocs;
-  char* d_inst = nullptr;
-  int2* d_items = nullptr;
-  int item_cap = 0;
-  int* d_counts = nullptr;  // items, face blocks, face entries, active instances
-  unsigned* d_ticket = nullptr;
-  int* d_face_prefix = nullptr;
-  int* d_face_inst = nullptr;
-  int* d_active = nullptr;
   std::vector<phono_handle*> slot;
   std::vector<int> remaining;
   cudaStream_t stream = nullptr;
-  cudaGraphExec_t graph = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   bool timed = false, dirty = true;
-  int grid_tiles = 0, grid_faces = 0, face_blocks = 0;
-  int streams = 0;  // PHONO_BATCH_STREAMS: per-instance launches on this many worker streams
+  int streams = 0;  // PHONO_BATCH_STREAMS: this many workers, every instance in its own shape; 0: the default scheme
   std::vector<cudaStream_t> workers;
   std::vector<cudaEvent_t> joins;
   cudaEvent_t fork = nullptr;
   std::vector<int> order;     // active slots, costliest first
   std::vector<int> step_end;  // per slot: the instance's budget end
-  std::vector<int> cut;       // persistent scheme, per slot: segment limit its device arguments were written with (-1: none)
-  std::vector<cudaGraphExec_t> igraph;  // streams scheme: per slot, 12 steps with its budget baked in
-  cudaStream_t capture = nullptr;       // streams scheme: capture stream (always idle)
+  std::vector<cudaGraphExec_t> igraph;  // per slot, 12 steps with its budget baked in
+  cudaStream_t capture = nullptr;       // capture stream (always idle)
 };
+constexpr int kBatchWorkers = 64;  // worker streams of the default scheme, at most one an instance
 
 static void drop_igraph(phono_batch* b, int s) {
   if (s < (int)b->igraph.size() && b->igraph[s]) {
@@ -1477,12 +1468,13 @@ static void batch_detach(phono_batch* b, const phono_handle* h) {
     }
 }
 
-// a default FP32 handle's tiles for single steps or for steps beside others
-static int reshape_own(phono_handle* h, bool alone) {
-  if (!h->own.tj) return PHONO_OK;
-  int rc = own_tiling(h, alone);
+// a default FP32 handle's tiles for single steps (0) or, with segments of at
+// most `limit` planes, for steps beside others
+static int reshape_own(phono_handle* h, int limit) {
+  h->own_limit = limit;
+  int rc = own_tiling(h, limit);
   if (!rc) rc = encode_tensor_maps(h, h->own);
-  if (h->graph) {
+  if (h->graph && !h->lent) {  // (a lent shape's is that of t)
     cudaGraphExecDestroy(h->graph);
     h->graph = nullptr;
   }
@@ -1492,7 +1484,8 @@ static int reshape_own(phono_handle* h, bool alone) {
 // the batch's work is done: the handle is on its own again
 static cudaError_t leave_batch(phono_handle* h) {
   h->batch = nullptr;
-  reshape_own(h, true);
+  if (h->lent) h->own = Tiling{}, h->lent = false;
+  if (h->own.tj) reshape_own(h, 0);
   if (!h->resplit) return cudaSuccess;
   h->resplit = false;
   return set_split(h, true);
@@ -1503,10 +1496,8 @@ static void batch_release(phono_batch* b) {
   if (b->stream) cudaStreamSynchronize(b->stream);
   for (phono_handle* h : b->slot)
     if (h) leave_batch(h);
-  if (b->graph) cudaGraphExecDestroy(b->graph);
   for (cudaGraphExec_t g : b->igraph)
     if (g) cudaGraphExecDestroy(g);
-  for (void* p : b->allocs) cudaFree(p);
   if (b->ev0) cudaEventDestroy(b->ev0);
   if (b->ev1) cudaEventDestroy(b->ev1);
   for (cudaEvent_t e : b->joins) cudaEventDestroy(e);
@@ -1517,148 +1508,63 @@ static void batch_release(phono_batch* b) {
   delete b;
 }
 
-static int balloc(phono_batch* b, void** p, size_t bytes) {
-  cudaError_t e = cudaMalloc(p, bytes);
-  if (e != cudaSuccess) {
-    *p = nullptr;
-    return fail(PHONO_ERR_NOMEM, std::string("cudaMalloc ") + std::to_string(bytes) + " bytes: " + cudaGetErrorString(e));
-  }
-  b->allocs.push_back(*p);
-  return PHONO_OK;
-}
-
-// BatchArgs over the batch's device tables (same layout for float and double)
-static BatchArgs<float> batch_args(const phono_batch* b, int step_off) {
-  BatchArgs<float> ba{};
-  ba.inst = reinterpret_cast<const StepArgs<float>*>(b->d_inst);
-  ba.items = b->d_items;
-  ba.counts = b->d_counts;
-  ba.ticket = b->d_ticket;
-  ba.face_prefix = b->d_face_prefix;
-  ba.face_inst = b->d_face_inst;
-  ba.active = b->d_active;
-  ba.step_off = step_off;
-  return ba;
-}
-static_assert(sizeof(BatchArgs<float>) == sizeof(BatchArgs<double>), "batch argument layouts differ");
 static_assert(PHONO_MAX_SEGMENTS == SEG_TABLE, "segment list limit and the kernel table differ");
 
-// a handle's tiles with every x segment cut evenly to at most `limit` planes (0: as they are)
-static Tiling cut_segments(const phono_handle* h, int limit) {
-  Tiling t = h->t;
-  if (!limit) return t;
-  const int planes = h->d.nx - 1;
-  std::vector<int> starts{0};
-  for (int q = 0, p = 0; q < t.nseg; q++) {
-    const int end = t.nseg <= SEG_TABLE ? t.seg_start[q + 1] : std::min(planes, p + t.xseg);
-    const int n = (end - p + limit - 1) / limit;
-    for (int c = 1; c <= n; c++) starts.push_back(p + (int)((long long)(end - p) * c / n));
-    p = end;
-  }
-  if ((int)starts.size() - 1 > SEG_TABLE) starts = segment_starts(planes, limit);  // even: beyond the table
-  t.xseg = limit;
-  t.n_tile = t.n_tile / t.nseg * ((int)starts.size() - 1);
-  t.nseg = (int)starts.size() - 1;
-  t.seg_start = starts;
-  return t;
-}
-
-// device arguments of the instance in slot s
-static int write_instance(phono_batch* b, int s, const Tiling& t) {
-  const phono_handle* h = b->slot[s];
-  char* dst = b->d_inst + (size_t)s * b->inst_size;
-  if (b->precision == PHONO_F32K) {
-    StepArgs<float> a = make_args<float>(h, t, 0);
-    a.step_end = b->step_end[s];
-    CK(cudaMemcpy(dst, &a, sizeof a, cudaMemcpyHostToDevice));
-  } else {
-    StepArgs<double> a = make_args<double>(h, t, 0);
-    a.step_end = b->step_end[s];
-    CK(cudaMemcpy(dst, &a, sizeof a, cudaMemcpyHostToDevice));
+// worker streams: as many as asked for, kept for the batch's lifetime
+static int need_workers(phono_batch* b, int want) {
+  if (!b->fork) CK(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming));
+  if (!b->capture) CK(cudaStreamCreateWithFlags(&b->capture, cudaStreamNonBlocking));
+  while ((int)b->workers.size() < want) {
+    cudaStream_t w = nullptr;
+    cudaEvent_t j = nullptr;
+    CK(cudaStreamCreateWithFlags(&w, cudaStreamNonBlocking));
+    cudaError_t e = cudaEventCreateWithFlags(&j, cudaEventDisableTiming);
+    if (e != cudaSuccess) {
+      cudaStreamDestroy(w);
+      return fail(PHONO_ERR_CUDA, std::string("cudaEventCreateWithFlags: ") + cudaGetErrorString(e));
+    }
+    b->workers.push_back(w);
+    b->joins.push_back(j);
   }
   return PHONO_OK;
 }
 
-// work items (costliest instances first), face-block prefix, active list
+// The active instances, the most node updates left first (each instance's
+// chunks are queued before the next one's), and the segment length of those
+// that pick their own tiles: as many blocks in all as stay resident (three an
+// SM), in segments of 3 to 24 planes.  A step of a small batch is the march of
+// one block (6 crystals of 55 k nodes: 15 us a step in segments of 3 planes,
+// 53 in 24), while a large one pays for the planes that segments share (24
+// crystals of 1.2 M nodes: 552 us in segments of 4 planes, 432 in 24).  An
+// instance's segments are cut anew, and its graph captured again, when the
+// length has changed by more than a factor of two.
 static int batch_rebuild(phono_batch* b) {
   std::vector<int> act;
+  double planes = 0;  // of all tile columns
   for (int s = 0; s < b->cap; s++)
-    if (b->slot[s] && b->remaining[s] > 0) act.push_back(s);
-  // persistent scheme: the largest instances' work items first (the tail of
-  // each step launch); streams scheme: the most remaining work first (node
-  // updates left), each instance's chunks queued before the next one's
+    if (b->slot[s] && b->remaining[s] > 0) {
+      act.push_back(s);
+      const phono_handle* h = b->slot[s];
+      const Tiling& t = h->own.tj ? h->own : h->t;
+      planes += (double)t.ntj * t.ntk * (h->d.nx - 1);
+    }
   auto cost = [&](int x) {
     const phono_handle* h = b->slot[x];
-    return b->streams ? (long long)h->d.nx * h->d.ny * h->d.nz * b->remaining[x] : (long long)h->t.n_tile;
+    return (long long)h->d.nx * h->d.ny * h->d.nz * b->remaining[x];
   };
   std::sort(act.begin(), act.end(), [&](int x, int y) {
     const long long cx = cost(x), cy = cost(y);
     return cx != cy ? cx > cy : x < y;
   });
-  b->order = act;
-  if (b->streams) {  // the instances' own launches: no work list
-    b->dirty = false;
-    return PHONO_OK;
-  }
-  std::vector<int2> items;
-  std::vector<int> prefix, finst;
-  int fb = 0;
-  // With fewer than three items a block, segments are cut
-  // to 12 planes, so that no block is left with a long one at the end of the
-  // launch (12 crystals of 6.2 M nodes, tiles of height 8: 184 us a step
-  // against 240 with their segments of 32 planes; 24 crystals of 29 M nodes
-  // fill the launch and stay at 730).
-  long long own_items = 0;
-  for (int s : act) own_items += b->slot[s]->t.n_tile;
-  const int limit = own_items < 3LL * b->grid_tiles ? 12 : 0;
-  for (int s : act)
-    if (b->cut[s] != limit) {
-      CK(cudaStreamSynchronize(b->stream));  // launches that read the old arguments
-      break;
-    }
+  const int limit = (int)std::min(std::max(planes / (3.0 * sm_count()), 3.0), 24.0);
   for (int s : act) {
-    const phono_handle* h = b->slot[s];
-    const Tiling t = cut_segments(h, limit);
-    for (int q = 0; q < t.n_tile; q++) items.push_back(make_int2(s, q));
-    if (b->cut[s] != limit) {
-      int rc = write_instance(b, s, t);
-      if (rc) return rc;
-      b->cut[s] = limit;
-    }
-    prefix.push_back(fb);
-    finst.push_back(s);
-    if (!writes_faces(b->precision == PHONO_F32K, b->tj, h->d.ny)) fb += (h->faces.off[12] + 255) / 256;
-  }
-  prefix.push_back(fb);
-  const int grid_faces = fb ? b->face_blocks : 0;  // no face launch where the tiles write the faces
-  if (grid_faces != b->grid_faces) {
-    b->grid_faces = grid_faces;
-    if (b->graph) cudaGraphExecDestroy(b->graph);  // captured with or without it
-    b->graph = nullptr;
-  }
-  if ((int)items.size() > b->item_cap) {
-    int cap = std::max<int>((int)items.size(), 2 * b->item_cap);
-    void* p = nullptr;
-    int rc = balloc(b, &p, (size_t)cap * sizeof(int2));
+    phono_handle* h = b->slot[s];
+    if (!h->own.tj || h->split || (h->own_limit && limit <= 2 * h->own_limit && h->own_limit <= 2 * limit)) continue;
+    int rc = reshape_own(h, limit);
     if (rc) return rc;
-    b->d_items = (int2*)p;
-    b->item_cap = cap;
-    if (b->graph) {  // the captured launches hold the old pointer
-      cudaGraphExecDestroy(b->graph);
-      b->graph = nullptr;
-    }
+    drop_igraph(b, s);
   }
-  int counts[4] = {(int)items.size(), fb, (int)finst.size(), (int)act.size()};
-  if (!items.empty())
-    CK(cudaMemcpyAsync(b->d_items, items.data(), items.size() * sizeof(int2), cudaMemcpyHostToDevice, b->stream));
-  CK(cudaMemcpyAsync(b->d_face_prefix, prefix.data(), prefix.size() * sizeof(int), cudaMemcpyHostToDevice, b->stream));
-  if (!finst.empty()) {
-    CK(cudaMemcpyAsync(b->d_face_inst, finst.data(), finst.size() * sizeof(int), cudaMemcpyHostToDevice, b->stream));
-    CK(cudaMemcpyAsync(b->d_active, act.data(), act.size() * sizeof(int), cudaMemcpyHostToDevice, b->stream));
-  }
-  CK(cudaMemcpyAsync(b->d_counts, counts, sizeof counts, cudaMemcpyHostToDevice, b->stream));
-  CK(cudaMemsetAsync(b->d_ticket, 0, sizeof(unsigned), b->stream));
-  CK(cudaStreamSynchronize(b->stream));  // host vectors go out of scope
+  b->order = act;
   b->dirty = false;
   return PHONO_OK;
 }
@@ -1670,17 +1576,7 @@ static cudaError_t chain_launch(phono_batch* b, int s, int step_off, cudaStream_
   return tile_step(h, step_off, b->step_end[s], h->separate_faces, st);
 }
 
-static cudaError_t batch_launch_steps(phono_batch* b, int first_off, int n) {
-  for (int s = 0; s < n; s++) {
-    BatchArgs<float> ba = batch_args(b, first_off + s);
-    cudaError_t e = batch_step_any(b->precision, &ba, b->tj, b->grid_tiles, b->grid_faces, b->stream);
-    if (e != cudaSuccess) return e;
-  }
-  BatchArgs<float> ba = batch_args(b, 0);
-  return batch_advance_any(b->precision, &ba, b->cap, n, b->stream);
-}
-
-// Streams scheme: the 12-step graph of the instance in slot s (its own step
+// The 12-step graph of the instance in slot s (its own step
 // kernels, as phono_step launches them, and a step-counter update clamped at
 // its budget), captured on the batch's idle capture stream
 static int capture_instance(phono_batch* b, int s) {
@@ -1703,14 +1599,14 @@ static int capture_instance(phono_batch* b, int s) {
   return PHONO_OK;
 }
 
-// Streams scheme: n steps of every active instance.  Instance q (costliest
+// n steps of every active instance.  Instance q (costliest
 // first) runs on worker q mod W; the host issues chunk by chunk (a 12-step
 // instance graph each, then the remainder step by step) across the instances
 // so that the workers progress together, and joins the workers back into the
 // batch stream only after the last chunk: an instance's next chunk starts as
 // soon as its previous one is done, whatever the others are doing.
 static cudaError_t streams_steps(phono_batch* b, int n) {
-  const int na = (int)b->order.size(), nw = std::min(na, b->streams);
+  const int na = (int)b->order.size(), nw = std::min(na, (int)b->workers.size());
   cudaError_t e = cudaEventRecord(b->fork, b->stream);
   for (int w = 0; w < nw && e == cudaSuccess; w++) e = cudaStreamWaitEvent(b->workers[w], b->fork, 0);
   const int full = n / kGraphSteps, rem = n % kGraphSteps;
@@ -1737,31 +1633,6 @@ static cudaError_t streams_steps(phono_batch* b, int n) {
   return e;
 }
 
-// Persistent scheme: 12-step graphs of the batch-wide launches (captured
-// once: the launches read the work list from device memory), then the
-// remainder step by step
-static int persistent_steps(phono_batch* b, int nsteps) {
-  if (!b->graph && nsteps >= kGraphSteps) {
-    cudaGraph_t g = nullptr;
-    CK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-    cudaError_t e = batch_launch_steps(b, 0, kGraphSteps);
-    cudaError_t e2 = cudaStreamEndCapture(b->stream, &g);
-    if (e != cudaSuccess || e2 != cudaSuccess) {
-      if (g) cudaGraphDestroy(g);
-      return fail(PHONO_ERR_CUDA, std::string("batch graph capture: ") + cudaGetErrorString(e != cudaSuccess ? e : e2));
-    }
-    e = cudaGraphInstantiate(&b->graph, g, 0);
-    cudaGraphDestroy(g);
-    if (e != cudaSuccess) return fail(PHONO_ERR_CUDA, std::string("cudaGraphInstantiate: ") + cudaGetErrorString(e));
-  }
-  CK(cudaEventRecord(b->ev0, b->stream));
-  const int full = nsteps / kGraphSteps, rem = nsteps % kGraphSteps;
-  for (int q = 0; q < full; q++) CK(cudaGraphLaunch(b->graph, b->stream));
-  if (rem) CK(batch_launch_steps(b, 0, rem));
-  CK(cudaEventRecord(b->ev1, b->stream));
-  return PHONO_OK;
-}
-
 extern "C" {
 
 int phono_batch_create(int capacity, int precision, int tile_j, phono_batch** out) {
@@ -1776,22 +1647,10 @@ int phono_batch_create(int capacity, int precision, int tile_j, phono_batch** ou
   b->cap = capacity;
   b->precision = precision;
   b->tj = tile_j;
-  b->inst_size = precision == PHONO_F32K ? sizeof(StepArgs<float>) : sizeof(StepArgs<double>);
   b->slot.assign(capacity, nullptr);
   b->remaining.assign(capacity, 0);
   b->step_end.assign(capacity, 0);
-  b->cut.assign(capacity, -1);
   b->igraph.assign(capacity, nullptr);
-#define BTRY(x)              \
-  do {                       \
-    int r_ = (x);            \
-    if (r_) {                \
-      std::string m_ = g_err; \
-      batch_release(b);      \
-      g_err = m_;            \
-      return r_;             \
-    }                        \
-  } while (0)
 #define BTRYC(x)                                                                      \
   do {                                                                                \
     cudaError_t e_ = (x);                                                             \
@@ -1803,21 +1662,6 @@ int phono_batch_create(int capacity, int precision, int tile_j, phono_batch** ou
   BTRYC(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking));
   BTRYC(cudaEventCreate(&b->ev0));
   BTRYC(cudaEventCreate(&b->ev1));
-  BTRY(balloc(b, (void**)&b->d_inst, b->inst_size * capacity));
-  BTRY(balloc(b, (void**)&b->d_counts, sizeof(int) * 4));
-  BTRY(balloc(b, (void**)&b->d_ticket, sizeof(unsigned)));
-  BTRY(balloc(b, (void**)&b->d_face_prefix, sizeof(int) * (capacity + 1)));
-  BTRY(balloc(b, (void**)&b->d_face_inst, sizeof(int) * capacity));
-  BTRY(balloc(b, (void**)&b->d_active, sizeof(int) * capacity));
-  BTRYC(cudaMemset(b->d_counts, 0, sizeof(int) * 4));
-  BTRYC(cudaMemset(b->d_ticket, 0, sizeof(unsigned)));
-  int bps = 0, dev = 0, nsm = 0;
-  BTRYC(batch_configure_any(precision, tile_j, &bps));
-  BTRYC(cudaGetDevice(&dev));
-  BTRYC(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-  b->grid_tiles = std::max(1, bps) * nsm;
-  b->face_blocks = 8 * nsm;
-#undef BTRY
 #undef BTRYC
   *out = b;
   return PHONO_OK;
@@ -1831,24 +1675,10 @@ int phono_batch_set_mode(phono_batch* b, int mode, int streams) {
   for (phono_handle* h : b->slot)
     if (h) return fail(PHONO_ERR_STATE, "the launch scheme of a batch is set while it is empty");
   CK(cudaStreamSynchronize(b->stream));
-  if (b->graph) {
-    cudaGraphExecDestroy(b->graph);
-    b->graph = nullptr;
-  }
   const int want = mode == PHONO_BATCH_STREAMS ? streams : 0;
-  if (!b->fork && want) CK(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming));
-  if (!b->capture && want) CK(cudaStreamCreateWithFlags(&b->capture, cudaStreamNonBlocking));
-  while ((int)b->workers.size() < want) {  // worker streams are kept for the batch's lifetime
-    cudaStream_t w = nullptr;
-    cudaEvent_t j = nullptr;
-    CK(cudaStreamCreateWithFlags(&w, cudaStreamNonBlocking));
-    cudaError_t e = cudaEventCreateWithFlags(&j, cudaEventDisableTiming);
-    if (e != cudaSuccess) {
-      cudaStreamDestroy(w);
-      return fail(PHONO_ERR_CUDA, std::string("cudaEventCreateWithFlags: ") + cudaGetErrorString(e));
-    }
-    b->workers.push_back(w);
-    b->joins.push_back(j);
+  if (want) {
+    int rc = need_workers(b, want);
+    if (rc) return rc;
   }
   b->streams = want;
   b->dirty = true;
@@ -1871,19 +1701,33 @@ int phono_batch_add(phono_batch* b, phono_handle* h, int nsteps) {
     if (s < 0 && !b->slot[q]) s = q;
   }
   if (s < 0) return fail(PHONO_ERR_NOMEM, "batch is full");
-  if (b->streams && reshape_own(h, false)) return PHONO_ERR_ARG;
-  // the persistent launch is a tile pass; beside others FP32's two launches
-  // only move more bytes (12 crystals: 120 us a step, 142 with the small ones split)
-  if (h->split && (!b->streams || b->precision == PHONO_F32K)) {
+  if (!b->streams) {
+    int members = 1;
+    for (const phono_handle* x : b->slot) members += x != nullptr;
+    int rc = need_workers(b, std::min(members, kBatchWorkers));
+    if (rc) return rc;
+  }
+  // beside others FP32's two launches only move more bytes (12 crystals: 120 us
+  // a step, 142 with the small ones split)
+  if (h->split && b->precision == PHONO_F32K) {
     CK(set_split(h, false));
     h->resplit = true;
   }
+  // In the default scheme FP32 instances step in tiles of the batch's choice
+  // (12 crystals of 6.2 M nodes: 98 us a step, 108 at height 8, 177 in one
+  // launch a step whose blocks took tiles of all instances from a list).
+  if (!h->own.tj && !b->streams && b->precision == PHONO_F32K) {
+    int rc = own_tiling(h, 24);
+    if (rc) return rc;
+    CK(configure_step_f32k(h->own.tj));
+    h->lent = true;
+  }
+  h->own_limit = 0;  // cut with the next work list
   CK(cudaStreamSynchronize(h->stream));
   CK(cudaStreamSynchronize(b->stream));
   b->slot[s] = h;
   b->remaining[s] = nsteps;
   b->step_end[s] = h->steps_done + nsteps;
-  b->cut[s] = -1;  // its device arguments are written with the next work list
   b->dirty = true;
   h->batch = b;
   return s;
@@ -1915,20 +1759,15 @@ int phono_batch_step(phono_batch* b, int nsteps) {
     int rc = batch_rebuild(b);
     if (rc) return rc;
   }
-  if (b->streams) {
-    if (nsteps >= kGraphSteps)
-      for (int s : b->order)
-        if (!b->igraph[s]) {
-          int rc = capture_instance(b, s);
-          if (rc) return rc;
-        }
-    CK(cudaEventRecord(b->ev0, b->stream));
-    CK(streams_steps(b, nsteps));
-    CK(cudaEventRecord(b->ev1, b->stream));
-  } else {
-    int rc = persistent_steps(b, nsteps);
-    if (rc) return rc;
-  }
+  if (nsteps >= kGraphSteps)
+    for (int s : b->order)
+      if (!b->igraph[s]) {
+        int rc = capture_instance(b, s);
+        if (rc) return rc;
+      }
+  CK(cudaEventRecord(b->ev0, b->stream));
+  CK(streams_steps(b, nsteps));
+  CK(cudaEventRecord(b->ev1, b->stream));
   b->timed = true;
   for (int s = 0; s < b->cap; s++) {
     if (!b->slot[s] || b->remaining[s] <= 0) continue;

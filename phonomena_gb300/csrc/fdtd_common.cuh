@@ -127,20 +127,6 @@ struct StepArgs {
   int skip_plane;
 };
 
-// Batched launch: many instances (each a StepArgs in device memory) share one
-// persistent tile launch and one face launch per step.
-template <class R>
-struct BatchArgs {
-  const StepArgs<R>* inst;  // [capacity] per-instance arguments
-  const int2* items;        // (instance, tile) work items, costliest first
-  const int* counts;        // [0] work items, [1] face blocks, [2] entries of face_prefix
-  unsigned* ticket;         // work-item counter; returns to 0 after every launch
-  const int* face_prefix;   // first face block of each listed instance (+ total)
-  const int* face_inst;     // instance of each listed entry
-  const int* active;        // [counts[3]] active instances (step-counter update)
-  int step_off;             // offset of this launch inside a captured chunk of steps
-};
-
 // arguments of the energy reduction (energy.cu)
 struct EnergyArgs {
   Geo g;

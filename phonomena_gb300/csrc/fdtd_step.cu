@@ -31,8 +31,6 @@
 //         Kahan-compensated displacement sum; explicit fmaf only.
 //  F64V - the F32K scheme in FP64.
 //
-// Batches (batch_step_kernel and friends) run the same tile pass over the
-// (instance, tile) work items of many instances in one persistent launch.
 #include <cstdio>
 #include "scheme.cuh"
 
@@ -260,11 +258,11 @@ __host__ __device__ constexpr bool vec_tile() { return sizeof(typename S::R) == 
 
 // the tile pass of one block
 template <class S, int TJ>
-__device__ __forceinline__ bool run_tile(const StepArgs<typename S::R>& a, unsigned char* base,
+__device__ __forceinline__ void run_tile(const StepArgs<typename S::R>& a, unsigned char* base,
                                          const Roles<typename S::R>& r, const typename S::R s, const int tt,
-                                         const int tid, const int b, const StepArgs<typename S::R>* maps) {
-  if constexpr (vec_tile<S, TJ>()) return tile_block_vec<TJ>(a, base, r, s, tt, tid, b, maps);
-  else return tile_block_rows<S, TJ>(a, base, r, s, tt, tid, b, maps);
+                                         const int tid, const int b) {
+  if constexpr (vec_tile<S, TJ>()) tile_block_vec<TJ>(a, base, r, s, tt, tid, b);
+  else tile_block_rows<S, TJ>(a, base, r, s, tt, tid, b);
 }
 
 // ---------------------------------------------------------------------------
@@ -272,10 +270,10 @@ __device__ __forceinline__ bool run_tile(const StepArgs<typename S::R>& a, unsig
 // ---------------------------------------------------------------------------
 // Resident blocks per SM the register allocation is made for (measured on
 // GB300 for the 256x256x128 crystal and the 64-crystal batch).  FP32: tile
-// height 4, 6 blocks of 128 threads (up to 85 registers); heights 8 and 16
-// (two rows a thread), 4 blocks of 128 or 2 of 256 threads (up to 128
-// registers).  FP64: 16 warps per SM.
-template <class R, int TJ, bool BATCH = false>
+// height 4, 6 blocks of 128 threads (up to 85 registers); heights 8 and 16, 5
+// blocks of 96 or 3 of 160 threads (up to 128 registers).  FP64: 16 warps per
+// SM.
+template <class R, int TJ>
 struct MinBlocks {
   static constexpr int value = sizeof(R) == 8 ? (TJ < 16 ? 16 / TJ : 1) : (TJ == 4 ? 6 : (TJ == 8 ? 5 : 3));
 };
@@ -310,7 +308,7 @@ __global__ void __launch_bounds__(step_threads<S, TJ>(), MinBlocks<typename S::R
   }
 
   // ---------------- tile blocks ----------------
-  run_tile<S, TJ>(a, base, r, s, tt, tid, blockIdx.x, &a);
+  run_tile<S, TJ>(a, base, r, s, tt, tid, blockIdx.x);
 }
 
 // ---------------------------------------------------------------------------
@@ -357,126 +355,6 @@ cudaError_t launch_step(const StepArgs<typename S::R>& a, int tj, int separate_f
     case 16: return launch_tj<S, 16>(a, separate_faces, st);
     default: return cudaErrorInvalidValue;
   }
-}
-
-// ---------------------------------------------------------------------------
-// batched instances: persistent tile kernel + face kernel + counter update
-// ---------------------------------------------------------------------------
-template <class S, int TJ>
-__global__ void __launch_bounds__(step_threads<S, TJ>(), MinBlocks<typename S::R, TJ, true>::value)
-    batch_step_kernel(const __grid_constant__ BatchArgs<typename S::R> ba) {
-  using R = typename S::R;
-  extern __shared__ __align__(128) unsigned char smem_raw[];
-  unsigned char* base = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);
-  __shared__ StepArgs<R> sa;  // the current item's instance arguments
-  __shared__ int item;
-  const int tid = threadIdx.y * TK + threadIdx.x;
-  const int n_items = __ldg(ba.counts);
-  for (;;) {
-    // each block takes items until one past the end; the counter wraps to 0
-    // after the last of the n_items + gridDim.x requests
-    if (tid == 0) item = (int)atomicInc(ba.ticket, (unsigned)(n_items + gridDim.x - 1));
-    __syncthreads();
-    const int it = item;
-    if (it >= n_items) break;
-    const int2 w = ba.items[it];
-    const int4* src4 = reinterpret_cast<const int4*>(ba.inst + w.x);
-    int4* dst4 = reinterpret_cast<int4*>(&sa);
-    for (int q = tid; q < (int)(sizeof(StepArgs<R>) / 16); q += step_threads<S, TJ>()) dst4[q] = src4[q];
-    __syncthreads();
-    const int tt = *sa.step_base + ba.step_off;
-    if (tt < sa.step_end) {
-      const Roles<R> r = roles<S>(sa, tt);
-      run_tile<S, TJ>(sa, base, r, (R)__ldg(sa.src + tt), tt, tid, w.y, ba.inst + w.x);
-    }
-    __syncthreads();  // sa and item are rewritten by the next iteration
-  }
-}
-
-template <class S>
-__global__ void __launch_bounds__(256) batch_face_kernel(const __grid_constant__ BatchArgs<typename S::R> ba) {
-  using R = typename S::R;
-  const int n_fb = __ldg(ba.counts + 1), n_ent = __ldg(ba.counts + 2);
-  for (int fb = blockIdx.x; fb < n_fb; fb += gridDim.x) {
-    int lo = 0, hi = n_ent - 1;  // last entry whose first block <= fb
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (__ldg(ba.face_prefix + mid) <= fb) lo = mid;
-      else hi = mid - 1;
-    }
-    const StepArgs<R>& a = ba.inst[__ldg(ba.face_inst + lo)];
-    const int tt = *a.step_base + ba.step_off;
-    if (tt >= a.step_end) continue;
-    const Roles<R> r = roles<S>(a, tt);
-    face_point<S>(a, r, (R)__ldg(a.src + tt), tt, (fb - __ldg(ba.face_prefix + lo)) * 256 + threadIdx.x, true);
-  }
-}
-
-// advance the step counter of every active instance by n, stopping at its budget
-template <class R>
-__global__ void batch_advance_kernel(const __grid_constant__ BatchArgs<R> ba, int n) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= __ldg(ba.counts + 3)) return;
-  const StepArgs<R>& a = ba.inst[__ldg(ba.active + q)];
-  int* c = const_cast<int*>(a.step_base);
-  *c = min(*c + n, a.step_end);
-}
-
-template <class S, int TJ>
-static cudaError_t batch_launch_tj(const BatchArgs<typename S::R>& ba, int grid_tiles, int grid_faces,
-                                   cudaStream_t st) {
-  batch_step_kernel<S, TJ>
-      <<<grid_tiles, dim3(TK, step_threads<S, TJ>() / TK), step_smem<S, TJ>(BATCH_TAB_ROWS), st>>>(ba);
-  if (grid_faces > 0) batch_face_kernel<S><<<grid_faces, 256, 0, st>>>(ba);
-  return cudaGetLastError();
-}
-
-template <class S>
-cudaError_t batch_step(const BatchArgs<typename S::R>& ba, int tj, int grid_tiles, int grid_faces, cudaStream_t st) {
-  switch (tj) {
-    case 4: return batch_launch_tj<S, 4>(ba, grid_tiles, grid_faces, st);
-    case 8: return batch_launch_tj<S, 8>(ba, grid_tiles, grid_faces, st);
-    case 16: return batch_launch_tj<S, 16>(ba, grid_tiles, grid_faces, st);
-    default: return cudaErrorInvalidValue;
-  }
-}
-
-template <class S, int TJ>
-static cudaError_t batch_configure_tj(int* blocks_per_sm) {
-  const int smem = (int)step_smem<S, TJ>(BATCH_TAB_ROWS);
-  cudaError_t e = cudaFuncSetAttribute(batch_step_kernel<S, TJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e != cudaSuccess) return e;
-  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, batch_step_kernel<S, TJ>, step_threads<S, TJ>(),
-                                                       smem);
-}
-
-template <class S>
-cudaError_t batch_configure(int tj, int* blocks_per_sm) {
-  switch (tj) {
-    case 4: return batch_configure_tj<S, 4>(blocks_per_sm);
-    case 8: return batch_configure_tj<S, 8>(blocks_per_sm);
-    case 16: return batch_configure_tj<S, 16>(blocks_per_sm);
-    default: return cudaErrorInvalidValue;
-  }
-}
-
-cudaError_t batch_step_any(int precision, const void* ba, int tj, int grid_tiles, int grid_faces, cudaStream_t st) {
-  if (precision == 0) return batch_step<F64>(*(const BatchArgs<double>*)ba, tj, grid_tiles, grid_faces, st);
-  if (precision == 2) return batch_step<F64V>(*(const BatchArgs<double>*)ba, tj, grid_tiles, grid_faces, st);
-  return batch_step<F32K>(*(const BatchArgs<float>*)ba, tj, grid_tiles, grid_faces, st);
-}
-
-cudaError_t batch_advance_any(int precision, const void* ba, int n_active_cap, int n, cudaStream_t st) {
-  const int blocks = (n_active_cap + 255) / 256;
-  if (precision == 1) batch_advance_kernel<float><<<blocks, 256, 0, st>>>(*(const BatchArgs<float>*)ba, n);
-  else batch_advance_kernel<double><<<blocks, 256, 0, st>>>(*(const BatchArgs<double>*)ba, n);
-  return cudaGetLastError();
-}
-
-cudaError_t batch_configure_any(int precision, int tj, int* blocks_per_sm) {
-  if (precision == 0) return batch_configure<F64>(tj, blocks_per_sm);
-  if (precision == 2) return batch_configure<F64V>(tj, blocks_per_sm);
-  return batch_configure<F32K>(tj, blocks_per_sm);
 }
 
 // non-template entry points for the C ABI translation unit

@@ -17,9 +17,9 @@
 #pragma once
 
 template <class S, int TJ>
-__device__ __forceinline__ bool tile_block_rows(const StepArgs<typename S::R>& a, unsigned char* base,
+__device__ __forceinline__ void tile_block_rows(const StepArgs<typename S::R>& a, unsigned char* base,
                                            const Roles<typename S::R>& r, const typename S::R s, const int tt,
-                                           const int tid, const int b, const StepArgs<typename S::R>* maps) {
+                                           const int tid, const int b) {
   using R = typename S::R;
   using P = SmemPlan<S, TJ>;
   using TF = TileShape<R, TJ>;
@@ -104,12 +104,12 @@ __device__ __forceinline__ bool tile_block_rows(const StepArgs<typename S::R>& a
     // plane that segment 0 loads): armed, no copy, so the wait on it runs out
     if (a.skip_plane >= 0 && p == a.skip_plane) return;
     // padded coordinates: k, j + 1, i + 1; the u tiles start at k0-KB (columns before 0: zeros), j0-1
-    tma_load_4d(uring + sl * SU, &maps->tm_u, k0 - KB, j0, p + 1, r.rcur * 3, &bars[sl]);
-    tma_load_3d(mring + sl * SM, &maps->tm_mat, k0, j0, p + 1, &bars[sl]);
+    tma_load_4d(uring + sl * SU, &a.tm_u, k0 - KB, j0, p + 1, r.rcur * 3, &bars[sl]);
+    tma_load_3d(mring + sl * SM, &a.tm_mat, k0, j0, p + 1, &bars[sl]);
     if (pw) {
       R* d = pwring + sl * P::PWS;
-      tma_load_4d(d, &maps->tm_pw0, k0, j0 + 1, p + 1, pw_buf, &bars[sl]);
-      if constexpr (S::kahan) tma_load_4d(d + 3 * P::PWC, &maps->tm_pw1, k0, j0 + 1, p + 1, pw_buf, &bars[sl]);
+      tma_load_4d(d, &a.tm_pw0, k0, j0 + 1, p + 1, pw_buf, &bars[sl]);
+      if constexpr (S::kahan) tma_load_4d(d + 3 * P::PWC, &a.tm_pw1, k0, j0 + 1, p + 1, pw_buf, &bars[sl]);
     }
   };
   bool ok = true;
@@ -515,13 +515,4 @@ __device__ __forceinline__ bool tile_block_rows(const StepArgs<typename S::R>& a
       }
     }
   }
-  // every issued plane has been waited for; the barriers may be set up
-  // again by the next tile of a persistent block, whose copies write the
-  // ring: order this thread's reads of it first (as before a refill)
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-  __syncthreads();
-  if (tid == 0)
-    for (int q = 0; q < NSLOT; q++) asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(smem_u32(&bars[q])) : "memory");
-  __syncthreads();
-  return ok;
 }

@@ -21,7 +21,7 @@
 //      ux of plane i will need.
 // Segment ends need only T1 of the first plane behind them.
 //
-// The face points are written here too (meshes of TILE_FACES_NY rows and
+// The face points are written here too (height 16, five rows of nodes and
 // more).  The halo warp of a block with a row next to y = 0 or y = N evaluates
 // that face's points of plane i-1 from the new state the block has just
 // written: it reads it behind the barrier of iteration i and uses it before
@@ -30,8 +30,9 @@
 // without, us a step: 512x512x256 cells 805 / 778, 256x256x128 122 / 118,
 // 160x128x64 25.8 / 24.5); the same from the registers of the updating threads
 // made their loop slower for every block (256x256x128: 138).  At height 8 the
-// halo warp has half the time for it, and the launch is the better one (12
-// crystals in a persistent batch 174 us a step with it, 208 without).
+// halo warp has half the time for it, and the launch is the better one (193x161x97
+// cells 62.5 us a step with it, 61.2 without, 12 crystals of 6.2 M nodes stepped
+// together 174 and 208).
 //
 // Bound by DRAM traffic on large meshes (512x512x256 cells: 778 us a step,
 // 6.37 TB/s of the 73 bytes a node, 94% of the measured copy bandwidth), and by
@@ -123,9 +124,8 @@ __device__ __forceinline__ float y_face_coef(const StepArgs<float>& a, int c, in
 }
 
 template <int TJ>
-__device__ __forceinline__ bool tile_block_vec(const StepArgs<float>& a, unsigned char* base, const Roles<float>& r,
-                                               const float s, const int tt, const int tid, const int b,
-                                               const StepArgs<float>* maps) {
+__device__ __forceinline__ void tile_block_vec(const StepArgs<float>& a, unsigned char* base, const Roles<float>& r,
+                                               const float s, const int tt, const int tid, const int b) {
   using P = VecPlan<TJ>;
   using S = F32K;
   constexpr int KW = P::KW, KB = P::KB, CW = P::CW, YO = CW, ZO = 2 * CW, NS = P::NS;
@@ -155,12 +155,12 @@ __device__ __forceinline__ bool tile_block_vec(const StepArgs<float>& a, unsigne
     mbar_expect_tx(&bars[sl], P::tx_bytes + (pw ? P::pw_bytes : 0u));
     // test hook (skip_plane >= 0; -1 is off): armed, no copy, so the wait on it runs out
     if (a.skip_plane >= 0 && p == a.skip_plane) return;
-    tma_load_4d(uring + sl * P::SU, &maps->tm_u, k0 - KB, j0, p + 1, sbuf, &bars[sl]);
-    tma_load_3d(mring + sl * P::SM, &maps->tm_mat, k0, j0, p + 1, &bars[sl]);
+    tma_load_4d(uring + sl * P::SU, &a.tm_u, k0 - KB, j0, p + 1, sbuf, &bars[sl]);
+    tma_load_3d(mring + sl * P::SM, &a.tm_mat, k0, j0, p + 1, &bars[sl]);
     if (pw) {
       float* d = pwring + sl * P::PWS;
-      tma_load_4d(d, &maps->tm_pw0, k0, j0 + 1, p, sbuf, &bars[sl]);
-      tma_load_4d(d + 3 * P::PWC, &maps->tm_pw1, k0, j0 + 1, p, sbuf, &bars[sl]);
+      tma_load_4d(d, &a.tm_pw0, k0, j0 + 1, p, sbuf, &bars[sl]);
+      tma_load_4d(d + 3 * P::PWC, &a.tm_pw1, k0, j0 + 1, p, sbuf, &bars[sl]);
     }
   };
   if (tid == 0) {
@@ -608,12 +608,4 @@ __device__ __forceinline__ bool tile_block_vec(const StepArgs<float>& a, unsigne
       mbar_wait(&bars[q % NS], (q / NS) & 1);
     }
   }
-  // every issued stage has been waited for; the barriers may be set up again
-  // by the next tile of a persistent block, whose copies write the ring
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-  __syncthreads();
-  if (tid == 0)
-    for (int q = 0; q < NS; q++) asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(smem_u32(&bars[q])) : "memory");
-  __syncthreads();
-  return ok;
 }

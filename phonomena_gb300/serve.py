@@ -4,8 +4,8 @@ Requests (a crystal to build, a step count, a surface-record interval) arrive
 over time.  One loop thread owns the GPU work: it admits waiting requests
 while a batch slot is free and their device footprint fits the memory budget,
 uploads their materials and source into device-resident simulations, steps
-every admitted simulation together in chunks of time steps (one persistent
-launch per step for the whole mix, ``phonomena_gb300.batch``), and at each
+every admitted simulation together in chunks of time steps
+(``phonomena_gb300.batch``), and at each
 chunk boundary streams out the surface traces of the requests that finished
 and frees their memory for the next ones.  Requests that arrive while others
 are on the GPU join the running batch at the next chunk boundary; each

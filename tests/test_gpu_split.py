@@ -128,10 +128,12 @@ def test_switching_forms_mid_run(gpu_lib, precision, tmp_path):
             assert np.array_equal(sim.download(k), w), k
 
 
-@pytest.mark.parametrize("precision", ["f64", "f32k"])
-def test_default_handles_through_a_persistent_batch(gpu_lib, precision):
-    """Odd step counts in, through and out of the persistent batch, whose tile
-    pass keeps v and the Kahan term in other buffers than the two-launch form."""
+@pytest.mark.parametrize("precision,shape", [("f64", {}), ("f32k", {}), ("f64v", {}), ("f32k", {"tile_j": 4, "x_segment": 8}),
+                                             ("f64", {"tile_j": 8, "x_segment": 8})])
+def test_handles_through_a_batch(gpu_lib, precision, shape):
+    """Odd step counts in, through and out of a batch, where FP32 handles take
+    other tiles, and the tile pass, which keeps v and the Kahan term in other
+    buffers than the two-launch form."""
     from phonomena_gb300.batch import Batch
     from phonomena_gb300.device import DeviceSimulation
 
@@ -139,7 +141,7 @@ def test_default_handles_through_a_persistent_batch(gpu_lib, precision):
     probs = [_problem(s, 7, 40) for s in ((21, 19, 37), (30, 12, 9))]
 
     def make(p):
-        sim = DeviceSimulation(p[0], p[1], TABLE, p[2], precision=precision, surface_mode="corrected", max_steps=40)
+        sim = DeviceSimulation(p[0], p[1], TABLE, p[2], precision=precision, surface_mode="corrected", max_steps=40, **shape)
         sim.set_source(p[3])
         return sim
 
@@ -163,3 +165,31 @@ def test_default_handles_through_a_persistent_batch(gpu_lib, precision):
                 for k in s.state_fields:
                     assert np.array_equal(s.download(k), ref.download(k)), (leave, k)
             s.close()
+
+
+def test_batch_that_grows(gpu_lib):
+    """A small instance whose segments are cut anew, in mid-run, when a large
+    one joins, and again when it has left."""
+    from phonomena_gb300.batch import Batch
+    from phonomena_gb300.device import DeviceSimulation
+
+    small, large = _problem((30, 21, 13), 2, 90), _problem((260, 250, 40), 3, 90)
+
+    def make(p):
+        sim = DeviceSimulation(p[0], p[1], TABLE, p[2], precision="f32k", surface_mode="corrected", max_steps=90)
+        sim.set_source(p[3])
+        return sim
+
+    with make(small) as a, make(large) as b, Batch(3, precision="f32k", tile_j=4) as batch:
+        batch.add(a, 77)
+        batch.step(25)
+        batch.add(b, 26)
+        batch.step(26)
+        batch.step(26)
+        batch.sync()
+        for sim, p, n in ((a, small, 77), (b, large, 26)):
+            with make(p) as ref:
+                ref.step(n)
+                ref.sync()
+                for k in sim.state_fields:
+                    assert np.array_equal(sim.download(k), ref.download(k)), (n, k)
