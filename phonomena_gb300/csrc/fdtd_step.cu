@@ -296,7 +296,10 @@ __global__ void __launch_bounds__(step_threads<S, TJ>(), MinBlocks<typename S::R
   unsigned char* base = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);
 
   const int tt = __ldg(a.step_base) + a.step_off;
-  if (tt >= a.step_end) return;  // a batched instance past its budget
+  if (tt >= a.step_end) {  // a batched instance past its budget
+    last_launch_done();
+    return;
+  }
   const Roles<R> r = roles<S>(a, tt);
   const R s = (R)__ldg(a.src + tt);
   const int tid = threadIdx.y * TK + threadIdx.x;
@@ -341,7 +344,21 @@ static cudaError_t launch_tj(const StepArgs<typename S::R>& a, int separate_face
   dim3 block(TK, NT / TK);
   // fused: face points handled by extra blocks of the same launch
   dim3 grid(a.n_tile_blocks + (separate_faces ? 0 : (nfaces + NT - 1) / NT));
-  if (separate_faces != 3) fdtd_step_kernel<S, TJ><<<grid, block, step_smem<S, TJ>(a.nmat), st>>>(a);
+  if (separate_faces != 3) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = step_smem<S, TJ>(a.nmat);
+    cfg.stream = st;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    // behind the tile launch of the step before, which wrote its faces too
+    cfg.numAttrs = separate_faces == 1 && nfaces == 0 && a.step_off > 0 ? 1 : 0;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, fdtd_step_kernel<S, TJ>, a);
+    if (e != cudaSuccess) return e;
+  }
   if ((separate_faces == 1 || separate_faces == 3) && nfaces > 0)
     fdtd_face_kernel<S><<<(nfaces + 255) / 256, 256, 0, st>>>(a);
   return cudaGetLastError();

@@ -357,4 +357,15 @@ __device__ __forceinline__ void record(const A& a, int tt, int i, int j, R val) 
   if (!isfinite(val)) atomicOr(a.err, 1);
 }
 
+// Programmatic launches: a launch may start (its index arithmetic and reads of
+// constants: material rows, spacings, the step counter, which changes between
+// chunks of launches only) once the blocks of the one ahead have ended or let
+// it, and waits here until that is complete before it touches the state.  The
+// state is read with plain loads from then on: it is not read-only over such a
+// launch's lifetime, as the non-coherent loads (__ldg) would need.  A block
+// that has nothing to do waits too: the launch behind it relies on this one
+// for all that came before.
+__device__ __forceinline__ void last_launch_done() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_next_launch() { asm volatile("griddepcontrol.launch_dependents;"); }
+
 }  // namespace phono

@@ -14,14 +14,6 @@ __device__ __forceinline__ SoftRec ldd(const SoftRec* p) {
 
 __device__ __forceinline__ int fdiv(int n, const FastDiv& f) { return (int)(__umulhi(2u * (unsigned)n, f.mult) >> f.shift); }
 
-// Programmatic launches: a launch may start (its index arithmetic and reads of
-// constants: material rows, spacings, the step counter, which changes between
-// chunks of launches only) once the blocks of the one ahead have ended, and
-// waits here until that is complete before it touches the state.  The state is
-// read with plain loads from then on: it is not read-only over such a launch's
-// lifetime, as the non-coherent loads (__ldg) would need.
-__device__ __forceinline__ void last_launch_done() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 // point n of an update launch: component and indices; whether it is next to a face
 template <class A>
 __device__ __forceinline__ bool update_point(const A& a, const Geo& g, int n, int& c, int& i, int& j, int& k) {

@@ -34,6 +34,12 @@
 // cells 62.5 us a step with it, 61.2 without, 12 crystals of 6.2 M nodes stepped
 // together 174 and 208).
 //
+// With the faces written here a step is one launch, and the next one is let in
+// when a block has finished its planes: its start (barriers, tables, spacings)
+// runs beside the last blocks of this one (whole runs without and with:
+// 160x128x64 cells, 300 steps 8.91 / 8.31 ms, 256x256x128, 360 steps 44.2 /
+// 43.7; let in at the start of a block, or one or two planes earlier, less).
+//
 // Bound by DRAM traffic on large meshes (512x512x256 cells: 778 us a step,
 // 6.37 TB/s of the 73 bytes a node, 94% of the measured copy bandwidth), and by
 // the latency of a plane (1.7 us for a block alone) with the ramp and tail of
@@ -168,6 +174,7 @@ __device__ __forceinline__ void tile_block_vec(const StepArgs<float>& a, unsigne
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
+  last_launch_done();
   int issued = ib - 2;  // last stage issued (halo warp's lane 0)
   const bool producer = halo && lane == 0;
   if (producer)
@@ -329,6 +336,7 @@ __device__ __forceinline__ void tile_block_vec(const StepArgs<float>& a, unsigne
       advance(i);
     }
     if (ok && fd && ie - ib >= 2) face_rows(ie - 2, false);
+    let_next_launch();
     __syncthreads();  // the last plane is written
     if (ok && fd && !(fc == 0 && ie == nx - 1)) face_rows(ie - 1, true);  // ux ends at plane nx-2, its x = N face
   } else {
@@ -534,7 +542,8 @@ __device__ __forceinline__ void tile_block_vec(const StepArgs<float>& a, unsigne
                                    S::sub(q < 3 ? t3[q < 3 ? q + 1 : 3] : t3k, t3[q]), q ? fdz[q] : uzc0);
           un[q] = update_value<S>(z0[q], Pw<float>{v[q], kc[q]}, dv, qz[q], a.dt, vn[q], cn[q]);
           if (i == 0) {  // z0 holds the source there: the state itself is in global memory
-            un[q] = row && k + q <= nz - 2 ? __ldg(r.cur(2) + o + q) : 0.f;
+            // (__ldcg: a plain load here costs registers, and the loop 4%)
+            un[q] = row && k + q <= nz - 2 ? __ldcg(r.cur(2) + o + q) : 0.f;
             vn[q] = v[q], cn[q] = kc[q];
           }
         }
@@ -570,6 +579,7 @@ __device__ __forceinline__ void tile_block_vec(const StepArgs<float>& a, unsigne
       }
       update_x(ie, t1, pwring + s0 * P::PWS, qx, fx_prev);
     }
+    let_next_launch();
     // x = N (with its y = 0, y = N and z = N edges): the rows of the plane next
     // to it, as written above (ux of plane nx-3 may be the segment before's)
     if (ok && ie >= nx - 2 && row && writes_faces(true, TJ, ny)) {
