@@ -18,7 +18,7 @@ ROOT = PKG.parent
 CSRC = PKG / "csrc"
 BUILD = PKG / "_build"
 LIB = BUILD / "libphono_gpu.so"
-SOURCES = ["fdtd_step.cu", "split_step.cu", "split_f32.cu", "energy.cu", "lattice.cu", "api.cu"]
+SOURCES = ["fdtd_step.cu", "split_step.cu", "split_f32.cu", "energy.cu", "lattice.cu", "readback.cu", "api.cu"]
 HEADERS = ["fdtd_common.cuh", "scheme.cuh", "split_common.cuh", "split_point.cuh", "soft_f64.cuh", "div_table.cuh", "tile_rows.cuh", "tile_vec.cuh"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 # No implicit FMA anywhere: device code uses explicit _rn intrinsics for the

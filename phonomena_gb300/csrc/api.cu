@@ -22,6 +22,8 @@ cudaError_t launch_split(int precision, const void* args, bool stress, bool afte
 cudaError_t launch_energy(const EnergyArgs& a, double2* partial, int nblocks, double* out, bool pairs, cudaStream_t st);
 cudaError_t launch_lattice_ids(uint8_t* mat, const Geo& g, int pitch, int ncx, int ncy, const double* radius,
                                const uint8_t* kind, int depth, uint8_t host, cudaStream_t st);
+cudaError_t launch_readback(const void* in, long long sx, long long sy, int ex, int ey, int ez, int es, void* out,
+                            cudaStream_t st);
 cudaError_t launch_inclusion_ids(uint8_t* mat, const Geo& g, const double* x, const double* y, const double4* incl,
                                  const int* kend, const uint8_t* id, int n, uint8_t host, cudaStream_t st);
 
@@ -520,9 +522,34 @@ static int check_desc(const phono_desc* d) {
   return PHONO_OK;
 }
 
+// fields from here on are read back into pinned memory by a kernel
+constexpr size_t kReadbackBytes = 128 << 10;
+
+// the device address of `bytes` bytes of pinned host memory at p; NULL where
+// it is any other memory
+static void* pinned_address(const void* p, size_t bytes) {
+  cudaPointerAttributes a{}, z{};
+  if (cudaPointerGetAttributes(&a, p) == cudaSuccess && a.type == cudaMemoryTypeHost && a.devicePointer &&
+      cudaPointerGetAttributes(&z, (const char*)p + bytes - 1) == cudaSuccess && z.type == cudaMemoryTypeHost &&
+      z.devicePointer == (char*)a.devicePointer + bytes - 1)
+    return a.devicePointer;
+  cudaGetLastError();
+  return nullptr;
+}
+
 // 3-D copy between a dense host array (ex, ey, ez) and the padded device layout
 static cudaError_t copy3d(phono_handle* h, void* dev, void* host, int c, bool to_dev) {
   int ex = h->d.nx - (c == 0), ey = h->d.ny - (c == 1), ez = h->d.nz - (c == 2);
+  // pinned memory is written by a kernel (readback.cu); pageable memory, an
+  // element off its own alignment and small fields take the strided copy (a run
+  // of 6500 nodes FP64, 58 KB a field: 1284 us, 1309 with the kernel)
+  const size_t bytes = (size_t)ex * ey * ez * h->es;
+  if (!to_dev && bytes >= kReadbackBytes && (uintptr_t)host % h->es == 0) {
+    if (void* to = pinned_address(host, bytes)) {
+      cudaError_t e = launch_readback((char*)dev + h->g.o0 * h->es, h->g.sx, h->g.sy, ex, ey, ez, h->es, to, h->stream);
+      return e == cudaSuccess ? cudaStreamSynchronize(h->stream) : e;
+    }
+  }
   cudaMemcpy3DParms p{};
   cudaPitchedPtr hp = make_cudaPitchedPtr(host, (size_t)ez * h->es, (size_t)ez * h->es, ey);
   cudaPitchedPtr dp = make_cudaPitchedPtr((char*)dev + h->g.o0 * h->es, (size_t)h->g.sy * h->es,
