@@ -57,6 +57,11 @@ static const int kEnergyBlocks = 1024;
 // ones FP64 takes less than the launches around it
 static const double kEnergyPairNodes = 200000;
 
+// the FP64 velocity form's two-launch step multiplies by constants in integer
+// arithmetic from here on (split_step.cu: 35 k nodes 9.5 us a step without and
+// 10.9 with it, 78 k nodes 13.9 and 13.4)
+static const double kSoftVelNodes = 60000;
+
 // tile decomposition of the tile pass and the TMA descriptors of its boxes
 struct Tiling {
   int tj = 0, xseg = 64, ntj = 0, ntk = 0, nseg = 0, n_tile = 0;
@@ -105,9 +110,9 @@ struct phono_handle {
   bool split = false;
   bool resplit = false;        // in a batch (tile pass): back to the two-launch form when it leaves
   char* stress = nullptr;      // leapfrog: the window
-  SoftRec* rec = nullptr;      // leapfrog: table entries as records, 16 per material
+  SoftRec* rec = nullptr;      // FP64: table entries as records, 16 per material
   int shared = 0;              // leapfrog: the normal stresses share terms (split_step.cu)
-  void* spd[6] = {};           // divisors of the two-launch step (records, or sp)
+  void* spd[6] = {};           // divisors of the two-launch step (FP64: records or factors, FP32: sp)
   double* vals = nullptr;      // leapfrog: values of all records
   cudaStream_t stream = nullptr;
   cudaGraphExec_t graph = nullptr;
@@ -215,15 +220,17 @@ static int upload_table(phono_handle* h, const double* table, int nmat, int id00
     t32.assign(t.begin(), t.end());
     CK(cudaMemcpyAsync(h->tab, t32.data(), t32.size() * 4, cudaMemcpyHostToDevice, h->stream));
   }
-  if (leapfrog) {  // the same entries for the two-launch step
+  if (h->rec) {  // the same entries for the two-launch step
+    for (size_t q = 0; q < t.size(); q++) rec.push_back(soft_record(t[q], false, (uint32_t)q));
+    CK(cudaMemcpyAsync(h->rec, rec.data(), rec.size() * sizeof(SoftRec), cudaMemcpyHostToDevice, h->stream));
+  }
+  if (leapfrog) {
     h->shared = 1;
     for (int m = 0; m < nmat; m++) {
       const double* c = table + m * PHONO_TABLE_COLS;
       auto same = [&](int p, int q) { return soft_bits(c[p]) == soft_bits(c[q]); };  // zeros with their signs
       h->shared &= same(3, 6) && same(1, 7) && same(2, 5);
     }
-    for (size_t q = 0; q < t.size(); q++) rec.push_back(soft_record(t[q], false, (uint32_t)q));
-    CK(cudaMemcpyAsync(h->rec, rec.data(), rec.size() * sizeof(SoftRec), cudaMemcpyHostToDevice, h->stream));
     CK(cudaMemcpyAsync(h->vals, t.data(), t.size() * 8, cudaMemcpyHostToDevice, h->stream));
   }
   CK(cudaMemcpyAsync(h->tab13, table, (size_t)nmat * PHONO_TABLE_COLS * 8, cudaMemcpyHostToDevice, h->stream));
@@ -304,6 +311,7 @@ static cudaError_t split_step(const phono_handle* h, int step_off, int step_end,
   a.rec = h->rec;
   a.vals = h->vals;
   a.shared = h->shared;
+  a.soft = (double)h->d.nx * h->d.ny * h->d.nz >= kSoftVelNodes;
   a.dtab = h->dtab;
   a.src = h->src;
   a.ubase = (R*)h->ubase;
@@ -374,7 +382,7 @@ static cudaError_t split_step(const phono_handle* h, int step_off, int step_end,
 
 static cudaError_t split_step_any(const phono_handle* h, int step_off, int step_end, cudaStream_t st) {
   if (h->d.precision == PHONO_F64) return split_step<double, SoftRec>(h, step_off, step_end, st);
-  if (h->d.precision == PHONO_F64V) return split_step<double, double>(h, step_off, step_end, st);
+  if (h->d.precision == PHONO_F64V) return split_step<double, SoftFactor>(h, step_off, step_end, st);
   return split_step<float, float>(h, step_off, step_end, st);
 }
 
@@ -410,7 +418,7 @@ static long long mat_row(int nz) { return round_up(MKOFF + nz + 1, 16); }
 // the tile pass.
 //  * FP64 (both schemes) is bound by the FP64 pipe: every mesh takes the
 //    two-launch form (256x256x128 cells: 1.07 ms a step against 2.0 for the
-//    best tile shape of the leapfrog, 1.03 against 1.17 for the velocity form).
+//    best tile shape of the leapfrog, 0.84 against 1.17 for the velocity form).
 //  * FP32 moves 60 more bytes a node than the tile pass, and wins only where
 //    a launch is too short to fill its pipeline (us a step, two launches
 //    against the default tiles: 7.5 / 10.1 at 78 k nodes, 9.2 / 9.7 at 139 k,
@@ -441,8 +449,8 @@ static size_t split_bytes(int nx, int ny, int nz, int precision) {
 // as the kernels use them (with one value 1 before and two after, so that the
 // tile pass reads the x spacings of its planes -1..nx without range tests;
 // the padding only reaches values whose results are discarded), their FP64
-// reciprocals (energy) and, for the leapfrog, the divisor table and the
-// records of the two-launch step with their values (16 per material id first).
+// reciprocals (energy) and, for FP64, the records of the two-launch step (16 per
+// material id first), for the leapfrog with their values and the divisor table.
 struct ConstBlock {
   size_t sp[6], rsp[6], spd[6], div, rec, vals, bytes;
 };
@@ -464,9 +472,11 @@ static ConstBlock const_block(int nx, int ny, int nz, int precision) {
       c.spd[a] = take((size_t)(lens[a] + 3) * sizeof(SoftRec));
       n += lens[a] + 1;
     }
-    c.rec = take(256 * 16 * sizeof(SoftRec));
     c.vals = take(n * 8);
+  } else if (precision == PHONO_F64V) {
+    for (int a = 0; a < 6; a++) c.spd[a] = take((size_t)(lens[a] + 3) * sizeof(SoftFactor));
   }
+  if (es == 8) c.rec = take(256 * 16 * sizeof(SoftRec));
   return c;
 }
 
@@ -900,7 +910,8 @@ int phono_create(const phono_desc* d, phono_handle** out) {
       h->h_sp0[a] = arrs[a][0];
       h->sp_host[a].assign(arrs[a], arrs[a] + lens[a]);
       h->sp[a] = dev + cb.sp[a] + h->es;
-      h->spd[a] = f64 ? (void*)((SoftRec*)(dev + cb.spd[a]) + 1) : h->sp[a];
+      const bool f64v = d->precision == PHONO_F64V;
+      h->spd[a] = f64 ? (void*)((SoftRec*)(dev + cb.spd[a]) + 1) : f64v ? (void*)((SoftFactor*)(dev + cb.spd[a]) + 1) : h->sp[a];
       h->rsp64[a] = (double*)(dev + cb.rsp[a]);
       SoftRec* rec = (SoftRec*)(host.data() + cb.spd[a]);
       const uint32_t one = nval;  // the padding's divisor
@@ -916,11 +927,12 @@ int phono_create(const phono_desc* d, phono_handle** out) {
           rec[q + 1] = soft_record(v, true, in ? nval : one);
           if (in) vals[nval++] = v;
         }
+        if (f64v) ((SoftFactor*)rec)[q + 1] = SoftFactor{soft_record(1.0 / v, false, 0), 1.0 / v, 0.0};
       }
       divisors.insert(divisors.end(), arrs[a], arrs[a] + lens[a]);
     }
+    if (h->es == 8) h->rec = (SoftRec*)(dev + cb.rec);
     if (f64) {
-      h->rec = (SoftRec*)(dev + cb.rec);
       h->vals = (double*)(dev + cb.vals);
       // divisor table (div_tab in div_table.cuh) over the distinct spacing
       // values and 1.0, the divisors the step uses

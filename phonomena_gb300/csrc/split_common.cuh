@@ -21,18 +21,25 @@ inline FastDiv fast_div(int d) {
   return FastDiv{(unsigned)((1ull << (31 + s)) / (unsigned)d + 1), s, d};
 }
 
-// R: element type; D: divisor as the scheme uses it (reciprocal, or the
-// record of soft_f64.cuh for the leapfrog).  Spacing arrays carry the value 1
-// at index -1 and two after the end.
+// a factor with its record (soft_f64.cuh)
+struct alignas(16) SoftFactor {
+  SoftRec rec;
+  double v, unused;
+};
+
+// R: element type; D: divisor as the scheme uses it (FP32: reciprocal; FP64
+// velocity form: reciprocal with its record; leapfrog: record).  Spacing
+// arrays carry the value 1 at index -1 and two after the end.
 template <class R, class D>
 struct SplitArgs {
   Geo g;
   const D *fdx, *fdy, *fdz, *sdx, *sdy, *sdz;
   const uint8_t* mat;
   const R* tab;          // velocity forms: 16 entries per material id
-  const SoftRec* rec;    // leapfrog: the same entries as records
+  const SoftRec* rec;    // FP64: the same entries as records
   const double* vals;    // leapfrog: values of the records (fallback division)
   int shared;            // leapfrog: c10 = c20, c01 = c21, c02 = c12 in every material
+  int soft;              // FP64 velocity form: products in integer arithmetic
   DivTable dtab;
   const double* src;
   R *ubase, *vbase, *cbase;

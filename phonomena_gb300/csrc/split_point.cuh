@@ -12,6 +12,9 @@ __device__ __forceinline__ SoftRec ldd(const SoftRec* p) {
   return SoftRec{v.x, v.y, v.z, v.w};
 }
 
+// (a caller that uses one part loads that part alone)
+__device__ __forceinline__ SoftFactor ldd(const SoftFactor* p) { return SoftFactor{ldd(&p->rec), ldd(&p->v), 0.0}; }
+
 __device__ __forceinline__ int fdiv(int n, const FastDiv& f) { return (int)(__umulhi(2u * (unsigned)n, f.mult) >> f.shift); }
 
 // point n of an update launch: component and indices; whether it is next to a face

@@ -10,36 +10,101 @@
 // through it in chunks.  The result is that of the tile pass, bit for bit.
 //
 // Bound (one GB300, us a step, the best tile shape of the tile pass first):
-// FP64 by instruction issue and the FP64 pipe together (18 FP64 of 1220
-// instructions a stress point; issue 61%, ALU 61%, FP64 pipe 57% busy); small
+// the FP64 leapfrog by instruction issue and the FP64 pipe together (18 FP64 of
+// 1220 instructions a stress point; issue 61%, ALU 61%, FP64 pipe 57% busy),
+// the FP64 velocity form by the FP64 pipe; small
 // meshes by two dependent launches (1.2 us each) of three or four L2
 // latencies.
 //   nodes       25x21x13   41x41x21   61x61x21   150x131x47  194x162x98  257x257x129
 //   F64         25 / 10.9  32 / 11.1  47 / 13.5  354 / 102   969 / 337   2012 / 924
-//   F64V        13 / 7.4   21 / 9.1   29 / 13.8  197 / 121   559 / 385   1174 / 1064
+//   F64V        13 / 7.4   21 / 9.1   29 / 13.4  197 / 98    559 / 307   1174 / 838
 //   F32K        9 / 5.3    10 / 5.7   12 / 6.7   (split_f32.cu; larger meshes: tile_vec.cuh)
 #include "split_point.cuh"
 
 namespace phono {
 
-// the velocity form in FP64: reciprocal spacings, coefficients as stored
+// an operand of a product in integer arithmetic: its value, and taken apart
+// where the integer path may take it
+struct SoftArg {
+  double x;
+  SoftNum n;
+  bool ok;
+};
+__device__ __forceinline__ SoftArg soft_arg(double x) {
+  SoftArg v;
+  v.x = x;
+  v.n = soft_split(x, v.ok);
+  return v;
+}
+__device__ __forceinline__ bool is_zero(double x) {
+  return ((uint32_t)__double2hiint(x) << 1 | (uint32_t)__double2loint(x)) == 0u;
+}
+// a zero's quotient or product keeps its sign (the other operand's sign is in `flip`)
+__device__ __forceinline__ double signed_zero(double x, uint32_t flip) {
+  return soft_double(((uint32_t)__double2hiint(x) ^ flip) & 0x80000000u, 0u);
+}
+
+// a call, so that nothing multiplies ahead of the branches around it
+__device__ __noinline__ double slow_mul(double x, double c) { return __dmul_rn(x, c); }
+
+// the velocity form in FP64: reciprocal spacings, coefficients as stored.  Of
+// its 63 FP64 operations a node 15 are products with a constant that no sum
+// takes in; SOFT: those run in integer arithmetic, 24 FP64 instructions a
+// stress point and 33 a node's update becoming 18 and 30 (the FP64 pipe, 85%
+// busy before, is still the bound at 78 and 67%).  A product is a chain of 25
+// instructions, so that meshes whose launches are a latency keep the plain
+// form.  us a step, plain / SOFT: 41x41x21 nodes 9.5 / 10.9, 61x61x21 13.9 /
+// 13.4, 81x71x31 26.1 / 22.7, 194x162x98 387 / 307, 257x257x129 1078 / 838.
+template <bool SOFT>
 struct VelOps {
   using Base = F64V;
   using R = double;
-  using D = R;
+  using D = SoftFactor;
   using Args = SplitArgs<R, D>;
-  static constexpr int STRESS_BLOCKS = 6, UPDATE_BLOCKS = 7;
-  static __device__ __forceinline__ void normals(const Args& a, int id, R d1, R d2, R d3, D x, D y, D z, R* t) {
-    const R* row = a.tab + 16 * id;
-    R c[9];
-    for (int q = 0; q < 9; q++) c[q] = __ldg(row + q);
-    for (int q = 0; q < 3; q++) t[q] = F64V::tn1(a.dtab, c + 3 * q, d1, d2, d3, x, y, z);
+  // resident blocks the registers are allotted for (SOFT, us a step on
+  // 256x256x128 cells): 9 and 8 838, 8 and 8 844, 6 and 7 877, 8 and 9 885
+  static constexpr int STRESS_BLOCKS = SOFT ? 9 : 6, UPDATE_BLOCKS = SOFT ? 8 : 7;
+  // x * c.  The result of a product may go into another one: the range that
+  // soft_arg tests leaves room for two factors (soft_f64.cuh).
+  template <class V>
+  static __device__ __forceinline__ SoftArg product(const SoftArg& x, const SoftRec& c, V value) {
+    SoftArg p;
+    if constexpr (!SOFT) {
+      p.x = __dmul_rn(x.x, value());
+      return p;
+    }
+    const bool fits = (int)c.hi < 0;
+    p.ok = x.ok && fits;
+    if (p.ok) {
+      p.n = soft_mul(x.n, c);
+      p.x = soft_join(p.n);
+    } else if (fits && is_zero(x.x)) {
+      p.x = signed_zero(x.x, c.de);
+    } else {
+      p.x = slow_mul(x.x, value());
+    }
+    return p;
   }
-  static __device__ __forceinline__ R shear(const Args& a, int id, int col, R d1, D x, R d2, D y) {
-    return F64V::ts(a.dtab, __ldg(a.tab + 16 * id + col), d1, x, d2, y);
+  static __device__ __forceinline__ SoftArg product(R x, const D& c) {
+    return product(soft_arg(x), c.rec, [&] { return c.v; });
   }
-  static __device__ __forceinline__ R div3(const Args& a, R d1, D x, R d2, D y, R d3, D z) {
-    return F64V::div3(a.dtab, d1, x, d2, y, d3, z);
+  static __device__ __forceinline__ void normals(const Args& a, int id, R d1, R d2, R d3, const D& x, const D& y, const D& z,
+                                                 R* t) {
+    const R* c = a.tab + 16 * id;
+    const SoftRec* rec = a.rec + 16 * id;
+    const R e1 = product(d1, x).x, e2 = product(d2, y).x;
+    const SoftArg e3 = product(d3, z);
+#pragma unroll
+    for (int q = 0; q < 3; q++)
+      t[q] = __fma_rn(__ldg(c + 3 * q), e1,
+                      __fma_rn(__ldg(c + 3 * q + 1), e2, product(e3, ldd(rec + 3 * q + 2), [&] { return __ldg(c + 3 * q + 2); }).x));
+  }
+  static __device__ __forceinline__ R shear(const Args& a, int id, int col, R d1, const D& x, R d2, const D& y) {
+    const R s = __fma_rn(d1, x.v, product(d2, y).x);
+    return product(soft_arg(s), ldd(a.rec + 16 * id + col), [&] { return __ldg(a.tab + 16 * id + col); }).x;
+  }
+  static __device__ __forceinline__ R div3(const Args& a, R d1, const D& x, R d2, const D& y, R d3, const D& z) {
+    return __fma_rn(d1, x.v, __fma_rn(d2, y.v, product(d3, z).x));
   }
   static __device__ __forceinline__ R update(const Args& a, int id, R u, Pw<R> pw, R dv, R& vn, R& cn) {
     return update_value<F64V>(u, pw, dv, __ldg(a.tab + 16 * id + 12), a.dt, vn, cn);
@@ -62,46 +127,28 @@ struct LeapOps {
   // resident blocks the registers are allotted for (us a step on 256x256x128
   // cells): 7 and 8 924, 6 and 8 954, 8 and 8 926, 7 and 7 962
   static constexpr int STRESS_BLOCKS = 7, UPDATE_BLOCKS = 8;
-  struct Num {
-    double x;
-    SoftNum n;
-    bool ok;
-  };
-  static __device__ __forceinline__ Num split(double x) {
-    Num v;
-    v.x = x;
-    v.n = soft_split(x, v.ok);
-    return v;
-  }
-  // a zero's quotient or product keeps its sign (the other operand's sign is in `flip`)
-  static __device__ __forceinline__ bool zero(double x) {
-    return ((uint32_t)__double2hiint(x) << 1 | (uint32_t)__double2loint(x)) == 0u;
-  }
-  static __device__ __forceinline__ double signed_zero(double x, uint32_t flip) {
-    return soft_double(((uint32_t)__double2hiint(x) ^ flip) & 0x80000000u, 0u);
-  }
   static __device__ __forceinline__ double divide(const Args& a, double x, const SoftRec& d) {
-    const Num v = split(x);
+    const SoftArg v = soft_arg(x);
     if (v.ok && (int)d.hi < 0) return soft_join(soft_div(v.n, d, [&] { return __ldg(a.vals + d.idx); }));
-    return zero(x) ? signed_zero(x, 0u) : slow_div(x, __ldg(a.vals + d.idx), a.dtab);
+    return is_zero(x) ? signed_zero(x, 0u) : slow_div(x, __ldg(a.vals + d.idx), a.dtab);
   }
   static __device__ __forceinline__ double times(const Args& a, double x, const SoftRec& c) {
-    const Num v = split(x);
+    const SoftArg v = soft_arg(x);
     if (v.ok && (int)c.hi < 0) return soft_join(soft_mul(v.n, c));
-    return zero(x) ? signed_zero(x, c.de) : __dmul_rn(__ldg(a.vals + c.idx), x);
+    return is_zero(x) ? signed_zero(x, c.de) : __dmul_rn(__ldg(a.vals + c.idx), x);
   }
   // (c * x) / d, both roundings
-  static __device__ __forceinline__ double scaled(const Args& a, const Num& v, const SoftRec& c, const SoftRec& d) {
+  static __device__ __forceinline__ double scaled(const Args& a, const SoftArg& v, const SoftRec& c, const SoftRec& d) {
     if (v.ok && (int)(c.hi & d.hi) < 0)
       return soft_join(soft_div(soft_mul(v.n, c), d, [&] { return __ldg(a.vals + d.idx); }));
-    if (zero(v.x)) return signed_zero(v.x, c.de);
+    if (is_zero(v.x)) return signed_zero(v.x, c.de);
     const double y = __dmul_rn(__ldg(a.vals + c.idx), v.x);
-    return zero(y) ? y : slow_div(y, __ldg(a.vals + d.idx), a.dtab);
+    return is_zero(y) ? y : slow_div(y, __ldg(a.vals + d.idx), a.dtab);
   }
   static __device__ __forceinline__ void normals(const Args& a, int id, R d1, R d2, R d3, const D& x, const D& y,
                                                  const D& z, R* t) {
     const SoftRec* c = a.rec + 16 * id;
-    const Num v1 = split(d1), v2 = split(d2), v3 = split(d3);
+    const SoftArg v1 = soft_arg(d1), v2 = soft_arg(d2), v3 = soft_arg(d3);
     if constexpr (SHARED) {
       const R x1 = scaled(a, v1, ldd(c + 3), x), y0 = scaled(a, v2, ldd(c + 1), y), z0 = scaled(a, v3, ldd(c + 2), z);
       t[0] = __dadd_rn(__dadd_rn(scaled(a, v1, ldd(c), x), y0), z0);
@@ -278,7 +325,10 @@ cudaError_t launch_split(int precision, const void* args, bool stress, bool afte
     if (((const LeapOps<false>::Args*)args)->shared) return launch_pass<LeapOps<true>>(args, stress, after_kernel, st);
     return launch_pass<LeapOps<false>>(args, stress, after_kernel, st);
   }
-  if (precision == 2) return launch_pass<VelOps>(args, stress, after_kernel, st);
+  if (precision == 2) {
+    if (((const VelOps<true>::Args*)args)->soft) return launch_pass<VelOps<true>>(args, stress, after_kernel, st);
+    return launch_pass<VelOps<false>>(args, stress, after_kernel, st);
+  }
   return launch_split_f32(args, stress, after_kernel, st);
 }
 
