@@ -22,6 +22,7 @@ cudaError_t launch_split(int precision, const void* args, bool stress, bool afte
 cudaError_t launch_energy(const EnergyArgs& a, double2* partial, int nblocks, double* out, bool pairs, cudaStream_t st);
 cudaError_t launch_lattice_ids(uint8_t* mat, const Geo& g, int pitch, int ncx, int ncy, const double* radius,
                                const uint8_t* kind, int depth, uint8_t host, cudaStream_t st);
+cudaError_t launch_unpack_ids(uint8_t* mat, const Geo& g, const uint8_t* dense, long long first, int rows, cudaStream_t st);
 cudaError_t launch_readback(const void* in, long long sx, long long sy, int ex, int ey, int ez, int es, void* out,
                             cudaStream_t st);
 cudaError_t launch_inclusion_ids(uint8_t* mat, const Geo& g, const double* x, const double* y, const double4* incl,
@@ -86,6 +87,7 @@ struct phono_handle {
   DivTable dtab{};        // FP64 leapfrog: reciprocal pairs of the mesh's divisors (tab null: none)
   std::vector<double> sp_host[6];  // raw spacings (ABC coefficients)
   uint8_t* mat = nullptr;
+  uint8_t* stage = nullptr;  // ids on their way from the host (stage_bytes)
   void* tab = nullptr;       // 16 R per material
   double* tab13 = nullptr;   // raw table (energy)
   double* src = nullptr;
@@ -171,7 +173,7 @@ static void abc_coeffs(const phono_handle* h, const double* row0, double out[8])
 }
 
 // the largest of n ids, 64 at a time: a byte at a time took most of a material
-// upload (160x128x64 cells: 812 us with it, 306 so)
+// upload (160x128x64 cells: 837 us with it, 416 without)
 static int largest_id(const uint8_t* id, size_t n) {
   uint8_t m[64] = {};
   size_t p = 0;
@@ -193,17 +195,25 @@ static int check_materials(const phono_handle* h, const uint8_t* mat, const doub
   return PHONO_OK;
 }
 
+// Ids pass through a stage of whole rows on the way to the padded layout, where
+// a kernel puts them: a strided copy moves a row (65 bytes, say) at a time (us
+// an upload, strided / staged: 41x41x21 nodes 45 / 31, 160x128x64 cells 416 / 89,
+// 256x256x128 2334 / 539, 512x512x256 11300 / 4100).
+static size_t stage_bytes(int nx, int ny, int nz) {
+  return (size_t)std::min<long long>((long long)nx * ny, std::max<long long>((4 << 20) / nz, 1)) * nz;
+}
+
 // ids into the padded layout, 16-entry device rows, raw rows, ABC coefficients
 static int upload_table(phono_handle* h, const double* table, int nmat, int id000);
 
 static int upload_materials(phono_handle* h, const uint8_t* mat, const double* table, int nmat) {
   const int nx = h->d.nx, ny = h->d.ny, nz = h->d.nz;
-  cudaMemcpy3DParms p{};
-  p.srcPtr = make_cudaPitchedPtr((void*)mat, nz, nz, ny);
-  p.dstPtr = make_cudaPitchedPtr(h->mat + h->g.mo0, h->g.msy, h->g.msy, ny + 2);
-  p.extent = make_cudaExtent(nz, ny, nx);
-  p.kind = cudaMemcpyHostToDevice;
-  CK(cudaMemcpy3DAsync(&p, h->stream));
+  const long long rows = (long long)nx * ny, step = (long long)stage_bytes(nx, ny, nz) / nz;
+  for (long long first = 0; first < rows; first += step) {
+    const int n = (int)std::min(step, rows - first);
+    CK(cudaMemcpyAsync(h->stage, mat + first * nz, (size_t)n * nz, cudaMemcpyHostToDevice, h->stream));
+    CK(launch_unpack_ids(h->mat, h->g, h->stage, first, n, h->stream));
+  }
   return upload_table(h, table, nmat, mat[0]);
 }
 
@@ -500,7 +510,7 @@ static size_t handle_bytes(int nx, int ny, int nz, int precision, int max_steps,
   const size_t fb = field_elems * es * 3 * nbuf;
   size_t total = r(fb) * (precision == PHONO_F64 ? 1 : 3);
   total += r(const_block(nx, ny, nz, precision).bytes);
-  total += r((size_t)(nx + 2) * (ny + 2) * mat_row(nz));
+  total += r((size_t)(nx + 2) * (ny + 2) * mat_row(nz)) + r(stage_bytes(nx, ny, nz));
   total += r((size_t)256 * 16 * es) + r((size_t)256 * PHONO_TABLE_COLS * 8);
   const int cap = max_steps > 0 ? max_steps : 1;
   total += r((size_t)cap * 8);
@@ -955,7 +965,8 @@ int phono_create(const phono_desc* d, phono_handle** out) {
   }
   // materials: padded id layout and the 16-entry device rows (capacity 256 ids)
   TRY(dalloc(h, (void**)&h->mat, h->mat_bytes));
-  TRYC(cudaMemset(h->mat, 0, h->mat_bytes));
+  TRY(dalloc(h, (void**)&h->stage, stage_bytes(nx, ny, nz)));
+  TRYC(cudaMemsetAsync(h->mat, 0, h->mat_bytes, h->stream));
   TRY(dalloc(h, &h->tab, (size_t)256 * 16 * h->es));
   // two-launch step; the leapfrog's window is zero outside the points the
   // stress pass writes, and a mesh whose window does not fit keeps to the tiles
@@ -978,7 +989,7 @@ int phono_create(const phono_desc* d, phono_handle** out) {
   // source table, surface records, counters
   int cap = d->max_steps > 0 ? d->max_steps : 1;
   TRY(dalloc(h, (void**)&h->src, (size_t)cap * 8));
-  TRYC(cudaMemset(h->src, 0, (size_t)cap * 8));
+  TRYC(cudaMemsetAsync(h->src, 0, (size_t)cap * 8, h->stream));
   h->nrec_cap = d->record_every > 0 ? d->max_steps / d->record_every : 0;
   if (h->nrec_cap > 0) {
     size_t sb = (size_t)h->nrec_cap * nx * ny * h->es;

@@ -78,4 +78,34 @@ cudaError_t launch_inclusion_ids(uint8_t* mat, const Geo& g, const double* x, co
   return cudaGetLastError();
 }
 
+// Dense ids of mesh rows [first, first + rows) into the padded layout, 8
+// bytes a thread (a padded row starts on 8 bytes; what follows its nz ids
+// stays).
+__global__ void unpack_ids_kernel(uint8_t* __restrict__ mat, const Geo g, const uint8_t* __restrict__ dense, long long first,
+                                  int rows, int words) {
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long long row = t / words;
+  const int k = (int)(t - row * words) * 8;
+  if (row >= rows) return;
+  const uint8_t* in = dense + row * g.nz + k;
+  const long long at = first + row, i = at / g.ny;
+  uint8_t* out = mat + g.mo0 + i * g.msx + (at - i * g.ny) * g.msy + k;
+  const int n = min(8, g.nz - k);
+  if (n == 8) {
+    uint2 w = make_uint2(0, 0);
+#pragma unroll
+    for (int q = 0; q < 4; q++) w.x |= (unsigned)in[q] << (8 * q), w.y |= (unsigned)in[q + 4] << (8 * q);
+    *reinterpret_cast<uint2*>(out) = w;
+  } else {
+    for (int q = 0; q < n; q++) out[q] = in[q];
+  }
+}
+
+cudaError_t launch_unpack_ids(uint8_t* mat, const Geo& g, const uint8_t* dense, long long first, int rows, cudaStream_t st) {
+  const int words = (g.nz + 7) / 8;
+  const long long blocks = ((long long)rows * words + 255) / 256;
+  unpack_ids_kernel<<<(unsigned)blocks, 256, 0, st>>>(mat, g, dense, first, rows, words);
+  return cudaGetLastError();
+}
+
 }  // namespace phono
