@@ -1665,7 +1665,7 @@ static int capture_instance(phono_batch* b, int s) {
 // batch stream only after the last chunk: an instance's next chunk starts as
 // soon as its previous one is done, whatever the others are doing.
 static cudaError_t streams_steps(phono_batch* b, int n) {
-  const int na = (int)b->order.size(), nw = std::min(na, (int)b->workers.size());
+  const int na = (int)b->order.size(), nw = std::min(na, b->streams ? b->streams : (int)b->workers.size());
   cudaError_t e = cudaEventRecord(b->fork, b->stream);
   for (int w = 0; w < nw && e == cudaSuccess; w++) e = cudaStreamWaitEvent(b->workers[w], b->fork, 0);
   const int full = n / kGraphSteps, rem = n % kGraphSteps;
