@@ -108,10 +108,11 @@ struct FacePoints {
 
 // the stress or update launch of the planes set in the arguments
 template <class F, class A>
-inline cudaError_t split_launch(F* kernel, const A& a, long long points, bool after_kernel, cudaStream_t st) {
+inline cudaError_t split_launch(F* kernel, const A& a, long long points, bool after_kernel, cudaStream_t st,
+                                int parts = 1) {
   if (points <= 0) return cudaSuccess;
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((unsigned)((points + SPLIT_THREADS - 1) / SPLIT_THREADS));
+  cfg.gridDim = dim3((unsigned)((points + SPLIT_THREADS - 1) / SPLIT_THREADS), (unsigned)parts);
   cfg.blockDim = dim3(SPLIT_THREADS);
   cfg.stream = st;
   cudaLaunchAttribute at{};

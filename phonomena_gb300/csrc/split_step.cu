@@ -16,8 +16,8 @@
 // meshes by two dependent launches (1.2 us each) of three or four L2
 // latencies.
 //   nodes       25x21x13   41x41x21   61x61x21   150x131x47  194x162x98  257x257x129
-//   F64         25 / 10.9  32 / 11.1  47 / 13.5  354 / 102   969 / 337   2012 / 924
-//   F64V        13 / 7.4   21 / 9.1   29 / 13.4  197 / 98    559 / 307   1174 / 838
+//   F64         25 / 8.4   32 / 10.8  47 / 13.5  354 / 102   969 / 337   2012 / 924
+//   F64V        13 / 7.2   21 / 9.1   29 / 13.4  197 / 98    559 / 307   1174 / 838
 //   F32K        9 / 5.3    10 / 5.7   12 / 6.7   (split_f32.cu; larger meshes: tile_vec.cuh)
 #include "split_point.cuh"
 
@@ -64,6 +64,7 @@ struct VelOps {
   // resident blocks the registers are allotted for (SOFT, us a step on
   // 256x256x128 cells): 9 and 8 838, 8 and 8 844, 6 and 7 877, 8 and 9 885
   static constexpr int STRESS_BLOCKS = SOFT ? 9 : 6, UPDATE_BLOCKS = SOFT ? 8 : 7;
+  static constexpr bool SMALL = !SOFT;  // stress points may be shared by threads
   // x * c.  The result of a product may go into another one: the range that
   // soft_arg tests leaves room for two factors (soft_f64.cuh).
   template <class V>
@@ -99,6 +100,12 @@ struct VelOps {
       t[q] = __fma_rn(__ldg(c + 3 * q), e1,
                       __fma_rn(__ldg(c + 3 * q + 1), e2, product(e3, ldd(rec + 3 * q + 2), [&] { return __ldg(c + 3 * q + 2); }).x));
   }
+  static __device__ __forceinline__ R normal(const Args& a, int id, int q, R d1, R d2, R d3, const D& x, const D& y, const D& z) {
+    const R* c = a.tab + 16 * id + 3 * q;
+    const R e1 = product(d1, x).x, e2 = product(d2, y).x;
+    const SoftArg e3 = product(d3, z);
+    return __fma_rn(__ldg(c), e1, __fma_rn(__ldg(c + 1), e2, product(e3, ldd(a.rec + 16 * id + 3 * q + 2), [&] { return __ldg(c + 2); }).x));
+  }
   static __device__ __forceinline__ R shear(const Args& a, int id, int col, R d1, const D& x, R d2, const D& y) {
     const R s = __fma_rn(d1, x.v, product(d2, y).x);
     return product(soft_arg(s), ldd(a.rec + 16 * id + col), [&] { return __ldg(a.tab + 16 * id + col); }).x;
@@ -127,6 +134,7 @@ struct LeapOps {
   // resident blocks the registers are allotted for (us a step on 256x256x128
   // cells): 7 and 8 924, 6 and 8 954, 8 and 8 926, 7 and 7 962
   static constexpr int STRESS_BLOCKS = 7, UPDATE_BLOCKS = 8;
+  static constexpr bool SMALL = true;
   static __device__ __forceinline__ double divide(const Args& a, double x, const SoftRec& d) {
     const SoftArg v = soft_arg(x);
     if (v.ok && (int)d.hi < 0) return soft_join(soft_div(v.n, d, [&] { return __ldg(a.vals + d.idx); }));
@@ -163,6 +171,11 @@ struct LeapOps {
                          scaled(a, v3, ldd(c + 3 * q + 2), z));
     }
   }
+  static __device__ __forceinline__ R normal(const Args& a, int id, int q, R d1, R d2, R d3, const D& x, const D& y, const D& z) {
+    const SoftRec* c = a.rec + 16 * id + 3 * q;
+    return __dadd_rn(__dadd_rn(scaled(a, soft_arg(d1), ldd(c), x), scaled(a, soft_arg(d2), ldd(c + 1), y)),
+                     scaled(a, soft_arg(d3), ldd(c + 2), z));
+  }
   static __device__ __forceinline__ R shear(const Args& a, int id, int col, R d1, const D& x, R d2, const D& y) {
     return times(a, __dadd_rn(divide(a, d1, x), divide(a, d2, y)), ldd(a.rec + 16 * id + col));
   }
@@ -179,8 +192,16 @@ struct LeapOps {
 // ---------------------------------------------------------------------------
 // stresses of planes [sa, sb): one thread per node of [sa, sb) x [0, ny-1) x
 // [0, nz-1).  Zero where the reference never writes (base_solver.py:329-433).
+//
+// PARTS: threads that share a point, in blocks of their own (blockIdx.y).  On a
+// mesh of few blocks the pass is the 1220 instructions of one thread after
+// another: two parts (normal and shear stresses) or six (a stress each)
+// shorten that chain, until the work done twice fills the chip.  us a step
+// with 1 / 2 / 6 parts: F64 25x21x13 nodes 11.9 / 9.8 / 8.4, 41x41x21 12.5 /
+// 10.8 / 10.8, 61x61x21 14.3 / 14.4 / 15.6, 101x101x41 44 / 46 / 58; F64V
+// 25x21x13 8.3 / 7.6 / 7.2, 41x41x21 9.5 / 9.5 / 9.8.
 // ---------------------------------------------------------------------------
-template <class O>
+template <class O, int PARTS>
 __global__ void __launch_bounds__(SPLIT_THREADS, O::STRESS_BLOCKS) split_stress_kernel(const __grid_constant__ typename O::Args a) {
   using R = typename O::R;
   using B = typename O::Base;
@@ -202,30 +223,44 @@ __global__ void __launch_bounds__(SPLIT_THREADS, O::STRESS_BLOCKS) split_stress_
   const bool kz = k == 0;
   const int up = kz ? 0 : 1;  // shear moduli of T4, T5: one layer down, except in the z = 0 row
   const bool i_n = i >= 1 && i <= nx - 2, i_s = i <= nx - 2, j_n = j >= 1;
+  const int part = PARTS == 1 ? 0 : (int)blockIdx.y;
+  // the stresses of this block, T1..T6
+  auto mine = [&](int q) { return PARTS == 1 || (PARTS == 2 ? part == q / 3 : part == q); };
   const R x0 = X[0], y0 = Y[0];
   R z0 = Z[0];
   if (i == 0 && (a.source_mode == 1 || kz)) z0 = (R)__ldg(a.src + tt);  // source overwrite (base_solver.py:251)
-  const R x_k = X[1], x_j = X[sy], y_k = Y[1], y_i = Y[sx], z_j = Z[sy], z_i = Z[sx];
+  const R x_k = mine(4) ? X[1] : R(0), x_j = mine(5) ? X[sy] : R(0), y_k = mine(3) ? Y[1] : R(0),
+          y_i = mine(5) ? Y[sx] : R(0), z_j = mine(3) ? Z[sy] : R(0), z_i = mine(4) ? Z[sx] : R(0);
   R t[6] = {R(0), R(0), R(0), R(0), R(0), R(0)};
-  if (i_n && j_n)
-    O::normals(a, M[0], B::sub(x0, *(X - sx)), B::sub(y0, *(Y - sy)), B::sub(z0, Z[-1]), ldd(a.sdx + (kz ? 0 : i - 1)),
-               ldd(a.sdy + (kz ? 0 : j - 1)), ldd(a.sdz + (kz ? 0 : k - 1)), t);
-  if (kz) t[2] = R(0);  // base_solver.py:418
+  if (i_n && j_n && (mine(0) || mine(1) || mine(2))) {
+    const R d1 = B::sub(x0, *(X - sx)), d2 = B::sub(y0, *(Y - sy)), d3 = B::sub(z0, Z[-1]);
+    const auto ax = ldd(a.sdx + (kz ? 0 : i - 1));
+    const auto ay = ldd(a.sdy + (kz ? 0 : j - 1));
+    const auto az = ldd(a.sdz + (kz ? 0 : k - 1));
+    if constexpr (PARTS == 6) t[0] = O::normal(a, M[0], part, d1, d2, d3, ax, ay, az);
+    else O::normals(a, M[0], d1, d2, d3, ax, ay, az, t);
+  }
+  if (kz) t[PARTS == 6 ? 0 : 2] = PARTS == 6 && part != 2 ? t[0] : R(0);  // base_solver.py:418
   // shears; the z = 0 row's substituted spacings are base_solver.py:420-433's
-  if (i_n)
+  if (i_n && mine(3))
     t[3] = O::shear(a, M[g.msy + up], 9, B::sub(y_k, y0), ldd(kz ? a.fdy : a.fdz + k), B::sub(z_j, z0),
                     ldd(kz ? a.fdz : a.fdy + j));
-  if (i_s && j_n)
+  if (i_s && j_n && mine(4))
     t[4] = O::shear(a, M[g.msx + up], 10, B::sub(x_k, x0), ldd(kz ? a.fdx : a.fdz + k), B::sub(z_i, z0),
                     ldd(kz ? a.fdz : a.fdx + i));
-  if (i_s)
+  if (i_s && mine(5))
     t[5] = O::shear(a, M[g.msx + g.msy], 11, B::sub(x_j, x0), ldd(kz ? a.fdx : a.fdy + j), B::sub(y_i, y0),
                     ldd(kz ? a.fdz : a.fdx + i));
   const unsigned to = (unsigned)(i % a.W) * a.tsx + (unsigned)(j * a.tsy + k);
+  if constexpr (PARTS == 6) {
+    if (part < 3) a.Ta[to + part * a.tcs] = t[0];
+    else a.Tb[to + (part - 3) * a.tcs] = part == 3 ? t[3] : part == 4 ? t[4] : t[5];
+    return;
+  }
 #pragma unroll
   for (int q = 0; q < 3; q++) {
-    a.Ta[to + q * a.tcs] = t[q];
-    a.Tb[to + q * a.tcs] = t[q + 3];
+    if (mine(q)) a.Ta[to + q * a.tcs] = t[q];
+    if (mine(q + 3)) a.Tb[to + q * a.tcs] = t[q + 3];
   }
 }
 
@@ -311,8 +346,13 @@ __global__ void __launch_bounds__(SPLIT_THREADS, O::UPDATE_BLOCKS) split_update_
 template <class O>
 static cudaError_t launch_pass(const void* args, bool stress, bool after_kernel, cudaStream_t st) {
   const typename O::Args& a = *(const typename O::Args*)args;
-  return stress ? split_launch(split_stress_kernel<O>, a, (long long)(a.sb - a.sa) * a.dy1.d * a.dz1.d, after_kernel, st)
-                : split_launch(split_update_kernel<O>, a, a.off[6], after_kernel, st);
+  if (!stress) return split_launch(split_update_kernel<O>, a, a.off[6], after_kernel, st);
+  const long long points = (long long)(a.sb - a.sa) * a.dy1.d * a.dz1.d;
+  if constexpr (O::SMALL) {
+    if (points < 20000) return split_launch(split_stress_kernel<O, 6>, a, points, after_kernel, st, 6);
+    if (points < 60000) return split_launch(split_stress_kernel<O, 2>, a, points, after_kernel, st, 2);
+  }
+  return split_launch(split_stress_kernel<O, 1>, a, points, after_kernel, st);
 }
 
 cudaError_t launch_split_f32(const void* args, bool stress, bool after_kernel, cudaStream_t st);
