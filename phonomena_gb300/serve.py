@@ -96,10 +96,12 @@ class GpuBackend:
     ``max_steps`` steps so that requests of any length share a key.
     """
 
-    def __init__(self, precision="f32k", capacity=128, tile_j=16, x_segment=0, max_steps=3000, streams=0):
+    def __init__(self, precision="f32k", capacity=128, tile_j=None, x_segment=0, max_steps=3000, streams=0):
         from .batch import Batch
 
         self.precision = precision
+        if tile_j is None:  # FP64 simulations of the default shape take the two-launch step
+            tile_j = 16 if precision == "f32k" or x_segment else 0
         self.tile_j = tile_j
         self.x_segment = x_segment
         self.max_steps = int(max_steps)
@@ -155,7 +157,7 @@ class GpuBackend:
         else:
             sim = DeviceSimulation(p.spacing, p.ids, p.table, p.dt, precision=self.precision,
                                    surface_mode="corrected", max_steps=k[1], record_every=k[2], tile_j=self.tile_j,
-                                   x_segment=self.x_segment or _x_segment(p.shape[0]))
+                                   x_segment=self.x_segment or (_x_segment(p.shape[0]) if self.tile_j else 0))
         sim.set_source(p.source)
         sim.pool_key = k
         slot = self.batch.add(sim, p.req.steps)
