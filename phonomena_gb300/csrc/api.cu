@@ -3,6 +3,7 @@
 #include <climits>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <vector>
 #include <algorithm>
@@ -87,7 +88,7 @@ struct phono_handle {
   DivTable dtab{};        // FP64 leapfrog: reciprocal pairs of the mesh's divisors (tab null: none)
   std::vector<double> sp_host[6];  // raw spacings (ABC coefficients)
   uint8_t* mat = nullptr;
-  uint8_t* stage = nullptr;  // ids on their way from the host (stage_bytes)
+  int dev = -1;              // the handle counts among the users of this device's stage (-1: not yet)
   void* tab = nullptr;       // 16 R per material
   double* tab13 = nullptr;   // raw table (energy)
   double* src = nullptr;
@@ -140,6 +141,7 @@ static int dalloc(phono_handle* h, void** p, size_t bytes) {
 }
 
 static void batch_detach(phono_batch* b, const phono_handle* h);
+static void leave_stage(phono_handle* h);
 
 static void release(phono_handle* h) {
   if (!h) return;
@@ -147,6 +149,7 @@ static void release(phono_handle* h) {
   if (h->graph) cudaGraphExecDestroy(h->graph);
   if (h->stream) cudaStreamSynchronize(h->stream);
   for (void* p : h->allocs) cudaFree(p);
+  leave_stage(h);
   if (h->ev0) cudaEventDestroy(h->ev0);
   if (h->ev1) cudaEventDestroy(h->ev1);
   if (h->stream) cudaStreamDestroy(h->stream);
@@ -195,12 +198,61 @@ static int check_materials(const phono_handle* h, const uint8_t* mat, const doub
   return PHONO_OK;
 }
 
-// Ids pass through a stage of whole rows on the way to the padded layout, where
-// a kernel puts them: a strided copy moves a row (65 bytes, say) at a time (us
-// an upload, strided / staged: 41x41x21 nodes 45 / 31, 160x128x64 cells 416 / 89,
-// 256x256x128 2334 / 539, 512x512x256 11300 / 4100).
-static size_t stage_bytes(int nx, int ny, int nz) {
-  return (size_t)std::min<long long>((long long)nx * ny, std::max<long long>((4 << 20) / nz, 1)) * nz;
+// From 256 KB on, ids pass through a stage of whole rows on the way to the
+// padded layout, where a kernel puts them: a strided copy moves a row (65 bytes,
+// say) at a time (us an upload, strided / staged: 160x128x64 cells 416 / 89,
+// 256x256x128 2334 / 539, 512x512x256 11300 / 4100).  One stage a device, made at
+// the first such upload and given back with the device's last handle; an upload
+// holds it until its copies are done.
+struct IdStage {
+  std::mutex m;
+  int users = 0;
+  uint8_t* p = nullptr;
+};
+static IdStage g_stage[32];
+constexpr size_t kStageBytes = 4 << 20, kStagedFrom = 256 << 10;
+
+static void join_stage(phono_handle* h) {
+  int dev = -1;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 32) return;
+  std::lock_guard<std::mutex> hold(g_stage[dev].m);
+  g_stage[dev].users++;
+  h->dev = dev;
+}
+static void leave_stage(phono_handle* h) {
+  if (h->dev < 0) return;
+  IdStage& g = g_stage[h->dev];
+  std::lock_guard<std::mutex> hold(g.m);
+  if (--g.users == 0 && g.p) {
+    cudaFree(g.p);
+    g.p = nullptr;
+  }
+  h->dev = -1;
+}
+
+// `staged`: the ids are in place (else nothing was done)
+static int upload_staged(phono_handle* h, const uint8_t* mat, bool& staged) {
+  const int nz = h->d.nz;
+  const long long rows = (long long)h->d.nx * h->d.ny, step = (long long)kStageBytes / nz;
+  if (h->dev < 0 || (size_t)rows * nz < kStagedFrom || step < 1) return PHONO_OK;
+  IdStage& g = g_stage[h->dev];
+  std::lock_guard<std::mutex> hold(g.m);
+  if (!g.p && cudaMalloc(&g.p, kStageBytes) != cudaSuccess) {
+    g.p = nullptr;
+    cudaGetLastError();
+    return PHONO_OK;
+  }
+  cudaError_t e = cudaSuccess;
+  for (long long first = 0; first < rows && e == cudaSuccess; first += step) {
+    const int n = (int)std::min(step, rows - first);
+    e = cudaMemcpyAsync(g.p, mat + first * nz, (size_t)n * nz, cudaMemcpyHostToDevice, h->stream);
+    if (e == cudaSuccess) e = launch_unpack_ids(h->mat, h->g, g.p, first, n, h->stream);
+  }
+  const cudaError_t done = cudaStreamSynchronize(h->stream);
+  CK(e);
+  CK(done);
+  staged = true;
+  return PHONO_OK;
 }
 
 // ids into the padded layout, 16-entry device rows, raw rows, ABC coefficients
@@ -208,11 +260,15 @@ static int upload_table(phono_handle* h, const double* table, int nmat, int id00
 
 static int upload_materials(phono_handle* h, const uint8_t* mat, const double* table, int nmat) {
   const int nx = h->d.nx, ny = h->d.ny, nz = h->d.nz;
-  const long long rows = (long long)nx * ny, step = (long long)stage_bytes(nx, ny, nz) / nz;
-  for (long long first = 0; first < rows; first += step) {
-    const int n = (int)std::min(step, rows - first);
-    CK(cudaMemcpyAsync(h->stage, mat + first * nz, (size_t)n * nz, cudaMemcpyHostToDevice, h->stream));
-    CK(launch_unpack_ids(h->mat, h->g, h->stage, first, n, h->stream));
+  bool staged = false;
+  if (const int rc = upload_staged(h, mat, staged)) return rc;
+  if (!staged) {
+    cudaMemcpy3DParms p{};
+    p.srcPtr = make_cudaPitchedPtr((void*)mat, nz, nz, ny);
+    p.dstPtr = make_cudaPitchedPtr(h->mat + h->g.mo0, h->g.msy, h->g.msy, ny + 2);
+    p.extent = make_cudaExtent(nz, ny, nx);
+    p.kind = cudaMemcpyHostToDevice;
+    CK(cudaMemcpy3DAsync(&p, h->stream));
   }
   return upload_table(h, table, nmat, mat[0]);
 }
@@ -510,7 +566,7 @@ static size_t handle_bytes(int nx, int ny, int nz, int precision, int max_steps,
   const size_t fb = field_elems * es * 3 * nbuf;
   size_t total = r(fb) * (precision == PHONO_F64 ? 1 : 3);
   total += r(const_block(nx, ny, nz, precision).bytes);
-  total += r((size_t)(nx + 2) * (ny + 2) * mat_row(nz)) + r(stage_bytes(nx, ny, nz));
+  total += r((size_t)(nx + 2) * (ny + 2) * mat_row(nz));
   total += r((size_t)256 * 16 * es) + r((size_t)256 * PHONO_TABLE_COLS * 8);
   const int cap = max_steps > 0 ? max_steps : 1;
   total += r((size_t)cap * 8);
@@ -965,8 +1021,8 @@ int phono_create(const phono_desc* d, phono_handle** out) {
   }
   // materials: padded id layout and the 16-entry device rows (capacity 256 ids)
   TRY(dalloc(h, (void**)&h->mat, h->mat_bytes));
-  TRY(dalloc(h, (void**)&h->stage, stage_bytes(nx, ny, nz)));
   TRYC(cudaMemsetAsync(h->mat, 0, h->mat_bytes, h->stream));
+  join_stage(h);
   TRY(dalloc(h, &h->tab, (size_t)256 * 16 * h->es));
   // two-launch step; the leapfrog's window is zero outside the points the
   // stress pass writes, and a mesh whose window does not fit keeps to the tiles
