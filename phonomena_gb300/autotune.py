@@ -173,11 +173,15 @@ def tune_batch(shapes, precision="f32k", steps=24, tile_js=TILE_J, use_cache=Tru
     shapes: mesh node counts (nx, ny, nz) of the instances, in batch order.
     streams: 0 times the default scheme, W > 0 the streams scheme on W
     worker streams (every instance at the chosen tile height).
-    Returns (tile_j, [x_segment per instance]).
+    Returns (tile_j, [x_segment per instance]); zeros where default handles,
+    which take the library's own choice, are fastest (not tried for FP32 in the
+    default scheme, where the batch picks the tiles anyway).
     """
     from .batch import Batch
 
     shapes = [tuple(int(v) for v in s) for s in shapes]
+    if streams or precision != "f32k":
+        tile_js = (0, *tile_js)
     key = _batch_key(precision, shapes) + ":" + ",".join(map(str, tile_js)) + (f":streams{streams}" if streams else "")
     if use_cache:
         hit = _load().get(key)
@@ -188,12 +192,13 @@ def tune_batch(shapes, precision="f32k", steps=24, tile_js=TILE_J, use_cache=Tru
     seg_cands = {nx: sorted({xs for xs in X_SEGMENTS if xs < nx - 1} | {nx - 1}) for nx in groups}
     n_timings = len(tile_js) * (len(X_SEGMENTS) + 1) + sum(len(c) for c in seg_cands.values())
     budget = (steps + 12) * (n_timings + 2)
-    sims = [_scratch(s, precision, budget) for s in shapes]
+    sims = [_scratch(s, precision, budget, tile_j=0, x_segment=0) for s in shapes]
     log = []
 
     def time_mix(tj, seg_by_nx):
         for sim in sims:
-            sim.set_tiling(tj, seg_by_nx[sim.nx])
+            if tj:
+                sim.set_tiling(tj, seg_by_nx[sim.nx])
         with Batch(len(sims), precision=precision, tile_j=tj, streams=streams) as b:
             for sim in sims:
                 b.add(sim, steps + 12)
@@ -209,6 +214,9 @@ def tune_batch(shapes, precision="f32k", steps=24, tile_js=TILE_J, use_cache=Tru
     try:
         best = None
         for tj in tile_js:
+            if not tj:  # first: a tile shape, once set, stays
+                best = (time_mix(0, dict.fromkeys(groups, 0)), 0, dict.fromkeys(groups, 0))
+                continue
             for xs in list(X_SEGMENTS) + [0]:  # 0: one segment per block column
                 seg = {nx: (min(xs, nx - 1) if xs else nx - 1) for nx in groups}
                 ms = time_mix(tj, seg)
@@ -216,7 +224,7 @@ def tune_batch(shapes, precision="f32k", steps=24, tile_js=TILE_J, use_cache=Tru
                     best = (ms, tj, dict(seg))
         ms_best, tj, seg = best
         for nx in reversed(groups):  # per-group refinement, largest x extent first
-            for xs in seg_cands[nx]:
+            for xs in seg_cands[nx] if tj else ():
                 if xs == seg[nx]:
                     continue
                 trial = dict(seg)
