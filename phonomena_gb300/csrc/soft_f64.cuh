@@ -171,6 +171,11 @@ SOFT_HD double soft_join(const SoftNum& n) {
   return soft_double(((n.hi >> 11) & 0xfffffu) | n.se, (n.lo >> 11) | (n.hi << 21));
 }
 
+// sign of a record's operand (its top bit): of a factor below 1/2 the exponent
+// that `de` adds is negative and borrows from the sign bit above it, which the
+// bit below the sign tells (|exponent| <= 129 of 2047)
+SOFT_HD uint32_t soft_sign(const SoftRec& c) { return (c.de ^ (c.de << 1)) & 0x80000000u; }
+
 // record of a divisor (div) or factor; idx: where the kernels find its value
 inline SoftRec soft_record(double v, bool div, uint32_t idx) {
   SoftRec r{0, 0, 0, idx};

@@ -39,7 +39,7 @@ __device__ __forceinline__ SoftArg soft_arg(double x) {
 __device__ __forceinline__ bool is_zero(double x) {
   return ((uint32_t)__double2hiint(x) << 1 | (uint32_t)__double2loint(x)) == 0u;
 }
-// a zero's quotient or product keeps its sign (the other operand's sign is in `flip`)
+// a zero's quotient or product keeps its sign (flip: the other operand's, in the top bit)
 __device__ __forceinline__ double signed_zero(double x, uint32_t flip) {
   return soft_double(((uint32_t)__double2hiint(x) ^ flip) & 0x80000000u, 0u);
 }
@@ -80,7 +80,7 @@ struct VelOps {
       p.n = soft_mul(x.n, c);
       p.x = soft_join(p.n);
     } else if (fits && is_zero(x.x)) {
-      p.x = signed_zero(x.x, c.de);
+      p.x = signed_zero(x.x, soft_sign(c));
     } else {
       p.x = slow_mul(x.x, value());
     }
@@ -143,13 +143,13 @@ struct LeapOps {
   static __device__ __forceinline__ double times(const Args& a, double x, const SoftRec& c) {
     const SoftArg v = soft_arg(x);
     if (v.ok && (int)c.hi < 0) return soft_join(soft_mul(v.n, c));
-    return is_zero(x) ? signed_zero(x, c.de) : __dmul_rn(__ldg(a.vals + c.idx), x);
+    return is_zero(x) ? signed_zero(x, soft_sign(c)) : __dmul_rn(__ldg(a.vals + c.idx), x);
   }
   // (c * x) / d, both roundings
   static __device__ __forceinline__ double scaled(const Args& a, const SoftArg& v, const SoftRec& c, const SoftRec& d) {
     if (v.ok && (int)(c.hi & d.hi) < 0)
       return soft_join(soft_div(soft_mul(v.n, c), d, [&] { return __ldg(a.vals + d.idx); }));
-    if (is_zero(v.x)) return signed_zero(v.x, c.de);
+    if (is_zero(v.x)) return signed_zero(v.x, soft_sign(c));
     const double y = __dmul_rn(__ldg(a.vals + c.idx), v.x);
     return is_zero(y) ? y : slow_div(y, __ldg(a.vals + d.idx), a.dtab);
   }
