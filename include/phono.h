@@ -248,9 +248,7 @@ int phono_upload_surface(phono_handle *h, int first, int count, const void *host
 int phono_elem_size(const phono_handle *h);
 
 /* Kinetic and strain energy of the current state, FP64 accumulation in a
- * fixed order (the same state gives the same bits; F32K meshes of 200,000
- * nodes and more form their terms in unevaluated pairs of floats, whose sums
- * are as accurate): out[0] = sum rho v^2 / 2
+ * fixed order (the same state gives the same bits): out[0] = sum rho v^2 / 2
  * over the interior displacement points, out[1] = sum T:e / 2 over the
  * reference's stress points, unit weights (no cell volume).  Blocks until
  * done.  No reference counterpart (error metric). */

@@ -20,7 +20,7 @@ cudaError_t launch_step_f32k(const StepArgs<float>& a, int tj, int n_face_blocks
 cudaError_t configure_step_f64v(int tj);
 cudaError_t launch_step_f64v(const StepArgs<double>& a, int tj, int n_face_blocks, cudaStream_t st);
 cudaError_t launch_split(int precision, const void* args, bool stress, bool after_kernel, cudaStream_t st);
-cudaError_t launch_energy(const EnergyArgs& a, double2* partial, int nblocks, double* out, bool pairs, cudaStream_t st);
+cudaError_t launch_energy(const EnergyArgs& a, double2* partial, int nblocks, double* out, int march_blocks, cudaStream_t st);
 cudaError_t launch_lattice_ids(uint8_t* mat, const Geo& g, int pitch, int ncx, int ncy, const double* radius,
                                const uint8_t* kind, int depth, uint8_t host, cudaStream_t st);
 cudaError_t launch_unpack_ids(uint8_t* mat, const Geo& g, const uint8_t* dense, long long first, int rows, cudaStream_t st);
@@ -55,9 +55,10 @@ void set_last_error(const char* msg) { g_err = msg; }
 
 static const int kGraphSteps = 12;  // multiple of 2 and 3: buffer rotations line up
 static const int kEnergyBlocks = 1024;
-// FP32 meshes from here on sum their energy in pairs of floats: on smaller
-// ones FP64 takes less than the launches around it
-static const double kEnergyPairNodes = 200000;
+// FP32 meshes from here on sum their energy marching along x: smaller ones have
+// too few columns for it (energy.cu: as fast at 108 k nodes, 78.6 to 67.4 us at
+// 207 k)
+static const double kEnergyMarchNodes = 200000;
 
 // the FP64 velocity form's two-launch step multiplies by constants in integer
 // arithmetic from here on (split_step.cu: 35 k nodes 9.5 us a step without and
@@ -1289,17 +1290,11 @@ int phono_energy(phono_handle* h, double out[2]) {
   a.mat = h->mat;
   a.tab = h->tab13;
   a.nmat = h->nmat;
-  const double n = (double)h->d.nx * h->d.ny * h->d.nz;
-  bool pairs = h->es == 4 && n >= kEnergyPairNodes;
-  for (;; pairs = false) {
-    CK(launch_energy(a, h->partial, kEnergyBlocks, h->energy_out, pairs, h->stream));
-    CK(cudaMemcpyAsync(out, h->energy_out, sizeof(double) * 2, cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaStreamSynchronize(h->stream));
-    // terms of 1e-6 to 1e30 on average keep every intermediate of the pairs
-    // within FP32's range (a pair's low part is 2^-48 of its term); a zero, tiny,
-    // huge or non-finite energy is computed again in FP64
-    if (!pairs || (out[0] > 1e-6 * n && out[0] < 1e30 && out[1] > 1e-6 * n && out[1] < 1e30)) return PHONO_OK;
-  }
+  const bool march = h->es == 4 && (double)h->d.nx * h->d.ny * h->d.nz >= kEnergyMarchNodes;
+  CK(launch_energy(a, h->partial, kEnergyBlocks, h->energy_out, march ? 2 * sm_count() : 0, h->stream));
+  CK(cudaMemcpyAsync(out, h->energy_out, sizeof(double) * 2, cudaMemcpyDeviceToHost, h->stream));
+  CK(cudaStreamSynchronize(h->stream));
+  return PHONO_OK;
 }
 
 int phono_reset(phono_handle* h) {

@@ -126,62 +126,20 @@ __global__ void __launch_bounds__(EN_THREADS, 4) energy_partial_kernel(EnergyArg
 }
 
 // ---------------------------------------------------------------------------
-// FP32 fields of large meshes: the same sums in pairs of floats (an
-// unevaluated sum h + l, 48 bits), on the FP32 pipe, whose rate is 64 times
-// the FP64 pipe's.  Differences of floats are exact pairs; constants enter as
-// three floats (72 bits) and the low parts' product is kept in squares, so
-// that no rounding is biased; a product or sum of pairs is off by 2^-47 of its
-// value at random, which over the terms of a large mesh averages out below
-// the FP64 rounding of the result (against 128-bit sums on meshes of 0.2 to 3 M
-// nodes: 2.6e-16 at most, 2.7e-16 for the FP64 kernel).  A thread's sums go to
-// FP64 every few planes (every 32: 9.6e-16).  Terms must stay clear of
-// the FP32 range: the caller checks the result and repeats in FP64 otherwise.
+// FP32 fields of large meshes: the same FP64 sums, marching along x with the
+// values of the last plane in registers, and FP32 values widened by integer
+// instructions: the conversion instruction runs at the FP64 pipe's rate.
 // ---------------------------------------------------------------------------
-struct Pair {
-  float h, l;
-};
-__device__ __forceinline__ Pair pair_diff(float x, float y) {  // x - y, exact (Knuth's two-sum)
-  const float d = __fsub_rn(x, y), t = __fsub_rn(d, x);
-  return Pair{d, __fsub_rn(__fsub_rn(x, __fsub_rn(d, t)), __fadd_rn(y, t))};
-}
-__device__ __forceinline__ Pair pair_fast(float h, float l) {  // |h| >= |l|
-  const float s = __fadd_rn(h, l);
-  return Pair{s, __fsub_rn(l, __fsub_rn(s, h))};
-}
-__device__ __forceinline__ Pair pair_add(Pair x, Pair y) {
-  const float s = __fadd_rn(x.h, y.h), t = __fsub_rn(s, x.h);
-  const float e = __fadd_rn(__fsub_rn(x.h, __fsub_rn(s, t)), __fsub_rn(y.h, t));
-  return pair_fast(s, __fadd_rn(e, __fadd_rn(x.l, y.l)));
-}
-__device__ __forceinline__ Pair pair_scale(Pair x, const float3 c) {  // x times a constant of three floats
-  const float p = __fmul_rn(x.h, c.x);
-  float e = __fmaf_rn(x.h, c.x, -p);
-  e = __fmaf_rn(x.h, c.z, e);
-  e = __fmaf_rn(x.l, c.y, e);
-  e = __fmaf_rn(x.h, c.y, e);
-  e = __fmaf_rn(x.l, c.x, e);
-  return pair_fast(p, e);
-}
-// sum += x * y
-__device__ __forceinline__ void pair_acc(Pair& sum, Pair x, Pair y) {
-  const float p = __fmul_rn(x.h, y.h);
-  float e = __fmaf_rn(x.h, y.h, -p);
-  e = __fmaf_rn(x.l, y.l, e);
-  e = __fmaf_rn(x.h, y.l, e);
-  e = __fmaf_rn(x.l, y.h, e);
-  const float s = __fadd_rn(sum.h, p), t = __fsub_rn(s, sum.h);
-  sum.l = __fadd_rn(sum.l, __fadd_rn(__fadd_rn(__fsub_rn(sum.h, __fsub_rn(s, t)), __fsub_rn(p, t)), e));
-  sum.h = s;
-}
-__device__ __forceinline__ float3 triple(double c) {
-  const float x = __double2float_rn(c);
-  const double r = __dsub_rn(c, (double)x);
-  const float y = __double2float_rn(r);
-  return make_float3(x, y, __double2float_rn(__dsub_rn(r, (double)y)));
+// a call, so that the conversion is not done ahead of the branches around it
+__device__ __noinline__ double convert(float x) { return (double)x; }
+__device__ __forceinline__ double widen(float x) {
+  const uint32_t u = __float_as_uint(x);
+  if ((u & 0x7fffffffu) - 0x00800000u < 0x7f000000u)  // normal: the exponent rebiased, the fraction moved
+    return __hiloint2double((int)((((uint32_t)((int)u >> 3)) & 0x8fffffffu) + 0x38000000u), (int)(u << 29));
+  return u << 1 ? convert(x) : __hiloint2double((int)u, 0);
 }
 
 constexpr int EN_PLANES = 64;  // most planes of an item
-constexpr int EN_FLUSH = 4;    // planes after which a thread's sums go to FP64: a pair's low part drifts by 2^-49 a term
 
 // what plane i of a column adds to the last plane's values
 struct EnPlane {
@@ -195,16 +153,16 @@ struct EnPlane {
 // A block takes (column tile of 8 rows x 32 z, 1/nit of the planes) items in a
 // fixed order; a warp owns a row of the tile, a lane a z column, and marches
 // along x with the values of the last plane in registers and those of the next
-// one on their way.  256x256x128 cells: 191 us, 1510 for the FP64 form, which the
-// FP64 pipe bounds; without the loads a plane ahead 380 us.  Bound by
-// instruction issue (71% of the slots, 430 instructions a node).
-__global__ void __launch_bounds__(EN_THREADS, 2) energy_pair_kernel(EnergyArgs a, int nit, double2* __restrict__ partial) {
-  extern __shared__ float4 ptab[];  // nmat rows of EN_COLS constants (x, y, z of a float4), then the x spacings of an item
-  float4* px = ptab + a.nmat * EN_COLS;
-  for (int q = threadIdx.x; q < a.nmat * EN_COLS; q += EN_THREADS) {
-    const float3 c = triple(en_coef(a.tab + 13 * (q / EN_COLS), q % EN_COLS));
-    ptab[q] = make_float4(c.x, c.y, c.z, 0.f);
-  }
+// one on their way.  Bound by the FP64 pipe: 39 operations a node, 0.54 ms of
+// its issue at 257x257x129 nodes.  us a call, energy_partial_kernel<float> / here:
+// 55 k nodes 41.6 / 53.7, 108 k 53.4 / 53.1, 207 k 78.6 / 67.4, 845 k 165 / 117,
+// 8.5 M 1063 / 631.  (Terms formed in pairs of floats took 216 there, but a
+// term was off by up to 2^-45, which shows when a state is a few values; here
+// it is as good as the other form's.)
+__global__ void __launch_bounds__(EN_THREADS, 2) energy_march_kernel(EnergyArgs a, int nit, double2* __restrict__ partial) {
+  extern __shared__ double etab[];  // nmat rows of EN_COLS constants, then the x spacings of an item
+  double* px = etab + a.nmat * EN_COLS;
+  for (int q = threadIdx.x; q < a.nmat * EN_COLS; q += EN_THREADS) etab[q] = en_coef(a.tab + 13 * (q / EN_COLS), q % EN_COLS);
   const Geo& g = a.g;
   const int nx = g.nx, ny = g.ny, nz = g.nz;
   const int lane = threadIdx.x & 31, row = threadIdx.x >> 5;
@@ -217,20 +175,19 @@ __global__ void __launch_bounds__(EN_THREADS, 2) energy_pair_kernel(EnergyArgs a
     __syncthreads();
     for (int q = threadIdx.x; q < 2 * (i1 - i0); q += EN_THREADS) {
       const int i = i0 + (q >> 1);  // 1/sdx[i-1], 1/fdx[i]
-      const float3 c = triple(q & 1 ? __ldg(a.rfdx + i) : (i >= 1 && i <= nx - 2 ? __ldg(a.rsdx + i - 1) : 0.0));
-      px[q] = make_float4(c.x, c.y, c.z, 0.f);
+      px[q] = q & 1 ? __ldg(a.rfdx + i) : (i >= 1 && i <= nx - 2 ? __ldg(a.rsdx + i - 1) : 0.0);
     }
     __syncthreads();
     const int j = jt * EN_WARPS + row, k = kt * 32 + lane;
     if (j > ny - 2 || k > nz - 2) continue;  // no term there
     const bool j_n = j >= 1, jy = j >= 1 && j <= ny - 3, kn = k >= 1, kz = k <= nz - 3;
-    const float3 rsy = triple(j_n ? __ldg(a.rsdy + j - 1) : 0.0), rfy = triple(__ldg(a.rfdy + j));
-    const float3 rsz = triple(kn ? __ldg(a.rsdz + k - 1) : 0.0), rfz = triple(__ldg(a.rfdz + k));
+    const double rsy = j_n ? __ldg(a.rsdy + j - 1) : 0.0, rfy = __ldg(a.rfdy + j);
+    const double rsz = kn ? __ldg(a.rsdz + k - 1) : 0.0, rfz = __ldg(a.rfdz + k);
     const long long o = g.o0 + (long long)i0 * sx + (long long)j * sy + k;
     const float *ux = (const float*)a.ux + o, *uy = (const float*)a.uy + o, *uz = (const float*)a.uz + o;
     const float *vx = (const float*)a.vx + o, *vy = (const float*)a.vy + o, *vz = (const float*)a.vz + o;
     const uint8_t* m = a.mat + g.mo0 + (long long)i0 * msx + (long long)j * msy + k;
-    float xm = __ldg(ux - sx), y0 = __ldg(uy), z0 = __ldg(uz);
+    double xm = widen(__ldg(ux - sx)), y0 = widen(__ldg(uy)), z0 = widen(__ldg(uz));
     int id = m[0], id_z = m[1], id_y = m[msy], id_yz = m[msy + 1];
     // the padding makes every neighbour of planes up to nx-1 readable
     auto read = [&] {
@@ -243,46 +200,36 @@ __global__ void __launch_bounds__(EN_THREADS, 2) energy_pair_kernel(EnergyArgs a
       ux += sx, uy += sx, uz += sx, vx += sx, vy += sx, vz += sx, m += msx;
       return p;
     };
-    Pair k2{0.f, 0.f}, s2{0.f, 0.f};
-    auto coef = [&](int mid, int q) {
-      const float4 c = ptab[EN_COLS * mid + q];
-      return make_float3(c.x, c.y, c.z);
-    };
+    auto square = [&](double& sum, int mid, int q, double x) { sum = __fma_rn(__dmul_rn(etab[EN_COLS * mid + q], x), x, sum); };
     EnPlane next = read();
     for (int i = i0; i < i1; i++) {
       const EnPlane p = next;
       if (i + 1 < i1) next = read();
       const bool i_n = i >= 1, in = i_n && j_n;  // i <= nx-2 here
+      const double x0 = widen(p.x0), y1 = widen(p.y1), z1 = widen(p.z1);
       // kinetic energy
-      auto kinetic = [&](int mid, float v) { pair_acc(k2, pair_scale(Pair{v, 0.f}, coef(mid, 9)), Pair{v, 0.f}); };
-      if (j_n && i <= nx - 3) kinetic(p.id, p.vx);
-      if (i_n && jy) kinetic(id_y, p.vy);
-      if (in && kz) kinetic(id_z, p.vz);
+      if (j_n && i <= nx - 3) square(ek, p.id, 9, widen(p.vx));
+      if (i_n && jy) square(ek, id_y, 9, widen(p.vy));
+      if (in && kz) square(ek, id_z, 9, widen(p.vz));
       if (kn) {
-        const float4 sx4 = px[2 * (i - i0)], fx4 = px[2 * (i - i0) + 1];
-        const float3 rsx = make_float3(sx4.x, sx4.y, sx4.z), rfx = make_float3(fx4.x, fx4.y, fx4.z);
+        const double rsx = px[2 * (i - i0)], rfx = px[2 * (i - i0) + 1];
         if (in) {
-          const Pair e1 = pair_scale(pair_diff(p.x0, xm), rsx), e2 = pair_scale(pair_diff(y0, p.yj), rsy),
-                     e3 = pair_scale(pair_diff(z0, p.zk), rsz);
-          pair_acc(s2, pair_add(pair_scale(e1, coef(id, 0)), pair_add(pair_scale(e2, coef(id, 3)), pair_scale(e3, coef(id, 4)))), e1);
-          pair_acc(s2, pair_add(pair_scale(e2, coef(id, 1)), pair_scale(e3, coef(id, 5))), e2);
-          pair_acc(s2, pair_scale(e3, coef(id, 2)), e3);
+          const double* c = etab + EN_COLS * id;
+          const double e1 = __dmul_rn(__dsub_rn(x0, xm), rsx), e2 = __dmul_rn(__dsub_rn(y0, widen(p.yj)), rsy),
+                       e3 = __dmul_rn(__dsub_rn(z0, widen(p.zk)), rsz);
+          es = __fma_rn(__fma_rn(c[0], e1, __fma_rn(c[3], e2, __dmul_rn(c[4], e3))), e1, es);
+          es = __fma_rn(__fma_rn(c[1], e2, __dmul_rn(c[5], e3)), e2, es);
+          square(es, id, 2, e3);
         }
-        auto shear = [&](int mid, int q, Pair d1, float3 r1, Pair d2, float3 r2) {
-          const Pair gam = pair_add(pair_scale(d1, r1), pair_scale(d2, r2));
-          pair_acc(s2, pair_scale(gam, coef(mid, q)), gam);
+        auto shear = [&](int mid, int q, double d1, double r1, double d2, double r2) {
+          square(es, mid, q, __fma_rn(d1, r1, __dmul_rn(d2, r2)));
         };
-        if (i_n) shear(id_yz, 6, pair_diff(p.yk, y0), rfz, pair_diff(p.zj, z0), rfy);
-        if (j_n) shear(p.id_z, 7, pair_diff(p.xk, p.x0), rfz, pair_diff(p.z1, z0), rfx);
-        shear(p.id_y, 8, pair_diff(p.xj, p.x0), rfy, pair_diff(p.y1, y0), rfx);
+        if (i_n) shear(id_yz, 6, __dsub_rn(widen(p.yk), y0), rfz, __dsub_rn(widen(p.zj), z0), rfy);
+        if (j_n) shear(p.id_z, 7, __dsub_rn(widen(p.xk), x0), rfz, __dsub_rn(z1, z0), rfx);
+        shear(p.id_y, 8, __dsub_rn(widen(p.xj), x0), rfy, __dsub_rn(y1, y0), rfx);
       }
-      xm = p.x0, y0 = p.y1, z0 = p.z1;
+      xm = x0, y0 = y1, z0 = z1;
       id = p.id, id_z = p.id_z, id_y = p.id_y, id_yz = p.id_yz;
-      if ((i + 1 - i0) % EN_FLUSH == 0 || i + 1 == i1) {
-        ek = __dadd_rn(ek, __dadd_rn((double)k2.h, (double)k2.l));
-        es = __dadd_rn(es, __dadd_rn((double)s2.h, (double)s2.l));
-        k2 = s2 = Pair{0.f, 0.f};
-      }
     }
   }
   block_partial(ek, es, partial + blockIdx.x);
@@ -313,11 +260,12 @@ __global__ void __launch_bounds__(EN_THREADS) energy_final_kernel(const double2*
 }
 
 // partial must hold nblocks double2 values; out two doubles (device).
-// pairs: FP32 fields in pairs of floats (energy_pair_kernel)
-cudaError_t launch_energy(const EnergyArgs& a, double2* partial, int nblocks, double* out, bool pairs, cudaStream_t st) {
-  if (pairs) {
-    const size_t smem = ((size_t)a.nmat * EN_COLS + 2 * EN_PLANES) * sizeof(float4);
-    nblocks = nblocks < 304 ? nblocks : 304;  // two resident blocks on each of 152 SMs
+// march_blocks > 0: FP32 fields by energy_march_kernel in that many blocks
+// (at most nblocks)
+cudaError_t launch_energy(const EnergyArgs& a, double2* partial, int nblocks, double* out, int march_blocks, cudaStream_t st) {
+  if (march_blocks > 0) {
+    const size_t smem = ((size_t)a.nmat * EN_COLS + 2 * EN_PLANES) * sizeof(double);
+    nblocks = nblocks < march_blocks ? nblocks : march_blocks;
     // x parts: as many items as fill the blocks' last round best
     const int tiles = ((a.g.nz + 30) / 32) * ((a.g.ny - 1 + EN_WARPS - 1) / EN_WARPS);
     const int least = (a.g.nx - 1 + EN_PLANES - 1) / EN_PLANES, most = (a.g.nx - 1 + 7) / 8;
@@ -329,7 +277,7 @@ cudaError_t launch_energy(const EnergyArgs& a, double2* partial, int nblocks, do
       const double use = 1.0 / (rounds * ((double)(a.g.nx - 1) / n + 2.0));
       if (use > best) best = use, nit = n;
     }
-    energy_pair_kernel<<<nblocks, EN_THREADS, smem, st>>>(a, nit, partial);
+    energy_march_kernel<<<nblocks, EN_THREADS, smem, st>>>(a, nit, partial);
   } else {
     const size_t smem = (size_t)a.nmat * EN_COLS * sizeof(double);
     if (a.f32)
