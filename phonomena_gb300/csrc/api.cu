@@ -204,9 +204,12 @@ static int check_materials(const phono_handle* h, const uint8_t* mat, const doub
 // say) at a time (us an upload, strided / staged: 160x128x64 cells 416 / 89,
 // 256x256x128 2334 / 539, 512x512x256 11300 / 4100).  One stage a device, made at
 // the first such upload and given back with the device's last handle; an upload
-// holds it until its copies are done.
+// holds it for its own copies alone: it waits for the handle's earlier work
+// before.  Handles come and go meanwhile (an upload's handle is a user, so that
+// the stage is not given back under it).
 struct IdStage {
-  std::mutex m;
+  std::mutex upload;  // held for an upload's copies
+  std::mutex count;   // held while a handle joins or leaves
   int users = 0;
   uint8_t* p = nullptr;
 };
@@ -216,14 +219,14 @@ constexpr size_t kStageBytes = 4 << 20, kStagedFrom = 256 << 10;
 static void join_stage(phono_handle* h) {
   int dev = -1;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 32) return;
-  std::lock_guard<std::mutex> hold(g_stage[dev].m);
+  std::lock_guard<std::mutex> hold(g_stage[dev].count);
   g_stage[dev].users++;
   h->dev = dev;
 }
 static void leave_stage(phono_handle* h) {
   if (h->dev < 0) return;
   IdStage& g = g_stage[h->dev];
-  std::lock_guard<std::mutex> hold(g.m);
+  std::lock_guard<std::mutex> hold(g.count);
   if (--g.users == 0 && g.p) {
     cudaFree(g.p);
     g.p = nullptr;
@@ -236,8 +239,9 @@ static int upload_staged(phono_handle* h, const uint8_t* mat, bool& staged) {
   const int nz = h->d.nz;
   const long long rows = (long long)h->d.nx * h->d.ny, step = (long long)kStageBytes / nz;
   if (h->dev < 0 || (size_t)rows * nz < kStagedFrom || step < 1) return PHONO_OK;
+  CK(cudaStreamSynchronize(h->stream));
   IdStage& g = g_stage[h->dev];
-  std::lock_guard<std::mutex> hold(g.m);
+  std::lock_guard<std::mutex> hold(g.upload);
   if (!g.p && cudaMalloc(&g.p, kStageBytes) != cudaSuccess) {
     g.p = nullptr;
     cudaGetLastError();

@@ -1,0 +1,46 @@
+"""Host code of the C ABI on a stand-in CUDA runtime."""
+import threading
+
+import pytest
+
+from host_abi import Handle, compile_host_abi
+
+
+@pytest.fixture(scope="module")
+def lib():
+    return compile_host_abi()
+
+
+@pytest.fixture
+def L(lib):
+    lib.fake_reset()
+    return lib
+
+
+def test_handles_do_not_wait_for_another_ones_steps(L):
+    """While an upload waits for the steps its own handle has queued, handles
+    of another thread are made, given ids of any size and destroyed."""
+    busy = Handle(L, (80, 70, 60), max_steps=1)  # ids above 256 KB: staged
+    L.fake_hold(busy.stream(), 1)
+    done = threading.Event()
+
+    def others():
+        for shape in ((9, 8, 7), (81, 70, 60)):
+            h = Handle(L, shape, max_steps=1)
+            assert h.rc == 0 and h.set_ids(5) == 0 and h.ids_arrived()
+            h.close()
+        done.set()
+
+    upload = threading.Thread(target=busy.set_ids, args=(3,))
+    upload.start()
+    upload.join(0.2)
+    assert upload.is_alive()
+    worker = threading.Thread(target=others)
+    worker.start()
+    free = done.wait(5.0)
+    L.fake_hold(busy.stream(), 0)
+    upload.join()
+    worker.join()
+    assert free and busy.ids_arrived()
+    busy.close()
+    assert L.fake_bytes(0) == 0 and L.fake_broken() == 0
