@@ -89,7 +89,8 @@ struct phono_handle {
   DivTable dtab{};        // FP64 leapfrog: reciprocal pairs of the mesh's divisors (tab null: none)
   std::vector<double> sp_host[6];  // raw spacings (ABC coefficients)
   uint8_t* mat = nullptr;
-  int dev = -1;              // the handle counts among the users of this device's stage (-1: not yet)
+  int dev = 0;               // the device the handle was made on
+  bool in_stage = false;     // it counts among the users of that device's stage
   void* tab = nullptr;       // 16 R per material
   double* tab13 = nullptr;   // raw table (energy)
   double* src = nullptr;
@@ -217,28 +218,44 @@ static IdStage g_stage[32];
 constexpr size_t kStageBytes = 4 << 20, kStagedFrom = 256 << 10;
 
 static void join_stage(phono_handle* h) {
-  int dev = -1;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 32) return;
-  std::lock_guard<std::mutex> hold(g_stage[dev].count);
-  g_stage[dev].users++;
-  h->dev = dev;
+  if (h->dev < 0 || h->dev >= 32) return;
+  std::lock_guard<std::mutex> hold(g_stage[h->dev].count);
+  g_stage[h->dev].users++;
+  h->in_stage = true;
 }
 static void leave_stage(phono_handle* h) {
-  if (h->dev < 0) return;
+  if (!h->in_stage) return;
   IdStage& g = g_stage[h->dev];
   std::lock_guard<std::mutex> hold(g.count);
   if (--g.users == 0 && g.p) {
     cudaFree(g.p);
     g.p = nullptr;
   }
-  h->dev = -1;
+  h->in_stage = false;
 }
+
+// A launch goes to a stream of the current device only; copies do not mind.
+// Calls that were copies make the handle's device current for their launches.
+struct OnDevice {
+  int back = -1;
+  cudaError_t err;
+  explicit OnDevice(int dev) {
+    int now = dev;
+    err = cudaGetDevice(&now);
+    if (err == cudaSuccess && now != dev && (err = cudaSetDevice(dev)) == cudaSuccess) back = now;
+  }
+  ~OnDevice() {
+    if (back >= 0) cudaSetDevice(back);
+  }
+};
 
 // `staged`: the ids are in place (else nothing was done)
 static int upload_staged(phono_handle* h, const uint8_t* mat, bool& staged) {
   const int nz = h->d.nz;
   const long long rows = (long long)h->d.nx * h->d.ny, step = (long long)kStageBytes / nz;
-  if (h->dev < 0 || (size_t)rows * nz < kStagedFrom || step < 1) return PHONO_OK;
+  if (!h->in_stage || (size_t)rows * nz < kStagedFrom || step < 1) return PHONO_OK;
+  const OnDevice here(h->dev);
+  CK(here.err);
   CK(cudaStreamSynchronize(h->stream));
   IdStage& g = g_stage[h->dev];
   std::lock_guard<std::mutex> hold(g.upload);
@@ -635,6 +652,8 @@ static cudaError_t copy3d(phono_handle* h, void* dev, void* host, int c, bool to
   // of 6500 nodes FP64, 58 KB a field: 1284 us, 1309 with the kernel)
   const size_t bytes = (size_t)ex * ey * ez * h->es;
   if (!to_dev && bytes >= kReadbackBytes && (uintptr_t)host % h->es == 0) {
+    const OnDevice here(h->dev);
+    if (here.err != cudaSuccess) return here.err;
     if (void* to = pinned_address(host, bytes)) {
       cudaError_t e = launch_readback((char*)dev + h->g.o0 * h->es, h->g.sx, h->g.sy, ex, ey, ez, h->es, to, h->stream);
       return e == cudaSuccess ? cudaStreamSynchronize(h->stream) : e;
@@ -937,7 +956,8 @@ int phono_create(const phono_desc* d, phono_handle** out) {
     return PHONO_ERR_ARG;
   }
 
-  cudaError_t e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
+  cudaError_t e = cudaGetDevice(&h->dev);
+  if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
   if (e != cudaSuccess) {
     delete h;
     return fail(PHONO_ERR_CUDA, std::string("cudaStreamCreate: ") + cudaGetErrorString(e));

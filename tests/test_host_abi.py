@@ -1,6 +1,8 @@
 """Host code of the C ABI on a stand-in CUDA runtime."""
+import ctypes
 import threading
 
+import numpy as np
 import pytest
 
 from host_abi import Handle, compile_host_abi
@@ -43,4 +45,29 @@ def test_handles_do_not_wait_for_another_ones_steps(L):
     worker.join()
     assert free and busy.ids_arrived()
     busy.close()
+    assert L.fake_bytes(0) == 0 and L.fake_broken() == 0
+
+
+def test_calls_with_another_device_current(L):
+    """Uploads of ids and reads into pinned memory use the handle's device and
+    leave the caller's current."""
+    shape = (80, 70, 60)
+    h = Handle(L, shape, max_steps=1)
+    field = np.random.default_rng(1).standard_normal((79, 70, 60)).astype(np.float32)
+    assert L.phono_upload(h.h, 0, field.ctypes.data, field.nbytes) == 0
+    got = np.zeros_like(field)
+    L.fake_pin(got.ctypes.data, got.nbytes)
+    small = Handle(L, (9, 8, 7), max_steps=1)
+    L.fake_device(1)
+    try:
+        assert h.set_ids(7) == 0, L.phono_last_error()
+        assert h.ids_arrived()
+        reads = L.fake_count(b"readback")
+        assert L.phono_download(h.h, 0, got.ctypes.data, got.nbytes) == 0, L.phono_last_error()
+        assert L.fake_count(b"readback") == reads + 1 and np.array_equal(got, field)
+        assert L.fake_current() == 1 and L.fake_bytes(1) == 0
+        h.close()
+        small.close()
+    finally:
+        L.fake_device(0)
     assert L.fake_bytes(0) == 0 and L.fake_broken() == 0
