@@ -148,8 +148,8 @@ static void leave_stage(phono_handle* h);
 static void release(phono_handle* h) {
   if (!h) return;
   if (h->batch) batch_detach(h->batch, h);
-  if (h->graph) cudaGraphExecDestroy(h->graph);
   if (h->stream) cudaStreamSynchronize(h->stream);
+  if (h->graph) cudaGraphExecDestroy(h->graph);
   for (void* p : h->allocs) cudaFree(p);
   leave_stage(h);
   if (h->ev0) cudaEventDestroy(h->ev0);
@@ -1694,6 +1694,7 @@ static int batch_rebuild(phono_batch* b) {
   for (int s : act) {
     phono_handle* h = b->slot[s];
     if (!h->own.tj || h->split || (h->own_limit && limit <= 2 * h->own_limit && h->own_limit <= 2 * limit)) continue;
+    if (b->igraph[s]) CK(cudaStreamSynchronize(b->stream));  // its graph may still run
     int rc = reshape_own(h, limit);
     if (rc) return rc;
     drop_igraph(b, s);

@@ -71,3 +71,26 @@ def test_calls_with_another_device_current(L):
     finally:
         L.fake_device(0)
     assert L.fake_bytes(0) == 0 and L.fake_broken() == 0
+
+
+def test_graphs_are_not_destroyed_while_they_run(L):
+    """An instance whose segments are cut anew, between calls that do not wait,
+    because a larger one has run out."""
+    small, large = Handle(L, (30, 21, 13)), Handle(L, (200, 200, 40))
+    b = ctypes.c_void_p()
+    assert L.phono_batch_create(2, 1, 4, ctypes.byref(b)) == 0
+    assert L.phono_batch_add(b, small.h, 90) >= 0 and L.phono_batch_add(b, large.h, 24) >= 0
+    graphs = L.fake_count(b"graph")
+    assert L.phono_batch_step(b, 24) == 0 and L.phono_batch_step(b, 24) == 0
+    assert L.fake_count(b"graph") > graphs and L.fake_broken() == 0
+    assert L.phono_batch_sync(b) == 0
+    L.phono_batch_destroy(b)
+    small.close()
+    large.close()
+
+
+def test_a_handle_is_destroyed_with_steps_queued(L):
+    h = Handle(L, (30, 21, 13))
+    assert L.phono_step(h.h, 24) == 0
+    h.close()
+    assert L.fake_broken() == 0
