@@ -99,10 +99,17 @@ typedef struct phono_desc {
 typedef struct phono_handle phono_handle;
 
 /* Device bytes phono_create would allocate for a mesh of nx*ny*nz nodes with
- * these settings (each allocation rounded up to 512 bytes): what a caller
- * admitting simulations against a memory budget charges per handle.  No
- * reference counterpart. */
+ * these settings and the default tile shape (each allocation rounded up to 512
+ * bytes): what a caller admitting simulations against a memory budget charges
+ * per handle.  No reference counterpart. */
 int phono_footprint(int nx, int ny, int nz, int precision, int max_steps, int record_every, size_t *bytes);
+/* The same for a handle made with this tile shape: FP64 ones with a shape have
+ * no stress window (up to 128 MB, or 36 planes of six stresses where those are
+ * more); phono_set_tiling and phono_set_segments free that of a handle made
+ * without.  Beside the handles' own memory a device holds one 4 MB stage while
+ * it has handles and one of them was given 256 KB of material ids or more. */
+int phono_footprint_shaped(int nx, int ny, int nz, int precision, int max_steps, int record_every, int tile_j, int x_segment,
+                           size_t *bytes);
 
 /* Allocate the device state (zero fields) for one simulation.
  * Replaces BaseSolver.init (base_solver.py:194-222). */

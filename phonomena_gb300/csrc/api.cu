@@ -579,8 +579,9 @@ static ConstBlock const_block(int nx, int ny, int nz, int precision) {
 }
 
 // Bytes of device memory phono_create allocates for a handle (each cudaMalloc
-// rounded up to 512 bytes).
-static size_t handle_bytes(int nx, int ny, int nz, int precision, int max_steps, int record_every) {
+// rounded up to 512 bytes).  shaped: it is made with a tile shape, and has no
+// stress window.
+static size_t handle_bytes(int nx, int ny, int nz, int precision, int max_steps, int record_every, bool shaped) {
   const int es = precision == PHONO_F32K ? 4 : 8;
   const int nbuf = precision == PHONO_F64 ? 3 : 2;
   auto r = [](size_t b) { return (b + 511) / 512 * 512; };
@@ -595,7 +596,7 @@ static size_t handle_bytes(int nx, int ny, int nz, int precision, int max_steps,
   const int nrec = record_every > 0 ? max_steps / record_every : 0;
   if (nrec > 0) total += r((size_t)nrec * nx * ny * es);
   total += r(sizeof(int) * 2) + r(sizeof(double2) * kEnergyBlocks) + r(sizeof(double) * 2);
-  total += r(split_bytes(nx, ny, nz, precision));
+  if (!shaped) total += r(split_bytes(nx, ny, nz, precision));
   return total;
 }
 
@@ -898,15 +899,20 @@ extern "C" {
 
 int phono_abi_version(void) { return PHONO_ABI_VERSION; }
 
-int phono_footprint(int nx, int ny, int nz, int precision, int max_steps, int record_every, size_t* bytes) {
+int phono_footprint_shaped(int nx, int ny, int nz, int precision, int max_steps, int record_every, int tile_j, int x_segment,
+                           size_t* bytes) {
   if (!bytes) return fail(PHONO_ERR_ARG, "bytes is NULL");
   if (nx < 3 || ny < 3 || nz < 3) return fail(PHONO_ERR_ARG, "nx, ny, nz must be >= 3 mesh nodes");
   if ((long long)nx * ny * nz > (1LL << 34)) return fail(PHONO_ERR_ARG, "grid too large");
   if (precision != PHONO_F64 && precision != PHONO_F32K && precision != PHONO_F64V)
     return fail(PHONO_ERR_ARG, "unknown precision");
   if (max_steps < 0 || record_every < 0) return fail(PHONO_ERR_ARG, "max_steps and record_every must be >= 0");
-  *bytes = handle_bytes(nx, ny, nz, precision, max_steps, record_every);
+  *bytes = handle_bytes(nx, ny, nz, precision, max_steps, record_every, tile_j || x_segment);
   return PHONO_OK;
+}
+
+int phono_footprint(int nx, int ny, int nz, int precision, int max_steps, int record_every, size_t* bytes) {
+  return phono_footprint_shaped(nx, ny, nz, precision, max_steps, record_every, 0, 0, bytes);
 }
 
 const char* phono_last_error(void) { return g_err.c_str(); }
@@ -1049,10 +1055,12 @@ int phono_create(const phono_desc* d, phono_handle** out) {
   TRYC(cudaMemsetAsync(h->mat, 0, h->mat_bytes, h->stream));
   join_stage(h);
   TRY(dalloc(h, &h->tab, (size_t)256 * 16 * h->es));
-  // two-launch step; the leapfrog's window is zero outside the points the
-  // stress pass writes, and a mesh whose window does not fit keeps to the tiles
-  h->win = split_window(nx, ny, nz, d->precision);
-  if (const size_t sb = split_bytes(nx, ny, nz, d->precision)) {
+  // two-launch step (a handle made with a tile shape never takes it); the
+  // leapfrog's window is zero outside the points the stress pass writes, and a
+  // mesh whose window does not fit keeps to the tiles
+  const bool shaped = d->tile_j || d->x_segment;
+  h->win = shaped ? 0 : split_window(nx, ny, nz, d->precision);
+  if (const size_t sb = shaped ? 0 : split_bytes(nx, ny, nz, d->precision)) {
     h->tsy = (int)round_up(SPLIT_KOFF + nz, 8);
     if (dalloc(h, (void**)&h->stress, sb)) {
       h->win = 0;
@@ -1062,7 +1070,7 @@ int phono_create(const phono_desc* d, phono_handle** out) {
       TRYC(cudaMemsetAsync(h->stress, 0, sb, h->stream));
     }
   }
-  h->split = h->win > 0 && !d->tile_j && !d->x_segment;
+  h->split = h->win > 0;
   TRY(dalloc(h, (void**)&h->tab13, (size_t)256 * PHONO_TABLE_COLS * 8));
   TRY(upload_materials(h, d->mat, d->table, d->nmat));
   TRY(encode_tensor_maps(h, h->t));
@@ -1519,6 +1527,12 @@ static int retile(phono_handle* h, int tj, int xseg, const std::vector<int>& sta
   h->t = t;
   h->own = Tiling();
   CK(set_split(h, false));
+  if (h->stress) {  // tiles from here on
+    h->allocs.erase(std::find(h->allocs.begin(), h->allocs.end(), h->stress));
+    CK(cudaFree(h->stress));
+    h->stress = nullptr;
+    h->win = 0;
+  }
   if (h->graph) {  // the captured launches hold the old grid and tensor maps
     cudaGraphExecDestroy(h->graph);
     h->graph = nullptr;

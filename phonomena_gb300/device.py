@@ -20,13 +20,13 @@ def field_shape(nx, ny, nz, comp):
     return (nx - (comp == 0), ny - (comp == 1), nz - (comp == 2))
 
 
-def footprint(shape, precision="f32k", max_steps=0, record_every=0):
-    """Device bytes a DeviceSimulation of this mesh shape allocates (phono_footprint)."""
+def footprint(shape, precision="f32k", max_steps=0, record_every=0, tile_j=0, x_segment=0):
+    """Device bytes a DeviceSimulation of this mesh and tile shape allocates (phono_footprint_shaped)."""
     L = _lib.load()
     out = ctypes.c_size_t()
     nx, ny, nz = (int(v) for v in shape)
-    check(L.phono_footprint(nx, ny, nz, _lib.PRECISIONS[precision], int(max_steps), int(record_every),
-                            ctypes.byref(out)))
+    check(L.phono_footprint_shaped(nx, ny, nz, _lib.PRECISIONS[precision], int(max_steps), int(record_every), int(tile_j),
+                                   1 if np.ndim(x_segment) else int(x_segment), ctypes.byref(out)))
     return int(out.value)
 
 

@@ -124,7 +124,7 @@ class GpuBackend:
     def footprint(self, shape, steps, record_every):
         from .device import footprint
 
-        return footprint(shape, self.precision, max(self.max_steps, int(steps)), record_every)
+        return footprint(shape, self.precision, max(self.max_steps, int(steps)), record_every, self.tile_j, self.x_segment)
 
     def _key_bytes(self, k):
         return self.footprint(k[0], k[1], k[2])

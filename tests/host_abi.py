@@ -33,7 +33,7 @@ def compile_host_abi():
                             ("phono_set_materials", ci, [vp, vp, vp, ci]), ("phono_download_materials", ci, [vp, vp, sz]),
                             ("phono_download", ci, [vp, ci, vp, sz]), ("phono_upload", ci, [vp, ci, vp, sz]),
                             ("phono_set_tiling", ci, [vp, ci, ci]), ("phono_last_error", ctypes.c_char_p, []),
-                            ("phono_footprint", ci, [ci] * 6 + [vp]),
+                            ("phono_footprint", ci, [ci] * 6 + [vp]), ("phono_footprint_shaped", ci, [ci] * 8 + [vp]),
                             ("phono_batch_create", ci, [ci, ci, ci, vp]), ("phono_batch_add", ci, [vp, vp, ci]),
                             ("phono_batch_remove", ci, [vp, ci]), ("phono_batch_step", ci, [vp, ci]),
                             ("phono_batch_sync", ci, [vp]), ("phono_batch_destroy", None, [vp]),

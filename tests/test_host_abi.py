@@ -94,3 +94,31 @@ def test_a_handle_is_destroyed_with_steps_queued(L):
     assert L.phono_step(h.h, 24) == 0
     h.close()
     assert L.fake_broken() == 0
+
+
+def test_memory_of_fp64_handles_with_a_tile_shape(L):
+    """The stress window of the two-launch step is held by the handles that
+    step that way alone, and the footprint of a handle is what it allocates."""
+    shape, out = (21, 70, 60), ctypes.c_size_t()
+    held = {}
+    for kw in ({}, {"tile_j": 8}, {"x_segment": 12}, {"tile_j": 16, "x_segment": -4}):
+        for precision, code in (("f64", 0), ("f64v", 2), ("f32k", 1)):
+            h = Handle(L, shape, precision, max_steps=30, **kw)
+            held[precision, bool(kw)] = L.fake_bytes(0)
+            assert L.phono_footprint_shaped(*shape, code, 30, 0, kw.get("tile_j", 0), kw.get("x_segment", 0),
+                                            ctypes.byref(out)) == 0
+            assert out.value == L.fake_bytes(0), (precision, kw)
+            if not kw:
+                assert L.phono_footprint(*shape, code, 30, 0, ctypes.byref(out)) == 0 and out.value == held[precision, False]
+                if precision == "f64":
+                    assert L.phono_step(h.h, 13) == 0 and L.phono_set_tiling(h.h, 8, 6) == 0 and L.phono_step(h.h, 13) == 0
+                    assert L.fake_bytes(0) == held["f64", False] - window(shape)
+            h.close()
+            assert L.fake_bytes(0) == 0 and L.fake_broken() == 0
+    assert held["f64", True] == held["f64", False] - window(shape)
+    assert held["f64v", True] == held["f64v", False] and held["f32k", True] == held["f32k", False]
+
+
+def window(shape):
+    """Bytes of the leapfrog's window: six stresses of rows padded to 64 bytes, the first 32 of them zeros."""
+    return -(-6 * shape[0] * shape[1] * -(-(4 + shape[2]) // 8) * 64 // 512) * 512
