@@ -702,10 +702,10 @@ static void* field_ptr(phono_handle* h, int field) {
 }
 
 // Switch a handle between the two-launch form (v and the Kahan term in buffer
-// 0) and the tile pass (in the buffer of the step's parity).
+// 0) and the tile pass (in the buffer of the step's parity).  On failure the
+// handle keeps its form: what may have been copied is the state it does not use.
 static cudaError_t set_split(phono_handle* h, bool on) {
   if (h->split == on) return cudaSuccess;
-  h->split = on;
   cudaError_t e = cudaSuccess;
   if (h->vbase && (h->steps_done & 1)) {
     const size_t n = 3 * h->field_elems * h->es;
@@ -713,6 +713,7 @@ static cudaError_t set_split(phono_handle* h, bool on) {
       if (e == cudaSuccess)
         e = cudaMemcpyAsync(on ? b : b + n, on ? b + n : b, n, cudaMemcpyDeviceToDevice, h->stream);
   }
+  if (e == cudaSuccess) h->split = on;
   return e;
 }
 
@@ -821,7 +822,7 @@ static std::vector<double> wave_lengths(double depth, int waves, double shortest
 // us at 12 planes, 917 at 57). Beside other
 // instances (a batch) there is no last wave to fill: even segments of at most
 // `limit` planes (0: alone), see batch_rebuild.
-static int own_tiling(phono_handle* h, int limit) {
+static int own_tiling(phono_handle* h, Tiling& t, int limit) {
   const int nsm = sm_count();
   const int planes = h->d.nx - 1, rows = h->d.ny - 1;
   const long long r16 = round_up(rows, 16), r8 = round_up(rows, 8);
@@ -846,8 +847,8 @@ static int own_tiling(phono_handle* h, int limit) {
   }
   const int nseg = (int)starts.size() - 1;
   // more segments than a launch describes by table: even ones
-  if (nseg > SEG_TABLE) return apply_tiling(h, h->own, tj, (planes + nseg - 1) / nseg, segment_starts(planes, (planes + nseg - 1) / nseg));
-  return apply_tiling(h, h->own, tj, kExplicitSegments, starts);
+  if (nseg > SEG_TABLE) return apply_tiling(h, t, tj, (planes + nseg - 1) / nseg, segment_starts(planes, (planes + nseg - 1) / nseg));
+  return apply_tiling(h, t, tj, kExplicitSegments, starts);
 }
 
 // TMA descriptors: a 4-D (k, j, i, array) map over the u allocation with a
@@ -954,7 +955,7 @@ int phono_create(const phono_desc* d, phono_handle** out) {
   // tiles: the shape the caller knows by default is height 4 for FP32, 8 for
   // FP64, and 24 planes per segment
   int rt = set_tiling(h, d->tile_j ? d->tile_j : (d->precision == PHONO_F32K ? 4 : 8), d->x_segment ? d->x_segment : 24);
-  if (!rt && d->precision == PHONO_F32K && !d->tile_j && !d->x_segment) rt = own_tiling(h, 0);
+  if (!rt && d->precision == PHONO_F32K && !d->tile_j && !d->x_segment) rt = own_tiling(h, h->own, 0);
   if (rt) {
     std::string m_ = g_err;
     delete h;
@@ -1617,26 +1618,39 @@ static void batch_detach(phono_batch* b, const phono_handle* h) {
 }
 
 // a default FP32 handle's tiles for single steps (0) or, with segments of at
-// most `limit` planes, for steps beside others
+// most `limit` planes, for steps beside others; it keeps those it has when the
+// new ones cannot be set up
 static int reshape_own(phono_handle* h, int limit) {
+  Tiling own;
+  int rc = own_tiling(h, own, limit);
+  if (!rc) rc = encode_tensor_maps(h, own);
+  if (rc) return rc;
+  h->own = own;
   h->own_limit = limit;
-  int rc = own_tiling(h, limit);
-  if (!rc) rc = encode_tensor_maps(h, h->own);
   if (h->graph && !h->lent) {  // (a lent shape's is that of t)
     cudaGraphExecDestroy(h->graph);
     h->graph = nullptr;
   }
-  return rc;
+  return PHONO_OK;
 }
 
-// the batch's work is done: the handle is on its own again
-static cudaError_t leave_batch(phono_handle* h) {
+// The batch's work is done: the handle is on its own again.  Where its own
+// tiles or form cannot be set up anew it steps on in those of the batch.
+static int leave_batch(phono_handle* h) {
   h->batch = nullptr;
   if (h->lent) h->own = Tiling{}, h->lent = false;
-  if (h->own.tj) reshape_own(h, 0);
-  if (!h->resplit) return cudaSuccess;
+  const bool resplit = h->resplit;
   h->resplit = false;
-  return set_split(h, true);
+  int rc = h->own.tj ? reshape_own(h, 0) : PHONO_OK;
+  if (resplit) {
+    const cudaError_t e = set_split(h, true);
+    if (e != cudaSuccess) rc = fail(PHONO_ERR_CUDA, std::string("leaving a batch: ") + cudaGetErrorString(e));
+  }
+  if (rc && h->graph) {  // captured in the form it had before
+    cudaGraphExecDestroy(h->graph);
+    h->graph = nullptr;
+  }
+  return rc;
 }
 
 static void batch_release(phono_batch* b) {
@@ -1856,24 +1870,26 @@ int phono_batch_add(phono_batch* b, phono_handle* h, int nsteps) {
     int rc = need_workers(b, std::min(members, kBatchWorkers));
     if (rc) return rc;
   }
-  // beside others FP32's two launches only move more bytes (12 crystals: 120 us
-  // a step, 142 with the small ones split)
-  if (h->split && b->precision == PHONO_F32K) {
-    CK(set_split(h, false));
-    h->resplit = true;
-  }
   // In the default scheme FP32 instances step in tiles of the batch's choice
   // (12 crystals of 6.2 M nodes: 98 us a step, 108 at height 8, 177 in one
   // launch a step whose blocks took tiles of all instances from a list).
-  if (!h->own.tj && !b->streams && b->precision == PHONO_F32K) {
-    int rc = own_tiling(h, 24);
+  const bool lend = !h->own.tj && !b->streams && b->precision == PHONO_F32K;
+  Tiling own;
+  if (lend) {
+    int rc = own_tiling(h, own, 24);  // (its tensor maps come with the next work list)
     if (rc) return rc;
-    CK(configure_step_f32k(h->own.tj));
-    h->lent = true;
+    CK(configure_step_f32k(own.tj));
   }
-  h->own_limit = 0;  // cut with the next work list
   CK(cudaStreamSynchronize(h->stream));
   CK(cudaStreamSynchronize(b->stream));
+  // beside others FP32's two launches only move more bytes (12 crystals: 120 us
+  // a step, 142 with the small ones split)
+  const bool resplit = h->split && b->precision == PHONO_F32K;
+  if (resplit) CK(set_split(h, false));
+  // nothing fails from here on: the handle is the batch's
+  h->resplit = resplit;
+  if (lend) h->own = own, h->lent = true;
+  h->own_limit = 0;  // cut with the next work list
   b->slot[s] = h;
   b->remaining[s] = nsteps;
   b->step_end[s] = h->steps_done + nsteps;
@@ -1885,12 +1901,12 @@ int phono_batch_add(phono_batch* b, phono_handle* h, int nsteps) {
 int phono_batch_remove(phono_batch* b, int s) {
   if (!b || s < 0 || s >= b->cap || !b->slot[s]) return fail(PHONO_ERR_ARG, "no instance in that slot");
   CK(cudaStreamSynchronize(b->stream));
-  CK(leave_batch(b->slot[s]));
+  phono_handle* h = b->slot[s];
   b->slot[s] = nullptr;
   b->remaining[s] = 0;
   b->dirty = true;
   drop_igraph(b, s);
-  return PHONO_OK;
+  return leave_batch(h);
 }
 
 int phono_batch_remaining(const phono_batch* b, int s) {

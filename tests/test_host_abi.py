@@ -122,3 +122,81 @@ def test_memory_of_fp64_handles_with_a_tile_shape(L):
 def window(shape):
     """Bytes of the leapfrog's window: six stresses of rows padded to 64 bytes, the first 32 of them zeros."""
     return -(-6 * shape[0] * shape[1] * -(-(4 + shape[2]) // 8) * 64 // 512) * 512
+
+
+@pytest.mark.parametrize("what", ["sync", "copy", "configure"])
+@pytest.mark.parametrize("shape,tile", [((30, 21, 13), 0), ((60, 70, 60), 0), ((60, 70, 60), 4)])
+def test_a_failed_join_leaves_the_handle_as_it_was(L, what, shape, tile):
+    ref = Handle(L, shape, tile_j=tile)
+    h = Handle(L, shape, tile_j=tile)
+    form = "split" if shape == (30, 21, 13) else "tile"
+    b = ctypes.c_void_p()
+    assert L.phono_batch_create(2, 1, 4, ctypes.byref(b)) == 0
+    assert L.phono_step(h.h, 1) == 0 and L.phono_step(ref.h, 1) == 0
+    for after in (1, 2):
+        L.fake_fail(what.encode(), after)
+        rc = L.phono_batch_add(b, h.h, 20)
+        L.fake_fail(what.encode(), 0)
+        if rc < 0:  # alone: the kernels it had
+            n = L.fake_count(form.encode())
+            assert L.phono_step(h.h, 3) == 0
+            steps = L.fake_count(form.encode()) - n
+            n = L.fake_count(form.encode())
+            assert L.phono_step(ref.h, 3) == 0
+            assert steps == L.fake_count(form.encode()) - n > 0
+        else:
+            assert L.phono_batch_step(b, 5) == 0 and L.phono_batch_remove(b, rc) == 0
+    slot = L.phono_batch_add(b, h.h, 20)
+    assert slot >= 0 and L.phono_batch_step(b, 20) == 0 and L.phono_batch_remove(b, slot) == 0
+    L.phono_batch_destroy(b)
+    for x in (h, ref):
+        x.close()
+    assert L.fake_broken() == 0
+
+
+def test_segments_that_cannot_be_cut_anew(L):
+    """Tensor maps that cannot be made while a batch is stepped or left: the
+    call reports it, nothing is launched without maps, and a later call works."""
+    small, large = Handle(L, (30, 21, 13)), Handle(L, (130, 150, 40))
+    b = ctypes.c_void_p()
+    assert L.phono_batch_create(2, 1, 4, ctypes.byref(b)) == 0
+    slots = [L.phono_batch_add(b, h.h, 40) for h in (small, large)]
+    for after in (1, 2, 5):
+        L.fake_fail(b"encode", after)
+        assert L.phono_batch_step(b, 5) < 0
+        L.fake_fail(b"encode", 0)
+    assert L.phono_batch_step(b, 5) == 0
+    L.fake_fail(b"encode", 1)
+    assert L.phono_batch_remove(b, slots[1]) < 0
+    L.fake_fail(b"encode", 0)
+    assert L.phono_step(large.h, 5) == 0  # out of the batch, in tiles that work
+    assert L.phono_batch_step(b, 5) == 0 and L.phono_batch_remove(b, slots[0]) == 0
+    assert L.phono_step(small.h, 20) == 0
+    L.phono_batch_destroy(b)
+    for h in (small, large):
+        h.close()
+    assert L.fake_broken() == 0
+
+
+@pytest.mark.parametrize("what", ["encode", "copy", "both"])
+def test_a_handle_that_cannot_take_its_form_back(L, what):
+    """A default FP32 handle whose own tiles or two-launch form cannot be set up
+    as it leaves a batch: reported, out of the batch, and a graph captured in
+    the form it had before is not replayed on the state of another."""
+    h = Handle(L, (30, 21, 13))
+    b = ctypes.c_void_p()
+    assert L.phono_batch_create(1, 1, 4, ctypes.byref(b)) == 0
+    assert L.phono_step(h.h, 13) == 0  # 12 of them by a graph of the two-launch form
+    slot = L.phono_batch_add(b, h.h, 20)
+    for name in ("encode", "copy") if what == "both" else (what,):
+        L.fake_fail(name.encode(), 1)
+    assert L.phono_batch_remove(b, slot) < 0
+    tiles, splits = L.fake_count(b"tile"), L.fake_count(b"split")
+    assert L.phono_step(h.h, 13) == 0
+    # 13 steps launched or captured anew, in one form
+    assert (L.fake_count(b"tile") - tiles, L.fake_count(b"split") - splits) == ((0, 26) if what == "encode" else (13, 0))
+    slot = L.phono_batch_add(b, h.h, 20)
+    assert slot >= 0 and L.phono_batch_step(b, 20) == 0 and L.phono_batch_remove(b, slot) == 0
+    L.phono_batch_destroy(b)
+    h.close()
+    assert L.fake_broken() == 0
