@@ -14,8 +14,9 @@ the same x extent, keeping a change only when the whole batch gets faster.
 
 Timing uses scratch simulations (zero material ids and zero source: the
 kernel's work does not depend on the values), so tuning never touches the
-caller's state.  Results are cached per (scheme, shapes, device) in a JSON
-file next to the built library, so a mesh or a mix is tuned once per machine.
+caller's state.  Results are cached per (scheme, shapes, candidates, device,
+kernel sources) in a JSON file next to the built library, so a mesh or a mix is
+tuned once per machine and again when the kernels change.
 
 tile_j sets the block (a 32 x tile_j tile: 32 x tile_j threads at height 4,
 two rows a thread at 8 and 16 in FP32; shared memory per block); the x
@@ -27,12 +28,15 @@ run while the GPU drains at the end of a launch short.
 """
 from __future__ import annotations
 
+import functools
 import hashlib
 import json
 import os
 from pathlib import Path
 
 import numpy as np
+
+from . import build
 
 CACHE = Path(__file__).resolve().parent / "_build" / "autotune.json"
 TILE_J = (4, 8, 16)
@@ -54,8 +58,19 @@ def _device_name():
         return "cuda"
 
 
-def _key(precision, shape):
-    return f"{precision}:{shape[0]}x{shape[1]}x{shape[2]}:{_device_name()}"
+@functools.lru_cache(None)
+def _kernels():
+    """Digest of the library's sources and of this file: a choice holds for the
+    kernels and the candidates it was timed with."""
+    h = hashlib.sha1()
+    for f in [build.CSRC / f for f in build.SOURCES + build.HEADERS] + [Path(__file__)]:
+        h.update(f.read_bytes() if f.exists() else b"")
+    return h.hexdigest()[:16]
+
+
+def _key(precision, shape, cands):
+    h = hashlib.sha1(json.dumps(cands).encode()).hexdigest()[:16]
+    return f"{precision}:{shape[0]}x{shape[1]}x{shape[2]}:{_device_name()}:{h}:{_kernels()}"
 
 
 def _load():
@@ -129,7 +144,8 @@ def candidates_for(shape, tile_js=TILE_J):
 def tune(spacing, mat, table, dt, precision="f32k", steps=None, candidates=None, use_cache=True, verbose=False):
     """Best (tile_j, x_segment) for this mesh and scheme; times each candidate."""
     shape = tuple(int(s) for s in np.shape(mat))
-    key = _key(precision, shape)
+    cands = [(0, 0)] + list(candidates or candidates_for(shape))  # (0, 0): the library's own choice, tiles or not
+    key = _key(precision, shape, cands)
     if use_cache:
         hit = _load().get(key)
         if hit:
@@ -137,7 +153,6 @@ def tune(spacing, mat, table, dt, precision="f32k", steps=None, candidates=None,
             return int(tj), (tuple(xs) if isinstance(xs, list) else int(xs))
     if steps is None:
         steps = 48 if precision == "f32k" else 12
-    cands = [(0, 0)] + list(candidates or candidates_for(shape))  # (0, 0): the library's own choice, tiles or not
     results = []
     sim = _scratch(shape, precision, (steps + 12) * len(cands) + 12, tile_j=0, x_segment=0)
     try:
@@ -164,7 +179,7 @@ def tune(spacing, mat, table, dt, precision="f32k", steps=None, candidates=None,
 
 def _batch_key(precision, shapes):
     h = hashlib.sha1(json.dumps(sorted(map(list, shapes))).encode()).hexdigest()[:16]
-    return f"batch:{precision}:{len(shapes)}:{h}:{_device_name()}"
+    return f"batch:{precision}:{len(shapes)}:{h}:{_device_name()}:{_kernels()}"
 
 
 def tune_batch(shapes, precision="f32k", steps=24, tile_js=TILE_J, use_cache=True, verbose=False, streams=0):
