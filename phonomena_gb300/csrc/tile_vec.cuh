@@ -129,6 +129,22 @@ __device__ __forceinline__ float y_face_coef(const StepArgs<float>& a, int c, in
   return dj < 0 ? a.abc[c == 1 ? 3 : 2] : a.abc[c == 1 ? 5 : 4];
 }
 
+// The block's barrier for its two kinds of warps, which reach it at statements
+// of their own: __syncthreads() has to be one statement for all threads, while
+// PTX's barrier counts those that arrive at barrier 0, wherever that is.
+// Aligned: the lanes of a warp are of one kind and come together (us for 360
+// steps on 256x256x128 cells: 43150, 52940 without).
+__device__ __forceinline__ void block_wait() { asm volatile("barrier.cta.sync.aligned 0;" ::: "memory"); }
+__device__ __forceinline__ bool block_any(bool x) {
+  uint32_t any;
+  asm volatile(
+      "{\n .reg .pred p, q;\n setp.ne.u32 p, %1, 0;\n barrier.cta.red.or.pred.aligned q, 0, p;\n selp.u32 %0, 1, 0, q;\n}\n"
+      : "=r"(any)
+      : "r"((uint32_t)x)
+      : "memory");
+  return any != 0;
+}
+
 template <int TJ>
 __device__ __forceinline__ void tile_block_vec(const StepArgs<float>& a, unsigned char* base, const Roles<float>& r,
                                                const float s, const int tt, const int tid, const int b) {
@@ -273,7 +289,7 @@ __device__ __forceinline__ void tile_block_vec(const StepArgs<float>& a, unsigne
       if (ok) xt_m = U[u_top], xr_m = col ? U[u_right] : 0.f;
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    __syncthreads();  // stage ib-1 is read
+    block_wait();  // stage ib-1 is read
     if (producer && ok && ib + 2 <= ie) {
       issue(ib + 2, 0);
       issued = ib + 2;
@@ -322,7 +338,7 @@ __device__ __forceinline__ void tile_block_vec(const StepArgs<float>& a, unsigne
       // barrier: order this thread's reads of it first (a barrier orders
       // shared-memory accesses of the block's threads only).
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      if (__syncthreads_or(!ok)) {
+      if (block_any(!ok)) {
         ok = false;
         break;
       }
@@ -337,7 +353,7 @@ __device__ __forceinline__ void tile_block_vec(const StepArgs<float>& a, unsigne
     }
     if (ok && fd && ie - ib >= 2) face_rows(ie - 2, false);
     let_next_launch();
-    __syncthreads();  // the last plane is written
+    block_wait();  // the last plane is written
     if (ok && fd && !(fc == 0 && ie == nx - 1)) face_rows(ie - 1, true);  // ux ends at plane nx-2, its x = N face
   } else {
     // ---------------- updating warps ----------------
@@ -409,7 +425,7 @@ __device__ __forceinline__ void tile_block_vec(const StepArgs<float>& a, unsigne
       }
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    __syncthreads();  // stage ib-1 is read: its slot is refilled with stage ib+2
+    block_wait();  // stage ib-1 is read: its slot is refilled with stage ib+2
 
     // ux of plane i-1 from T1 of plane i (base_solver.py:441-447, 495-501)
     auto update_x = [&](int i, const float (&t1)[4], const float* pw, const float (&qd)[4], const float fxm) {
@@ -496,7 +512,7 @@ __device__ __forceinline__ void tile_block_vec(const StepArgs<float>& a, unsigne
         }
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // before the refill of plane i's slot (see above)
-      if (__syncthreads_or(!ok)) {
+      if (block_any(!ok)) {
         ok = false;
         break;
       }
@@ -604,7 +620,7 @@ __device__ __forceinline__ void tile_block_vec(const StepArgs<float>& a, unsigne
         out.write(a, r, tt, c, p + 1, j, k, u);
       }
     }
-    __syncthreads();  // see the halo warp
+    block_wait();  // see the halo warp
   }
   if (!ok && producer) {
     // A wait ran out: flag it and drain the copies this block issued, so that
