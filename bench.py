@@ -53,7 +53,7 @@ def parse():
     p.add_argument("--batch-streams", type=int, default=64,
                    help="batch and serving: worker streams of the streams batch scheme (0: the default scheme only)")
     p.add_argument("--requests", type=int, default=2000, help="serve: FP32K requests")
-    p.add_argument("--rate", type=float, default=0.0, help="serve: FP32K arrivals per second (0: 70%% load)")
+    p.add_argument("--rate", type=float, default=0.0, help="serve: FP32K arrivals per second (0: 70%% of 45 Gcell/s)")
     p.add_argument("--requests-f64", type=int, default=40, help="serve: plain FP64 requests")
     p.add_argument("--budget-gb", type=float, default=150.0, help="serve: device memory budget")
     p.add_argument("--cells", default="256,256,128")
@@ -475,7 +475,10 @@ def bench_batch(args, rank, world, local, torch, dist):
         print(json.dumps(line), flush=True)
 
 
-SERVE_GCELL = {"f32k": 45.0, "f64": 4.0}  # batched throughputs the offered loads refer to
+# Gcell/s that the offered loads are fractions of: fixed, so that the arrival
+# rates stay comparable; and the batched throughputs measured (--workload batch)
+SERVE_GCELL = {"f32k": 45.0, "f64": 4.0}
+BATCH_GCELL = {"f32k": 71.5, "f64": 9.4}
 
 
 def serve_stream(precision, n, rate, seed, budget_gb, streams=0):
@@ -503,9 +506,9 @@ def serve_stream(precision, n, rate, seed, budget_gb, streams=0):
     return out
 
 
-def serve_summary(r, load):
+def serve_summary(r, load, precision):
     """The served-stream figures of the benchmark line."""
-    return {"load": load, "rate": r["rate_per_s"], "requests": r["requests"], "p50": round(r["p50_s"], 4),
+    return {"load": load, "load_of_throughput": round(load * SERVE_GCELL[precision] / BATCH_GCELL[precision], 2), "rate": r["rate_per_s"], "requests": r["requests"], "p50": round(r["p50_s"], 4),
             "p95": round(r["p95_s"], 4), "p99": round(r["p99_s"], 4),
             "gcell_per_s": round(r["gcell_updates_per_s"], 4), "offered_gcell_per_s": r["offered_gcell_per_s"],
             "failed": r["failed"], "rejected": r["rejected"], "peak_active": r["peak_active"],
@@ -513,8 +516,8 @@ def serve_summary(r, load):
 
 
 def bench_serve(args, rank, world, local, torch, dist):
-    """FP32K and plain FP64 request streams, each at about 70% of its own
-    batched throughput (serve_stream)."""
+    """FP32K and plain FP64 request streams, each at 70% of its scheme's
+    reference rate (SERVE_GCELL; serve_stream)."""
     from phonomena_gb300 import serve
 
     rate32 = args.rate or serve.rate_for_load(SERVE_GCELL["f32k"], 0.7)
@@ -530,8 +533,8 @@ def bench_serve(args, rank, world, local, torch, dist):
             "unit": "Gcell-updates/s", "n_gpus": world, "steps": 1, "warmup": 0,
             "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f32",
             "data": "synthetic (seeded request stream)",
-            "config": {"workload": f"Poisson stream of {args.requests} requests at {rate32:.3f}/s (70% of "
-                                   f"{SERVE_GCELL['f32k']} Gcell/s offered), sizes {{64..192}}^2 x {{32..96}} cells "
+            "config": {"workload": f"Poisson stream of {args.requests} requests at {rate32:.3f}/s ("
+                                   f"{rate32 * serve.mean_work() / 1e9:.1f} Gcell/s offered), sizes {{64..192}}^2 x {{32..96}} cells "
                                    "plus 5% 512x512x128, 500-3000 steps, uz surface every 10 steps, "
                                    f"{args.budget_gb:.0f} GB device budget, continuous batching",
                        "parallelism": f"replicas x{world}"},
@@ -543,22 +546,23 @@ def bench_serve(args, rank, world, local, torch, dist):
 
 def serve_study(args, rank):
     """The serve object of the default line: FP32K streams at the offered
-    loads of --serve-loads, a plain FP64 stream at 70% of its throughput."""
+    loads of --serve-loads, a plain FP64 stream at load 0.7 (SERVE_GCELL)."""
     from phonomena_gb300 import serve
 
     loads = [float(v) for v in args.serve_loads.split(",") if v]
     out = {"workload": "Poisson request streams: sizes {64..192}^2 x {32..96} cells plus 5% 512x512x128, "
                        "500-3000 steps, uz surface every 10 steps, continuous batching, "
-                       f"{args.budget_gb:.0f} GB device budget; load = offered work / the scheme's batched "
-                       f"throughput ({SERVE_GCELL['f32k']} Gcell/s FP32K, {SERVE_GCELL['f64']} FP64)",
+                       f"{args.budget_gb:.0f} GB device budget; load = offered work / a fixed rate "
+                       f"({SERVE_GCELL['f32k']} Gcell/s FP32K, {SERVE_GCELL['f64']} FP64); of the batched throughput "
+                       f"({BATCH_GCELL['f32k']} and {BATCH_GCELL['f64']}) it is load_of_throughput",
            "f32k": [], "fp64": []}
     for q, load in enumerate(loads):
         rate = serve.rate_for_load(SERVE_GCELL["f32k"], load)
         out["f32k"].append(serve_summary(serve_stream("f32k", args.serve_requests, rate, rank + 10 * q,
-                                                      args.budget_gb, streams=args.batch_streams), load))
+                                                      args.budget_gb, streams=args.batch_streams), load, "f32k"))
     rate64 = serve.rate_for_load(SERVE_GCELL["f64"], 0.7)
     out["fp64"].append(serve_summary(serve_stream("f64", args.serve_requests_f64, rate64, rank + 1000,
-                                                  args.budget_gb, streams=args.batch_streams), 0.7))
+                                                  args.budget_gb, streams=args.batch_streams), 0.7, "f64"))
     out["batch_scheme"] = "streams" if args.batch_streams > 0 else "default"
     return out
 

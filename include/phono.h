@@ -91,9 +91,10 @@ typedef struct phono_desc {
   int source_mode;               /* PHONO_SOURCE_* */
   int max_steps;                 /* capacity: source samples and surface records */
   int record_every;              /* record uz[:, :, 0] after every k-th step; 0 = off */
-  int tile_j;                    /* tile height along y: 4, 8 or 16; 0 = default (F32K 4, else 8) */
-  int x_segment;                 /* planes per block segment; -L: L-plane segments, the last 2L planes in four shorter ones; 0 = default (24).
-                                  * Both 0: the form of phono_step that suits the mesh, not necessarily tiles */
+  int tile_j;                    /* tile height along y: 4, 8 or 16; 0 = default (F32K 4, else 8, where x_segment is given) */
+  int x_segment;                 /* planes per block segment; -L: L-plane segments, the last 2L planes in four shorter ones;
+                                  * 0 = default (24, where tile_j is given).  Both 0: the form of phono_step that suits the
+                                  * mesh, tiles of a height and segments of the library's choice or no tiles at all */
 } phono_desc;
 
 typedef struct phono_handle phono_handle;
@@ -121,7 +122,7 @@ int phono_create(const phono_desc *desc, phono_handle **out);
 int phono_set_source(phono_handle *h, const double *samples, int n);
 
 /* Advance nsteps time steps; per step a tile launch and a face launch (one
- * launch when ny == 3), or in the two-launch form a stress launch and an
+ * launch in F32K at height 16, and when ny == 3), or in the two-launch form a stress launch and an
  * update launch per chunk of planes, replayed from captured CUDA graphs of 12
  * steps.  The two-launch form is that of handles with the default tile shape
  * (tile_j = x_segment = 0) in FP64, and in FP32 up to 170,000 nodes.  Otherwise

@@ -18,8 +18,9 @@ caller's state.  Results are cached per (scheme, shapes, candidates, device,
 kernel sources) in a JSON file next to the built library, so a mesh or a mix is
 tuned once per machine and again when the kernels change.
 
-tile_j sets the block (a 32 x tile_j tile: 32 x tile_j threads at height 4,
-two rows a thread at 8 and 16 in FP32; shared memory per block); the x
+tile_j sets the block (a 32 x tile_j tile: 32 x tile_j threads, in FP32 at
+heights 8 and 16 four z points a thread and a warp for the tile's halo; shared
+memory per block); the x
 segment sets how many x planes a block marches and thereby the number of
 blocks (several waves of the 152 SMs vs. the re-read of two halo planes per
 segment).  Blocks are dispatched segment by segment, so segments that

@@ -106,7 +106,7 @@ struct phono_handle {
   Tiling own;                  // a default handle's own shape (own.tj 0: t)
   int own_limit = 0;           // longest segment of it in a batch (0: alone)
   bool lent = false;           // not a default handle: own is its batch's choice
-  int n_face = 0, separate_faces = 1;
+  int separate_faces = 1;
   FaceTable faces{};
   // two-launch step (split_step.cu): stress window of `win` planes (0: this
   // mesh has none).  split: the handle steps that way (default tile shape);
@@ -771,7 +771,6 @@ static int apply_tiling(phono_handle* h, Tiling& t, int tj, int xseg, const std:
   t.nseg = nseg;
   t.n_tile = (int)ntile;
   h->faces = faces;
-  h->n_face = (int)nface;
   // faces in a second launch that reads the tile pass's interior values; the
   // chain end of a face point can itself be a face point only when ny == 3
   h->separate_faces = ny >= 4 ? 1 : 0;

@@ -35,7 +35,7 @@ constexpr int SEG_TABLE = 64;  // x segments a launch describes by table (more: 
 constexpr int MKOFF = 8;    // material front pad in k (bytes)
 constexpr int MKW = 48;     // material tile width in k (bytes): k0-8 .. k0+40
 constexpr int TAB_ROWS_MAX = 256;  // material rows a table may hold (uint8 ids)
-constexpr int BATCH_TAB_ROWS = 32;  // material rows of a batched instance
+constexpr int BATCH_TAB_ROWS = 32;  // most material rows of a batched instance (part of phono_batch_add's contract)
 
 constexpr int VEC_TJ = 8;         // the FP32 tile pass is the vectorised one from this tile height on
 // It writes the face points itself (no face launch) on meshes with no row next

@@ -1,21 +1,25 @@
 // Elastic FDTD step for GB300 (sm_103a).
 //
 // One time step of phonomena's staggered-grid solver
-// (simulation/base_solver.py:245-266) is a tile launch and a face launch:
+// (simulation/base_solver.py:245-266) as a tile pass; the other form, which FP64
+// and small FP32 handles take by default, is split_step.cu's.
 //
-//  * tile blocks (tile_rows.cuh): a (TJ x 32) tile of the
-//    (y, z) plane marches along x over a segment of planes.  Planes of u (all
-//    three components, 1-node halo), of the material ids and of the pointwise
-//    state of the own points (u_old, or v and the Kahan term) stream into a
-//    4-slot shared-memory ring through TMA (cp.async.bulk.tensor, completion
-//    on an mbarrier per slot).  Each iteration evaluates the six stresses of
-//    the current plane once (plus the halo stresses the neighbours need) into
-//    shared memory and writes the new state of the plane.  Stresses are never
-//    written to global memory.  The tile pass also writes the z = N face
-//    point above every (i, j) that is on no x / y face.
+//  * tile blocks: a (TJ x 32) tile of the (y, z) plane marches along x over a
+//    segment of planes.  Planes of u (all three components, 1-node halo), of
+//    the material ids and of the pointwise state of the own points (u_old, or v
+//    and the Kahan term) stream into a shared-memory ring through TMA
+//    (cp.async.bulk.tensor, completion on an mbarrier per slot).  Each iteration
+//    evaluates the six stresses of the current plane once (plus the halo
+//    stresses the neighbours need) and writes the new state of the plane.
+//    Stresses are never written to global memory.  FP32 tiles of height 8 and 16
+//    hold them in registers (tile_vec.cuh: four z points a thread, a 3-slot
+//    ring), the others in shared memory (tile_rows.cuh: one z point a thread, a
+//    4-slot ring).  The tile pass also writes the z = N face point above every
+//    (i, j) that is on no x / y face, and in FP32 at height 16 (ny >= 5) all
+//    face points: then a step is this launch alone.
 //
-//  * face points (fdtd_face_kernel, a second launch; for ny == 3, extra
-//    blocks of the same launch): the x = N, y = 0, y = N faces and the z = N
+//  * face points otherwise (fdtd_face_kernel, a second launch; for ny == 3,
+//    extra blocks of the same launch): the x = N, y = 0, y = N faces and the z = N
 //    points on them (simulation/base_solver.py:540-554).  The reference
 //    applies the faces one after another, each reading the plane next to it
 //    as left by the earlier faces; the final value of a face point is thus a

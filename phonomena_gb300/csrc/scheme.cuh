@@ -99,9 +99,6 @@ __device__ __forceinline__ long long fidx(const Geo& g, int i, int j, int k) {
 __device__ __forceinline__ int ext_x(const Geo& g, int c) { return g.nx - (c == 0); }
 __device__ __forceinline__ int ext_y(const Geo& g, int c) { return g.ny - (c == 1); }
 __device__ __forceinline__ int ext_z(const Geo& g, int c) { return g.nz - (c == 2); }
-__device__ __forceinline__ bool on_face(const Geo& g, int c, int i, int j, int k) {
-  return i == ext_x(g, c) - 1 || j == 0 || j == ext_y(g, c) - 1 || k == ext_z(g, c) - 1;
-}
 // points the reference's interior update or z=0 row writes
 // (base_solver.py:441-463,495-516)
 __device__ __forceinline__ bool in_v0(const Geo& g, int c, int i, int j, int k) {

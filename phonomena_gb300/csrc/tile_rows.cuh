@@ -100,7 +100,7 @@ __device__ __forceinline__ void tile_block_rows(const StepArgs<typename S::R>& a
     const int q = p - ibase, sl = q & (NSLOT - 1);
     const bool pw = p >= ib && p < ie;
     mbar_expect_tx(&bars[sl], P::tx_bytes + (pw ? P::pw_bytes : 0u));
-    // test hook (skip_plane >= 0; -1 is off_i, and plane -1 is a real padding
+    // test hook (skip_plane >= 0; -1 is off, and plane -1 is a real padding
     // plane that segment 0 loads): armed, no copy, so the wait on it runs out
     if (a.skip_plane >= 0 && p == a.skip_plane) return;
     // padded coordinates: k, j + 1, i + 1; the u tiles start at k0-KB (columns before 0: zeros), j0-1
@@ -247,7 +247,7 @@ __device__ __forceinline__ void tile_block_rows(const StepArgs<typename S::R>& a
     const R* U0 = uslot(i);
     const R* Up = uslot(i + 1);
     const uint8_t* Mp = mslot(i + 1);
-      t5m = R(0);
+    t5m = R(0);
     t6m = R(0);
     if (i_s && j_n && k_in) {  // T5 (base_solver.py:360-365, 425-428)
       const R c = tab[16 * Mp[Lm + (kz ? 0 : 1)] + 10];
@@ -307,10 +307,10 @@ __device__ __forceinline__ void tile_block_rows(const StepArgs<typename S::R>& a
     const R* Up = uslot(i + 1);
     const uint8_t* M0 = mslot(i);
     const uint8_t* Mp = mslot(i + 1);
-    // own stresses of plane i, row by row, each ring value read once
+    // own stresses of plane i, each ring value read once
     R uxc, uyc, uzc, uxc_up, t1c, t2c, t3c, t4c, t5c, t6c;
     int idp_c, idp_z, idp_y;
-      uxc = U0[XO + Lu];
+    uxc = U0[XO + Lu];
     uyc = uyc_n;
     uzc = uzc_n;
     uyc_n = Up[YO + Lu];

@@ -82,9 +82,11 @@ class DeviceSimulation:
         h = ctypes.c_void_p()
         check(L.phono_create(ctypes.byref(d), ctypes.byref(h)))
         self._h = h
+        # the library picks the step's form and tiles; tile_j and x_segment then
+        # are what a batch compares and set_tiling keeps, not what steps
+        self._default_shape = not tile_j and not x_segment and segments is None
         self.tile_j = int(tile_j) or (4 if precision == "f32k" else 8)
         self.x_segment = int(x_segment) or 24
-        self._default_shape = not tile_j and not x_segment and segments is None  # the library picks the step's form
         self.surface_mode, self.bc, self.source_mode = surface_mode, bc, source_mode
         self._source = None
         if segments is not None:

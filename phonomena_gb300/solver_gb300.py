@@ -68,7 +68,7 @@ class Solver(_Base):
     def __init__(self):
         super().__init__(logger)
         self.name = "gb300"
-        self.description = ("<p>GB300 solver: one fused sm_103a kernel per time step, graph-replayed, "
+        self.description = ("<p>GB300 solver: hand-written sm_103a step kernels, graph-replayed, "
                             "fields resident in HBM. precision f64 matches the default solver bit for bit; "
                             "f32k is FP32 with Kahan-compensated displacement.</p>")
         self.cfg = {**cfg, **self.cfg}
