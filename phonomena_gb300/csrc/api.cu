@@ -1055,22 +1055,6 @@ int phono_create(const phono_desc* d, phono_handle** out) {
   TRYC(cudaMemsetAsync(h->mat, 0, h->mat_bytes, h->stream));
   join_stage(h);
   TRY(dalloc(h, &h->tab, (size_t)256 * 16 * h->es));
-  // two-launch step (a handle made with a tile shape never takes it); the
-  // leapfrog's window is zero outside the points the stress pass writes, and a
-  // mesh whose window does not fit keeps to the tiles
-  const bool shaped = d->tile_j || d->x_segment;
-  h->win = shaped ? 0 : split_window(nx, ny, nz, d->precision);
-  if (const size_t sb = shaped ? 0 : split_bytes(nx, ny, nz, d->precision)) {
-    h->tsy = (int)round_up(SPLIT_KOFF + nz, 8);
-    if (dalloc(h, (void**)&h->stress, sb)) {
-      h->win = 0;
-      cudaGetLastError();
-      g_err.clear();
-    } else {
-      TRYC(cudaMemsetAsync(h->stress, 0, sb, h->stream));
-    }
-  }
-  h->split = h->win > 0;
   TRY(dalloc(h, (void**)&h->tab13, (size_t)256 * PHONO_TABLE_COLS * 8));
   TRY(upload_materials(h, d->mat, d->table, d->nmat));
   TRY(encode_tensor_maps(h, h->t));
@@ -1090,6 +1074,22 @@ int phono_create(const phono_desc* d, phono_handle** out) {
   TRYC(cudaMemsetAsync(h->step_base, 0, sizeof(int) * 2, h->stream));
   TRY(dalloc(h, (void**)&h->partial, sizeof(double2) * kEnergyBlocks));
   TRY(dalloc(h, (void**)&h->energy_out, sizeof(double) * 2));
+  // two-launch step (a handle made with a tile shape never takes it); the
+  // leapfrog's window is zero outside the points the stress pass writes.  It
+  // comes last: a handle that fits the memory without it keeps to the tiles.
+  const bool shaped = d->tile_j || d->x_segment;
+  h->win = shaped ? 0 : split_window(nx, ny, nz, d->precision);
+  if (const size_t sb = shaped ? 0 : split_bytes(nx, ny, nz, d->precision)) {
+    h->tsy = (int)round_up(SPLIT_KOFF + nz, 8);
+    if (dalloc(h, (void**)&h->stress, sb)) {
+      h->win = 0;
+      cudaGetLastError();
+      g_err.clear();
+    } else {
+      TRYC(cudaMemsetAsync(h->stress, 0, sb, h->stream));
+    }
+  }
+  h->split = h->win > 0;
   TRYC(cudaStreamSynchronize(h->stream));
 #undef TRY
 #undef TRYC

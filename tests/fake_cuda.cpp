@@ -38,6 +38,7 @@ std::map<char*, Block> g_mem, g_pinned;
 std::map<std::string, int> g_fail, g_count;
 std::set<Stream*> g_streams;
 int g_broken = 0;
+size_t g_limit = 0;  // bytes all allocations may take (0: any)
 thread_local int g_dev = 0;
 Stream* S(cudaStream_t s) { return reinterpret_cast<Stream*>(s); }
 Event* E(cudaEvent_t e) { return reinterpret_cast<Event*>(e); }
@@ -121,7 +122,9 @@ void fake_fail(const char* what, int after) {  // the after-th call of its kind 
 void fake_reset() {
   g_fail.clear();
   g_broken = 0;
+  g_limit = 0;
 }
+void fake_limit(size_t bytes) { g_limit = bytes; }
 void fake_device(int dev) { g_dev = dev; }
 int fake_current() { return g_dev; }
 int fake_broken() { return g_broken; }
@@ -141,7 +144,7 @@ cudaError_t cudaGetDevice(int* d) { return *d = g_dev, cudaSuccess; }
 cudaError_t cudaSetDevice(int d) { return g_dev = d, cudaSuccess; }
 cudaError_t cudaDeviceGetAttribute(int* v, enum cudaDeviceAttr, int) { return *v = 152, cudaSuccess; }
 cudaError_t cudaMalloc(void** p, size_t n) {
-  if (fails("malloc")) return cudaErrorMemoryAllocation;
+  if (fails("malloc") || (g_limit && fake_bytes(g_dev) + (n + 511) / 512 * 512 > g_limit)) return cudaErrorMemoryAllocation;
   *p = std::calloc(n, 1);
   std::lock_guard<std::mutex> hold(g_m);
   g_mem[(char*)*p] = Block{n, g_dev};

@@ -37,7 +37,7 @@ def compile_host_abi():
                             ("phono_batch_create", ci, [ci, ci, ci, vp]), ("phono_batch_add", ci, [vp, vp, ci]),
                             ("phono_batch_remove", ci, [vp, ci]), ("phono_batch_step", ci, [vp, ci]),
                             ("phono_batch_sync", ci, [vp]), ("phono_batch_destroy", None, [vp]),
-                            ("fake_reset", None, []), ("fake_hold", None, [vp, ci]), ("fake_fail", None, [ctypes.c_char_p, ci]),
+                            ("fake_reset", None, []), ("fake_limit", None, [sz]), ("fake_hold", None, [vp, ci]), ("fake_fail", None, [ctypes.c_char_p, ci]),
                             ("fake_device", None, [ci]), ("fake_current", ci, []), ("fake_broken", ci, []),
                             ("fake_count", ci, [ctypes.c_char_p]), ("fake_bytes", sz, [ci]), ("fake_pin", None, [vp, sz])):
         f = getattr(L, name)
@@ -51,12 +51,12 @@ TABLE = np.array([[224e9, 64e9, 64e9, 64e9, 224e9, 64e9, 64e9, 64e9, 224e9, 80e9
 class Handle:
     """A handle of uniform spacing; calls return the C ABI's codes."""
 
-    def __init__(self, L, shape, precision="f32k", max_steps=100, tile_j=0, x_segment=0, seed=0):
+    def __init__(self, L, shape, precision="f32k", max_steps=100, tile_j=0, x_segment=0, seed=0, record_every=0):
         self.L, self.shape = L, shape
         self.ids = np.random.default_rng(seed).integers(0, len(TABLE), shape, dtype=np.uint8)
         arrs = [np.full(n - d, 1e-5) for d in (1, 2) for n in shape]
         d = _lib.PhonoDesc(*shape, *(a.ctypes.data for a in arrs), self.ids.ctypes.data, TABLE.ctypes.data, len(TABLE), 1e-10,
-                           _lib.PRECISIONS[precision], 1, 0, 0, max_steps, 0, tile_j, x_segment)
+                           _lib.PRECISIONS[precision], 1, 0, 0, max_steps, record_every, tile_j, x_segment)
         h = ctypes.c_void_p()
         self.rc = L.phono_create(ctypes.byref(d), ctypes.byref(h))
         self.h = h

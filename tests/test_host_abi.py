@@ -119,6 +119,21 @@ def test_memory_of_fp64_handles_with_a_tile_shape(L):
     assert held["f64v", True] == held["f64v", False] and held["f32k", True] == held["f32k", False]
 
 
+def test_the_window_comes_after_what_a_handle_cannot_do_without(L):
+    """A handle that fits the device's memory without the stress window is made,
+    and steps by tiles."""
+    shape, out = (21, 70, 60), ctypes.c_size_t()
+    assert L.phono_footprint_shaped(*shape, 0, 30, 1, 8, 0, ctypes.byref(out)) == 0
+    for spare, form in ((0, b"tile"), (window(shape) - 512, b"tile"), (window(shape), b"split")):
+        L.fake_limit(out.value + spare)
+        h = Handle(L, shape, "f64", max_steps=30, record_every=1)
+        assert h.rc == 0, L.phono_last_error()
+        n = L.fake_count(form)
+        assert L.phono_step(h.h, 5) == 0 and L.fake_count(form) > n
+        h.close()
+    assert L.fake_bytes(0) == 0 and L.fake_broken() == 0
+
+
 def window(shape):
     """Bytes of the leapfrog's window: six stresses of rows padded to 64 bytes, the first 32 of them zeros."""
     return -(-6 * shape[0] * shape[1] * -(-(4 + shape[2]) // 8) * 64 // 512) * 512
