@@ -36,7 +36,8 @@ namespace phono {
 // known operand: divisor or factor.  hi has its top bit set, except for
 // records the integer path must not take (zero factors, exponents out of
 // range), where hi = lo = 0.  de: what the operand adds to the sign/exponent
-// word of x when Q has its top bit set (one less in the exponent otherwise);
+// word of x when Q has its top bit set (one less in the exponent otherwise), and
+// SOFT_BIAS, which keeps its exponent positive and its top bit the sign;
 // idx: the operand itself at vals[idx].
 struct alignas(16) SoftRec {
   uint32_t lo, hi, de, idx;
@@ -80,6 +81,7 @@ SOFT_HD double soft_double(uint32_t hi, uint32_t lo) {
 // normal
 constexpr uint32_t SOFT_EXP_MIN = 300, SOFT_EXP_SPAN = 1400;
 constexpr int SOFT_REC_EXP = 128;
+constexpr uint32_t SOFT_BIAS = 2u * SOFT_REC_EXP << 20;
 
 SOFT_HD SoftNum soft_split(double x, bool& ok) {
   const uint64_t u = soft_bits(x);
@@ -147,7 +149,7 @@ SOFT_HD SoftNum soft_mul(const SoftNum& x, const SoftRec& c) {
   SoftNum n;
   n.hi = (uint32_t)(r >> 32);
   n.lo = (uint32_t)r;
-  n.se = x.se + c.de - (up ? 0u : 1u << 20);
+  n.se = x.se + c.de - (up ? SOFT_BIAS : SOFT_BIAS + (1u << 20));
   return n;
 }
 
@@ -163,7 +165,7 @@ SOFT_HD SoftNum soft_div(const SoftNum& x, const SoftRec& d, B b) {
   SoftNum n;
   n.hi = (uint32_t)(r >> 32);
   n.lo = (uint32_t)r;
-  n.se = x.se + d.de - (up ? 0u : 1u << 20);
+  n.se = x.se + d.de - (up ? SOFT_BIAS : SOFT_BIAS + (1u << 20));
   return n;
 }
 
@@ -171,10 +173,8 @@ SOFT_HD double soft_join(const SoftNum& n) {
   return soft_double(((n.hi >> 11) & 0xfffffu) | n.se, (n.lo >> 11) | (n.hi << 21));
 }
 
-// sign of a record's operand (its top bit): of a factor below 1/2 the exponent
-// that `de` adds is negative and borrows from the sign bit above it, which the
-// bit below the sign tells (|exponent| <= 129 of 2047)
-SOFT_HD uint32_t soft_sign(const SoftRec& c) { return (c.de ^ (c.de << 1)) & 0x80000000u; }
+// the sign of a record's operand, in the top bit
+SOFT_HD uint32_t soft_sign(const SoftRec& c) { return c.de; }
 
 // record of a divisor (div) or factor; idx: where the kernels find its value
 inline SoftRec soft_record(double v, bool div, uint32_t idx) {
@@ -189,10 +189,10 @@ inline SoftRec soft_record(double v, bool div, uint32_t idx) {
   if (div) {
     const unsigned __int128 q = ((unsigned __int128)1 << 116) / m;  // 2^64 * 2^52 / m, in (2^63, 2^64]
     f = q >> 64 ? ~0ull : (uint64_t)q;
-    r.de = (uint32_t)(1023 - ex) << 20;
+    r.de = SOFT_BIAS + ((uint32_t)(1023 - ex) << 20);
   } else {
     f = m << 11;
-    r.de = sign + ((uint32_t)(ex - 1022) << 20);
+    r.de = SOFT_BIAS + sign + ((uint32_t)(ex - 1022) << 20);
   }
   r.hi = (uint32_t)(f >> 32);
   r.lo = (uint32_t)f;
