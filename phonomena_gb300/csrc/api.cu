@@ -132,8 +132,26 @@ struct phono_handle {
 
 static long long round_up(long long x, long long m) { return (x + m - 1) / m * m; }
 
+// a leapfrog handle that keeps to tiles has no use for its stress window
+static cudaError_t drop_window(phono_handle* h) {
+  if (!h->stress) return cudaSuccess;
+  h->allocs.erase(std::find(h->allocs.begin(), h->allocs.end(), h->stress));
+  const cudaError_t e = cudaFree(h->stress);
+  h->stress = nullptr;
+  h->win = 0;
+  h->split = false;
+  return e;
+}
+
+// memory of a handle that is being made: where it does not fit beside the stress
+// window, the handle does without the window
 static int dalloc(phono_handle* h, void** p, size_t bytes) {
   cudaError_t e = cudaMalloc(p, bytes);
+  if (e != cudaSuccess && h->stress) {
+    cudaGetLastError();
+    drop_window(h);
+    e = cudaMalloc(p, bytes);
+  }
   if (e != cudaSuccess) {
     *p = nullptr;
     return fail(PHONO_ERR_NOMEM, std::string("cudaMalloc ") + std::to_string(bytes) + " bytes: " + cudaGetErrorString(e));
@@ -1055,6 +1073,23 @@ int phono_create(const phono_desc* d, phono_handle** out) {
   TRYC(cudaMemsetAsync(h->mat, 0, h->mat_bytes, h->stream));
   join_stage(h);
   TRY(dalloc(h, &h->tab, (size_t)256 * 16 * h->es));
+  // two-launch step (a handle made with a tile shape never takes it); the
+  // leapfrog's window is zero outside the points the stress pass writes, and a
+  // mesh whose window does not fit keeps to the tiles.  (Made after the rest, small
+  // windows lie where the steps take 1% longer.)
+  const bool shaped = d->tile_j || d->x_segment;
+  h->win = shaped ? 0 : split_window(nx, ny, nz, d->precision);
+  if (const size_t sb = shaped ? 0 : split_bytes(nx, ny, nz, d->precision)) {
+    h->tsy = (int)round_up(SPLIT_KOFF + nz, 8);
+    if (dalloc(h, (void**)&h->stress, sb)) {
+      h->win = 0;
+      cudaGetLastError();
+      g_err.clear();
+    } else {
+      TRYC(cudaMemsetAsync(h->stress, 0, sb, h->stream));
+    }
+  }
+  h->split = h->win > 0;
   TRY(dalloc(h, (void**)&h->tab13, (size_t)256 * PHONO_TABLE_COLS * 8));
   TRY(upload_materials(h, d->mat, d->table, d->nmat));
   TRY(encode_tensor_maps(h, h->t));
@@ -1074,22 +1109,6 @@ int phono_create(const phono_desc* d, phono_handle** out) {
   TRYC(cudaMemsetAsync(h->step_base, 0, sizeof(int) * 2, h->stream));
   TRY(dalloc(h, (void**)&h->partial, sizeof(double2) * kEnergyBlocks));
   TRY(dalloc(h, (void**)&h->energy_out, sizeof(double) * 2));
-  // two-launch step (a handle made with a tile shape never takes it); the
-  // leapfrog's window is zero outside the points the stress pass writes.  It
-  // comes last: a handle that fits the memory without it keeps to the tiles.
-  const bool shaped = d->tile_j || d->x_segment;
-  h->win = shaped ? 0 : split_window(nx, ny, nz, d->precision);
-  if (const size_t sb = shaped ? 0 : split_bytes(nx, ny, nz, d->precision)) {
-    h->tsy = (int)round_up(SPLIT_KOFF + nz, 8);
-    if (dalloc(h, (void**)&h->stress, sb)) {
-      h->win = 0;
-      cudaGetLastError();
-      g_err.clear();
-    } else {
-      TRYC(cudaMemsetAsync(h->stress, 0, sb, h->stream));
-    }
-  }
-  h->split = h->win > 0;
   TRYC(cudaStreamSynchronize(h->stream));
 #undef TRY
 #undef TRYC
@@ -1527,12 +1546,7 @@ static int retile(phono_handle* h, int tj, int xseg, const std::vector<int>& sta
   h->t = t;
   h->own = Tiling();
   CK(set_split(h, false));
-  if (h->stress) {  // tiles from here on
-    h->allocs.erase(std::find(h->allocs.begin(), h->allocs.end(), h->stress));
-    CK(cudaFree(h->stress));
-    h->stress = nullptr;
-    h->win = 0;
-  }
+  CK(drop_window(h));
   if (h->graph) {  // the captured launches hold the old grid and tensor maps
     cudaGraphExecDestroy(h->graph);
     h->graph = nullptr;
