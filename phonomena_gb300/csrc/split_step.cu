@@ -10,11 +10,12 @@
 // through it in chunks.  The result is that of the tile pass, bit for bit.
 //
 // Bound (one GB300, us a step, the best tile shape of the tile pass first):
-// the FP64 leapfrog by instruction issue and the FP64 pipe together (18 FP64 of
-// 1220 instructions a stress point; issue 61%, ALU 61%, FP64 pipe 57% busy),
-// the FP64 velocity form by the FP64 pipe; small
-// meshes by two dependent launches (1.2 us each) of three or four L2
-// latencies.
+// the FP64 leapfrog by latency: of 1214 instructions a stress point 18 are FP64,
+// and with the 25 warps an SM that the registers leave (28 in the update) issue
+// is 60% busy, ALU 59 (45), FP64 pipe 58 (56), with 2.6 stalls an issue on a
+// dependent instruction and 2.7 (3.3) on loads; the FP64 velocity form by the
+// FP64 pipe; small meshes by two dependent launches (1.2 us each) of three or
+// four L2 latencies.
 //   nodes       25x21x13   41x41x21   61x61x21   150x131x47  194x162x98  257x257x129
 //   F64         25 / 8.4   32 / 10.8  47 / 13.5  354 / 102   969 / 337   2012 / 924
 //   F64V        13 / 7.2   21 / 9.1   29 / 13.4  197 / 98    559 / 307   1174 / 838
