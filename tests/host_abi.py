@@ -22,8 +22,9 @@ def compile_host_abi():
     src.write_text('#include "fake_prelude.h"\n' + text.replace("../../include/", ""))
     lib = out / f"libhost_abi.{os.getpid()}.so"
     cuda = Path(build.nvcc()).resolve().parents[1] / "include"
-    subprocess.run(["g++", "-O1", "-std=c++17", "-ffp-contract=off", "-w", "-shared", "-fPIC", "-pthread", "-I", str(cuda),
-                    "-I", str(HERE), "-I", str(build.CSRC), "-I", str(build.ROOT / "include"), str(src),
+    # (-Bsymbolic: a CUDA runtime that the process has loaded, as torch does, must not take the calls)
+    subprocess.run(["g++", "-O1", "-std=c++17", "-ffp-contract=off", "-w", "-shared", "-fPIC", "-pthread", "-Wl,-Bsymbolic",
+                    "-I", str(cuda), "-I", str(HERE), "-I", str(build.CSRC), "-I", str(build.ROOT / "include"), str(src),
                     str(HERE / "fake_cuda.cpp"), "-o", str(lib)], check=True)
     L = ctypes.CDLL(str(lib))
     lib.unlink()
