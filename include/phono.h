@@ -331,7 +331,10 @@ int phono_batch_create(int capacity, int precision, int tile_j, phono_batch **ou
 #define PHONO_BATCH_PERSISTENT 0
 #define PHONO_BATCH_STREAMS 1
 int phono_batch_set_mode(phono_batch *b, int mode, int streams);
-/* Attach h for nsteps more steps; returns the slot (>= 0) or an error code. */
+/* Attach h (of at most 32 materials) for nsteps more steps; returns the slot
+ * (>= 0) or an error code, after which h is as it was.  phono_batch_remove
+ * takes it out in any case; an error then says that h steps on in the batch's
+ * tiles. */
 int phono_batch_add(phono_batch *b, phono_handle *h, int nsteps);
 int phono_batch_remove(phono_batch *b, int slot);
 /* Steps an instance still has to take (0 when done). */

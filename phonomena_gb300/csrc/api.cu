@@ -56,8 +56,8 @@ void set_last_error(const char* msg) { g_err = msg; }
 static const int kGraphSteps = 12;  // multiple of 2 and 3: buffer rotations line up
 static const int kEnergyBlocks = 1024;
 // FP32 meshes from here on sum their energy marching along x: smaller ones have
-// too few columns for it (energy.cu: as fast at 108 k nodes, 78.6 to 67.4 us at
-// 207 k)
+// too few columns for it (energy.cu: 42.8 us a call without and 53.2 with it at
+// 108 k nodes, 78.3 and 67.1 at 207 k)
 static const double kEnergyMarchNodes = 200000;
 
 // the FP64 velocity form's two-launch step multiplies by constants in integer

@@ -155,8 +155,8 @@ struct EnPlane {
 // along x with the values of the last plane in registers and those of the next
 // one on their way.  Bound by the FP64 pipe: 39 operations a node, 0.54 ms of
 // its issue at 257x257x129 nodes.  us a call, energy_partial_kernel<float> / here:
-// 55 k nodes 41.6 / 53.7, 108 k 53.4 / 53.1, 207 k 78.6 / 67.4, 845 k 165 / 117,
-// 8.5 M 1063 / 631.  (Terms formed in pairs of floats took 216 there, but a
+// 55 k nodes 40.0 / 53.9, 108 k 42.8 / 53.2, 207 k 78.3 / 67.1, 845 k 166 / 116,
+// 8.5 M 1066 / 633.  (Terms formed in pairs of floats took 216 there, but a
 // term was off by up to 2^-45, which shows when a state is a few values; here
 // it is as good as the other form's.)
 __global__ void __launch_bounds__(EN_THREADS, 2) energy_march_kernel(EnergyArgs a, int nit, double2* __restrict__ partial) {
@@ -280,6 +280,11 @@ cudaError_t launch_energy(const EnergyArgs& a, double2* partial, int nblocks, do
     energy_march_kernel<<<nblocks, EN_THREADS, smem, st>>>(a, nit, partial);
   } else {
     const size_t smem = (size_t)a.nmat * EN_COLS * sizeof(double);
+    // no block without a row: its table and its sums took longer than the rows
+    // of a small mesh (us a call: 2.0 k nodes 32.4 / 27.7, 35 k 40.4 / 31.3); the
+    // partials left out are zeros
+    const long long rows = ((long long)a.g.nx * a.g.ny + EN_WARPS - 1) / EN_WARPS;
+    if (rows < nblocks) nblocks = (int)rows;
     if (a.f32)
       energy_partial_kernel<float><<<nblocks, EN_THREADS, smem, st>>>(a, partial);
     else
